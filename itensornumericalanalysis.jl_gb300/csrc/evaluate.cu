@@ -19,127 +19,22 @@
 //      nor overflow.
 //   4. k_combine: product over the roots of the forest, times 2^exponent.
 #include <algorithm>
+#include <memory>
 #include <type_traits>
 
+#include "eval_tree.cuh"
 #include "evaluate.cuh"
+#include "rows.cuh"
 
 namespace tnfa {
-
-// ----------------------------------------------------------- digitize ----
-struct DigitEntry {
-  int col;     // column of X
-  int base;
-  int vertex;
-  int stride;  // weight of this leg inside the vertex's site value
-  double invb; // base^-digit, correctly rounded
-  int start;   // first digit of a (variable, part): reload the remainder
-};
-
-__global__ void k_digitize(const double* __restrict__ X, int ncols, int Pc,
-                           const DigitEntry* __restrict__ prog, int nprog, uint8_t* __restrict__ S,
-                           int64_t ldS, int* __restrict__ err) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < Pc; p += gridDim.x * blockDim.x) {
-    double xr = 0.0;
-    for (int e = 0; e < nprog; ++e) {
-      DigitEntry d = prog[e];
-      if (d.start) {
-        xr = X[(int64_t)p * ncols + d.col];
-        if (!(xr >= 0.0) || !isfinite(xr)) {
-          atomicOr(err, 1);
-          xr = 0.0;
-        }
-      }
-      // Largest digit value v with xr >= v * base^-digit; subtract it.
-      int dig = 0;
-      for (int v = d.base - 1; v >= 1; --v) {
-        double t = (double)v * d.invb;
-        if (xr >= t) {
-          dig = v;
-          xr -= t;
-          break;
-        }
-      }
-      uint8_t* sp = S + (int64_t)d.vertex * ldS + p;
-      *sp = (uint8_t)(*sp + dig * d.stride);
-    }
-  }
-}
-
-// ----------------------------------------------------------- grouping ----
-__global__ void k_group_count(const uint8_t* __restrict__ S, int Pc, int ng, int* __restrict__ cnt) {
-  __shared__ int h[256];
-  for (int i = threadIdx.x; i < ng; i += blockDim.x) h[i] = 0;
-  __syncthreads();
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < Pc; p += gridDim.x * blockDim.x)
-    atomicAdd(&h[S[p]], 1);
-  __syncthreads();
-  for (int i = threadIdx.x; i < ng; i += blockDim.x)
-    if (h[i]) atomicAdd(&cnt[i], h[i]);
-}
-
-// Single thread: offsets, tile starts and scatter cursors from the counts.
-__global__ void k_group_scan(int* meta, int ng, int tp) {
-  int* off = meta;
-  int* cnt = meta + ng;
-  int* ts = meta + 2 * ng;
-  int* cur = meta + 3 * ng + 1;
-  int o = 0, t = 0;
-  for (int g = 0; g < ng; ++g) {
-    off[g] = o;
-    cur[g] = o;
-    ts[g] = t;
-    o += cnt[g];
-    t += (cnt[g] + tp - 1) / tp;
-  }
-  ts[ng] = t;
-}
-
-// Identity grouping (vertex without site legs).
-__global__ void k_group_identity(int* meta, int Pc, int tp) {
-  meta[0] = 0;
-  meta[1] = Pc;
-  meta[2] = 0;
-  meta[3] = (Pc + tp - 1) / tp;
-  meta[4] = 0;
-}
-
-constexpr int SCATTER_ITEMS = 8;
-__global__ void k_group_scatter(const uint8_t* __restrict__ S, int Pc, int ng, int* __restrict__ cur,
-                                int* __restrict__ perm) {
-  __shared__ int h[256];
-  __shared__ int base[256];
-  for (int i = threadIdx.x; i < ng; i += blockDim.x) h[i] = 0;
-  __syncthreads();
-  int p0 = blockIdx.x * blockDim.x * SCATTER_ITEMS;
-  int loc[SCATTER_ITEMS];
-  int grp[SCATTER_ITEMS];
-#pragma unroll
-  for (int i = 0; i < SCATTER_ITEMS; ++i) {
-    int p = p0 + i * blockDim.x + threadIdx.x;
-    grp[i] = -1;
-    if (p < Pc) {
-      grp[i] = S[p];
-      loc[i] = atomicAdd(&h[grp[i]], 1);
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < ng; i += blockDim.x) base[i] = h[i] ? atomicAdd(&cur[i], h[i]) : 0;
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < SCATTER_ITEMS; ++i) {
-    int p = p0 + i * blockDim.x + threadIdx.x;
-    if (grp[i] >= 0) perm[base[grp[i]] + loc[i]] = p;
-  }
-}
 
 // ------------------------------------------------------- contraction ----
 template <class T>
 __device__ inline bool locate_tile(const VertexJob<T>& j, int tp, int b, int& row0, int& nrows,
                                    int& g) {
-  int ng = j.ngroups;
+  const int ng = j.ngroups;
   if (b >= j.tile_start[ng]) return false;
-  int gg = 0;
-  while (gg + 1 < ng && j.tile_start[gg + 1] <= b) ++gg;
+  const int gg = find_group(j.tile_start, ng, b);
   g = gg;
   row0 = j.grp_off[gg] + (b - j.tile_start[gg]) * tp;
   nrows = min(tp, j.grp_off[gg] + j.grp_cnt[gg] - row0);
@@ -185,8 +80,7 @@ __device__ void load_children(const VertexJob<T>& j, const int* pts, int nrows, 
         const int r = idx / s.dim, i = idx - r * s.dim;
         v[u] = Sc<T>::zero();
         if (idx < n && r < nrows) {
-          const int p = pts[r];
-          v[u] = s.S ? s.ptr[(int64_t)s.S[p] * s.dim + i] : s.ptr[(int64_t)p * s.dim + i];
+          v[u] = s.ptr[(int64_t)s.idx(pts[r]) * s.dim + i];
         }
       }
 #pragma unroll
@@ -211,7 +105,7 @@ __device__ void load_children(const VertexJob<T>& j, const int* pts, int nrows, 
       int ex = (m > 0) ? Frexp<decltype(m)>::e(m) : 0;
       if (ex != 0)
         for (int i = lane; i < s.dim; i += 32) row[i] = Sc<T>::scale2(row[i], -ex);
-      if (lane == 0) atomicAdd(&eacc[r], ex + (s.exps ? s.exps[pts[r]] : 0));
+      if (lane == 0) atomicAdd(&eacc[r], ex + (s.exps ? s.exps[s.idx(pts[r])] : 0));
     }
     off += s.dim;
   }
@@ -308,7 +202,8 @@ __global__ void __launch_bounds__(256) k_contract_gemm(const VertexJob<T> j) {
     }
   }
   if (blockIdx.y == 0)
-    for (int r = threadIdx.x; r < nrows; r += blockDim.x) j.out_exp[pts[r]] = eacc[r];
+    for (int r = threadIdx.x; r < nrows; r += blockDim.x)
+      j.out_exp[pts[r]] = eacc[r] + (j.gexp ? j.gexp[g] : 0);
 }
 
 // Narrow outputs (chi_a <= 16): one warp per point, lanes split K, shuffle
@@ -379,46 +274,7 @@ __global__ void __launch_bounds__(256) k_contract_narrow(const VertexJob<T> j) {
     }
     if (lane == 0) j.out[(int64_t)p * j.chi_a + q] = v;
   }
-  if (lane == 0) j.out_exp[p] = eacc[r];
-}
-
-// ------------------------------------------------------------ combine ----
-template <class T>
-__device__ inline void write_out(void* out, int kind, int64_t p, int64_t P, T v, int e);
-template <>
-__device__ inline void write_out<double>(void* out, int kind, int64_t p, int64_t P, double v, int e) {
-  if (kind == TNFA_OUT_F64) {
-    ((double*)out)[p] = scalbn(v, e);
-  } else if (kind == TNFA_OUT_F32) {
-    ((float*)out)[p] = (float)scalbn(v, e);
-  } else {  // scaled f32
-    int ex = 0;
-    double m = frexp(v, &ex);
-    ((float*)out)[p] = (float)m;
-    ((int*)((float*)out + P))[p] = (v == 0.0) ? 0 : e + ex;
-  }
-}
-template <>
-__device__ inline void write_out<float>(void* out, int kind, int64_t p, int64_t P, float v, int e) {
-  write_out<double>(out, kind, p, P, (double)v, e);
-}
-template <>
-__device__ inline void write_out<cplx>(void* out, int kind, int64_t p, int64_t P, cplx v, int e) {
-  ((cplx*)out)[p] = cplx{scalbn(v.re, e), scalbn(v.im, e)};
-}
-
-template <class T>
-__global__ void k_combine(const T* __restrict__ rootv, const int* __restrict__ roote, int nroots,
-                          int Pc, void* out, int kind, int64_t P, int64_t p0) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < Pc; p += gridDim.x * blockDim.x) {
-    T v = Sc<T>::one();
-    int e = 0;
-    for (int r = 0; r < nroots; ++r) {
-      v = v * rootv[(int64_t)r * Pc + p];
-      e += roote[(int64_t)r * Pc + p];
-    }
-    write_out<T>(out, kind, p0 + p, P, v, e);
-  }
+  if (lane == 0) j.out_exp[p] = eacc[r] + (j.gexp ? j.gexp[g] : 0);
 }
 
 // --------------------------------------------- fused small-bond path ----
@@ -443,7 +299,7 @@ constexpr int FUSED_MAXV = 128;
 
 template <class T, int CHI>
 __global__ void __launch_bounds__(128) k_eval_fused(
-    const double* __restrict__ X, int ncols, int Pc, const DigitEntry* __restrict__ prog, int nprog,
+    const double* __restrict__ X, int ncols, int Pc, const DigitRun* __restrict__ prog, int nprog,
     const FusedStep* __restrict__ steps, int nsteps, const T* __restrict__ tensors, int n_elem,
     int V, int nslots, size_t off_msg, size_t off_prog, size_t off_steps, void* out, int kind,
     int64_t P, int64_t p0, int* __restrict__ err) {
@@ -452,7 +308,7 @@ __global__ void __launch_bounds__(128) k_eval_fused(
   // place (a few hundred KB at most: they stay in L1 / L2)
   const T* ts = off_msg ? (const T*)smem_raw : tensors;
   T* msg = (T*)(smem_raw + off_msg);
-  DigitEntry* pg = (DigitEntry*)(smem_raw + off_prog);
+  DigitRun* pg = (DigitRun*)(smem_raw + off_prog);
   FusedStep* st = (FusedStep*)(smem_raw + off_steps);
   if (off_msg)
     for (int i = threadIdx.x; i < n_elem; i += blockDim.x) ((T*)smem_raw)[i] = tensors[i];
@@ -462,29 +318,9 @@ __global__ void __launch_bounds__(128) k_eval_fused(
   const int tpb = blockDim.x, tid = threadIdx.x;
   auto M = [&](int slot, int k) -> T& { return msg[((size_t)slot * CHI + k) * tpb + tid]; };
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < Pc; p += gridDim.x * blockDim.x) {
-    uint8_t dg[FUSED_MAXV];
+    int dg[FUSED_MAXV];
     for (int v = 0; v < V; ++v) dg[v] = 0;
-    double xr = 0.0;
-    for (int e = 0; e < nprog; ++e) {
-      const DigitEntry d = pg[e];
-      if (d.start) {
-        xr = X[(int64_t)p * ncols + d.col];
-        if (!(xr >= 0.0) || !isfinite(xr)) {
-          atomicOr(err, 1);
-          xr = 0.0;
-        }
-      }
-      int dig = 0;
-      for (int v = d.base - 1; v >= 1; --v) {
-        const double t = (double)v * d.invb;
-        if (xr >= t) {
-          dig = v;
-          xr -= t;
-          break;
-        }
-      }
-      dg[d.vertex] = (uint8_t)(dg[d.vertex] + dig * d.stride);
-    }
+    digit_codes(X + (int64_t)p * ncols, pg, nprog, dg, 1, 0, V, err);
     T val = Sc<T>::one();
     int ex_acc = 0;
     for (int i = 0; i < nsteps; ++i) {
@@ -610,7 +446,7 @@ static FusedPlan make_fused_plan(const Topo& T, size_t tsize, size_t nprog, int6
   const bool ts_smem = (size_t)T.n_elem * tsize <= 96 * 1024;
   F.off_msg = ts_smem ? al((size_t)T.n_elem * tsize) : 0;
   F.off_prog = al(F.off_msg + (size_t)F.tpb * per_thread);
-  F.off_steps = al(F.off_prog + nprog * sizeof(DigitEntry));
+  F.off_steps = al(F.off_prog + nprog * sizeof(DigitRun));
   F.smem = F.off_steps + F.steps.size() * sizeof(FusedStep);
   F.ok = F.smem <= 200 * 1024;
   return F;
@@ -619,7 +455,7 @@ static FusedPlan make_fused_plan(const Topo& T, size_t tsize, size_t nprog, int6
 template <class T>
 static void launch_fused(tnfa_ctx* ctx, const FusedPlan& F, const FusedStep* dsteps, const T* tensors,
                          const Topo& Tp, const double* Xc, int ncols, int Pc,
-                         const DigitEntry* dprog, int nprog, void* o, int kind, int64_t Pout,
+                         const DigitRun* dprog, int nprog, void* o, int kind, int64_t Pout,
                          int64_t pofs, int* derr) {
   const int tpb = F.tpb;
   const unsigned grid = grid_for(Pc, tpb, ctx->sm_count * (2048 / tpb));
@@ -771,215 +607,17 @@ static int contract_tile_rows(int chi_a, int sumdim, size_t tsize) {
   return chi_a <= 16 ? 8 : gemm_tile(chi_a, sumdim, tsize).tp;
 }
 
-template <class T>
-static void evaluate_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double* X,
-                          int64_t P, int ncols, const std::vector<DigitEntry>& prog, int xmem,
-                          void* out, int out_kind, int out_mem, bool use_tc,
-                          bool use_oz = false) {
-  const Topo& Tp = net->topo;
-  const int V = Tp.V;
-  EvalPlan plan = make_plan(Tp);
-  const int nroots = (int)plan.roots.size();
-  size_t out_elem = out_kind == TNFA_OUT_F64 ? 8 : out_kind == TNFA_OUT_F32 ? 4
-                    : out_kind == TNFA_OUT_F32_SCALED ? 8 : 16;
-  size_t per_point = (size_t)plan.nslots * (plan.chimax * sizeof(T) + sizeof(int)) + V + 4 +
-                     (xmem == TNFA_MEM_HOST ? ncols * 8 : 0) + nroots * (sizeof(T) + 4) +
-                     (out_mem == TNFA_MEM_HOST ? out_elem : 0);
-  int64_t Pc_max = (int64_t)(ctx->eval_budget / per_point);
-  Pc_max = std::max<int64_t>(256, std::min<int64_t>(Pc_max, int64_t(1) << 30));
-  Pc_max = (Pc_max / 256) * 256;
-  const int64_t Pc_alloc = std::min<int64_t>(P, Pc_max);
-  const int Pcap = (int)std::max<int64_t>(Pc_alloc, 1);
+// Digits of a network for the given variable list, in the order the digit map
+// takes them (variable, part, digit).
+struct DigitRef {
+  int col, base, vertex, digit;
+  int stride;   // weight of this leg inside the vertex's site value
+  double invb;  // base^-digit, correctly rounded
+  int start;    // first digit of a (variable, part)
+};
 
-  DBuf dprog(ctx, prog.size() * sizeof(DigitEntry));
-  if (!prog.empty())
-    TNFA_CUDA(cudaMemcpyAsync(dprog.p, prog.data(), prog.size() * sizeof(DigitEntry),
-                              cudaMemcpyHostToDevice, ctx->stream));
-  DBuf dS(ctx, (size_t)V * Pcap);
-  DBuf dperm(ctx, (size_t)Pcap * 4);
-  int maxsd = 1;
-  for (int v = 0; v < V; ++v) maxsd = std::max(maxsd, Tp.site_dim[v]);
-  DBuf dmeta(ctx, group_meta_ints(maxsd) * 4);
-  DBuf derr(ctx, 4);
-  TNFA_CUDA(cudaMemsetAsync(derr.p, 0, 4, ctx->stream));
-  const size_t slot_vals = (size_t)Pcap * plan.chimax;
-  DBuf dslots(ctx, (size_t)plan.nslots * slot_vals * sizeof(T));
-  DBuf dslote(ctx, (size_t)plan.nslots * Pcap * sizeof(int));
-  DBuf droot(ctx, (size_t)nroots * Pcap * sizeof(T));
-  DBuf droote(ctx, (size_t)nroots * Pcap * sizeof(int));
-  DBuf dX(ctx, xmem == TNFA_MEM_HOST ? (size_t)Pcap * ncols * 8 : 0);
-  DBuf dout(ctx, out_mem == TNFA_MEM_HOST ? (size_t)Pcap * out_elem : 0);
-  std::vector<int> root_index(V, -1);
-  for (int r = 0; r < nroots; ++r) root_index[plan.roots[r]] = r;
-  // small bonds everywhere: the whole tree per thread in one launch
-  const FusedPlan F = make_fused_plan(Tp, sizeof(T), prog.size(), std::min<int64_t>(P, Pcap));
-  DBuf dsteps;
-  if (F.ok) {
-    dsteps = DBuf(ctx, F.steps.size() * sizeof(FusedStep));
-    TNFA_CUDA(cudaMemcpyAsync(dsteps.p, F.steps.data(), F.steps.size() * sizeof(FusedStep),
-                              cudaMemcpyHostToDevice, ctx->stream));
-  }
-
-  for (int64_t p0 = 0; p0 < P; p0 += Pcap) {
-    const int Pc = (int)std::min<int64_t>(Pcap, P - p0);
-    const double* Xc;
-    if (xmem == TNFA_MEM_HOST) {
-      TNFA_CUDA(cudaMemcpyAsync(dX.p, X + p0 * ncols, (size_t)Pc * ncols * 8,
-                                cudaMemcpyHostToDevice, ctx->stream));
-      Xc = dX.as<double>();
-    } else {
-      Xc = X + p0 * ncols;
-    }
-    if (F.ok) {
-      void* o = out_mem == TNFA_MEM_HOST ? dout.p : out;
-      launch_fused<T>(ctx, F, dsteps.as<FusedStep>(), tensors, Tp, Xc, ncols, Pc,
-                      dprog.as<DigitEntry>(), (int)prog.size(), o, out_kind,
-                      out_mem == TNFA_MEM_HOST ? Pc : P, out_mem == TNFA_MEM_HOST ? 0 : p0,
-                      derr.as<int>());
-    } else {
-    TNFA_CUDA(cudaMemsetAsync(dS.p, 0, (size_t)V * Pcap, ctx->stream));
-    if (!prog.empty()) {
-      KernelScope ks(ctx, "digitize", 0.0, (double)Pc * (ncols * 8.0 + V));
-      k_digitize<<<grid_for(Pc, 256, 8 * 152 * 8), 256, 0, ctx->stream>>>(
-          Xc, ncols, Pc, dprog.as<DigitEntry>(), (int)prog.size(), dS.as<uint8_t>(), (int64_t)Pcap,
-          derr.as<int>());
-      TNFA_LAUNCH_CHECK();
-    }
-    for (int v : plan.order) {
-      VertexJob<T> j{};
-      j.nchild = (int)Tp.children[v].size();
-      TNFA_CHECK(j.nchild <= EVAL_MAXC, TNFA_ERR_UNSUPPORTED,
-                 "vertex degree above " + std::to_string(EVAL_MAXC) + " children");
-      int64_t K = 1;
-      int sumdim = 0;
-      int cdims[EVAL_MAXC];
-      for (int i = 0; i < j.nchild; ++i) {
-        int c = Tp.children[v][i];
-        ChildSrc<T>& s = j.ch[i];
-        s.dim = Tp.link[c];
-        cdims[i] = s.dim;
-        sumdim += s.dim;
-        K *= s.dim;
-        if (plan.fused_leaf[c]) {
-          s.ptr = tensors + Tp.off[c];
-          s.exps = nullptr;
-          s.S = dS.as<uint8_t>() + (int64_t)c * Pcap;
-        } else {
-          s.ptr = (const T*)dslots.p + (size_t)plan.slot[c] * slot_vals;
-          s.exps = dslote.as<int>() + (size_t)plan.slot[c] * Pcap;
-          s.S = nullptr;
-        }
-      }
-      TNFA_CHECK(K < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
-      j.K = (int)K;
-      j.chi_a = Tp.link[v];
-      j.site_dim = Tp.site_dim[v];
-      j.B = tensors + Tp.off[v];
-      j.Pc = Pc;
-      if (Tp.parent[v] < 0) {
-        j.out = (T*)droot.p + (size_t)root_index[v] * Pcap;
-        j.out_exp = droote.as<int>() + (size_t)root_index[v] * Pcap;
-      } else {
-        j.out = (T*)dslots.p + (size_t)plan.slot[v] * slot_vals;
-        j.out_exp = dslote.as<int>() + (size_t)plan.slot[v] * Pcap;
-      }
-      const bool tc = use_tc && j.site_dim <= 256 && tc_vertex_eligible(j.nchild, cdims, j.chi_a);
-      const bool oz = use_oz && oz_vertex_eligible(j.nchild, cdims, j.chi_a);
-      // SIMT shapes: the tile kept by the autotuner for this shape, else the rule's
-      std::vector<GemmTile> cand;
-      std::string key;
-      int tp = tc   ? tc_tile_rows()
-               : oz ? oz_tile_rows()
-                    : contract_tile_rows(j.chi_a, sumdim, sizeof(T));
-      if (!tc && !oz && j.chi_a > 16) {
-        cand = gemm_tile_candidates(j.chi_a, sumdim, sizeof(T));
-        key = std::string("simt:") + FamilyName<T>::v + ":" + std::to_string(j.chi_a) + ":";
-        for (int i = 0; i < j.nchild; ++i) key += std::to_string(cdims[i]) + (i + 1 < j.nchild ? "x" : "");
-        const int kept = tuned_choice(ctx, key);
-        tp = cand[kept >= 0 ? kept : 0].tp;
-      }
-      const int ng = j.site_dim;
-      int* meta = dmeta.as<int>();
-      j.ngroups = ng;
-      j.grp_off = meta;
-      j.grp_cnt = meta + ng;
-      j.tile_start = meta + 2 * ng;
-      if (ng == 1) {
-        KernelScope ks(ctx, "group", 0.0, 0.0);
-        k_group_identity<<<1, 1, 0, ctx->stream>>>(meta, Pc, tp);
-        TNFA_LAUNCH_CHECK();
-        j.perm = nullptr;
-      } else {
-        TNFA_CHECK(ng <= 256, TNFA_ERR_UNSUPPORTED, "site dimension above 256 per vertex");
-        const uint8_t* Sv = dS.as<uint8_t>() + (int64_t)v * Pcap;
-        TNFA_CUDA(cudaMemsetAsync(meta + ng, 0, ng * sizeof(int), ctx->stream));
-        KernelScope ks(ctx, "group", 0.0, (double)Pc * 6.0);
-        k_group_count<<<grid_for(Pc, 256, 4 * 152), 256, 0, ctx->stream>>>(Sv, Pc, ng, meta + ng);
-        k_group_scan<<<1, 1, 0, ctx->stream>>>(meta, ng, tp);
-        unsigned gs = (unsigned)((Pc + 256 * SCATTER_ITEMS - 1) / (256 * SCATTER_ITEMS));
-        k_group_scatter<<<gs, 256, 0, ctx->stream>>>(Sv, Pc, ng, meta + 3 * ng + 1, dperm.as<int>());
-        TNFA_LAUNCH_CHECK();
-        j.perm = dperm.as<int>();
-      }
-      if constexpr (std::is_same<T, float>::value) {
-        if (tc) {
-          tc_contract_vertex(ctx, net, v, j, tp, derr.as<int>());
-          continue;
-        }
-      }
-      if constexpr (std::is_same<T, double>::value) {
-        if (oz) {
-          oz_contract_vertex(ctx, net, v, j, tp, derr.as<int>());
-          continue;
-        }
-      }
-      if (cand.empty()) {
-        launch_contract<T>(ctx, j, Pc);
-        continue;
-      }
-      int cur_tp = tp;
-      tune(ctx, key, (int)cand.size(), 2.0 * Pc * (double)j.K * j.chi_a, [&](int i) {
-        if (cand[i].tp != cur_tp) {  // tile table for this candidate's rows per tile
-          if (ng == 1) k_group_identity<<<1, 1, 0, ctx->stream>>>(meta, Pc, cand[i].tp);
-          else k_group_scan<<<1, 1, 0, ctx->stream>>>(meta, ng, cand[i].tp);
-          TNFA_LAUNCH_CHECK();
-          cur_tp = cand[i].tp;
-        }
-        launch_contract<T>(ctx, j, Pc, &cand[i]);
-      });
-    }
-    void* o = out_mem == TNFA_MEM_HOST ? dout.p : out;
-    int64_t Pout = out_mem == TNFA_MEM_HOST ? Pc : P;
-    int64_t pofs = out_mem == TNFA_MEM_HOST ? 0 : p0;
-    KernelScope ksc(ctx, "combine", 0.0, (double)Pc * nroots * (sizeof(T) + 4.0));
-    k_combine<T><<<grid_for(Pc, 256, 8192), 256, 0, ctx->stream>>>(
-        (const T*)droot.p, droote.as<int>(), nroots, Pc, o, out_kind, Pout, pofs);
-    TNFA_LAUNCH_CHECK();
-    }
-    if (out_mem == TNFA_MEM_HOST) {
-      if (out_kind == TNFA_OUT_F32_SCALED) {
-        TNFA_CUDA(cudaMemcpyAsync((float*)out + p0, dout.p, (size_t)Pc * 4, cudaMemcpyDeviceToHost,
-                                  ctx->stream));
-        TNFA_CUDA(cudaMemcpyAsync((int*)((float*)out + P) + p0, (float*)dout.p + Pc, (size_t)Pc * 4,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-      } else {
-        TNFA_CUDA(cudaMemcpyAsync((char*)out + p0 * out_elem, dout.p, (size_t)Pc * out_elem,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-      }
-    }
-  }
-  int herr = 0;
-  TNFA_CUDA(cudaMemcpyAsync(&herr, derr.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
-  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
-  TNFA_CHECK((herr & 2) == 0, TNFA_ERR_TIMEOUT,
-             "a tensor-core pipeline wait ran out of its iteration budget");
-  TNFA_CHECK(herr == 0, TNFA_ERR_DOMAIN,
-             "a coordinate is negative or not finite (the digit map needs x >= 0)");
-}
-
-// Digit program of a network for the given variable list.
-static std::vector<DigitEntry> make_digit_program(const Topo& T, int n_dims, const int32_t* dims,
-                                                  int* ncols_out) {
+static std::vector<DigitRef> make_digit_program(const Topo& T, int n_dims, const int32_t* dims,
+                                                int* ncols_out) {
   bool has_imag = false;
   int L = T.leg_off[T.V];
   for (int l = 0; l < L; ++l) {
@@ -1005,7 +643,8 @@ static std::vector<DigitEntry> make_digit_program(const Topo& T, int n_dims, con
     if (a.kind != b.kind) return a.kind < b.kind;
     return a.digit < b.digit;
   });
-  std::vector<DigitEntry> prog;
+  std::vector<DigitRef> prog;
+  prog.reserve(refs.size());
   for (size_t i = 0; i < refs.size(); ++i) {
     const LegRef& r = refs[i];
     bool start = (i == 0 || refs[i - 1].var != r.var || refs[i - 1].kind != r.kind);
@@ -1023,16 +662,931 @@ static std::vector<DigitEntry> make_digit_program(const Topo& T, int n_dims, con
     double bk = 1.0;
     for (int k = 0; k < r.digit; ++k) bk *= base;
     TNFA_CHECK(bk < 9007199254740992.0, TNFA_ERR_UNSUPPORTED, "base^digit above 2^53");
-    DigitEntry d;
+    DigitRef d;
     d.col = has_imag ? 2 * col + (r.kind == TNFA_LEG_IMAG ? 1 : 0) : col;
     d.base = base;
     d.vertex = r.vertex;
+    d.digit = r.digit;
     d.stride = r.stride;
     d.invb = 1.0 / bk;
     d.start = start ? 1 : 0;
     prog.push_back(d);
   }
   return prog;
+}
+
+// The digits as runs that add to codes: the digit of vertex v counts
+// mult[v] * stride in code slot[v].  A column in base 2 throughout becomes bit
+// fields (neighbouring digits whose strides double or halve join one field).
+static std::vector<DigitRun> make_runs(const std::vector<DigitRef>& prog, const std::vector<int>& slot,
+                                       const std::vector<int>& mult) {
+  std::vector<DigitRun> runs;
+  for (size_t i = 0; i < prog.size();) {
+    size_t e = i + 1;
+    while (e < prog.size() && !prog[e].start) ++e;
+    bool binary = true;
+    for (size_t k = i; k < e; ++k) binary &= prog[k].base == 2;
+    for (size_t k = i; k < e; ++k) {
+      const DigitRef& d = prog[k];
+      const int w = mult[d.vertex] * d.stride, s = slot[d.vertex];
+      if (binary && k > i && runs.back().slot == s && runs.back().n < 31) {
+        DigitRun& r = runs.back();
+        if ((r.n == 1 || !r.rev) && (int64_t)w * 2 == r.w) {
+          r.w = w;
+          r.n += 1;
+          continue;
+        }
+        if ((r.n == 1 || r.rev) && (int64_t)r.w << r.n == w) {
+          r.rev = 1;
+          r.n += 1;
+          continue;
+        }
+      }
+      DigitRun r{};
+      r.col = d.col;
+      r.slot = s;
+      r.w = w;
+      r.first = (short)d.digit;
+      r.n = 1;
+      r.base = (short)d.base;
+      r.bits = binary;
+      r.start = k == i;
+      r.invb = d.invb;
+      runs.push_back(r);
+    }
+    i = e;
+  }
+  return runs;
+}
+
+// The fused small-bond kernel keeps every vertex's site value by itself.
+static std::vector<DigitRun> make_fused_runs(const Topo& T, const std::vector<DigitRef>& prog) {
+  std::vector<int> slot(T.V), mult(T.V, 1);
+  for (int v = 0; v < T.V; ++v) slot[v] = v;
+  return make_runs(prog, slot, mult);
+}
+
+static size_t digitize_smem(int n, int block) { return (size_t)n * block * sizeof(int); }
+
+// Codes of Pc points into C[slot][ldC].
+static void launch_digitize(tnfa_ctx* ctx, const double* X, int ncols, int Pc, const DigitRun* runs,
+                            int nruns, int nslots, int* C, int64_t ldC, int* err) {
+  const int block = nslots <= 48 ? 256 : 64;
+  const int per = block == 256 ? 48 : 192;
+  for (int s0 = 0; s0 < nslots; s0 += per) {
+    const int s1 = std::min(nslots, s0 + per);
+    KernelScope ks(ctx, "digitize", 0.0, (double)Pc * (ncols * 8.0 + 4.0 * (s1 - s0)));
+    k_digitize<<<grid_for(Pc, block, 8 * 152 * 8), block, digitize_smem(s1 - s0, block), ctx->stream>>>(
+        X, ncols, Pc, runs, nruns, C, ldC, s0, s1, err);
+    TNFA_LAUNCH_CHECK();
+  }
+}
+
+// Groups Pc points by key (null: one group); meta as in group_meta_ints.
+static const int* launch_group(tnfa_ctx* ctx, const int* key, int Pc, int ng, int tp, int* meta, int* perm) {
+  KernelScope ks(ctx, "group", 0.0, key ? (double)Pc * 12.0 : 0.0);
+  if (!key) {
+    k_group_identity<<<1, 1, 0, ctx->stream>>>(meta, Pc, tp);
+    TNFA_LAUNCH_CHECK();
+    return nullptr;
+  }
+  TNFA_CUDA(cudaMemsetAsync(meta + ng, 0, ng * sizeof(int), ctx->stream));
+  const size_t sm = ng <= GROUP_SMEM ? ng * sizeof(int) : 0;
+  k_group_count<<<grid_for(Pc, 256, 4 * 152), 256, sm, ctx->stream>>>(key, Pc, ng, meta + ng);
+  k_group_scan<<<1, 1024, 0, ctx->stream>>>(meta, ng, tp);
+  const unsigned gs = (unsigned)((Pc + 256 * SCATTER_ITEMS - 1) / (256 * SCATTER_ITEMS));
+  k_group_scatter<<<gs, 256, 2 * sm, ctx->stream>>>(key, Pc, ng, meta + 3 * ng + 1, perm);
+  TNFA_LAUNCH_CHECK();
+  return perm;
+}
+static void launch_retile(tnfa_ctx* ctx, bool keyed, int Pc, int ng, int tp, int* meta) {
+  if (keyed) k_group_scan<<<1, 1024, 0, ctx->stream>>>(meta, ng, tp);
+  else k_group_identity<<<1, 1, 0, ctx->stream>>>(meta, Pc, tp);
+  TNFA_LAUNCH_CHECK();
+}
+
+// ------------------------------------------------- row-gather launches ----
+// Tiles of k_rows_gemm by type, largest first.
+template <class T> struct RowTiles;
+template <> struct RowTiles<float> {
+  static constexpr int n = 3;
+  static constexpr int rm[3] = {8, 4, 2}, cn[3] = {4, 2, 1};
+};
+template <> struct RowTiles<double> {
+  static constexpr int n = 3;
+  static constexpr int rm[3] = {4, 2, 1}, cn[3] = {2, 1, 1};
+};
+template <> struct RowTiles<cplx> {
+  static constexpr int n = 2;
+  static constexpr int rm[2] = {2, 1}, cn[2] = {1, 1};
+};
+
+template <class T>
+static int64_t row_blocks(const RowJob<T>& j, int tile) {
+  const int tm = 8 * RowTiles<T>::rm[tile], tn = 32 * RowTiles<T>::cn[tile];
+  const int64_t nbn = (j.N + tn - 1) / tn;
+  if (j.rpg > 0) return (int64_t)(j.rows / j.rpg) * ((j.rpg + tm - 1) / tm) * nbn;
+  return ((int64_t)(j.rows + tm - 1) / tm + j.ngroups) * nbn;
+}
+
+// The largest tile that still gives every SM two blocks, else the smallest:
+// short tables are bound by the SMs they reach, not by the tile's reuse.
+template <class T>
+static int row_tile(tnfa_ctx* ctx, const std::vector<RowJob<T>>& jobs) {
+  for (int t = 0; t + 1 < RowTiles<T>::n; ++t) {
+    int64_t nb = 0;
+    for (const auto& j : jobs) nb += row_blocks(j, t);
+    if (nb >= 2 * ctx->sm_count) return t;
+  }
+  return RowTiles<T>::n - 1;
+}
+
+template <class T>
+static void launch_rows(tnfa_ctx* ctx, int tile, int64_t blocks, const RowJob<T>& one,
+                        const RowJob<T>* jobs, const int* first, int njobs) {
+  TNFA_CHECK(blocks < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
+  auto go = [&](auto kern) { kern<<<(unsigned)blocks, 256, 0, ctx->stream>>>(one, jobs, first, njobs); };
+  if constexpr (std::is_same<T, float>::value) {
+    if (tile == 0) go(k_rows_gemm<T, 8, 4>);
+    else if (tile == 1) go(k_rows_gemm<T, 4, 2>);
+    else go(k_rows_gemm<T, 2, 1>);
+  } else if constexpr (std::is_same<T, double>::value) {
+    if (tile == 0) go(k_rows_gemm<T, 4, 2>);
+    else if (tile == 1) go(k_rows_gemm<T, 2, 1>);
+    else go(k_rows_gemm<T, 1, 1>);
+  } else {
+    if (tile == 0) go(k_rows_gemm<T, 2, 1>);
+    else go(k_rows_gemm<T, 1, 1>);
+  }
+  TNFA_LAUNCH_CHECK();
+}
+
+// ------------------------------------------------------------- engine ----
+// Scratch handed out in 256-byte pieces from one block (or counted, base null).
+struct Carve {
+  unsigned char* base = nullptr;
+  size_t used = 0;
+  template <class U> U* take(size_t n) {
+    const size_t off = (used + 255) & ~(size_t)255;
+    used = off + n * sizeof(U);
+    return reinterpret_cast<U*>(base + off);
+  }
+};
+
+// One evaluation call: the schedule of eval_tree.cuh laid out over scratch,
+// then run.  Tables are built level by level (all row products of a level in
+// one launch) once per call; the points follow in chunks: codes, the messages
+// that have one row per point, the dot products at the centre.
+template <class T>
+class EvalEngine {
+ public:
+  EvalEngine(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const std::vector<DigitRef>& prog,
+             int ncols, int64_t P, bool use_tc, bool use_oz, size_t budget)
+      : ctx_(ctx), net_(net), tensors_(tensors), topo_(net->topo), prog_(prog), ncols_(ncols), P_(P),
+        use_tc_(use_tc), use_oz_(use_oz) {
+    const int V = topo_.V;
+    EvalTreeOptions o;
+    o.points = (double)P;
+    o.rule = use_tc ? CentreRule::ROOT : use_oz ? CentreRule::ROOT_EDGE : CentreRule::ANY_EDGE;
+    o.absorb = !use_tc;
+    if (use_tc || use_oz) {
+      o.tensor_ok.assign(V, 0);
+      for (int v = 0; v < V; ++v) {
+        int cd[EVAL_MAXC];
+        const auto& kids = topo_.children[v];
+        if (kids.size() > (size_t)EVAL_MAXC) continue;
+        bool aligned = true;  // leaf rows are read in place, 16 bytes at a time by the FP32 kernels
+        for (size_t i = 0; i < kids.size(); ++i) {
+          cd[i] = topo_.link[kids[i]];
+          if (topo_.children[kids[i]].empty())
+            aligned &= ((uintptr_t)(tensors + topo_.off[kids[i]]) & 15) == 0 && cd[i] % 4 == 0;
+        }
+        o.tensor_ok[v] = use_tc ? aligned && tc_vertex_eligible((int)kids.size(), cd, topo_.link[v])
+                                : oz_vertex_eligible((int)kids.size(), cd, topo_.link[v]);
+      }
+    }
+    // Tables take at most half the scratch: the row bound shrinks until they
+    // fit.  Every digit code stays within 31 bits.
+    double rows = std::min((double)P, 134217728.0);
+    for (;;) {
+      o.table_rows = rows;
+      o.table_elems = std::min(1073741824.0, (double)(budget / 2) / sizeof(T));
+      tree_ = EvalTreeBuilder(topo_, o).build();
+      if (table_bytes() <= budget / 2 || o.rule == CentreRule::ROOT && rows < 1) break;
+      rows = std::floor(rows / 4);
+      if (rows < 1) {  // the stored order, nothing but points
+        o.rule = CentreRule::ROOT;
+        o.absorb = false;
+      }
+    }
+    plan();
+    per_point_ = (size_t)nmsg_ * (msg_chi_ * sizeof(T) + sizeof(int)) + (size_t)ncodes_ * 4 + (npp_ ? 4 : 0);
+    const size_t tab = scratch(0);
+    const size_t left = budget > tab ? budget - tab : 0;
+    int64_t pc = per_point_ ? (int64_t)(left / per_point_) / 256 * 256 : int64_t(1) << 30;
+    Pc_ = (int)std::min<int64_t>(P, std::max<int64_t>(256, std::min<int64_t>(pc, int64_t(1) << 30)));
+  }
+
+  int chunk() const { return Pc_; }
+  void set_chunk(int pc) { Pc_ = pc; }
+  size_t per_point() const { return per_point_; }
+  // Bytes of scratch for chunks of pc points.
+  size_t scratch(int64_t pc) {
+    Carve c;
+    lay_out(c, pc);
+    return c.used + 256;
+  }
+
+  // Lays the call out over scratch at base (scratch(chunk()) bytes, 256-byte
+  // aligned) and fills the host image of the job tables.
+  void bind(void* base) {
+    Carve c;
+    c.base = (unsigned char*)base;
+    lay_out(c, Pc_);
+    fill_blob();
+  }
+  int* err_flag() const { return err_; }
+  // The job tables and the cleared error flag go to the scratch (stream order).
+  void upload() {
+    h2d(ctx_, blob_, host_.data(), host_.size());
+    clear_error();
+  }
+  void clear_error() { TNFA_CUDA(cudaMemsetAsync(err_, 0, 4, ctx_->stream)); }
+
+  // Tables: permuted tensors, then every level.
+  void tables() {
+    if (!moves_.empty()) {
+      int64_t n = 1;
+      for (const auto& m : moves_) n = std::max(n, m.n);
+      KernelScope ks(ctx_, "move", 0.0, 0.0);
+      k_move<T><<<dim3(grid_for(n, 256, 1024), (unsigned)moves_.size()), 256, 0, ctx_->stream>>>(dmoves_);
+      TNFA_LAUNCH_CHECK();
+    }
+    for (size_t l = 0; l < levels_.size(); ++l) {
+      Level& L = levels_[l];
+      if (!L.rows.empty()) {
+        double fl = 0;
+        std::string key = std::string("simt:") + FamilyName<T>::v + ":rows";
+        for (const auto& j : L.rows) fl += 2.0 * (double)j.rows * j.N * j.K;
+        const bool tuned = fl >= ctx_->autotune_min_work;
+        if (tuned)
+          for (const auto& j : L.rows)
+            key += ":" + std::to_string(j.rows) + "x" + std::to_string(j.N) + "x" + std::to_string(j.K);
+        const int rule = row_tile(ctx_, L.rows);
+        auto go = [&](int i) {
+          const int t = i == 0 ? rule : i <= rule ? i - 1 : i;
+          KernelScope ks(ctx_, FamilyName<T>::v, fl, 0.0);
+          launch_rows<T>(ctx_, t, L.first[t].back(), RowJob<T>{}, L.drows, L.dfirst[t], (int)L.rows.size());
+        };
+        if (tuned) tune(ctx_, key, RowTiles<T>::n, fl, go);
+        else go(0);
+      }
+      for (int v : L.verts) contract_table(v);
+    }
+    if (!norms_.empty()) {
+      int n = 1;
+      for (const auto& m : norms_) n = std::max(n, m.rows);
+      k_norm_rows<T><<<dim3(grid_for(n, 32, 1024), (unsigned)norms_.size()), 256, 0, ctx_->stream>>>(dnorms_);
+      TNFA_LAUNCH_CHECK();
+    }
+  }
+
+  // Points [p0, p0 + n) of the call, X the chunk's coordinates.
+  void points(const double* X, int n, void* out, int kind, int64_t Pout, int64_t pofs) {
+    if (ncodes_ > 0)
+      launch_digitize(ctx_, X, ncols_, n, druns_, (int)runs_.size(), ncodes_, codes_, Pc_, err_);
+    for (int v : tree_.order)
+      if (!tree_.v[v].tabled) contract_points(v, n);
+    centre(X, n, out, kind, Pout, pofs);
+  }
+
+ private:
+  struct Level {
+    std::vector<RowJob<T>> rows;
+    std::vector<int> verts;  // table vertices of the multi-child kernels
+    RowJob<T>* drows = nullptr;
+    std::vector<int> first[3];
+    int* dfirst[3] = {nullptr, nullptr, nullptr};
+  };
+
+  size_t table_bytes() const {
+    double b = 0;
+    for (int v = 0; v < topo_.V; ++v) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.tabled && !e.leaf) b += (double)e.N * (e.chi * sizeof(T) + 4);
+      if (e.absorb) b += absorbed_rows(v) * (e.W / tree_chi(e.kids.back(), v) * sizeof(T) + 4);
+      if (e.moved) b += (double)topo_.size(v) * sizeof(T);
+    }
+    return (size_t)std::min(b, 1e18);
+  }
+  int tree_chi(int w, int) const { return tree_.v[w].chi; }
+  double absorbed_rows(int v) const {
+    return (double)topo_.site_dim[v] * (double)tree_.v[tree_.v[v].kids.back()].N;
+  }
+
+  // Codes, message slots and table levels of the schedule.
+  void plan() {
+    const int V = topo_.V;
+    slot_.assign(V, -1);
+    mult_.assign(V, 1);
+    key_slot_.assign(V, -1);
+    row_slot_.assign(V, -1);
+    msg_.assign(V, -1);
+    npp_ = 0;
+    for (int v = 0; v < V; ++v) npp_ += !tree_.v[v].tabled;
+    int n = 0;
+    for (int v : tree_.order) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.tabled) continue;
+      const int ab = e.absorb ? e.kids.back() : -1;
+      if (e.absorb || topo_.site_dim[v] > 1) {
+        key_slot_[v] = slot_[v] = n++;
+        mult_[v] = e.absorb ? (int)tree_.v[ab].N : 1;
+        if (e.absorb) assign(ab, slot_[v], 1);
+      } else {
+        slot_[v] = -2;  // one site value, no digits
+      }
+      for (int w : e.kids)
+        if (w != ab && tree_.v[w].tabled) assign(w, row_slot_[w] = n++, 1);
+    }
+    for (const auto& c : tree_.comps)
+      for (int v : {c.a, c.b})
+        if (v >= 0 && tree_.v[v].tabled) assign(v, row_slot_[v] = n++, 1);
+    nslots_ = n;
+    // all sides are tables: the centre kernel takes the digits itself, as long
+    // as its shared memory holds them
+    fused_ = npp_ == 0 && n <= 16 && prog_.size() <= 256;
+    ncodes_ = fused_ ? 0 : n;
+    runs_ = make_runs(prog_, slot_, mult_);
+    // message slots (rows per point), reused once read; the output's is taken
+    // before the kids' are given back, so it never shares memory with them
+    std::vector<int> free_slots;
+    nmsg_ = 0;
+    msg_chi_ = 1;
+    for (int v : tree_.order) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.tabled) continue;
+      if (free_slots.empty()) free_slots.push_back(nmsg_++);
+      msg_[v] = free_slots.back();
+      free_slots.pop_back();
+      msg_chi_ = std::max(msg_chi_, e.chi);
+      for (int w : e.kids)
+        if (!tree_.v[w].tabled) free_slots.push_back(msg_[w]);
+    }
+    max_group_ = 1;
+    for (int v = 0; v < V; ++v)
+      if (!tree_.v[v].tabled)
+        max_group_ = std::max<int64_t>(max_group_, tree_.v[v].absorb ? (int64_t)absorbed_rows(v) : topo_.site_dim[v]);
+    // levels
+    lvl_.assign(V, 0);
+    lvl_m_.assign(V, 0);
+    int top = 0;
+    for (int v : tree_.order) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.leaf) continue;
+      int l = 0;
+      for (size_t i = 0; i < e.kids.size(); ++i) {
+        const bool ab = e.absorb && i + 1 == e.kids.size();
+        if (ab) lvl_m_[v] = lvl_[e.kids[i]] + 1;
+        l = std::max(l, ab ? lvl_m_[v] : tree_.v[e.kids[i]].tabled ? lvl_[e.kids[i]] : 0);
+      }
+      if (e.tabled) lvl_[v] = l + 1;
+      top = std::max({top, lvl_m_[v], e.tabled ? lvl_[v] : 0});
+    }
+    levels_.assign(top + 1, Level{});
+    for (int v : tree_.order) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.leaf) continue;
+      if (e.absorb) levels_[lvl_m_[v]].rows.emplace_back();
+      if (!e.tabled) continue;
+      if (row_form(v)) levels_[lvl_[v]].rows.emplace_back();
+      else levels_[lvl_[v]].verts.push_back(v);
+    }
+  }
+  // One kid besides the absorbed one: the row-gather kernel.
+  bool row_form(int v) const {
+    const EvalVertex& e = tree_.v[v];
+    return !e.tensor && (int)e.kids.size() - (e.absorb ? 1 : 0) == 1;
+  }
+  // Digit codes of everything below v: v's site value first, then the absorbed
+  // kid, then the others in order, the last one fastest.
+  void assign(int v, int s, int64_t m) {
+    const EvalVertex& e = tree_.v[v];
+    const int nk = (int)e.kids.size() - (e.absorb ? 1 : 0);
+    for (int i = nk - 1; i >= 0; --i) {
+      assign(e.kids[i], s, m);
+      m *= tree_.v[e.kids[i]].N;
+    }
+    if (e.absorb) {
+      assign(e.kids.back(), s, m);
+      m *= tree_.v[e.kids.back()].N;
+    }
+    slot_[v] = s;
+    mult_[v] = (int)m;
+  }
+
+  void lay_out(Carve& c, int64_t pc) {
+    const int V = topo_.V;
+    err_ = c.take<int>(1);
+    // the job tables (sizes known from the plan)
+    druns_ = c.take<DigitRun>(runs_.size());
+    blob_ = (unsigned char*)druns_;
+    moves_.clear();
+    int nmove = 0, nnorm = 0;
+    for (int v = 0; v < V; ++v) nmove += needs_move(v);
+    for (const auto& cc : tree_.comps)
+      for (int v : {cc.a, cc.b}) nnorm += v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf;
+    dmoves_ = c.take<MoveJob>(nmove);
+    dnorms_ = c.take<NormJob<T>>(nnorm);
+    dcentre_ = c.take<CentreJob<T>>(tree_.comps.size());
+    for (auto& L : levels_) {
+      L.drows = c.take<RowJob<T>>(L.rows.size());
+      for (int t = 0; t < RowTiles<T>::n; ++t) L.dfirst[t] = c.take<int>(L.rows.size() + 1);
+    }
+    tmeta_.assign(V, nullptr);
+    ttile_.assign(V, 0);
+    for (const auto& L : levels_)
+      for (int v : L.verts) tmeta_[v] = c.take<int>(group_meta_ints(table_groups(v)));
+    blob_bytes_ = c.used - (size_t)(blob_ - c.base);
+    // tensors and tables
+    ten_.assign(V, nullptr);
+    tab_.assign(V, nullptr);
+    tabe_.assign(V, nullptr);
+    abs_.assign(V, nullptr);
+    abse_.assign(V, nullptr);
+    for (int v = 0; v < V; ++v) {
+      const EvalVertex& e = tree_.v[v];
+      ten_[v] = needs_move(v) ? c.take<T>(topo_.size(v)) : const_cast<T*>(tensors_ + topo_.off[v]);
+      if (e.leaf) {
+        tab_[v] = ten_[v];
+      } else if (e.tabled) {
+        tab_[v] = c.take<T>((size_t)e.N * e.chi);
+        tabe_[v] = c.take<int>(e.N);
+      }
+      if (e.absorb) {
+        const int64_t r = (int64_t)absorbed_rows(v);
+        abs_[v] = c.take<T>((size_t)(r * (int64_t)(e.W / tree_.v[e.kids.back()].chi)));
+        abse_[v] = c.take<int>(r);
+      }
+    }
+    // per point
+    codes_ = c.take<int>((size_t)ncodes_ * pc);
+    perm_ = c.take<int>(npp_ ? pc : 0);
+    meta_ = c.take<int>(npp_ ? group_meta_ints((int)max_group_) : 0);
+    mval_ = c.take<T>((size_t)nmsg_ * pc * msg_chi_);
+    mexp_ = c.take<int>((size_t)nmsg_ * pc);
+    ld_ = pc;
+  }
+  bool needs_move(int v) const { return tree_.v[v].moved; }
+  int table_groups(int v) const {
+    return tree_.v[v].absorb ? (int)absorbed_rows(v) : topo_.site_dim[v];
+  }
+
+  RowIdx table_row(int div, int64_t mod) const {
+    RowIdx r;
+    r.div = div;
+    r.mod = (int)mod;
+    return r;
+  }
+
+  void fill_blob() {
+    host_.assign(blob_bytes_, 0);
+    auto put = [&](const void* dev, const void* src, size_t n) {
+      if (n) std::memcpy(host_.data() + ((const unsigned char*)dev - blob_), src, n);
+    };
+    put(druns_, runs_.data(), runs_.size() * sizeof(DigitRun));
+    moves_.clear();
+    norms_.clear();
+    for (int v = 0; v < topo_.V; ++v) {
+      const EvalVertex& e = tree_.v[v];
+      if (!needs_move(v)) continue;
+      std::vector<int> shape{topo_.site_dim[v], topo_.link[v]};
+      for (int c : topo_.children[v]) shape.push_back(topo_.link[c]);
+      TNFA_CHECK(shape.size() <= (size_t)MOVE_MAXD, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
+      std::vector<int64_t> str(shape.size(), 1);
+      for (int i = (int)shape.size() - 2; i >= 0; --i) str[i] = str[i + 1] * shape[i + 1];
+      MoveJob m{};
+      m.src = tensors_ + topo_.off[v];
+      m.dst = ten_[v];
+      m.n = topo_.size(v);
+      m.nd = (int)e.axes.size();
+      for (int i = 0; i < m.nd; ++i) {
+        m.dim[i] = shape[e.axes[i]];
+        m.str[i] = str[e.axes[i]];
+      }
+      moves_.push_back(m);
+    }
+    put(dmoves_, moves_.data(), moves_.size() * sizeof(MoveJob));
+    std::vector<CentreJob<T>> cj;
+    for (const auto& c : tree_.comps) {
+      CentreJob<T> j{};
+      j.chi = tree_.v[c.a].chi;
+      j.a = side(c.a);
+      if (c.b >= 0) j.b = side(c.b);
+      cj.push_back(j);
+      for (int v : {c.a, c.b})
+        if (v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf)
+          norms_.push_back({tab_[v], tabe_[v], (int)tree_.v[v].N, tree_.v[v].chi});
+    }
+    put(dcentre_, cj.data(), cj.size() * sizeof(CentreJob<T>));
+    put(dnorms_, norms_.data(), norms_.size() * sizeof(NormJob<T>));
+    centre_chi_ = 1;
+    centre_vec_ = true;
+    constexpr int vec = 16 / sizeof(T);
+    for (const auto& j : cj) {
+      centre_chi_ = std::max(centre_chi_, j.chi);
+      centre_vec_ &= j.chi % vec == 0 && ((uintptr_t)j.a.ptr & 15) == 0 && ((uintptr_t)j.b.ptr & 15) == 0;
+    }
+    for (auto& L : levels_) L.rows.clear();
+    for (int v : tree_.order) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.leaf) continue;
+      if (e.absorb) {
+        const int w = e.kids.back();
+        const EvalVertex& k = tree_.v[w];
+        RowJob<T> j{};
+        j.A = tab_[w];
+        j.Aexp = tabe_[w];
+        j.aidx = table_row(1, k.N);
+        j.B = ten_[v];
+        j.out = abs_[v];
+        j.out_exp = abse_[v];
+        j.K = k.chi;
+        j.N = (int)(e.W / k.chi);
+        j.rpg = (int)k.N;
+        j.rows = topo_.site_dim[v] * j.rpg;
+        levels_[lvl_m_[v]].rows.push_back(j);
+      }
+      if (e.tabled && row_form(v)) {
+        const int w = e.kids[0];
+        const EvalVertex& k = tree_.v[w];
+        RowJob<T> j{};
+        j.A = tab_[w];
+        j.Aexp = tabe_[w];
+        j.aidx = table_row(1, k.N);
+        j.B = e.absorb ? abs_[v] : ten_[v];
+        j.gexp = e.absorb ? abse_[v] : nullptr;
+        j.out = tab_[v];
+        j.out_exp = tabe_[v];
+        j.K = k.chi;
+        j.N = e.chi;
+        j.rpg = (int)k.N;
+        j.rows = (int)e.N;
+        levels_[lvl_[v]].rows.push_back(j);
+      }
+      if (tmeta_[v]) {  // uniform groups of a multi-child table
+        const int ng = table_groups(v), m = (int)(e.N / ng);
+        std::vector<int> g(group_meta_ints(ng));
+        const int tp = ttile_[v] = table_tile_rows(v);
+        for (int i = 0; i < ng; ++i) {
+          g[i] = i * m;
+          g[ng + i] = m;
+          g[2 * ng + i] = i * ((m + tp - 1) / tp);
+        }
+        g[3 * ng] = ng * ((m + tp - 1) / tp);
+        put(tmeta_[v], g.data(), g.size() * sizeof(int));
+      }
+    }
+    for (auto& L : levels_) {
+      put(L.drows, L.rows.data(), L.rows.size() * sizeof(RowJob<T>));
+      for (int t = 0; t < RowTiles<T>::n; ++t) {
+        L.first[t].assign(1, 0);
+        int64_t b = 0;
+        for (const auto& j : L.rows) {
+          b += row_blocks(j, t);
+          TNFA_CHECK(b < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
+          L.first[t].push_back((int)b);
+        }
+        put(L.dfirst[t], L.first[t].data(), L.first[t].size() * sizeof(int));
+      }
+    }
+  }
+
+  CentreSide<T> side(int v) const {
+    const EvalVertex& e = tree_.v[v];
+    CentreSide<T> s{};
+    s.slot = -1;
+    if (e.tabled) {
+      s.ptr = tab_[v];
+      s.exps = tabe_[v];
+      if (fused_) s.slot = row_slot_[v];
+      else s.idx.codes = codes_ + (int64_t)row_slot_[v] * ld_;
+      s.scale = e.leaf;
+    } else {
+      s.ptr = mval_ + (int64_t)msg_[v] * ld_ * msg_chi_;
+      s.exps = mexp_ + (int64_t)msg_[v] * ld_;
+      s.scale = 1;
+    }
+    return s;
+  }
+
+  // The multi-child job of vertex v (table rows or points), without groups.
+  VertexJob<T> vertex_job(int v) const {
+    const EvalVertex& e = tree_.v[v];
+    VertexJob<T> j{};
+    const int nk = (int)e.kids.size() - (e.absorb ? 1 : 0);
+    TNFA_CHECK(nk <= EVAL_MAXC, TNFA_ERR_UNSUPPORTED,
+               "vertex degree above " + std::to_string(EVAL_MAXC) + " children");
+    j.nchild = nk;
+    int64_t K = 1;
+    int div = 1;
+    for (int i = nk - 1; i >= 0; --i) {
+      const EvalVertex& k = tree_.v[e.kids[i]];
+      ChildSrc<T>& s = j.ch[i];
+      s.dim = k.chi;
+      K *= k.chi;
+      if (k.tabled) {
+        s.ptr = tab_[e.kids[i]];
+        s.exps = tabe_[e.kids[i]];
+        if (e.tabled) {
+          s.idx.div = div;
+          s.idx.mod = (int)k.N;
+          div *= (int)k.N;
+        } else {
+          s.idx.codes = codes_ + (int64_t)row_slot_[e.kids[i]] * ld_;
+        }
+      } else {
+        s.ptr = mval_ + (int64_t)msg_[e.kids[i]] * ld_ * msg_chi_;
+        s.exps = mexp_ + (int64_t)msg_[e.kids[i]] * ld_;
+      }
+    }
+    TNFA_CHECK(K < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
+    j.K = (int)K;
+    j.chi_a = e.chi;
+    j.B = e.absorb ? abs_[v] : ten_[v];
+    j.gexp = e.absorb ? abse_[v] : nullptr;
+    j.site_dim = j.ngroups = e.absorb ? (int)absorbed_rows(v) : topo_.site_dim[v];
+    if (e.tabled) {
+      j.out = tab_[v];
+      j.out_exp = tabe_[v];
+      j.Pc = (int)e.N;
+    } else {
+      j.out = mval_ + (int64_t)msg_[v] * ld_ * msg_chi_;
+      j.out_exp = mexp_ + (int64_t)msg_[v] * ld_;
+    }
+    return j;
+  }
+  int job_sumdim(int v) const {
+    const EvalVertex& e = tree_.v[v];
+    int s = 0;
+    for (size_t i = 0; i + (e.absorb ? 1 : 0) < e.kids.size(); ++i) s += tree_.v[e.kids[i]].chi;
+    return s;
+  }
+  std::vector<GemmTile> vertex_tiles(int v, std::string* key) const {
+    const EvalVertex& e = tree_.v[v];
+    if (e.tensor || e.chi <= 16) return {};
+    *key = std::string("simt:") + FamilyName<T>::v + ":" + std::to_string(e.chi) + ":";
+    const int nk = (int)e.kids.size() - (e.absorb ? 1 : 0);
+    for (int i = 0; i < nk; ++i)
+      *key += std::to_string(tree_.v[e.kids[i]].chi) + (i + 1 < nk ? "x" : "");
+    return gemm_tile_candidates(e.chi, job_sumdim(v), sizeof(T));
+  }
+  int table_tile_rows(int v) const {
+    if (tree_.v[v].tensor) return use_tc_ ? tc_tile_rows() : oz_tile_rows();
+    std::string key;
+    const auto cand = vertex_tiles(v, &key);
+    if (cand.empty()) return contract_tile_rows(tree_.v[v].chi, job_sumdim(v), sizeof(T));
+    const int kept = tuned_choice(ctx_, key);
+    return cand[kept >= 0 ? kept : 0].tp;
+  }
+
+  // Runs a multi-child job whose groups are in meta with tile rows tp.
+  void contract_vertex(int v, VertexJob<T>& j, int* meta, bool keyed, int tp) {
+    const int ng = j.ngroups;
+    j.grp_off = meta;
+    j.grp_cnt = meta + ng;
+    j.tile_start = meta + 2 * ng;
+    if (tree_.v[v].tensor) {
+      if constexpr (std::is_same<T, float>::value) {
+        tc_contract_vertex(ctx_, net_, v, j, tp, err_);
+        return;
+      }
+      if constexpr (std::is_same<T, double>::value) {
+        oz_contract_vertex(ctx_, net_, v, j, tp, err_);
+        return;
+      }
+    }
+    std::string key;
+    const auto cand = vertex_tiles(v, &key);
+    if (cand.empty()) {
+      launch_contract<T>(ctx_, j, j.Pc);
+      return;
+    }
+    int cur = tp;
+    tune(ctx_, key, (int)cand.size(), 2.0 * j.Pc * (double)j.K * j.chi_a, [&](int i) {
+      if (cand[i].tp != cur) {  // tile table for this candidate's rows per tile
+        launch_retile(ctx_, keyed, j.Pc, ng, cand[i].tp, meta);
+        cur = cand[i].tp;
+      }
+      launch_contract<T>(ctx_, j, j.Pc, &cand[i]);
+    });
+  }
+
+  void contract_table(int v) {
+    VertexJob<T> j = vertex_job(v);
+    contract_vertex(v, j, tmeta_[v], true, ttile_[v]);
+  }
+
+  RowJob<T> point_rows(int v, int n) const {
+    const EvalVertex& e = tree_.v[v];
+    const int w = e.kids[0];
+    const EvalVertex& k = tree_.v[w];
+    RowJob<T> j{};
+    if (k.tabled) {
+      j.A = tab_[w];
+      j.Aexp = tabe_[w];
+      j.aidx.codes = codes_ + (int64_t)row_slot_[w] * ld_;
+    } else {
+      j.A = mval_ + (int64_t)msg_[w] * ld_ * msg_chi_;
+      j.Aexp = mexp_ + (int64_t)msg_[w] * ld_;
+    }
+    j.B = e.absorb ? abs_[v] : ten_[v];
+    j.gexp = e.absorb ? abse_[v] : nullptr;
+    j.out = mval_ + (int64_t)msg_[v] * ld_ * msg_chi_;
+    j.out_exp = mexp_ + (int64_t)msg_[v] * ld_;
+    j.K = k.chi;
+    j.N = e.chi;
+    j.rows = n;
+    j.ngroups = e.absorb ? (int)absorbed_rows(v) : topo_.site_dim[v];
+    j.grp_off = meta_;
+    j.grp_cnt = meta_ + j.ngroups;
+    j.tile_start = meta_ + 2 * j.ngroups;
+    return j;
+  }
+
+  void contract_points(int v, int n) {
+    const EvalVertex& e = tree_.v[v];
+    const int* key = key_slot_[v] >= 0 ? codes_ + (int64_t)key_slot_[v] * ld_ : nullptr;
+    if (!row_form(v)) {
+      VertexJob<T> j = vertex_job(v);
+      j.Pc = n;
+      const int tp = table_tile_rows(v);
+      j.perm = launch_group(ctx_, key, n, j.ngroups, tp, meta_, perm_);
+      contract_vertex(v, j, meta_, key != nullptr, tp);
+      return;
+    }
+    RowJob<T> j = point_rows(v, n);
+    const double fl = 2.0 * n * (double)j.N * j.K;
+    const int rule = group_tile(j);
+    const std::string tkey = std::string("simt:") + FamilyName<T>::v + ":points:" + std::to_string(j.N) + "x" +
+                             std::to_string(j.K) + ":" + std::to_string(j.ngroups > 1024 ? n / j.ngroups : 0);
+    const int kept = tuned_choice(ctx_, tkey);
+    auto tile_of = [&](int i) { return i == 0 ? rule : i <= rule ? i - 1 : i; };
+    int cur = 8 * RowTiles<T>::rm[tile_of(kept >= 0 ? kept : 0)];
+    j.perm = launch_group(ctx_, key, n, j.ngroups, cur, meta_, perm_);
+    tune(ctx_, tkey, RowTiles<T>::n, fl, [&](int i) {
+      const int t = tile_of(i), tp = 8 * RowTiles<T>::rm[t];
+      if (tp != cur) {
+        launch_retile(ctx_, key != nullptr, n, j.ngroups, tp, meta_);
+        cur = tp;
+      }
+      KernelScope ks(ctx_, FamilyName<T>::v, fl, (double)sizeof(T) * n * (j.N + j.K));
+      launch_rows<T>(ctx_, t, row_blocks(j, t), j, nullptr, nullptr, 0);
+    });
+  }
+  int group_tile(const RowJob<T>& j) const { return row_tile<T>(ctx_, {j}); }
+
+  void centre(const double* X, int n, void* out, int kind, int64_t Pout, int64_t pofs) {
+    const int ns = fused_ ? nslots_ : 0;
+    const size_t sm = 256 * (sizeof(T) + 4) + (size_t)ns * 1024 + (fused_ ? runs_.size() * sizeof(DigitRun) : 0);
+    KernelScope ks(ctx_, "centre", 2.0 * n * centre_chi_, (double)n * (ncols_ * 8.0 + 8.0));
+    const unsigned grid = grid_for(n, 256, ctx_->sm_count * 8);
+    auto go = [&](auto kern) {
+      kern<<<grid, 256, sm, ctx_->stream>>>(X, ncols_, n, druns_, (int)runs_.size(), ns, dcentre_,
+                                           (int)tree_.comps.size(), out, kind, Pout, pofs, err_);
+    };
+    constexpr int vec = 16 / sizeof(T);
+    if constexpr (vec > 1) {
+      if (centre_vec_) {
+        const int lanes = (centre_chi_ + vec - 1) / vec;
+        if (lanes <= 1) go(k_centre<T, 1, vec>);
+        else if (lanes <= 2) go(k_centre<T, 2, vec>);
+        else if (lanes <= 4) go(k_centre<T, 4, vec>);
+        else go(k_centre<T, 8, vec>);
+        TNFA_LAUNCH_CHECK();
+        return;
+      }
+    }
+    if (centre_chi_ <= 2) go(k_centre<T, 1, 1>);
+    else if (centre_chi_ <= 8) go(k_centre<T, 2, 1>);
+    else go(k_centre<T, 8, 1>);
+    TNFA_LAUNCH_CHECK();
+  }
+
+  tnfa_ctx* ctx_;
+  const tnfa_net* net_;
+  const T* tensors_;
+  const Topo& topo_;
+  const std::vector<DigitRef>& prog_;
+  int ncols_;
+  int64_t P_;
+  bool use_tc_, use_oz_;
+  EvalTree tree_;
+  std::vector<int> ttile_;  // tile rows that the group table of a table vertex was made for
+  std::vector<int> slot_, mult_, key_slot_, row_slot_, msg_, lvl_, lvl_m_;
+  std::vector<DigitRun> runs_;
+  std::vector<Level> levels_;
+  int nslots_ = 0, ncodes_ = 0, nmsg_ = 0, msg_chi_ = 1, npp_ = 0, Pc_ = 0, centre_chi_ = 1;
+  int64_t max_group_ = 1, ld_ = 0;
+  bool fused_ = false, centre_vec_ = false;
+  size_t per_point_ = 0, blob_bytes_ = 0;
+  std::vector<unsigned char> host_;
+  std::vector<MoveJob> moves_;
+  std::vector<NormJob<T>> norms_;
+  // scratch
+  int* err_ = nullptr;
+  unsigned char* blob_ = nullptr;
+  DigitRun* druns_ = nullptr;
+  MoveJob* dmoves_ = nullptr;
+  NormJob<T>* dnorms_ = nullptr;
+  CentreJob<T>* dcentre_ = nullptr;
+  std::vector<int*> tmeta_, tabe_, abse_;
+  std::vector<T*> ten_, tab_, abs_;
+  int *codes_ = nullptr, *perm_ = nullptr, *meta_ = nullptr, *mexp_ = nullptr;
+  T* mval_ = nullptr;
+};
+
+static size_t out_elem_size(int out_kind) {
+  return out_kind == TNFA_OUT_F64 ? 8 : out_kind == TNFA_OUT_F32 ? 4 : out_kind == TNFA_OUT_F32_SCALED ? 8 : 16;
+}
+
+static void check_eval_error(tnfa_ctx* ctx, const int* derr) {
+  int herr = 0;
+  TNFA_CUDA(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
+  TNFA_CHECK((herr & 2) == 0, TNFA_ERR_TIMEOUT,
+             "a tensor-core pipeline wait ran out of its iteration budget");
+  TNFA_CHECK(herr == 0, TNFA_ERR_DOMAIN,
+             "a coordinate is negative or not finite (the digit map needs x >= 0)");
+}
+
+template <class T>
+static void evaluate_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double* X,
+                          int64_t P, int ncols, const std::vector<DigitRef>& prog, int xmem,
+                          void* out, int out_kind, int out_mem, bool use_tc,
+                          bool use_oz = false) {
+  const size_t out_elem = out_elem_size(out_kind);
+  const size_t staged = (xmem == TNFA_MEM_HOST ? ncols * 8 : 0) + (out_mem == TNFA_MEM_HOST ? out_elem : 0);
+  // small bonds everywhere: the whole tree per thread in one launch
+  const FusedPlan F = make_fused_plan(net->topo, sizeof(T), prog.size(), P);
+  std::unique_ptr<EvalEngine<T>> E;
+  std::vector<DigitRun> runs;
+  int64_t Pcap;
+  if (F.ok) {
+    runs = make_fused_runs(net->topo, prog);
+    Pcap = staged ? std::max<int64_t>(256, (int64_t)(ctx->eval_budget / staged) / 256 * 256) : int64_t(1) << 30;
+  } else {
+    E.reset(new EvalEngine<T>(ctx, net, tensors, prog, ncols, P, use_tc, use_oz, ctx->eval_budget));
+    Pcap = E->chunk();
+    if (staged) Pcap = std::min(Pcap, std::max<int64_t>(256, (int64_t)(ctx->eval_budget / staged) / 256 * 256));
+  }
+  Pcap = std::max<int64_t>(1, std::min<int64_t>({P, Pcap, int64_t(1) << 30}));
+  DBuf dX(ctx, xmem == TNFA_MEM_HOST ? (size_t)Pcap * ncols * 8 : 0);
+  DBuf dout(ctx, out_mem == TNFA_MEM_HOST ? (size_t)Pcap * out_elem : 0);
+  DBuf derr(ctx, 4), arena, dprog, dsteps;
+  int* err;
+  if (F.ok) {
+    dprog = DBuf(ctx, std::max<size_t>(runs.size(), 1) * sizeof(DigitRun));
+    h2d(ctx, dprog.p, runs.data(), runs.size() * sizeof(DigitRun));
+    dsteps = DBuf(ctx, F.steps.size() * sizeof(FusedStep));
+    h2d(ctx, dsteps.p, F.steps.data(), F.steps.size() * sizeof(FusedStep));
+    err = derr.as<int>();
+    TNFA_CUDA(cudaMemsetAsync(err, 0, 4, ctx->stream));
+  } else {
+    E->set_chunk((int)Pcap);
+    arena = DBuf(ctx, E->scratch(Pcap));
+    E->bind(arena.p);
+    E->upload();
+    E->tables();
+    err = E->err_flag();
+  }
+  for (int64_t p0 = 0; p0 < P; p0 += Pcap) {
+    const int Pc = (int)std::min<int64_t>(Pcap, P - p0);
+    const double* Xc = X + p0 * ncols;
+    if (xmem == TNFA_MEM_HOST) {
+      TNFA_CUDA(cudaMemcpyAsync(dX.p, Xc, (size_t)Pc * ncols * 8, cudaMemcpyHostToDevice, ctx->stream));
+      Xc = dX.as<double>();
+    }
+    void* o = out_mem == TNFA_MEM_HOST ? dout.p : out;
+    const int64_t Pout = out_mem == TNFA_MEM_HOST ? Pc : P, pofs = out_mem == TNFA_MEM_HOST ? 0 : p0;
+    if (F.ok)
+      launch_fused<T>(ctx, F, dsteps.as<FusedStep>(), tensors, net->topo, Xc, ncols, Pc,
+                      dprog.as<DigitRun>(), (int)runs.size(), o, out_kind, Pout, pofs, err);
+    else
+      E->points(Xc, Pc, o, out_kind, Pout, pofs);
+    if (out_mem == TNFA_MEM_HOST) {
+      if (out_kind == TNFA_OUT_F32_SCALED) {
+        TNFA_CUDA(cudaMemcpyAsync((float*)out + p0, dout.p, (size_t)Pc * 4, cudaMemcpyDeviceToHost,
+                                  ctx->stream));
+        TNFA_CUDA(cudaMemcpyAsync((int*)((float*)out + P) + p0, (float*)dout.p + Pc, (size_t)Pc * 4,
+                                  cudaMemcpyDeviceToHost, ctx->stream));
+      } else {
+        TNFA_CUDA(cudaMemcpyAsync((char*)out + p0 * out_elem, dout.p, (size_t)Pc * out_elem,
+                                  cudaMemcpyDeviceToHost, ctx->stream));
+      }
+    }
+  }
+  check_eval_error(ctx, err);
 }
 
 }  // namespace tnfa
@@ -1056,7 +1610,7 @@ extern "C" int tnfa_evaluate(tnfa_ctx* ctx, const tnfa_net* net, const double* X
   for (int v = 0; v < net->topo.V; ++v)
     TNFA_CHECK(net->topo.site_dim[v] <= 256, TNFA_ERR_UNSUPPORTED, "site dimension above 256");
   int ncols = 0;
-  std::vector<DigitEntry> prog = make_digit_program(net->topo, n_dims, dims, &ncols);
+  std::vector<DigitRef> prog = make_digit_program(net->topo, n_dims, dims, &ncols);
   if (net->dtype == TNFA_C128) {
     TNFA_CHECK(out_kind == TNFA_OUT_C128, TNFA_ERR_DTYPE, "complex networks need TNFA_OUT_C128");
     TNFA_CHECK(precision == TNFA_PREC_F64, TNFA_ERR_UNSUPPORTED,
@@ -1135,189 +1689,123 @@ unsigned char* noalloc_base(int device) {
   return addr[device];
 }
 
-struct Carve {
-  unsigned char* base;
-  size_t cap, used = 0;
-  size_t take_off(size_t bytes) {
-    const size_t off = (used + 255) & ~(size_t)255;
-    used = off + bytes;
-    return off;
-  }
-  void* take(size_t bytes) {
-    const size_t off = take_off(bytes);
-    TNFA_CHECK(used <= cap, TNFA_ERR_INVALID_ARGUMENT, "scratch overflow");
-    return base + off;
-  }
-};
-
-// The pieces evaluate_noalloc_impl carves for P points, in order: digit
-// program, fused schedule, digits, permutation, group tables, error flag,
-// message slots, slot exponents, root values, root exponents.  The fused
-// small-bond path needs only the program, its schedule and the error flag.
-template <class T>
-std::array<size_t, 10> noalloc_sizes(const tnfa_net* net, const EvalPlan& plan, int64_t P,
-                                     size_t prog_entries, const FusedPlan& F) {
-  const Topo& Tp = net->topo;
-  const int V = Tp.V;
-  const int nroots = (int)plan.roots.size();
-  int maxsd = 1;
-  for (int v = 0; v < V; ++v) maxsd = std::max(maxsd, Tp.site_dim[v]);
-  const size_t slot_vals = (size_t)P * plan.chimax;
-  if (F.ok)
-    return {prog_entries * sizeof(DigitEntry), F.steps.size() * sizeof(FusedStep), 0, 0, 0, 4,
-            0, 0, 0, 0};
-  return {prog_entries * sizeof(DigitEntry),
-          0,
-          (size_t)V * P,
-          (size_t)P * 4,
-          group_meta_ints(maxsd) * 4,
-          4,
-          (size_t)plan.nslots * slot_vals * sizeof(T),
-          (size_t)plan.nslots * P * sizeof(int),
-          (size_t)nroots * P * sizeof(T),
-          (size_t)nroots * P * sizeof(int)};
-}
-
-// Scratch bytes evaluate_noalloc_impl carves for P points (256-byte aligned pieces).
+// Scratch bytes by which a request is accepted: digit program, fused schedule,
+// digits, permutation, group tables, error flag, message slots of every point
+// and root values, in 256-byte pieces.  The calls that fit are part of the
+// interface; the schedule itself works in chunks that fit (FixedRun).
 template <class T>
 size_t noalloc_bytes(const tnfa_net* net, int64_t P, size_t prog_entries) {
-  Carve dry{nullptr, ~(size_t)0};
-  const FusedPlan F = make_fused_plan(net->topo, sizeof(T), prog_entries, P);
-  for (size_t s : noalloc_sizes<T>(net, make_plan(net->topo), P, prog_entries, F)) dry.take_off(s);
+  const Topo& Tp = net->topo;
+  const FusedPlan F = make_fused_plan(Tp, sizeof(T), prog_entries, P);
+  const EvalPlan plan = make_plan(Tp);
+  const size_t nroots = plan.roots.size();
+  int maxsd = 1;
+  for (int v = 0; v < Tp.V; ++v) maxsd = std::max(maxsd, Tp.site_dim[v]);
+  std::array<size_t, 10> sizes{prog_entries * 32, 0, 0, 0, 0, 4, 0, 0, 0, 0};
+  if (F.ok) {
+    sizes[1] = F.steps.size() * sizeof(FusedStep);
+  } else {
+    sizes[2] = (size_t)Tp.V * P;
+    sizes[3] = (size_t)P * 4;
+    sizes[4] = group_meta_ints(maxsd) * 4;
+    sizes[6] = (size_t)plan.nslots * P * plan.chimax * sizeof(T);
+    sizes[7] = (size_t)plan.nslots * P * sizeof(int);
+    sizes[8] = nroots * P * sizeof(T);
+    sizes[9] = nroots * P * sizeof(int);
+  }
+  Carve dry;
+  for (size_t s : sizes) dry.take<unsigned char>(s);
   return dry.used;
 }
 
-// The evaluation kernels over scratch carved from [base, base + cap).  With
-// check, the digit program is copied in from the host and the call ends by
-// reading the error flag (a host sync); without it (stream capture), the
-// program must already sit at the start of the scratch and the call only
-// enqueues work.  *err_flag receives the device address of the error flag.
+// An evaluation over scratch that the caller owns: stage() sends the job
+// tables there, enqueue() runs the kernels (and nothing else, so that it can
+// be captured).
 template <class T>
-void evaluate_noalloc_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double* X,
-                           int64_t P64, int ncols, const std::vector<DigitEntry>& prog, void* out,
-                           int out_kind, unsigned char* base, size_t cap, bool check,
-                           int** err_flag = nullptr) {
-  const Topo& Tp = net->topo;
-  const int V = Tp.V;
-  EvalPlan plan = make_plan(Tp);
-  const int nroots = (int)plan.roots.size();
-  // Dry run of the carving to size the request before touching the device.
-  const int64_t P = P64;
-  const size_t slot_vals = (size_t)P * plan.chimax;
-  const FusedPlan F = make_fused_plan(Tp, sizeof(T), prog.size(), P);
-  const std::array<size_t, 10> sizes = noalloc_sizes<T>(net, plan, P, prog.size(), F);
-  Carve dry{nullptr, cap};
-  for (size_t s : sizes) dry.take_off(s);
-  if (dry.used > cap) {
-    const size_t per_point = (dry.used - prog.size() * sizeof(DigitEntry)) / (size_t)std::max<int64_t>(P, 1) + 1;
+class FixedRun {
+ public:
+  FixedRun(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const std::vector<DigitRef>& prog, int ncols,
+           int64_t P, size_t budget)
+      : ctx_(ctx), net_(net), tensors_(tensors), ncols_(ncols), P_(P),
+        F_(make_fused_plan(net->topo, sizeof(T), prog.size(), P)) {
+    if (F_.ok) {
+      runs_ = make_fused_runs(net->topo, prog);
+      return;
+    }
+    E_.reset(new EvalEngine<T>(ctx, net, tensors, prog, ncols, P, false, false, budget));
+    int pc = E_->chunk();
+    while (pc > 1 && E_->scratch(pc) > budget) pc = std::max(1, pc / 2);
+    E_->set_chunk(pc);
+  }
+  size_t bytes() {
+    if (!F_.ok) return E_->scratch(E_->chunk());
+    Carve c;
+    lay_out(c);
+    return c.used + 256;
+  }
+  void bind(void* base) {
+    Carve c;
+    c.base = (unsigned char*)base;
+    if (F_.ok) lay_out(c);
+    else E_->bind(base);
+  }
+  void stage() {
+    if (F_.ok) {
+      h2d(ctx_, dprog_, runs_.data(), runs_.size() * sizeof(DigitRun));
+      h2d(ctx_, dsteps_, F_.steps.data(), F_.steps.size() * sizeof(FusedStep));
+    } else {
+      E_->upload();
+    }
+  }
+  int* err_flag() const { return F_.ok ? err_ : E_->err_flag(); }
+  void enqueue(const double* X, void* out, int out_kind) {
+    TNFA_CUDA(cudaMemsetAsync(err_flag(), 0, 4, ctx_->stream));
+    if (F_.ok) {
+      launch_fused<T>(ctx_, F_, dsteps_, tensors_, net_->topo, X, ncols_, (int)P_, dprog_, (int)runs_.size(), out,
+                      out_kind, P_, 0, err_);
+      return;
+    }
+    E_->tables();
+    for (int64_t p0 = 0; p0 < P_; p0 += E_->chunk())
+      E_->points(X + p0 * ncols_, (int)std::min<int64_t>(E_->chunk(), P_ - p0), out, out_kind, P_, p0);
+  }
+
+ private:
+  void lay_out(Carve& c) {
+    dprog_ = c.take<DigitRun>(runs_.size());
+    dsteps_ = c.take<FusedStep>(F_.steps.size());
+    err_ = c.take<int>(1);
+  }
+  tnfa_ctx* ctx_;
+  const tnfa_net* net_;
+  const T* tensors_;
+  int ncols_;
+  int64_t P_;
+  FusedPlan F_;
+  std::vector<DigitRun> runs_;
+  std::unique_ptr<EvalEngine<T>> E_;
+  DigitRun* dprog_ = nullptr;
+  FusedStep* dsteps_ = nullptr;
+  int* err_ = nullptr;
+};
+
+template <class T>
+void evaluate_noalloc_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double* X, int64_t P,
+                           int ncols, const std::vector<DigitRef>& prog, void* out, int out_kind) {
+  const size_t need = noalloc_bytes<T>(net, P, prog.size());
+  if (need > NOALLOC_BYTES) {
+    const size_t per_point = (need - prog.size() * 32) / (size_t)std::max<int64_t>(P, 1) + 1;
     fail(TNFA_ERR_INVALID_ARGUMENT,
-         "tnfa_evaluate_noalloc: " + std::to_string(P) + " points need " +
-             std::to_string(dry.used) + " bytes of scratch, above the fixed " +
-             std::to_string(cap) + "; this network allows about " +
-             std::to_string(cap / per_point) + " points per call");
+         "tnfa_evaluate_noalloc: " + std::to_string(P) + " points need " + std::to_string(need) +
+             " bytes of scratch, above the fixed " + std::to_string(NOALLOC_BYTES) +
+             "; this network allows about " + std::to_string(NOALLOC_BYTES / per_point) + " points per call");
   }
-  Carve cv{base, cap};
-  DigitEntry* dprog = (DigitEntry*)cv.take(sizes[0]);
-  FusedStep* dsteps = (FusedStep*)cv.take(sizes[1]);
-  uint8_t* dS = (uint8_t*)cv.take(sizes[2]);
-  int* dperm = (int*)cv.take(sizes[3]);
-  int* meta = (int*)cv.take(sizes[4]);
-  int* derr = (int*)cv.take(sizes[5]);
-  T* slots = (T*)cv.take(sizes[6]);
-  int* slote = (int*)cv.take(sizes[7]);
-  T* rootv = (T*)cv.take(sizes[8]);
-  int* roote = (int*)cv.take(sizes[9]);
-  const int Pc = (int)P;
-  // the array keeps the previous call's contents: clear what must start at 0
-  if (err_flag) *err_flag = derr;
-  TNFA_CUDA(cudaMemsetAsync(derr, 0, 4, ctx->stream));
-  if (F.ok) {
-    if (check) {
-      if (!prog.empty())
-        TNFA_CUDA(cudaMemcpyAsync(dprog, prog.data(), sizes[0], cudaMemcpyHostToDevice, ctx->stream));
-      TNFA_CUDA(cudaMemcpyAsync(dsteps, F.steps.data(), sizes[1], cudaMemcpyHostToDevice, ctx->stream));
-    }
-    launch_fused<T>(ctx, F, dsteps, tensors, Tp, X, ncols, Pc, dprog, (int)prog.size(), out, out_kind,
-                    P, 0, derr);
-  } else {
-  TNFA_CUDA(cudaMemsetAsync(dS, 0, (size_t)V * P, ctx->stream));
-  if (!prog.empty()) {
-    if (check)
-      TNFA_CUDA(cudaMemcpyAsync(dprog, prog.data(), sizes[0], cudaMemcpyHostToDevice, ctx->stream));
-    k_digitize<<<grid_for(Pc, 256, 8 * 152 * 8), 256, 0, ctx->stream>>>(
-        X, ncols, Pc, dprog, (int)prog.size(), dS, (int64_t)P, derr);
-    TNFA_LAUNCH_CHECK();
-  }
-  std::vector<int> root_index(V, -1);
-  for (int r = 0; r < nroots; ++r) root_index[plan.roots[r]] = r;
-  for (int v : plan.order) {
-    VertexJob<T> j{};
-    j.nchild = (int)Tp.children[v].size();
-    TNFA_CHECK(j.nchild <= EVAL_MAXC, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
-    int64_t K = 1;
-    int sumdim = 0;
-    for (int i = 0; i < j.nchild; ++i) {
-      const int c = Tp.children[v][i];
-      ChildSrc<T>& s = j.ch[i];
-      s.dim = Tp.link[c];
-      sumdim += s.dim;
-      K *= s.dim;
-      if (plan.fused_leaf[c]) {
-        s.ptr = tensors + Tp.off[c];
-        s.exps = nullptr;
-        s.S = dS + (int64_t)c * P;
-      } else {
-        s.ptr = slots + (size_t)plan.slot[c] * slot_vals;
-        s.exps = slote + (size_t)plan.slot[c] * P;
-        s.S = nullptr;
-      }
-    }
-    TNFA_CHECK(K < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
-    j.K = (int)K;
-    j.chi_a = Tp.link[v];
-    j.site_dim = Tp.site_dim[v];
-    j.B = tensors + Tp.off[v];
-    j.Pc = Pc;
-    if (Tp.parent[v] < 0) {
-      j.out = rootv + (size_t)root_index[v] * P;
-      j.out_exp = roote + (size_t)root_index[v] * P;
-    } else {
-      j.out = slots + (size_t)plan.slot[v] * slot_vals;
-      j.out_exp = slote + (size_t)plan.slot[v] * P;
-    }
-    const int tp = contract_tile_rows(j.chi_a, sumdim, sizeof(T));
-    const int ng = j.site_dim;
-    j.ngroups = ng;
-    j.grp_off = meta;
-    j.grp_cnt = meta + ng;
-    j.tile_start = meta + 2 * ng;
-    if (ng == 1) {
-      k_group_identity<<<1, 1, 0, ctx->stream>>>(meta, Pc, tp);
-      TNFA_LAUNCH_CHECK();
-      j.perm = nullptr;
-    } else {
-      TNFA_CHECK(ng <= 256, TNFA_ERR_UNSUPPORTED, "site dimension above 256 per vertex");
-      const uint8_t* Sv = dS + (int64_t)v * P;
-      TNFA_CUDA(cudaMemsetAsync(meta + ng, 0, ng * sizeof(int), ctx->stream));
-      k_group_count<<<grid_for(Pc, 256, 4 * 152), 256, 0, ctx->stream>>>(Sv, Pc, ng, meta + ng);
-      k_group_scan<<<1, 1, 0, ctx->stream>>>(meta, ng, tp);
-      const unsigned gs = (unsigned)((Pc + 256 * SCATTER_ITEMS - 1) / (256 * SCATTER_ITEMS));
-      k_group_scatter<<<gs, 256, 0, ctx->stream>>>(Sv, Pc, ng, meta + 3 * ng + 1, dperm);
-      TNFA_LAUNCH_CHECK();
-      j.perm = dperm;
-    }
-    launch_contract<T>(ctx, j, Pc);
-  }
-  k_combine<T><<<grid_for(Pc, 256, 8192), 256, 0, ctx->stream>>>(rootv, roote, nroots, Pc, out,
-                                                                   out_kind, P, 0);
-  TNFA_LAUNCH_CHECK();
-  }
-  if (!check) return;
-  int herr = 0;
-  TNFA_CUDA(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, ctx->stream));
-  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
-  TNFA_CHECK(herr == 0, TNFA_ERR_DOMAIN,
-             "a coordinate is negative or not finite (the digit map needs x >= 0)");
+  FixedRun<T> run(ctx, net, tensors, prog, ncols, P, NOALLOC_BYTES);
+  TNFA_CHECK(run.bytes() <= NOALLOC_BYTES, TNFA_ERR_INVALID_ARGUMENT, "scratch overflow");
+  run.bind(noalloc_base(ctx->device));
+  run.stage();
+  run.enqueue(X, out, out_kind);
+  check_eval_error(ctx, run.err_flag());
 }
 
 }  // namespace
@@ -1337,22 +1825,22 @@ extern "C" int tnfa_evaluate_noalloc(tnfa_ctx* ctx, const tnfa_net* net, const d
   for (int v = 0; v < net->topo.V; ++v)
     TNFA_CHECK(net->topo.site_dim[v] <= 256, TNFA_ERR_UNSUPPORTED, "site dimension above 256");
   int ncols = 0;
-  std::vector<DigitEntry> prog = make_digit_program(net->topo, n_dims, dims, &ncols);
+  std::vector<DigitRef> prog = make_digit_program(net->topo, n_dims, dims, &ncols);
   if (net->dtype == TNFA_C128) {
     TNFA_CHECK(out_kind == TNFA_OUT_C128 && precision == TNFA_PREC_F64, TNFA_ERR_DTYPE,
                "complex networks: TNFA_OUT_C128 and TNFA_PREC_F64");
     evaluate_noalloc_impl<cplx>(ctx, net, (const cplx*)net->d, X, n_points, ncols, prog, out,
-                                out_kind, noalloc_base(ctx->device), NOALLOC_BYTES, true);
+                                out_kind);
   } else {
     TNFA_CHECK(out_kind == TNFA_OUT_F64 || out_kind == TNFA_OUT_F32 ||
                    out_kind == TNFA_OUT_F32_SCALED,
                TNFA_ERR_DTYPE, "real networks need a real output kind");
     if (precision == TNFA_PREC_F64 && net->dtype == TNFA_F64)
       evaluate_noalloc_impl<double>(ctx, net, (const double*)net->d, X, n_points, ncols, prog, out,
-                                    out_kind, noalloc_base(ctx->device), NOALLOC_BYTES, true);
+                                    out_kind);
     else if (precision == TNFA_PREC_F32 && net->dtype == TNFA_F32)
       evaluate_noalloc_impl<float>(ctx, net, (const float*)net->d, X, n_points, ncols, prog, out,
-                                   out_kind, noalloc_base(ctx->device), NOALLOC_BYTES, true);
+                                   out_kind);
     else
       fail(TNFA_ERR_UNSUPPORTED,
            "tnfa_evaluate_noalloc computes in the network's own type: TNFA_PREC_F64 on FP64 "
@@ -1390,20 +1878,21 @@ void plan_free(tnfa_eval_plan* p) {
 
 template <class T>
 void plan_build(tnfa_eval_plan* p, const T* tensors, const double* X, int ncols,
-                const std::vector<DigitEntry>& prog, void* out, int out_kind) {
+                const std::vector<DigitRef>& prog, void* out, int out_kind) {
   tnfa_ctx* ctx = p->ctx;
-  const size_t bytes = noalloc_bytes<T>(p->net, p->n_points, prog.size());
-  TNFA_CUDA(cudaMalloc(&p->scratch, bytes));
+  FixedRun<T> run(ctx, p->net, tensors, prog, ncols, p->n_points, ctx->eval_budget);
+  TNFA_CUDA(cudaMalloc(&p->scratch, run.bytes()));
+  run.bind(p->scratch);
+  p->derr = run.err_flag();
   // one eager run: validates the inputs, sets kernel attributes, stages the
-  // digit program at the start of the scratch (where the capture expects it)
-  evaluate_noalloc_impl<T>(ctx, p->net, tensors, X, p->n_points, ncols, prog, out, out_kind,
-                           (unsigned char*)p->scratch, bytes, true, &p->derr);
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
-  TNFA_CUDA(cudaStreamBeginCapture(ctx->stream, mode));
+  // job tables in the scratch (where the capture expects them)
+  run.stage();
+  run.enqueue(X, out, out_kind);
+  check_eval_error(ctx, p->derr);
+  TNFA_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   ctx->capturing = true;
   try {
-    evaluate_noalloc_impl<T>(ctx, p->net, tensors, X, p->n_points, ncols, prog, out, out_kind,
-                             (unsigned char*)p->scratch, bytes, false);
+    run.enqueue(X, out, out_kind);
   } catch (...) {
     ctx->capturing = false;
     cudaGraph_t g = nullptr;
@@ -1435,7 +1924,7 @@ extern "C" int tnfa_eval_plan_create(tnfa_ctx* ctx, const tnfa_net* net, const d
   for (int v = 0; v < net->topo.V; ++v)
     TNFA_CHECK(net->topo.site_dim[v] <= 256, TNFA_ERR_UNSUPPORTED, "site dimension above 256");
   int ncols = 0;
-  std::vector<DigitEntry> prog = make_digit_program(net->topo, n_dims, dims, &ncols);
+  std::vector<DigitRef> prog = make_digit_program(net->topo, n_dims, dims, &ncols);
   tnfa_eval_plan* p = new tnfa_eval_plan;
   p->ctx = ctx;
   ctx->refs += 1;
@@ -1637,32 +2126,18 @@ __global__ void k_vjp_seed(const double* __restrict__ dout, const T* __restrict_
 // Group the points of a chunk by the site value of vertex v (fills the job's
 // group fields; tp = tile rows of the kernel that will consume them).
 template <class T>
-void group_by_site(tnfa_ctx* ctx, VertexJob<T>& j, const uint8_t* Sv, int Pc, int ng, int tp,
-                   int* meta, int* perm) {
+void group_by_site(tnfa_ctx* ctx, VertexJob<T>& j, const int* key, int Pc, int ng, int tp, int* meta,
+                   int* perm) {
   j.ngroups = ng;
   j.grp_off = meta;
   j.grp_cnt = meta + ng;
   j.tile_start = meta + 2 * ng;
-  if (ng == 1) {
-    k_group_identity<<<1, 1, 0, ctx->stream>>>(meta, Pc, tp);
-    TNFA_LAUNCH_CHECK();
-    j.perm = nullptr;
-    return;
-  }
-  TNFA_CHECK(ng <= 256, TNFA_ERR_UNSUPPORTED, "site dimension above 256 per vertex");
-  TNFA_CUDA(cudaMemsetAsync(meta + ng, 0, ng * sizeof(int), ctx->stream));
-  KernelScope ks(ctx, "group", 0.0, (double)Pc * 6.0);
-  k_group_count<<<grid_for(Pc, 256, 4 * 152), 256, 0, ctx->stream>>>(Sv, Pc, ng, meta + ng);
-  k_group_scan<<<1, 1, 0, ctx->stream>>>(meta, ng, tp);
-  const unsigned gs = (unsigned)((Pc + 256 * SCATTER_ITEMS - 1) / (256 * SCATTER_ITEMS));
-  k_group_scatter<<<gs, 256, 0, ctx->stream>>>(Sv, Pc, ng, meta + 3 * ng + 1, perm);
-  TNFA_LAUNCH_CHECK();
-  j.perm = perm;
+  j.perm = launch_group(ctx, ng > 1 ? key : nullptr, Pc, ng, tp, meta, perm);
 }
 
 template <class T>
 void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double* X, int64_t P,
-              int ncols, const std::vector<DigitEntry>& prog, int xmem, const double* dout,
+              int ncols, const std::vector<DigitRef>& prog, int xmem, const double* dout,
               int dout_mem, T* dT) {
   const Topo& Tp = net->topo;
   const int V = Tp.V;
@@ -1670,7 +2145,7 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
   const int nroots = (int)plan.roots.size();
   std::vector<int> root_index(V, -1);
   for (int r = 0; r < nroots; ++r) root_index[plan.roots[r]] = r;
-  size_t per_point = V + 4 + (xmem == TNFA_MEM_HOST ? ncols * 8 : 0) +
+  size_t per_point = V * 4 + 4 + (xmem == TNFA_MEM_HOST ? ncols * 8 : 0) +
                      (dout_mem == TNFA_MEM_HOST ? 8 : 0) + nroots * (sizeof(T) + 4);
   for (int v = 0; v < V; ++v) per_point += 2 * ((size_t)Tp.link[v] * sizeof(T) + 4);
   int64_t Pc_max = (int64_t)(ctx->eval_budget / per_point);
@@ -1678,11 +2153,10 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
   const int Pcap = (int)std::max<int64_t>(std::min<int64_t>(P, (Pc_max / 256) * 256), 1);
   int maxsd = 1;
   for (int v = 0; v < V; ++v) maxsd = std::max(maxsd, Tp.site_dim[v]);
-  DBuf dprog(ctx, prog.size() * sizeof(DigitEntry));
-  if (!prog.empty())
-    TNFA_CUDA(cudaMemcpyAsync(dprog.p, prog.data(), prog.size() * sizeof(DigitEntry),
-                              cudaMemcpyHostToDevice, ctx->stream));
-  DBuf dS(ctx, (size_t)V * Pcap), dperm(ctx, (size_t)Pcap * 4);
+  const std::vector<DigitRun> runs = make_fused_runs(Tp, prog);
+  DBuf dprog(ctx, std::max<size_t>(runs.size(), 1) * sizeof(DigitRun));
+  h2d(ctx, dprog.p, runs.data(), runs.size() * sizeof(DigitRun));
+  DBuf dS(ctx, (size_t)V * Pcap * 4), dperm(ctx, (size_t)Pcap * 4);
   DBuf dmeta(ctx, group_meta_ints(maxsd) * 4), derr(ctx, 4);
   TNFA_CUDA(cudaMemsetAsync(derr.p, 0, 4, ctx->stream));
   std::vector<DBuf> in(V), ine(V), E(V), Ee(V);
@@ -1704,11 +2178,10 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
     if (plan.fused_leaf[c]) {
       s.ptr = tensors + Tp.off[c];
       s.exps = nullptr;
-      s.S = dS.as<uint8_t>() + (int64_t)c * Pcap;
+      s.idx.codes = dS.as<int>() + (int64_t)c * Pcap;
     } else {
       s.ptr = in[c].as<T>();
       s.exps = ine[c].as<int>();
-      s.S = nullptr;
     }
     return s;
   };
@@ -1724,14 +2197,8 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
       TNFA_CUDA(cudaMemcpyAsync(ddout.p, dc, (size_t)Pc * 8, cudaMemcpyHostToDevice, ctx->stream));
       dc = ddout.as<double>();
     }
-    TNFA_CUDA(cudaMemsetAsync(dS.p, 0, (size_t)V * Pcap, ctx->stream));
-    if (!prog.empty()) {
-      KernelScope ks(ctx, "digitize", 0.0, (double)Pc * (ncols * 8.0 + V));
-      k_digitize<<<grid_for(Pc, 256, 8 * 152 * 8), 256, 0, ctx->stream>>>(
-          Xc, ncols, Pc, dprog.as<DigitEntry>(), (int)prog.size(), dS.as<uint8_t>(), (int64_t)Pcap,
-          derr.as<int>());
-      TNFA_LAUNCH_CHECK();
-    }
+    launch_digitize(ctx, Xc, ncols, Pc, dprog.as<DigitRun>(), (int)runs.size(), V, dS.as<int>(), Pcap,
+                    derr.as<int>());
     // forward: inside messages of every non-leaf vertex
     for (int v : plan.order) {
       VertexJob<T> j{};
@@ -1756,7 +2223,7 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
         j.out = in[v].as<T>();
         j.out_exp = ine[v].as<int>();
       }
-      group_by_site(ctx, j, dS.as<uint8_t>() + (int64_t)v * Pcap, Pc, j.site_dim,
+      group_by_site(ctx, j, dS.as<int>() + (int64_t)v * Pcap, Pc, j.site_dim,
                     contract_tile_rows(j.chi_a, sumdim, sizeof(T)), meta, dperm.as<int>());
       launch_contract<T>(ctx, j, Pc);
     }
@@ -1796,7 +2263,6 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
         ChildSrc<T> e{};
         e.ptr = E[v].as<T>();
         e.exps = Ee[v].as<int>();
-        e.S = nullptr;
         e.dim = Tp.link[v];
         j.ch[j.nchild++] = e;
         int64_t K = e.dim;
@@ -1815,7 +2281,7 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
         j.Pc = Pc;
         j.out = E[c].as<T>();
         j.out_exp = Ee[c].as<int>();
-        group_by_site(ctx, j, dS.as<uint8_t>() + (int64_t)v * Pcap, Pc, j.site_dim,
+        group_by_site(ctx, j, dS.as<int>() + (int64_t)v * Pcap, Pc, j.site_dim,
                       contract_tile_rows(j.chi_a, sumdim, sizeof(T)), meta, dperm.as<int>());
         launch_contract<T>(ctx, j, Pc);
       }
@@ -1826,7 +2292,6 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
       ChildSrc<T> e{};
       e.ptr = E[v].as<T>();
       e.exps = Ee[v].as<int>();
-      e.S = nullptr;
       e.dim = Tp.link[v];
       j.ch[j.nchild++] = e;
       int64_t K = e.dim;
@@ -1843,7 +2308,7 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
       j.site_dim = Tp.site_dim[v];
       j.Pc = Pc;
       constexpr int TP = 64;
-      group_by_site(ctx, j, dS.as<uint8_t>() + (int64_t)v * Pcap, Pc, j.site_dim, TP, meta,
+      group_by_site(ctx, j, dS.as<int>() + (int64_t)v * Pcap, Pc, j.site_dim, TP, meta,
                     dperm.as<int>());
       const size_t sm = (size_t)sumdim * TP * sizeof(T) + TP * sizeof(T) + 2 * TP * sizeof(int);
       TNFA_CHECK(sm <= 200 * 1024, TNFA_ERR_UNSUPPORTED, "bonds too large for the gradient kernel");
@@ -1892,7 +2357,7 @@ extern "C" int tnfa_evaluate_vjp(tnfa_ctx* ctx, const tnfa_net* net, const doubl
   for (int v = 0; v < net->topo.V; ++v)
     TNFA_CHECK(net->topo.site_dim[v] <= 256, TNFA_ERR_UNSUPPORTED, "site dimension above 256");
   int ncols = 0;
-  std::vector<DigitEntry> prog = make_digit_program(net->topo, n_dims, dims, &ncols);
+  std::vector<DigitRef> prog = make_digit_program(net->topo, n_dims, dims, &ncols);
   const size_t es = dtype_size(net->dtype);
   const size_t bytes = (size_t)net->topo.n_elem * es;
   DBuf acc;

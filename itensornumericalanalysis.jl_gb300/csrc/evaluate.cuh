@@ -9,18 +9,28 @@ namespace tnfa {
 
 constexpr int EVAL_MAXC = 8;  // children per vertex handled by one contraction
 
-// Where a child's message row for point p comes from: a message buffer
-// (row p of a Pc x dim matrix plus a base-2 exponent per row) or, for a leaf
-// child fused into its parent, row S[p] of the leaf tensor itself.
+// Row of a message (or leaf tensor) that item p reads: a code per item, a
+// digit group of the item's own number ((p / div) % mod), or p itself.
+struct RowIdx {
+  const int* codes = nullptr;
+  int div = 0, mod = 0;
+  __device__ __forceinline__ int operator()(int p) const {
+    if (codes) return codes[p];
+    return div ? (p / div) % mod : p;
+  }
+};
+
+// A child's message: rows of dim entries with a base-2 exponent each, and the
+// row that item p reads (its own, or a table's by the digit code).
 template <class T>
 struct ChildSrc {
   const T* ptr;
-  const int* exps;     // null for a fused leaf
-  const uint8_t* S;    // site index of the leaf per point; null for a message
+  const int* exps;  // per row; null for a leaf tensor
+  RowIdx idx;
   int dim;
 };
 
-// One vertex contraction over all points of a chunk:
+// One vertex contraction over all points of a chunk (or rows of a table):
 //   out[p, a] = sum_k A[p, k] * T_v[s_p][a][k],  A[p, k] = prod_c m_c[p, k_c]
 // (k = mixed radix over the children, first child most significant), with
 // the points grouped by their site value s_p (grp_*) so that a tile of rows
@@ -37,6 +47,7 @@ struct VertexJob {
   const int* grp_off;  // [ngroups]
   const int* grp_cnt;  // [ngroups]
   const int* tile_start;  // [ngroups + 1]
+  const int* gexp;     // exponent of the group's tensor slice; null = zero
   int ngroups;
   int Pc;
 };

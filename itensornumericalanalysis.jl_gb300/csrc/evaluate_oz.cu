@@ -71,10 +71,10 @@ constexpr int OZ_SMEM = OZ_SLOTS * OZ_SLOT_BYTES + OZ_STAGES * OZ_B_BYTES + 1024
 struct OzParams {
   const double* m1_ptr;  // first child: message rows or (fused leaf) tensor rows
   const int* m1_exp;
-  const uint8_t* m1_S;
+  RowIdx m1_idx;
   const double* m2_ptr;  // second child
   const int* m2_exp;
-  const uint8_t* m2_S;
+  RowIdx m2_idx;
   int chi_a, chi1, site_dim;
   const int* bexp;  // [site][chi_a] base-2 exponents of the tensor slabs
   double* out;      // Pc x chi_a
@@ -241,10 +241,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const int h = warp >> 2;
     const bool valid = m < nrows;
     const int p = valid ? (P.perm ? P.perm[row0 + m] : row0 + m) : 0;
-    const double* m1row =
-        P.m1_S ? P.m1_ptr + (int64_t)P.m1_S[p] * P.chi1 : P.m1_ptr + (int64_t)p * P.chi1;
-    const double* m2row =
-        P.m2_S ? P.m2_ptr + (int64_t)P.m2_S[p] * CHI2 : P.m2_ptr + (int64_t)p * CHI2;
+    const int i1 = valid ? P.m1_idx(p) : 0, i2 = valid ? P.m2_idx(p) : 0;
+    const double* m1row = P.m1_ptr + (int64_t)i1 * P.chi1;
+    const double* m2row = P.m2_ptr + (int64_t)i2 * CHI2;
     // Row exponents: 2^E bounds |row| strictly.  The two threads of a row
     // scan one half each and meet in shared memory (the start of the A
     // region, free until the planes are written).
@@ -268,7 +267,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     if (E1 == INT_MIN) E1 = 0;
     if (E2 == INT_MIN) E2 = 0;
     asm volatile("bar.sync 1, 256;" ::: "memory");  // every row read before A overwrites
-    const int e_in = valid ? ((P.m1_exp ? P.m1_exp[p] : 0) + (P.m2_exp ? P.m2_exp[p] : 0)) : 0;
+    const int e_in = (P.m1_exp ? P.m1_exp[i1] : 0) + (P.m2_exp ? P.m2_exp[i2] : 0);
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     bool ok = true;
     uint32_t u = 0;  // accumulator unit, in the MMA issuer's order
@@ -645,10 +644,10 @@ void oz_contract_vertex(tnfa_ctx* ctx, const tnfa_net* net, int v, const VertexJ
   OzParams p{};
   p.m1_ptr = j.ch[0].ptr;
   p.m1_exp = j.ch[0].exps;
-  p.m1_S = j.ch[0].S;
+  p.m1_idx = j.ch[0].idx;
   p.m2_ptr = j.ch[1].ptr;
   p.m2_exp = j.ch[1].exps;
-  p.m2_S = j.ch[1].S;
+  p.m2_idx = j.ch[1].idx;
   p.chi_a = j.chi_a;
   p.chi1 = chi1;
   p.site_dim = j.site_dim;

@@ -42,10 +42,10 @@ constexpr int TC_ERR_TIMEOUT = ptx::ERR_TIMEOUT;
 struct TcParams {
   const float* m1_ptr;   // child 1 rows (message or leaf tensor); null: chi1 = 1
   const int* m1_exp;
-  const uint8_t* m1_S;
+  RowIdx m1_idx;
   const float* m2_ptr;   // child 2 rows
   const int* m2_exp;
-  const uint8_t* m2_S;
+  RowIdx m2_idx;
   int chi1, chi2, N, K;
   float* out;
   int* out_exp;
@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const bool valid = m < nrows;
     const int p = valid ? (P.perm ? P.perm[row0 + m] : row0 + m) : 0;
     float m2r[HALF];
-    const float* m2row = P.m2_S ? P.m2_ptr + (int64_t)P.m2_S[p] * CHI2
-                                : P.m2_ptr + (int64_t)p * CHI2;
+    const int i1 = valid && P.m1_ptr ? P.m1_idx(p) : 0, i2 = valid ? P.m2_idx(p) : 0;
+    const float* m2row = P.m2_ptr + (int64_t)i2 * CHI2;
 #pragma unroll
     for (int j = 0; j < HALF; ++j) {
       // columns [32h, 32h+32) of every 64-wide block of c
@@ -127,16 +127,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       m2r[j] = valid ? m2row[c] : 0.0f;
     }
     const float* m1row = nullptr;
-    if (P.m1_ptr)
-      m1row = P.m1_S ? P.m1_ptr + (int64_t)P.m1_S[p] * P.chi1 : P.m1_ptr + (int64_t)p * P.chi1;
+    if (P.m1_ptr) m1row = P.m1_ptr + (int64_t)i1 * P.chi1;
     const int nb = BILIN ? 1 : P.chi1;
-    const int e_in = valid ? ((P.m1_exp ? P.m1_exp[p] : 0) + (P.m2_exp ? P.m2_exp[p] : 0)) : 0;
+    const int e_in = (P.m1_exp ? P.m1_exp[i1] : 0) + (P.m2_exp ? P.m2_exp[i2] : 0);
     constexpr int CPB = CHI2 / TC_KC;  // chunks per value of b
     bool ok = true;
     // m1[p, b] is consumed once per b; it is loaded four at a time one group
     // ahead so the global-load latency hides behind the previous group.
     const bool use_m1 = !BILIN && m1row && valid;
-    const bool vec4 = use_m1 && (P.chi1 % 4 == 0);
+    const bool vec4 = use_m1 && (P.chi1 % 4 == 0) && ((uintptr_t)m1row & 15) == 0;
     float4 grp = make_float4(1.f, 1.f, 1.f, 1.f), nxt = grp;
     if (vec4) nxt = *reinterpret_cast<const float4*>(m1row);
     for (int bb = 0; bb < nb && ok; ++bb) {
@@ -378,8 +377,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int h = warp >> 2;
     const bool valid = m < nrows;
     const int p = valid ? (P.perm ? P.perm[row0 + m] : row0 + m) : 0;
-    const float* m2row =
-        P.m2_S ? P.m2_ptr + (int64_t)P.m2_S[p] * CHI2 : P.m2_ptr + (int64_t)p * CHI2;
+    const int i1 = valid ? P.m1_idx(p) : 0, i2 = valid ? P.m2_idx(p) : 0;
+    const float* m2row = P.m2_ptr + (int64_t)i2 * CHI2;
     // thread (m, h) writes columns [32h, 32h + 32) of every 64-wide chunk
 #pragma unroll
     for (int kc = 0; kc < KCH; ++kc) {
@@ -413,9 +412,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     fence_proxy_async();
     mbar_arrive(&a_ready);
 
-    const float* m1row =
-        P.m1_S ? P.m1_ptr + (int64_t)P.m1_S[p] * P.chi1 : P.m1_ptr + (int64_t)p * P.chi1;
-    const int e_in = valid ? ((P.m1_exp ? P.m1_exp[p] : 0) + (P.m2_exp ? P.m2_exp[p] : 0)) : 0;
+    const float* m1row = P.m1_ptr + (int64_t)i1 * P.chi1;
+    const int e_in = (P.m1_exp ? P.m1_exp[i1] : 0) + (P.m2_exp ? P.m2_exp[i2] : 0);
     float acc[ACC];
 #pragma unroll
     for (int i = 0; i < ACC; ++i) acc[i] = 0.f;
@@ -697,12 +695,12 @@ void tc_contract_vertex(tnfa_ctx* ctx, const tnfa_net* net, int v, const VertexJ
   const ChildSrc<float>& c2 = j.ch[j.nchild - 1];
   p.m2_ptr = c2.ptr;
   p.m2_exp = c2.exps;
-  p.m2_S = c2.S;
+  p.m2_idx = c2.idx;
   p.chi2 = c2.dim;
   if (j.nchild == 2) {
     p.m1_ptr = j.ch[0].ptr;
     p.m1_exp = j.ch[0].exps;
-    p.m1_S = j.ch[0].S;
+    p.m1_idx = j.ch[0].idx;
     p.chi1 = j.ch[0].dim;
   } else {
     p.chi1 = 1;
