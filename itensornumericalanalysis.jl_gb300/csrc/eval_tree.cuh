@@ -51,6 +51,7 @@ struct EvalTreeOptions {
   double table_rows = 1;        // a message with at most this many combinations is a table
   double table_elems = 1e18;    // bound on the elements of one absorbed tensor
   bool absorb = true;
+  bool balance = false;         // choose the centre by the costlier side, not the sum
   std::vector<char> tensor_ok;  // vertices the tensor-core kernel takes in the stored axis order
   double tensor_speed = 40.0;   // its rate over the CUDA cores' (measured: 46 for MIXED)
 };
@@ -107,7 +108,7 @@ class EvalTreeBuilder {
         if (c != v) all += D[c];
       U[v] = all + cost(p, v, nullptr);
       if (o_.rule == CentreRule::ROOT || (o_.rule == CentreRule::ROOT_EDGE && p != r)) continue;
-      const double c = D[v] + U[v] + o_.points * T_.link[v];
+      const double c = (o_.balance ? std::max(D[v], U[v]) : D[v] + U[v]) + o_.points * T_.link[v];
       if (c < best[r]) best[r] = c, a[r] = p, b[r] = v;
     }
     for (int v = 0; v < V; ++v)

@@ -277,205 +277,30 @@ __global__ void __launch_bounds__(256) k_contract_narrow(const VertexJob<T> j) {
   if (lane == 0) j.out_exp[p] = eacc[r] + (j.gexp ? j.gexp[g] : 0);
 }
 
-// --------------------------------------------- fused small-bond path ----
-// For networks whose bonds are all small (chi <= 16, or chi <= 32 on paths),
-// one thread walks its point through the whole tree: digits from the digit
-// program, then the vertices in post-order, each a chain of small
-// matrix-vector products against the network's tensors held in shared
-// memory, the messages in shared memory ([slot][entry][thread], conflict
-// free), each message rescaled by a power of two with the exponent carried.
-// One launch per chunk instead of about four per vertex, and no message
-// traffic through HBM.
-struct FusedStep {
-  int off;       // element offset of the vertex tensor in the shared copy
-  int vertex;
-  int chi_a;     // parent bond (1 at a root)
-  int nchild;    // 0, 1 or 2
-  int d1, d2;    // child bonds (1 when absent)
-  int in1, in2;  // message slots of the children
-  int out;       // message slot of this vertex; -1 at a root
-};
+// ------------------------------------------------- small-bond networks ----
+// TNFA_EVAL_FUSED=0 turns the one-launch kernels off (the walk, and digits
+// taken by the centre kernel).
+static bool fused_allowed() {
+  const char* env = getenv("TNFA_EVAL_FUSED");
+  return !(env && *env == '0');
+}
 constexpr int FUSED_MAXV = 128;
 
-template <class T, int CHI>
-__global__ void __launch_bounds__(128) k_eval_fused(
-    const double* __restrict__ X, int ncols, int Pc, const DigitRun* __restrict__ prog, int nprog,
-    const FusedStep* __restrict__ steps, int nsteps, const T* __restrict__ tensors, int n_elem,
-    int V, int nslots, size_t off_msg, size_t off_prog, size_t off_steps, void* out, int kind,
-    int64_t P, int64_t p0, int* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // the tensors in shared memory when they fit (off_msg > 0), else read in
-  // place (a few hundred KB at most: they stay in L1 / L2)
-  const T* ts = off_msg ? (const T*)smem_raw : tensors;
-  T* msg = (T*)(smem_raw + off_msg);
-  DigitRun* pg = (DigitRun*)(smem_raw + off_prog);
-  FusedStep* st = (FusedStep*)(smem_raw + off_steps);
-  if (off_msg)
-    for (int i = threadIdx.x; i < n_elem; i += blockDim.x) ((T*)smem_raw)[i] = tensors[i];
-  for (int i = threadIdx.x; i < nprog; i += blockDim.x) pg[i] = prog[i];
-  for (int i = threadIdx.x; i < nsteps; i += blockDim.x) st[i] = steps[i];
-  __syncthreads();
-  const int tpb = blockDim.x, tid = threadIdx.x;
-  auto M = [&](int slot, int k) -> T& { return msg[((size_t)slot * CHI + k) * tpb + tid]; };
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < Pc; p += gridDim.x * blockDim.x) {
-    int dg[FUSED_MAXV];
-    for (int v = 0; v < V; ++v) dg[v] = 0;
-    digit_codes(X + (int64_t)p * ncols, pg, nprog, dg, 1, 0, V, err);
-    T val = Sc<T>::one();
-    int ex_acc = 0;
-    for (int i = 0; i < nsteps; ++i) {
-      const FusedStep s = st[i];
-      const int K = s.d1 * s.d2;
-      const T* Tv = ts + s.off + (int64_t)dg[s.vertex] * s.chi_a * K;
-      // the last child's message in registers; the first child's (two
-      // children) read from its slot inside the loop, which the output slot
-      // never aliases (it is taken before the children's slots are freed)
-      const int dl = s.nchild == 2 ? s.d2 : s.d1;
-      const int il = s.nchild == 2 ? s.in2 : s.in1;
-      T ml[CHI];
-#pragma unroll
-      for (int c = 0; c < CHI; ++c) ml[c] = (s.nchild > 0 && c < dl) ? M(il, c) : Sc<T>::zero();
-      decltype(Sc<T>::absmax(Sc<T>::zero())) mx = 0;
-      T rv = Sc<T>::zero();
-      for (int a = 0; a < s.chi_a; ++a) {
-        const T* Ta = Tv + (int64_t)a * K;
-        T acc = Sc<T>::zero();
-        if (s.nchild == 0) {
-          acc = Ta[0];
-        } else if (s.nchild == 1) {
-#pragma unroll
-          for (int c = 0; c < CHI; ++c)
-            if (c < dl) acc = Sc<T>::fma(Ta[c], ml[c], acc);
-        } else {
-          for (int b = 0; b < s.d1; ++b) {
-            const T* Tb = Ta + b * dl;
-            T in = Sc<T>::zero();
-#pragma unroll
-            for (int c = 0; c < CHI; ++c)
-              if (c < dl) in = Sc<T>::fma(Tb[c], ml[c], in);
-            acc = Sc<T>::fma(M(s.in1, b), in, acc);
-          }
-        }
-        if (s.out < 0) {
-          rv = acc;  // a root: its parent bond is 1
-        } else {
-          M(s.out, a) = acc;
-          mx = max(mx, Sc<T>::absmax(acc));
-        }
-      }
-      if (s.out < 0) {
-        val = val * rv;
-        continue;
-      }
-      const int ex = mx > 0 ? Frexp<decltype(mx)>::e(mx) : 0;
-      ex_acc += ex;
-      if (ex != 0)
-        for (int a = 0; a < s.chi_a; ++a) M(s.out, a) = Sc<T>::scale2(M(s.out, a), -ex);
-    }
-    write_out<T>(out, kind, p0 + p, P, val, ex_acc);
-  }
-}
-
-struct FusedPlan {
-  bool ok = false;
-  int chi = 0;  // CHI of the kernel
-  int nslots = 0, tpb = 0;
-  std::vector<FusedStep> steps;
-  size_t off_msg = 0, off_prog = 0, off_steps = 0, smem = 0;
-};
-
-// Whether the fused kernel takes this network, and its schedule (post-order,
-// message slots recycled as children are consumed) and shared-memory layout.
-static FusedPlan make_fused_plan(const Topo& T, size_t tsize, size_t nprog, int64_t npoints) {
-  FusedPlan F;
-  const char* env = getenv("TNFA_EVAL_FUSED");
-  if (env && *env == '0') return F;
-  if (T.V > FUSED_MAXV) return F;
+// Networks whose points a thread can walk: every bond <= 16 (<= 32 on paths),
+// at most two children per vertex, 64 KB of messages per 32 points.  A thread
+// per point: above bond 8 a few thousand points leave the GPU mostly idle,
+// where the per-vertex kernels spread a point over a warp.
+static bool small_bonds(const Topo& T, size_t tsize, int64_t npoints) {
+  if (!fused_allowed() || T.V > FUSED_MAXV) return false;
   int chimax = 1, maxch = 0;
   for (int v = 0; v < T.V; ++v) {
     chimax = std::max(chimax, T.link[v]);
     maxch = std::max(maxch, (int)T.children[v].size());
-    if (T.site_dim[v] > 256) return F;
+    if (T.site_dim[v] > 256) return false;
   }
-  if (maxch > 2 || chimax > 32 || (chimax > 16 && maxch > 1)) return F;
-  // a thread per point: above chi 8 a few thousand points leave the GPU
-  // mostly idle, where the per-vertex kernels spread a point over a warp
-  if (chimax > 8 && npoints < 32768) return F;
-  if (T.n_elem * (int64_t)tsize > 4 * 1024 * 1024) return F;
-  F.chi = chimax <= 2 ? 2 : chimax <= 4 ? 4 : chimax <= 8 ? 8 : chimax <= 16 ? 16 : 32;
-  std::vector<int> slot(T.V, -1), free_slots;
-  int n = 0;
-  for (int r : T.roots()) {
-    std::vector<std::pair<int, int>> stack{{r, 0}};
-    while (!stack.empty()) {
-      auto& [v, i] = stack.back();
-      if (i < (int)T.children[v].size()) {
-        const int c = T.children[v][i++];
-        stack.push_back({c, 0});
-        continue;
-      }
-      FusedStep s{};
-      s.off = (int)T.off[v];
-      s.vertex = v;
-      s.chi_a = T.link[v];
-      s.nchild = (int)T.children[v].size();
-      s.d1 = s.nchild >= 1 ? T.link[T.children[v][0]] : 1;
-      s.d2 = s.nchild >= 2 ? T.link[T.children[v][1]] : 1;
-      s.in1 = s.nchild >= 1 ? slot[T.children[v][0]] : 0;
-      s.in2 = s.nchild >= 2 ? slot[T.children[v][1]] : 0;
-      // the output slot is taken before the children's are released, so it
-      // never aliases a message the step still reads
-      if (T.parent[v] >= 0) {
-        if (free_slots.empty()) free_slots.push_back(n++);
-        s.out = slot[v] = free_slots.back();
-        free_slots.pop_back();
-      } else {
-        s.out = -1;
-      }
-      for (int c : T.children[v]) free_slots.push_back(slot[c]);
-      F.steps.push_back(s);
-      stack.pop_back();
-    }
-  }
-  F.nslots = std::max(n, 1);
-  auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
-  // threads per block: as many as keep the messages within 64 KB, 32..128
-  const size_t per_thread = (size_t)F.nslots * F.chi * tsize;
-  F.tpb = (int)std::min<size_t>(128, std::max<size_t>(32, (64 * 1024 / per_thread) / 32 * 32));
-  if ((size_t)F.tpb * per_thread > 64 * 1024) return F;
-  const bool ts_smem = (size_t)T.n_elem * tsize <= 96 * 1024;
-  F.off_msg = ts_smem ? al((size_t)T.n_elem * tsize) : 0;
-  F.off_prog = al(F.off_msg + (size_t)F.tpb * per_thread);
-  F.off_steps = al(F.off_prog + nprog * sizeof(DigitRun));
-  F.smem = F.off_steps + F.steps.size() * sizeof(FusedStep);
-  F.ok = F.smem <= 200 * 1024;
-  return F;
-}
-
-template <class T>
-static void launch_fused(tnfa_ctx* ctx, const FusedPlan& F, const FusedStep* dsteps, const T* tensors,
-                         const Topo& Tp, const double* Xc, int ncols, int Pc,
-                         const DigitRun* dprog, int nprog, void* o, int kind, int64_t Pout,
-                         int64_t pofs, int* derr) {
-  const int tpb = F.tpb;
-  const unsigned grid = grid_for(Pc, tpb, ctx->sm_count * (2048 / tpb));
-  double fl = 0;
-  for (const auto& s : F.steps) fl += 2.0 * s.chi_a * s.d1 * s.d2;
-  KernelScope ks(ctx, "eval_fused", fl * Pc, (double)Pc * (ncols * 8.0 + 8.0));
-  auto go = [&](auto kern) {
-    TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F.smem));
-    kern<<<grid, tpb, F.smem, ctx->stream>>>(Xc, ncols, Pc, dprog, nprog, dsteps, (int)F.steps.size(),
-                                             tensors, (int)Tp.n_elem, Tp.V, F.nslots, F.off_msg,
-                                             F.off_prog, F.off_steps, o, kind, Pout, pofs, derr);
-  };
-  switch (F.chi) {
-    case 2: go(k_eval_fused<T, 2>); break;
-    case 4: go(k_eval_fused<T, 4>); break;
-    case 8: go(k_eval_fused<T, 8>); break;
-    case 16: go(k_eval_fused<T, 16>); break;
-    default: go(k_eval_fused<T, 32>); break;
-  }
-  TNFA_LAUNCH_CHECK();
+  if (maxch > 2 || chimax > 32 || (chimax > 16 && maxch > 1)) return false;
+  if (chimax > 8 && npoints < 32768) return false;
+  return T.n_elem * (int64_t)tsize <= 4 * 1024 * 1024;
 }
 
 // -------------------------------------------------------------- driver ----
@@ -719,8 +544,8 @@ static std::vector<DigitRun> make_runs(const std::vector<DigitRef>& prog, const 
   return runs;
 }
 
-// The fused small-bond kernel keeps every vertex's site value by itself.
-static std::vector<DigitRun> make_fused_runs(const Topo& T, const std::vector<DigitRef>& prog) {
+// Every vertex's site value as a code of its own.
+static std::vector<DigitRun> make_site_runs(const Topo& T, const std::vector<DigitRef>& prog) {
   std::vector<int> slot(T.V), mult(T.V, 1);
   for (int v = 0; v < T.V; ++v) slot[v] = v;
   return make_runs(prog, slot, mult);
@@ -801,11 +626,28 @@ static int row_tile(tnfa_ctx* ctx, const std::vector<RowJob<T>>& jobs) {
   return RowTiles<T>::n - 1;
 }
 
+// Jobs with their first blocks (first has one entry more): in the launch's
+// parameters when they fit, else from the device tables.
 template <class T>
-static void launch_rows(tnfa_ctx* ctx, int tile, int64_t blocks, const RowJob<T>& one,
-                        const RowJob<T>* jobs, const int* first, int njobs) {
+static RowPack<T> pack_rows(const std::vector<RowJob<T>>& jobs, const std::vector<int>& first, const RowJob<T>* djobs,
+                            const int* dfirst) {
+  RowPack<T> p{};
+  p.total = (int)jobs.size();
+  if (jobs.size() <= (size_t)ROW_PACK) {
+    p.n = p.total;
+    std::copy(jobs.begin(), jobs.end(), p.j);
+    std::copy(first.begin(), first.end(), p.f);
+  } else {
+    p.jobs = djobs;
+    p.first = dfirst;
+  }
+  return p;
+}
+
+template <class T>
+static void launch_rows(tnfa_ctx* ctx, int tile, int64_t blocks, const RowPack<T>& pack) {
   TNFA_CHECK(blocks < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
-  auto go = [&](auto kern) { kern<<<(unsigned)blocks, 256, 0, ctx->stream>>>(one, jobs, first, njobs); };
+  auto go = [&](auto kern) { kern<<<(unsigned)blocks, 256, 0, ctx->stream>>>(pack); };
   if constexpr (std::is_same<T, float>::value) {
     if (tile == 0) go(k_rows_gemm<T, 8, 4>);
     else if (tile == 1) go(k_rows_gemm<T, 4, 2>);
@@ -820,6 +662,31 @@ static void launch_rows(tnfa_ctx* ctx, int tile, int64_t blocks, const RowJob<T>
   }
   TNFA_LAUNCH_CHECK();
 }
+
+// Products of the thread-per-row kernel: fewer columns than a tile's 32 lanes.
+template <class T>
+static bool small_rows(const RowJob<T>& j) {
+  return j.rpg > 0 && j.K <= 32 && j.N < 32 && (int64_t)j.rows * ((j.N + 3) / 4) < (int64_t(1) << 31);
+}
+template <class T>
+static int64_t small_blocks(const RowJob<T>& j) {
+  return ((int64_t)j.rows * ((j.N + 3) / 4) + 127) / 128;
+}
+template <class T>
+static void launch_small_rows(tnfa_ctx* ctx, int64_t blocks, int kmax, const RowPack<T>& pack) {
+  auto go = [&](auto kern) { kern<<<(unsigned)blocks, 128, 0, ctx->stream>>>(pack); };
+  if (kmax <= 4) go(k_rows_small<T, 4>);
+  else if (kmax <= 8) go(k_rows_small<T, 8>);
+  else if (kmax <= 16) go(k_rows_small<T, 16>);
+  else go(k_rows_small<T, 32>);
+  TNFA_LAUNCH_CHECK();
+}
+
+// Multiply-adds per second of the walk, for choosing between it and tables.
+template <class T> struct WalkRate;
+template <> struct WalkRate<float> { static constexpr double v = 4e12; };
+template <> struct WalkRate<double> { static constexpr double v = 3e11; };
+template <> struct WalkRate<cplx> { static constexpr double v = 8e10; };
 
 // ------------------------------------------------------------- engine ----
 // Scratch handed out in 256-byte pieces from one block (or counted, base null).
@@ -868,13 +735,27 @@ class EvalEngine {
     // Tables take at most half the scratch: the row bound shrinks until they
     // fit.  Every digit code stays within 31 bits.
     double rows = std::min((double)P, 134217728.0);
+    small_ = !use_tc && !use_oz && small_bonds(topo_, sizeof(T), P);
+    if (small_) {
+      // Points that a thread walks cost one launch; a level of tables costs
+      // another (about 3 us).  Up to about 20 us of walking there are no tables;
+      // beyond, a table of half as many rows as points or less pays.
+      double w = 0;
+      for (int v = 0; v < V; ++v) {
+        double x = topo_.link[v];
+        for (int c : topo_.children[v]) x *= topo_.link[c];
+        w += x;
+      }
+      o.balance = true;
+      rows = w * P <= 20e-6 * WalkRate<T>::v ? 0 : std::floor(rows / 2);
+    }
     for (;;) {
       o.table_rows = rows;
       o.table_elems = std::min(1073741824.0, (double)(budget / 2) / sizeof(T));
       tree_ = EvalTreeBuilder(topo_, o).build();
-      if (table_bytes() <= budget / 2 || o.rule == CentreRule::ROOT && rows < 1) break;
+      if (table_bytes() <= budget / 2 || rows < 1) break;
       rows = std::floor(rows / 4);
-      if (rows < 1) {  // the stored order, nothing but points
+      if (rows < 1 && !small_) {  // the stored order, nothing but points
         o.rule = CentreRule::ROOT;
         o.absorb = false;
       }
@@ -906,10 +787,9 @@ class EvalEngine {
     fill_blob();
   }
   int* err_flag() const { return err_; }
-  // The job tables and the cleared error flag go to the scratch (stream order).
+  // The job tables go to the scratch (stream order).
   void upload() {
     h2d(ctx_, blob_, host_.data(), host_.size());
-    clear_error();
   }
   void clear_error() { TNFA_CUDA(cudaMemsetAsync(err_, 0, 4, ctx_->stream)); }
 
@@ -922,8 +802,35 @@ class EvalEngine {
       k_move<T><<<dim3(grid_for(n, 256, 1024), (unsigned)moves_.size()), 256, 0, ctx_->stream>>>(dmoves_);
       TNFA_LAUNCH_CHECK();
     }
+    if (!hgroups_.empty()) {
+      KernelScope ks(ctx_, FamilyName<T>::v, 0.0, 0.0);
+      const size_t sm = head_elems_ * sizeof(T) + head_exps_ * 4 + head_jobs_ * sizeof(HeadJob);
+      auto go = [&](auto kern) {
+        if (sm > 48 * 1024)
+          TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        // exponents of a side within +-range: its entries stay far from the type's limits
+        kern<<<(unsigned)hgroups_.size(), 256, sm, ctx_->stream>>>(dhblocks_, dhcopies_, dhjobs_, head_elems_,
+                                                                    head_exps_, head_jobs_, plain_,
+                                                                    sizeof(T) == 4 ? 40 : 400);
+      };
+      if (head_k_ <= 4) go(k_head<T, 4>);
+      else if (head_k_ <= 8) go(k_head<T, 8>);
+      else if (head_k_ <= 16) go(k_head<T, 16>);
+      else go(k_head<T, 32>);
+      TNFA_LAUNCH_CHECK();
+    }
     for (size_t l = 0; l < levels_.size(); ++l) {
       Level& L = levels_[l];
+      if (!L.small.empty()) {
+        double fl = 0;
+        int kmax = 1;
+        for (const auto& j : L.small) {
+          fl += 2.0 * (double)j.rows * j.N * j.K;
+          kmax = std::max(kmax, j.K);
+        }
+        KernelScope ks(ctx_, FamilyName<T>::v, fl, 0.0);
+        launch_small_rows<T>(ctx_, L.sfirst.back(), kmax, pack_rows(L.small, L.sfirst, L.dsmall, L.dsfirst));
+      }
       if (!L.rows.empty()) {
         double fl = 0;
         std::string key = std::string("simt:") + FamilyName<T>::v + ":rows";
@@ -936,7 +843,7 @@ class EvalEngine {
         auto go = [&](int i) {
           const int t = i == 0 ? rule : i <= rule ? i - 1 : i;
           KernelScope ks(ctx_, FamilyName<T>::v, fl, 0.0);
-          launch_rows<T>(ctx_, t, L.first[t].back(), RowJob<T>{}, L.drows, L.dfirst[t], (int)L.rows.size());
+          launch_rows<T>(ctx_, t, L.first[t].back(), pack_rows(L.rows, L.first[t], L.drows, L.dfirst[t]));
         };
         if (tuned) tune(ctx_, key, RowTiles<T>::n, fl, go);
         else go(0);
@@ -953,6 +860,10 @@ class EvalEngine {
 
   // Points [p0, p0 + n) of the call, X the chunk's coordinates.
   void points(const double* X, int n, void* out, int kind, int64_t Pout, int64_t pofs) {
+    if (walk_) {
+      walk(X, n, out, kind, Pout, pofs);
+      return;
+    }
     if (ncodes_ > 0)
       launch_digitize(ctx_, X, ncols_, n, druns_, (int)runs_.size(), ncodes_, codes_, Pc_, err_);
     for (int v : tree_.order)
@@ -965,6 +876,11 @@ class EvalEngine {
     std::vector<RowJob<T>> rows;
     std::vector<int> verts;  // table vertices of the multi-child kernels
     RowJob<T>* drows = nullptr;
+    std::vector<RowJob<T>> small;  // of the thread-per-row kernel
+    RowJob<T>* dsmall = nullptr;
+    std::vector<int> sfirst;
+    int* dsfirst = nullptr;
+    int njobs = 0;
     std::vector<int> first[3];
     int* dfirst[3] = {nullptr, nullptr, nullptr};
   };
@@ -975,7 +891,7 @@ class EvalEngine {
       const EvalVertex& e = tree_.v[v];
       if (e.tabled && !e.leaf) b += (double)e.N * (e.chi * sizeof(T) + 4);
       if (e.absorb) b += absorbed_rows(v) * (e.W / tree_chi(e.kids.back(), v) * sizeof(T) + 4);
-      if (e.moved) b += (double)topo_.size(v) * sizeof(T);
+      if (e.moved) b += (double)topo_.size(v) * sizeof(T);  // (more than a walk needs)
     }
     return (size_t)std::min(b, 1e18);
   }
@@ -1015,9 +931,16 @@ class EvalEngine {
     nslots_ = n;
     // all sides are tables: the centre kernel takes the digits itself, as long
     // as its shared memory holds them
-    fused_ = npp_ == 0 && n <= 16 && prog_.size() <= 256;
-    ncodes_ = fused_ ? 0 : n;
+    fused_ = fused_allowed() && npp_ == 0 && n <= 16 && prog_.size() <= 256;
     runs_ = make_runs(prog_, slot_, mult_);
+    walk_ = small_ && npp_ > 0 && plan_walk();
+    ncodes_ = fused_ || walk_ ? 0 : n;
+    if (walk_) {
+      nmsg_ = 0;
+      msg_chi_ = max_group_ = 1;
+      plan_levels();
+      return;
+    }
     // message slots (rows per point), reused once read; the output's is taken
     // before the kids' are given back, so it never shares memory with them
     std::vector<int> free_slots;
@@ -1037,29 +960,150 @@ class EvalEngine {
     for (int v = 0; v < V; ++v)
       if (!tree_.v[v].tabled)
         max_group_ = std::max<int64_t>(max_group_, tree_.v[v].absorb ? (int64_t)absorbed_rows(v) : topo_.site_dim[v]);
-    // levels
+    plan_levels();
+  }
+
+  // The walk's schedule: steps of side 0, then side 1, message slots, and the
+  // points per block that its shared memory allows.
+  bool plan_walk() {
+    const int V = topo_.V;
+    std::vector<int> side(V, 0);
+    for (const auto& c : tree_.comps)
+      if (c.b >= 0) side[c.b] = 1;
+    for (size_t i = tree_.order.size(); i-- > 0;) {
+      const int v = tree_.order[i];
+      for (int w : tree_.v[v].kids) side[w] = side[v];
+    }
+    wsteps_.clear();
+    wchi_ = 1;
+    nstage_ = 0;
+    nsteps0_ = 0;
+    int nmsg = 0;
+    for (int sd = 0; sd < 2; ++sd) {
+      std::vector<int> free_slots;
+      for (int v : tree_.order) {
+        const EvalVertex& e = tree_.v[v];
+        if (e.tabled || side[v] != sd) continue;
+        const int nk = (int)e.kids.size() - (e.absorb ? 1 : 0);
+        if (nk > 2) return false;
+        WalkVertex w;
+        w.v = v;
+        w.nk = nk;
+        w.d1 = nk == 2 ? tree_.v[e.kids[0]].chi : 1;
+        w.d2 = nk >= 1 ? tree_.v[e.kids[nk - 1]].chi : 1;
+        wchi_ = std::max({wchi_, e.chi, w.d1, w.d2});
+        if (free_slots.empty()) free_slots.push_back(nmsg++);
+        msg_[v] = free_slots.back();
+        free_slots.pop_back();
+        for (int i = 0; i < nk; ++i)
+          if (!tree_.v[e.kids[i]].tabled) free_slots.push_back(msg_[e.kids[i]]);
+        wsteps_.push_back(w);
+      }
+      if (sd == 0) nsteps0_ = (int)wsteps_.size();
+    }
+    // the sides of a vertex centre and tables at the centre
+    for (const auto& c : tree_.comps) wchi_ = std::max(wchi_, tree_.v[c.a].chi);
+    if (wchi_ > 32) return false;
+    wchi_ = wchi_ <= 2 ? 2 : wchi_ <= 4 ? 4 : wchi_ <= 8 ? 8 : wchi_ <= 16 ? 16 : 32;
+    wmsg_ = nmsg;
+    nstage_ = (size_t)topo_.n_elem * sizeof(T) <= 64 * 1024 ? (int)topo_.n_elem : 0;
+    // points per block: spread over the SMs first, then as many as the shared
+    // memory allows two blocks per SM with
+    wtp_ = P_ <= 32 * 2 * ctx_->sm_count ? 32 : P_ <= 64 * 4 * ctx_->sm_count ? 64 : 128;
+    while (wtp_ > 32 && walk_bytes() > 100 * 1024) wtp_ /= 2;
+    // lanes per point: up to four while the points alone do not give every
+    // scheduler (four per SM) a warp
+    wlanes_ = 1;
+    if (wchi_ <= 8)
+      while (wlanes_ < std::min(4, wchi_) && 2 * P_ * wlanes_ < 128 * 2 * (int64_t)ctx_->sm_count) wlanes_ *= 2;
+    if (wlanes_ > 1) wtp_ = 32 / wlanes_ * (wlanes_ == 4 ? 2 : 1);
+    return walk_bytes() <= 200 * 1024;
+  }
+  size_t walk_bytes() const {
+    return walk_smem<T>(wchi_, wtp_, nstage_, wmsg_, nslots_, (int)runs_.size(), (int)wsteps_.size(),
+                        (int)tree_.comps.size());
+  }
+
+  // Multiply-adds of one table product that a single block finishes in less
+  // than a launch takes (an SM does 2 FP64 or 128 FP32 a clock), and the shared
+  // memory of a block's tensors and tables.
+  static constexpr double kHeadWork = sizeof(T) == 4 ? 65536 : sizeof(T) == 8 ? 6144 : 1536;
+  static constexpr int kHeadK = 32;
+  static constexpr int64_t kHeadBytes = 96 * 1024;
+  int table_pitch(int chi) const { return chi | 1; }  // odd: rows start in different banks
+
+  void plan_levels() {
+    const int V = topo_.V;
     lvl_.assign(V, 0);
     lvl_m_.assign(V, 0);
+    // head vertices: every product of the subtree is small
+    head_.assign(V, 0);
+    plain_of_.assign(V, -1);
+    std::vector<int> reader(V, -1);
+    std::vector<int64_t> bytes(V, 0);
+    for (int v : tree_.order) {
+      const EvalVertex& e = tree_.v[v];
+      for (int w : e.kids) reader[w] = v;
+      bytes[v] = topo_.size(v) * (int64_t)sizeof(T);
+      if (e.leaf || !e.tabled || !row_form(v)) continue;
+      bool ok = e.kids.size() <= 2;
+      for (int w : e.kids) {
+        ok &= tree_.v[w].leaf || head_[w];
+        bytes[v] += bytes[w];
+      }
+      const double row_k = tree_.v[e.kids[0]].chi;
+      ok &= row_k <= kHeadK && (double)e.N * e.chi * row_k <= kHeadWork;
+      bytes[v] += e.N * (table_pitch(e.chi) * (int64_t)sizeof(T) + 4) + sizeof(HeadJob);
+      if (e.absorb) {
+        const int64_t r = (int64_t)absorbed_rows(v), k = tree_.v[e.kids.back()].chi;
+        ok &= k <= kHeadK && r * e.W <= kHeadWork;
+        bytes[v] += r * ((int64_t)(e.W / k) * (int64_t)sizeof(T) + 4) + sizeof(HeadJob);
+      }
+      head_[v] = ok && bytes[v] <= kHeadBytes;
+    }
+    hgroups_.clear();
+    nhead_copies_ = 0;
+    for (int v : tree_.order) {
+      if (!head_[v] || (reader[v] >= 0 && head_[reader[v]])) continue;
+      std::vector<int> g, todo{v};
+      while (!todo.empty()) {
+        const int x = todo.back();
+        todo.pop_back();
+        g.push_back(x);
+        for (int w : tree_.v[x].kids) {
+          if (head_[w]) todo.push_back(w);
+          else ++nhead_copies_;  // a leaf
+        }
+      }
+      nhead_copies_ += (int)g.size();
+      std::reverse(g.begin(), g.end());
+      plain_of_[v] = (int)hgroups_.size();
+      hgroups_.push_back(g);
+    }
     int top = 0;
+    nhead_jobs_ = 0;
     for (int v : tree_.order) {
       const EvalVertex& e = tree_.v[v];
       if (e.leaf) continue;
+      // (levels inside the head order its jobs; to the launches it is level 0)
+      auto lv = [&](int w) { return !head_[v] && head_[w] ? 0 : tree_.v[w].tabled ? lvl_[w] : 0; };
       int l = 0;
       for (size_t i = 0; i < e.kids.size(); ++i) {
         const bool ab = e.absorb && i + 1 == e.kids.size();
-        if (ab) lvl_m_[v] = lvl_[e.kids[i]] + 1;
-        l = std::max(l, ab ? lvl_m_[v] : tree_.v[e.kids[i]].tabled ? lvl_[e.kids[i]] : 0);
+        if (ab) lvl_m_[v] = lv(e.kids[i]) + 1;
+        l = std::max(l, ab ? lvl_m_[v] : lv(e.kids[i]));
       }
       if (e.tabled) lvl_[v] = l + 1;
-      top = std::max({top, lvl_m_[v], e.tabled ? lvl_[v] : 0});
+      if (head_[v]) nhead_jobs_ += e.absorb ? 2 : 1;
+      else top = std::max({top, lvl_m_[v], e.tabled ? lvl_[v] : 0});
     }
     levels_.assign(top + 1, Level{});
     for (int v : tree_.order) {
       const EvalVertex& e = tree_.v[v];
-      if (e.leaf) continue;
-      if (e.absorb) levels_[lvl_m_[v]].rows.emplace_back();
+      if (e.leaf || head_[v]) continue;
+      if (e.absorb) levels_[lvl_m_[v]].njobs += 1;
       if (!e.tabled) continue;
-      if (row_form(v)) levels_[lvl_[v]].rows.emplace_back();
+      if (row_form(v)) levels_[lvl_[v]].njobs += 1;
       else levels_[lvl_[v]].verts.push_back(v);
     }
   }
@@ -1095,13 +1139,20 @@ class EvalEngine {
     int nmove = 0, nnorm = 0;
     for (int v = 0; v < V; ++v) nmove += needs_move(v);
     for (const auto& cc : tree_.comps)
-      for (int v : {cc.a, cc.b}) nnorm += v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf;
+      for (int v : {cc.a, cc.b}) nnorm += !walk_ && v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf && !head_[v];
     dmoves_ = c.take<MoveJob>(nmove);
     dnorms_ = c.take<NormJob<T>>(nnorm);
     dcentre_ = c.take<CentreJob<T>>(tree_.comps.size());
+    dwalk_ = c.take<unsigned char>(
+        walk_ ? walk_blob<T>((int)runs_.size(), (int)wsteps_.size(), (int)tree_.comps.size()) : 0);
+    dhblocks_ = c.take<HeadBlock<T>>(hgroups_.size());
+    dhcopies_ = c.take<HeadCopy<T>>(nhead_copies_);
+    dhjobs_ = c.take<HeadJob>(nhead_jobs_);
     for (auto& L : levels_) {
-      L.drows = c.take<RowJob<T>>(L.rows.size());
-      for (int t = 0; t < RowTiles<T>::n; ++t) L.dfirst[t] = c.take<int>(L.rows.size() + 1);
+      L.drows = c.take<RowJob<T>>(L.njobs);
+      L.dsmall = c.take<RowJob<T>>(L.njobs);
+      L.dsfirst = c.take<int>(L.njobs + 1);
+      for (int t = 0; t < RowTiles<T>::n; ++t) L.dfirst[t] = c.take<int>(L.njobs + 1);
     }
     tmeta_.assign(V, nullptr);
     ttile_.assign(V, 0);
@@ -1129,15 +1180,28 @@ class EvalEngine {
         abse_[v] = c.take<int>(r);
       }
     }
+    plain_ = c.take<int>(hgroups_.size());
     // per point
     codes_ = c.take<int>((size_t)ncodes_ * pc);
-    perm_ = c.take<int>(npp_ ? pc : 0);
-    meta_ = c.take<int>(npp_ ? group_meta_ints((int)max_group_) : 0);
+    perm_ = c.take<int>(npp_ && !walk_ ? pc : 0);
+    meta_ = c.take<int>(npp_ && !walk_ ? group_meta_ints((int)max_group_) : 0);
     mval_ = c.take<T>((size_t)nmsg_ * pc * msg_chi_);
     mexp_ = c.take<int>((size_t)nmsg_ * pc);
     ld_ = pc;
   }
-  bool needs_move(int v) const { return tree_.v[v].moved; }
+  // (a walked vertex is read through strides; an absorbing one needs the kid last)
+  bool needs_move(int v) const {
+    const EvalVertex& e = tree_.v[v];
+    return e.moved && !head_[v] && (e.absorb || !(walk_ && !e.tabled));
+  }
+  // Strides of the stored tensor of v in the order its axes are read.
+  std::vector<int64_t> stored_strides(int v) const {
+    std::vector<int64_t> str(2 + topo_.children[v].size(), 1), out;
+    for (int i = (int)str.size() - 2; i >= 0; --i)
+      str[i] = str[i + 1] * (i == 0 ? topo_.link[v] : topo_.link[topo_.children[v][i - 1]]);
+    for (int a : tree_.v[v].axes) out.push_back(str[a]);
+    return out;
+  }
   int table_groups(int v) const {
     return tree_.v[v].absorb ? (int)absorbed_rows(v) : topo_.site_dim[v];
   }
@@ -1157,39 +1221,25 @@ class EvalEngine {
     put(druns_, runs_.data(), runs_.size() * sizeof(DigitRun));
     moves_.clear();
     norms_.clear();
-    for (int v = 0; v < topo_.V; ++v) {
-      const EvalVertex& e = tree_.v[v];
-      if (!needs_move(v)) continue;
-      std::vector<int> shape{topo_.site_dim[v], topo_.link[v]};
-      for (int c : topo_.children[v]) shape.push_back(topo_.link[c]);
-      TNFA_CHECK(shape.size() <= (size_t)MOVE_MAXD, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
-      std::vector<int64_t> str(shape.size(), 1);
-      for (int i = (int)shape.size() - 2; i >= 0; --i) str[i] = str[i + 1] * shape[i + 1];
-      MoveJob m{};
-      m.src = tensors_ + topo_.off[v];
-      m.dst = ten_[v];
-      m.n = topo_.size(v);
-      m.nd = (int)e.axes.size();
-      for (int i = 0; i < m.nd; ++i) {
-        m.dim[i] = shape[e.axes[i]];
-        m.str[i] = str[e.axes[i]];
-      }
-      moves_.push_back(m);
-    }
+    for (int v = 0; v < topo_.V; ++v)
+      if (needs_move(v)) moves_.push_back(move_job(v));
     put(dmoves_, moves_.data(), moves_.size() * sizeof(MoveJob));
+    if (walk_) fill_walk(put);
     std::vector<CentreJob<T>> cj;
     for (const auto& c : tree_.comps) {
+      if (walk_) break;
       CentreJob<T> j{};
       j.chi = tree_.v[c.a].chi;
       j.a = side(c.a);
       if (c.b >= 0) j.b = side(c.b);
       cj.push_back(j);
       for (int v : {c.a, c.b})
-        if (v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf)
+        if (!walk_ && v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf && !head_[v])
           norms_.push_back({tab_[v], tabe_[v], (int)tree_.v[v].N, tree_.v[v].chi});
     }
     put(dcentre_, cj.data(), cj.size() * sizeof(CentreJob<T>));
     put(dnorms_, norms_.data(), norms_.size() * sizeof(NormJob<T>));
+    fill_head(put);
     centre_chi_ = 1;
     centre_vec_ = true;
     constexpr int vec = 16 / sizeof(T);
@@ -1197,43 +1247,17 @@ class EvalEngine {
       centre_chi_ = std::max(centre_chi_, j.chi);
       centre_vec_ &= j.chi % vec == 0 && ((uintptr_t)j.a.ptr & 15) == 0 && ((uintptr_t)j.b.ptr & 15) == 0;
     }
-    for (auto& L : levels_) L.rows.clear();
+    for (auto& L : levels_) {
+      L.rows.clear();
+      L.small.clear();
+    }
+    auto add = [&](Level& L, const RowJob<T>& j) { (small_rows(j) ? L.small : L.rows).push_back(j); };
     for (int v : tree_.order) {
       const EvalVertex& e = tree_.v[v];
       if (e.leaf) continue;
-      if (e.absorb) {
-        const int w = e.kids.back();
-        const EvalVertex& k = tree_.v[w];
-        RowJob<T> j{};
-        j.A = tab_[w];
-        j.Aexp = tabe_[w];
-        j.aidx = table_row(1, k.N);
-        j.B = ten_[v];
-        j.out = abs_[v];
-        j.out_exp = abse_[v];
-        j.K = k.chi;
-        j.N = (int)(e.W / k.chi);
-        j.rpg = (int)k.N;
-        j.rows = topo_.site_dim[v] * j.rpg;
-        levels_[lvl_m_[v]].rows.push_back(j);
-      }
-      if (e.tabled && row_form(v)) {
-        const int w = e.kids[0];
-        const EvalVertex& k = tree_.v[w];
-        RowJob<T> j{};
-        j.A = tab_[w];
-        j.Aexp = tabe_[w];
-        j.aidx = table_row(1, k.N);
-        j.B = e.absorb ? abs_[v] : ten_[v];
-        j.gexp = e.absorb ? abse_[v] : nullptr;
-        j.out = tab_[v];
-        j.out_exp = tabe_[v];
-        j.K = k.chi;
-        j.N = e.chi;
-        j.rpg = (int)k.N;
-        j.rows = (int)e.N;
-        levels_[lvl_[v]].rows.push_back(j);
-      }
+      if (head_[v]) continue;
+      if (e.absorb) add(levels_[lvl_m_[v]], absorb_job(v));
+      if (e.tabled && row_form(v)) add(levels_[lvl_[v]], table_job(v));
       if (tmeta_[v]) {  // uniform groups of a multi-child table
         const int ng = table_groups(v), m = (int)(e.N / ng);
         std::vector<int> g(group_meta_ints(ng));
@@ -1249,6 +1273,15 @@ class EvalEngine {
     }
     for (auto& L : levels_) {
       put(L.drows, L.rows.data(), L.rows.size() * sizeof(RowJob<T>));
+      put(L.dsmall, L.small.data(), L.small.size() * sizeof(RowJob<T>));
+      L.sfirst.assign(1, 0);
+      int64_t sb = 0;
+      for (const auto& j : L.small) {
+        sb += small_blocks(j);
+        TNFA_CHECK(sb < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
+        L.sfirst.push_back((int)sb);
+      }
+      put(L.dsfirst, L.sfirst.data(), L.sfirst.size() * sizeof(int));
       for (int t = 0; t < RowTiles<T>::n; ++t) {
         L.first[t].assign(1, 0);
         int64_t b = 0;
@@ -1260,6 +1293,265 @@ class EvalEngine {
         put(L.dfirst[t], L.first[t].data(), L.first[t].size() * sizeof(int));
       }
     }
+  }
+
+  template <class Put>
+  void fill_walk(Put& put) {
+    std::vector<WalkStep<T>> st;
+    const bool reg = wchi_ <= 8;
+    for (size_t at_ = 0; at_ < wsteps_.size(); ++at_) {
+      const WalkVertex& w = wsteps_[at_];
+      const EvalVertex& e = tree_.v[w.v];
+      WalkStep<T> s{};
+      s.B = e.absorb ? abs_[w.v] : ten_[w.v];
+      s.gexp = e.absorb ? abse_[w.v] : nullptr;
+      s.key = key_slot_[w.v];
+      s.chi_a = e.chi;
+      s.d1 = w.d1;
+      s.d2 = w.d2;
+      s.c1 = s.c2 = -1;
+      for (int i = 0; i < w.nk; ++i) {
+        const int k = e.kids[i];
+        const bool last = i + 1 == w.nk, tab = tree_.v[k].tabled;
+        (last ? s.t2 : s.t1) = tab ? tab_[k] : nullptr;
+        (last ? s.e2 : s.e1) = tab ? tabe_[k] : nullptr;
+        (last ? s.c2 : s.c1) = tab ? row_slot_[k] : msg_[k];
+        // the previous step's message, still in registers
+        if (reg && last && !tab && at_ != (size_t)nsteps0_ && at_ > 0 && wsteps_[at_ - 1].v == k) s.c2 = -2;
+      }
+      if (e.absorb || !e.moved) {
+        s.s2 = 1;
+        s.s1 = w.d2;
+        s.sa = w.d1 * w.d2;
+        s.sg = e.chi * s.sa;
+      } else {  // the stored tensor's strides in the order read
+        const std::vector<int64_t> str = stored_strides(w.v);
+        // axes: sites, (a root's parent axis of dimension 1,) up, kids
+        const int at = (int)str.size() - w.nk;
+        s.sg = (int)str[0];
+        s.sa = e.up >= 0 ? (int)str[at - 1] : 0;
+        s.s1 = w.nk == 2 ? (int)str[at] : 0;
+        s.s2 = w.nk >= 1 ? (int)str[at + w.nk - 1] : 0;
+      }
+      s.out = msg_[w.v];
+      s.stage = nstage_ && !e.absorb && ten_[w.v] == tensors_ + topo_.off[w.v] ? (int)topo_.off[w.v] : -1;
+      st.push_back(s);
+    }
+    // a message that only the next step reads, from registers, is not stored
+    for (size_t i = 0; i + 1 < st.size(); ++i)
+      if (st[i + 1].c2 == -2) st[i].out = -1;
+    unsigned char* at = dwalk_;
+    put(at, runs_.data(), runs_.size() * sizeof(DigitRun));
+    at += runs_.size() * sizeof(DigitRun);
+    put(at, st.data(), st.size() * sizeof(WalkStep<T>));
+    at += st.size() * sizeof(WalkStep<T>);
+    std::vector<WalkSide<T>> sd;
+    for (const auto& c : tree_.comps)
+      for (int v : {c.a, c.b}) {
+        WalkSide<T> s{};
+        if (v >= 0) {
+          const EvalVertex& e = tree_.v[v];
+          s.chi = e.chi;
+          s.tab = e.tabled ? tab_[v] : nullptr;
+          s.exps = e.tabled ? tabe_[v] : nullptr;
+          s.at = e.tabled ? row_slot_[v] : msg_[v];
+        }
+        sd.push_back(s);
+      }
+    put(at, sd.data(), sd.size() * sizeof(WalkSide<T>));
+  }
+
+  void walk(const double* X, int n, void* out, int kind, int64_t Pout, int64_t pofs) {
+    WalkParams<T> W{};
+    W.X = X;
+    W.blob = dwalk_;
+    W.tensors = tensors_;
+    W.out = out;
+    W.err = err_;
+    W.P = Pout;
+    W.p0 = pofs;
+    W.ncols = ncols_;
+    W.Pc = n;
+    W.nruns = (int)runs_.size();
+    W.nslots = nslots_;
+    W.nsteps0 = nsteps0_;
+    W.nsteps = (int)wsteps_.size();
+    W.ncomp = (int)tree_.comps.size();
+    W.nmsg = wmsg_;
+    W.nstage = nstage_;
+    W.kind = kind;
+    const size_t sm = walk_bytes();
+    double fl = 0;
+    for (const auto& w : wsteps_) fl += 2.0 * tree_.v[w.v].chi * w.d1 * w.d2;
+    KernelScope ks(ctx_, "eval_fused", fl * n, (double)n * (ncols_ * 8.0 + 8.0));
+    const int per_sm = std::max(1, std::min((int)(220 * 1024 / std::max<size_t>(sm, 1)), 1024 / (wtp_ * wlanes_)));
+    const unsigned grid = grid_for(n, wtp_, ctx_->sm_count * per_sm);
+    auto go = [&](auto kern) {
+      if (sm > 48 * 1024)
+        TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      kern<<<grid, 2 * wtp_ * wlanes_, sm, ctx_->stream>>>(W);
+    };
+    if (wchi_ == 2) wlanes_ == 1 ? go(k_walk<T, 2, 1>) : go(k_walk<T, 2, 2>);
+    else if (wchi_ == 4) wlanes_ == 1 ? go(k_walk<T, 4, 1>) : wlanes_ == 2 ? go(k_walk<T, 4, 2>) : go(k_walk<T, 4, 4>);
+    else if (wchi_ == 8) wlanes_ == 1 ? go(k_walk<T, 8, 1>) : wlanes_ == 2 ? go(k_walk<T, 8, 2>) : go(k_walk<T, 8, 4>);
+    else if (wchi_ == 16) go(k_walk<T, 16, 1>);
+    else go(k_walk<T, 32, 1>);
+    TNFA_LAUNCH_CHECK();
+  }
+
+  MoveJob move_job(int v) const {
+    const EvalVertex& e = tree_.v[v];
+    std::vector<int> shape{topo_.site_dim[v], topo_.link[v]};
+    for (int c : topo_.children[v]) shape.push_back(topo_.link[c]);
+    TNFA_CHECK(shape.size() <= (size_t)MOVE_MAXD, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
+    const std::vector<int64_t> str = stored_strides(v);
+    MoveJob m{};
+    m.src = tensors_ + topo_.off[v];
+    m.dst = ten_[v];
+    m.n = topo_.size(v);
+    m.nd = (int)e.axes.size();
+    for (int i = 0; i < m.nd; ++i) {
+      m.dim[i] = shape[e.axes[i]];
+      m.str[i] = str[i];
+    }
+    return m;
+  }
+  // The absorption of the last kid's table into the tensor of v.
+  RowJob<T> absorb_job(int v) const {
+    const EvalVertex& e = tree_.v[v];
+    const int w = e.kids.back();
+    const EvalVertex& k = tree_.v[w];
+    RowJob<T> j{};
+    j.A = tab_[w];
+    j.Aexp = tabe_[w];
+    j.aidx = table_row(1, k.N);
+    j.B = ten_[v];
+    j.out = abs_[v];
+    j.out_exp = abse_[v];
+    j.K = k.chi;
+    j.N = (int)(e.W / k.chi);
+    j.rpg = (int)k.N;
+    j.rows = topo_.site_dim[v] * j.rpg;
+    return j;
+  }
+  // The table of v from its one kid (besides the absorbed one).
+  RowJob<T> table_job(int v) const {
+    const EvalVertex& e = tree_.v[v];
+    const int w = e.kids[0];
+    const EvalVertex& k = tree_.v[w];
+    RowJob<T> j{};
+    j.A = tab_[w];
+    j.Aexp = tabe_[w];
+    j.aidx = table_row(1, k.N);
+    j.B = e.absorb ? abs_[v] : ten_[v];
+    j.gexp = e.absorb ? abse_[v] : nullptr;
+    j.out = tab_[v];
+    j.out_exp = tabe_[v];
+    j.K = k.chi;
+    j.N = e.chi;
+    j.rpg = (int)k.N;
+    j.rows = (int)e.N;
+    return j;
+  }
+  template <class Put>
+  void fill_head(Put& put) {
+    std::vector<HeadBlock<T>> hb;
+    std::vector<HeadCopy<T>> cp;
+    std::vector<HeadJob> jobs;
+    head_k_ = 1;
+    head_elems_ = head_exps_ = head_jobs_ = 0;
+    for (const auto& g : hgroups_) {
+      HeadBlock<T> h{};
+      int at = 0, ea = 0;
+      h.copy0 = (int)cp.size();
+      h.job0 = (int)jobs.size();
+      std::vector<int> ten(topo_.V, -1), tab(topo_.V, -1), te(topo_.V, -1);
+      auto stage = [&](int v) {
+        cp.push_back({tensors_ + topo_.off[v], at, (int)topo_.size(v)});
+        ten[v] = at;
+        at += (int)topo_.size(v);
+      };
+      for (int v : g) {
+        stage(v);
+        for (int w : tree_.v[v].kids)
+          if (tree_.v[w].leaf) {
+            stage(w);
+            tab[w] = ten[w];
+          }
+      }
+      for (int v : g) {
+        const EvalVertex& e = tree_.v[v];
+        const std::vector<int64_t> str = stored_strides(v);
+        const int nk = (int)e.kids.size(), up = e.up >= 0 ? (int)str[str.size() - nk - 1] : 0;
+        int mo = -1, me = -1;
+        auto rows_of = [&](HeadJob& j, int w) {
+          j.A = tab[w];
+          j.Aexp = te[w];
+          j.lda = tree_.v[w].leaf ? tree_.v[w].chi : table_pitch(tree_.v[w].chi);
+          j.K = tree_.v[w].chi;
+          j.rpg = (int)tree_.v[w].N;
+        };
+        if (e.absorb) {  // columns (up, the other kid)
+          HeadJob j{};
+          rows_of(j, e.kids[1]);
+          j.B = ten[v];
+          j.gexp = -1;
+          j.bg = (int)str[0];
+          j.n2 = tree_.v[e.kids[0]].chi;
+          j.N = e.chi * j.n2;
+          j.bn1 = up;
+          j.bn2 = (int)str[str.size() - 2];
+          j.bk = (int)str.back();
+          j.rows = topo_.site_dim[v] * j.rpg;
+          j.out = mo = at;
+          j.ldo = j.N;
+          j.oexp = me = ea;
+          at += j.rows * j.N;
+          ea += j.rows;
+          j.level = lvl_m_[v];
+          jobs.push_back(j);
+        }
+        HeadJob j{};
+        rows_of(j, e.kids[0]);
+        j.N = j.n2 = e.chi;
+        j.B = e.absorb ? mo : ten[v];
+        j.gexp = e.absorb ? me : -1;
+        j.bk = e.absorb ? 1 : (int)str.back();
+        j.bn2 = e.absorb ? j.K : up;
+        j.bg = e.absorb ? j.N * j.K : (int)str[0];
+        j.rows = (int)e.N;
+        j.out = tab[v] = at;
+        j.ldo = table_pitch(e.chi);
+        j.oexp = te[v] = ea;
+        at += j.rows * j.ldo;
+        ea += j.rows;
+        j.level = lvl_[v];
+        jobs.push_back(j);
+      }
+      h.copy1 = (int)cp.size();
+      h.job1 = (int)jobs.size();
+      std::stable_sort(jobs.begin() + h.job0, jobs.end(),
+                       [](const HeadJob& x, const HeadJob& y) { return x.level < y.level; });
+      const int v = g.back();
+      h.tab = tab_[v];
+      h.exps = tabe_[v];
+      h.top = tab[v];
+      h.topexp = te[v];
+      h.chi = tree_.v[v].chi;
+      h.ld = table_pitch(h.chi);
+      h.rows = (int)tree_.v[v].N;
+      h.plain = (int)hb.size();
+      for (const auto& c : tree_.comps) h.centre |= !walk_ && (c.a == v || c.b == v);
+      hb.push_back(h);
+      head_elems_ = std::max(head_elems_, at);
+      head_exps_ = std::max(head_exps_, ea);
+      head_jobs_ = std::max(head_jobs_, h.job1 - h.job0);
+    }
+    for (const auto& j : jobs) head_k_ = std::max(head_k_, j.K);
+    head_elems_ += head_elems_ & 1;  // the exponents and jobs behind stay aligned
+    put(dhblocks_, hb.data(), hb.size() * sizeof(HeadBlock<T>));
+    put(dhcopies_, cp.data(), cp.size() * sizeof(HeadCopy<T>));
+    put(dhjobs_, jobs.data(), jobs.size() * sizeof(HeadJob));
   }
 
   CentreSide<T> side(int v) const {
@@ -1441,15 +1733,72 @@ class EvalEngine {
         cur = tp;
       }
       KernelScope ks(ctx_, FamilyName<T>::v, fl, (double)sizeof(T) * n * (j.N + j.K));
-      launch_rows<T>(ctx_, t, row_blocks(j, t), j, nullptr, nullptr, 0);
+      launch_rows<T>(ctx_, t, row_blocks(j, t), pack_rows<T>({j}, {0, 0}, nullptr, nullptr));
     });
   }
   int group_tile(const RowJob<T>& j) const { return row_tile<T>(ctx_, {j}); }
 
+  void centre_pair(const double* X, int n, void* out, int kind, int64_t Pout, int64_t pofs) {
+    const int a = tree_.comps[0].a, b = tree_.comps[0].b;
+    PairParams<T> W{};
+    W.X = X;
+    W.out = out;
+    W.err = err_;
+    W.P = Pout;
+    W.p0 = pofs;
+    W.A = tab_[a];
+    W.B = tab_[b];
+    W.ea = tabe_[a];
+    W.eb = tabe_[b];
+    W.ncols = ncols_;
+    W.Pc = n;
+    W.nruns = (int)runs_.size();
+    W.chi = tree_.v[a].chi;
+    W.sa = row_slot_[a];
+    W.sb = row_slot_[b];
+    W.kind = kind;
+    W.scale = tree_.v[a].leaf || tree_.v[b].leaf;
+    std::copy(runs_.begin(), runs_.end(), W.runs);
+    KernelScope ks(ctx_, "eval_fused", 2.0 * n * W.chi, (double)n * (ncols_ * 8.0 + 8.0));
+    W.na = (int)tree_.v[a].N;
+    W.nb = (int)tree_.v[b].N;
+    W.pa = plain_of_[a] >= 0 && !walk_ ? plain_ + plain_of_[a] : nullptr;
+    W.pb = plain_of_[b] >= 0 && !walk_ ? plain_ + plain_of_[b] : nullptr;
+    constexpr int vec = 16 / sizeof(T);
+    // short rows gathered by many points: from shared memory, if 4 blocks of it
+    // fit an SM and every copied row is read about 8 times or more
+    const size_t sm = ((size_t)(W.na + W.nb) * W.chi + 2 * vec) * sizeof(T);
+    const bool shared = W.chi * sizeof(T) <= 64 && sm <= 48 * 1024 &&
+                        (double)n >= 8.0 * (W.na + W.nb) * ctx_->sm_count;
+    const unsigned grid = grid_for(n, 256, ctx_->sm_count * (shared ? 4 : 8));
+    auto go = [&](auto kern, auto kern_sm) {
+      if (shared) kern_sm<<<grid, 256, sm, ctx_->stream>>>(W);
+      else kern<<<grid, 256, 0, ctx_->stream>>>(W);
+    };
+    if constexpr (vec > 1) {
+      if (centre_vec_) {
+        const int lanes = (W.chi + vec - 1) / vec;
+        if (lanes <= 2) go(k_centre_pair<T, 1, vec, false>, k_centre_pair<T, 1, vec, true>);
+        else if (lanes <= 4) go(k_centre_pair<T, 4, vec, false>, k_centre_pair<T, 4, vec, true>);
+        else go(k_centre_pair<T, 8, vec, false>, k_centre_pair<T, 8, vec, false>);
+        TNFA_LAUNCH_CHECK();
+        return;
+      }
+    }
+    if (W.chi <= 4) go(k_centre_pair<T, 1, 1, false>, k_centre_pair<T, 1, 1, true>);
+    else if (W.chi <= 8) go(k_centre_pair<T, 4, 1, false>, k_centre_pair<T, 4, 1, true>);
+    else go(k_centre_pair<T, 8, 1, false>, k_centre_pair<T, 8, 1, true>);
+    TNFA_LAUNCH_CHECK();
+  }
+
   void centre(const double* X, int n, void* out, int kind, int64_t Pout, int64_t pofs) {
     const int ns = fused_ ? nslots_ : 0;
     const size_t sm = 256 * (sizeof(T) + 4) + (size_t)ns * 1024 + (fused_ ? runs_.size() * sizeof(DigitRun) : 0);
-    KernelScope ks(ctx_, "centre", 2.0 * n * centre_chi_, (double)n * (ncols_ * 8.0 + 8.0));
+    if (fused_ && tree_.comps.size() == 1 && tree_.comps[0].b >= 0 && runs_.size() <= (size_t)CENTRE_RUNS) {
+      centre_pair(X, n, out, kind, Pout, pofs);
+      return;
+    }
+    KernelScope ks(ctx_, fused_ ? "eval_fused" : "centre", 2.0 * n * centre_chi_, (double)n * (ncols_ * 8.0 + 8.0));
     const unsigned grid = grid_for(n, 256, ctx_->sm_count * 8);
     auto go = [&](auto kern) {
       kern<<<grid, 256, sm, ctx_->stream>>>(X, ncols_, n, druns_, (int)runs_.size(), ns, dcentre_,
@@ -1488,7 +1837,22 @@ class EvalEngine {
   std::vector<Level> levels_;
   int nslots_ = 0, ncodes_ = 0, nmsg_ = 0, msg_chi_ = 1, npp_ = 0, Pc_ = 0, centre_chi_ = 1;
   int64_t max_group_ = 1, ld_ = 0;
-  bool fused_ = false, centre_vec_ = false;
+  bool fused_ = false, centre_vec_ = false, small_ = false, walk_ = false;
+  struct WalkVertex {
+    int v, nk, d1, d2;
+  };
+  std::vector<WalkVertex> wsteps_;
+  int wchi_ = 1, wmsg_ = 0, wtp_ = 32, wlanes_ = 1, nstage_ = 0, nsteps0_ = 0;
+  unsigned char* dwalk_ = nullptr;
+  // head of the tables: groups of vertices by block
+  std::vector<char> head_;
+  std::vector<int> plain_of_;  // head block of its top vertex
+  std::vector<std::vector<int>> hgroups_;
+  int nhead_jobs_ = 0, nhead_copies_ = 0, head_k_ = 1, head_elems_ = 0, head_exps_ = 0, head_jobs_ = 0;
+  int* plain_ = nullptr;  // per head block: its rows carry no exponents
+  HeadBlock<T>* dhblocks_ = nullptr;
+  HeadCopy<T>* dhcopies_ = nullptr;
+  HeadJob* dhjobs_ = nullptr;
   size_t per_point_ = 0, blob_bytes_ = 0;
   std::vector<unsigned char> host_;
   std::vector<MoveJob> moves_;
@@ -1527,39 +1891,18 @@ static void evaluate_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, 
                           bool use_oz = false) {
   const size_t out_elem = out_elem_size(out_kind);
   const size_t staged = (xmem == TNFA_MEM_HOST ? ncols * 8 : 0) + (out_mem == TNFA_MEM_HOST ? out_elem : 0);
-  // small bonds everywhere: the whole tree per thread in one launch
-  const FusedPlan F = make_fused_plan(net->topo, sizeof(T), prog.size(), P);
-  std::unique_ptr<EvalEngine<T>> E;
-  std::vector<DigitRun> runs;
-  int64_t Pcap;
-  if (F.ok) {
-    runs = make_fused_runs(net->topo, prog);
-    Pcap = staged ? std::max<int64_t>(256, (int64_t)(ctx->eval_budget / staged) / 256 * 256) : int64_t(1) << 30;
-  } else {
-    E.reset(new EvalEngine<T>(ctx, net, tensors, prog, ncols, P, use_tc, use_oz, ctx->eval_budget));
-    Pcap = E->chunk();
-    if (staged) Pcap = std::min(Pcap, std::max<int64_t>(256, (int64_t)(ctx->eval_budget / staged) / 256 * 256));
-  }
-  Pcap = std::max<int64_t>(1, std::min<int64_t>({P, Pcap, int64_t(1) << 30}));
+  EvalEngine<T> E(ctx, net, tensors, prog, ncols, P, use_tc, use_oz, ctx->eval_budget);
+  int64_t Pcap = E.chunk();
+  if (staged) Pcap = std::min(Pcap, std::max<int64_t>(256, (int64_t)(ctx->eval_budget / staged) / 256 * 256));
+  Pcap = std::max<int64_t>(1, std::min(P, Pcap));
   DBuf dX(ctx, xmem == TNFA_MEM_HOST ? (size_t)Pcap * ncols * 8 : 0);
   DBuf dout(ctx, out_mem == TNFA_MEM_HOST ? (size_t)Pcap * out_elem : 0);
-  DBuf derr(ctx, 4), arena, dprog, dsteps;
-  int* err;
-  if (F.ok) {
-    dprog = DBuf(ctx, std::max<size_t>(runs.size(), 1) * sizeof(DigitRun));
-    h2d(ctx, dprog.p, runs.data(), runs.size() * sizeof(DigitRun));
-    dsteps = DBuf(ctx, F.steps.size() * sizeof(FusedStep));
-    h2d(ctx, dsteps.p, F.steps.data(), F.steps.size() * sizeof(FusedStep));
-    err = derr.as<int>();
-    TNFA_CUDA(cudaMemsetAsync(err, 0, 4, ctx->stream));
-  } else {
-    E->set_chunk((int)Pcap);
-    arena = DBuf(ctx, E->scratch(Pcap));
-    E->bind(arena.p);
-    E->upload();
-    E->tables();
-    err = E->err_flag();
-  }
+  E.set_chunk((int)Pcap);
+  DBuf arena(ctx, E.scratch(Pcap));
+  E.bind(arena.p);
+  E.upload();
+  E.clear_error();
+  E.tables();
   for (int64_t p0 = 0; p0 < P; p0 += Pcap) {
     const int Pc = (int)std::min<int64_t>(Pcap, P - p0);
     const double* Xc = X + p0 * ncols;
@@ -1569,11 +1912,7 @@ static void evaluate_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, 
     }
     void* o = out_mem == TNFA_MEM_HOST ? dout.p : out;
     const int64_t Pout = out_mem == TNFA_MEM_HOST ? Pc : P, pofs = out_mem == TNFA_MEM_HOST ? 0 : p0;
-    if (F.ok)
-      launch_fused<T>(ctx, F, dsteps.as<FusedStep>(), tensors, net->topo, Xc, ncols, Pc,
-                      dprog.as<DigitRun>(), (int)runs.size(), o, out_kind, Pout, pofs, err);
-    else
-      E->points(Xc, Pc, o, out_kind, Pout, pofs);
+    E.points(Xc, Pc, o, out_kind, Pout, pofs);
     if (out_mem == TNFA_MEM_HOST) {
       if (out_kind == TNFA_OUT_F32_SCALED) {
         TNFA_CUDA(cudaMemcpyAsync((float*)out + p0, dout.p, (size_t)Pc * 4, cudaMemcpyDeviceToHost,
@@ -1586,7 +1925,7 @@ static void evaluate_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, 
       }
     }
   }
-  check_eval_error(ctx, err);
+  check_eval_error(ctx, E.err_flag());
 }
 
 }  // namespace tnfa
@@ -1696,14 +2035,13 @@ unsigned char* noalloc_base(int device) {
 template <class T>
 size_t noalloc_bytes(const tnfa_net* net, int64_t P, size_t prog_entries) {
   const Topo& Tp = net->topo;
-  const FusedPlan F = make_fused_plan(Tp, sizeof(T), prog_entries, P);
   const EvalPlan plan = make_plan(Tp);
   const size_t nroots = plan.roots.size();
   int maxsd = 1;
   for (int v = 0; v < Tp.V; ++v) maxsd = std::max(maxsd, Tp.site_dim[v]);
   std::array<size_t, 10> sizes{prog_entries * 32, 0, 0, 0, 0, 4, 0, 0, 0, 0};
-  if (F.ok) {
-    sizes[1] = F.steps.size() * sizeof(FusedStep);
+  if (small_bonds(Tp, sizeof(T), P)) {
+    sizes[1] = (size_t)Tp.V * 36;
   } else {
     sizes[2] = (size_t)Tp.V * P;
     sizes[3] = (size_t)P * 4;
@@ -1726,67 +2064,26 @@ class FixedRun {
  public:
   FixedRun(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const std::vector<DigitRef>& prog, int ncols,
            int64_t P, size_t budget)
-      : ctx_(ctx), net_(net), tensors_(tensors), ncols_(ncols), P_(P),
-        F_(make_fused_plan(net->topo, sizeof(T), prog.size(), P)) {
-    if (F_.ok) {
-      runs_ = make_fused_runs(net->topo, prog);
-      return;
-    }
-    E_.reset(new EvalEngine<T>(ctx, net, tensors, prog, ncols, P, false, false, budget));
-    int pc = E_->chunk();
-    while (pc > 1 && E_->scratch(pc) > budget) pc = std::max(1, pc / 2);
-    E_->set_chunk(pc);
+      : ncols_(ncols), P_(P), E_(ctx, net, tensors, prog, ncols, P, false, false, budget) {
+    int pc = E_.chunk();
+    while (pc > 1 && E_.scratch(pc) > budget) pc = std::max(1, pc / 2);
+    E_.set_chunk(pc);
   }
-  size_t bytes() {
-    if (!F_.ok) return E_->scratch(E_->chunk());
-    Carve c;
-    lay_out(c);
-    return c.used + 256;
-  }
-  void bind(void* base) {
-    Carve c;
-    c.base = (unsigned char*)base;
-    if (F_.ok) lay_out(c);
-    else E_->bind(base);
-  }
-  void stage() {
-    if (F_.ok) {
-      h2d(ctx_, dprog_, runs_.data(), runs_.size() * sizeof(DigitRun));
-      h2d(ctx_, dsteps_, F_.steps.data(), F_.steps.size() * sizeof(FusedStep));
-    } else {
-      E_->upload();
-    }
-  }
-  int* err_flag() const { return F_.ok ? err_ : E_->err_flag(); }
+  size_t bytes() { return E_.scratch(E_.chunk()); }
+  void bind(void* base) { E_.bind(base); }
+  void stage() { E_.upload(); }
+  int* err_flag() const { return E_.err_flag(); }
   void enqueue(const double* X, void* out, int out_kind) {
-    TNFA_CUDA(cudaMemsetAsync(err_flag(), 0, 4, ctx_->stream));
-    if (F_.ok) {
-      launch_fused<T>(ctx_, F_, dsteps_, tensors_, net_->topo, X, ncols_, (int)P_, dprog_, (int)runs_.size(), out,
-                      out_kind, P_, 0, err_);
-      return;
-    }
-    E_->tables();
-    for (int64_t p0 = 0; p0 < P_; p0 += E_->chunk())
-      E_->points(X + p0 * ncols_, (int)std::min<int64_t>(E_->chunk(), P_ - p0), out, out_kind, P_, p0);
+    E_.clear_error();
+    E_.tables();
+    for (int64_t p0 = 0; p0 < P_; p0 += E_.chunk())
+      E_.points(X + p0 * ncols_, (int)std::min<int64_t>(E_.chunk(), P_ - p0), out, out_kind, P_, p0);
   }
 
  private:
-  void lay_out(Carve& c) {
-    dprog_ = c.take<DigitRun>(runs_.size());
-    dsteps_ = c.take<FusedStep>(F_.steps.size());
-    err_ = c.take<int>(1);
-  }
-  tnfa_ctx* ctx_;
-  const tnfa_net* net_;
-  const T* tensors_;
   int ncols_;
   int64_t P_;
-  FusedPlan F_;
-  std::vector<DigitRun> runs_;
-  std::unique_ptr<EvalEngine<T>> E_;
-  DigitRun* dprog_ = nullptr;
-  FusedStep* dsteps_ = nullptr;
-  int* err_ = nullptr;
+  EvalEngine<T> E_;
 };
 
 template <class T>
@@ -2153,7 +2450,7 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
   const int Pcap = (int)std::max<int64_t>(std::min<int64_t>(P, (Pc_max / 256) * 256), 1);
   int maxsd = 1;
   for (int v = 0; v < V; ++v) maxsd = std::max(maxsd, Tp.site_dim[v]);
-  const std::vector<DigitRun> runs = make_fused_runs(Tp, prog);
+  const std::vector<DigitRun> runs = make_site_runs(Tp, prog);
   DBuf dprog(ctx, std::max<size_t>(runs.size(), 1) * sizeof(DigitRun));
   h2d(ctx, dprog.p, runs.data(), runs.size() * sizeof(DigitRun));
   DBuf dS(ctx, (size_t)V * Pcap * 4), dperm(ctx, (size_t)Pcap * 4);

@@ -2,6 +2,8 @@
 // codes, the one-child contraction over gathered rows, permuted tensor
 // copies, and the dot product at the centre.
 #pragma once
+#include <climits>
+
 #include "evaluate.cuh"
 
 namespace tnfa {
@@ -47,9 +49,9 @@ __device__ __forceinline__ void digit_codes(const double* __restrict__ Xp, const
     const DigitRun d = runs[e];
     if (d.start) {
       xr = Xp[d.col];
-      const unsigned hi = (unsigned)((unsigned long long)__double_as_longlong(xr) >> 32);
-      const bool neg = (hi >> 31) && xr != 0.0;
-      if (neg || (hi & 0x7FF00000u) == 0x7FF00000u) {  // negative, infinite or NaN
+      const unsigned long long xb = (unsigned long long)__double_as_longlong(xr);
+      // negative (not -0), infinite or NaN
+      if (xb > 0x8000000000000000ull || (xb & 0x7FF0000000000000ull) == 0x7FF0000000000000ull) {
         atomicOr(err, 1);
         xr = 0.0;
       }
@@ -269,13 +271,38 @@ struct RowJob {
   T* out;
   int* out_exp;
   int K, N, rows;
-  int rpg;  // > 0: uniform groups
+  int rpg;  // > 0: uniform groups, and row(q) = q % rpg
   const int* perm;  // null: identity
   const int* grp_off;
   const int* grp_cnt;
   const int* tile_start;
   int ngroups;
 };
+
+// Up to ROW_PACK jobs travel in the launch's parameters (no load stands before
+// a job's own operands); longer lists are read from the job table.
+constexpr int ROW_PACK = 8;
+template <class T>
+struct RowPack {
+  const RowJob<T>* jobs;
+  const int* first;  // first block of every job, and the end
+  int n;             // 0: in the table
+  int total;         // jobs
+  RowJob<T> j[ROW_PACK];
+  int f[ROW_PACK + 1];
+};
+template <class T>
+__device__ __forceinline__ int find_job(const RowPack<T>& p, int b, RowJob<T>& j) {
+  if (p.n) {
+    int i = 0;
+    while (i + 1 < p.n && p.f[i + 1] <= b) ++i;
+    j = p.j[i];
+    return b - p.f[i];
+  }
+  const int i = find_group(p.first, p.total, b);
+  j = p.jobs[i];
+  return b - p.first[i];
+}
 
 // A block: TM = 8 RM rows x TN = 32 CN columns, 8 warps of RM rows each (a
 // warp without valid rows skips the products, so short groups cost their own
@@ -284,20 +311,14 @@ struct RowJob {
 // compute bound and small ones spread over more SMs; FP32 takes 64 x 128
 // (8 x 4 accumulators per thread: 12 shared-memory words per 32 FMAs).
 template <class T, int RM, int CN>
-__global__ void __launch_bounds__(256) k_rows_gemm(const RowJob<T> one, const RowJob<T>* __restrict__ jobs,
-                                                   const int* __restrict__ first, int njobs) {
+__global__ void __launch_bounds__(256) k_rows_gemm(const __grid_constant__ RowPack<T> pack) {
   constexpr int TM = 8 * RM, TN = 32 * CN, KC = 32;
   constexpr int LA = TM + (sizeof(T) == 4 ? 4 : 2), LB = TN + (sizeof(T) == 4 ? 4 : 2);
   __shared__ __align__(16) T As[KC * LA];
   __shared__ __align__(16) T Bs[KC * LB];
   __shared__ int arow[TM], item[TM], rex[TM];
-  int b = blockIdx.x;
-  RowJob<T> j = one;
-  if (njobs > 0) {
-    const int i = find_group(first, njobs, b);
-    j = jobs[i];
-    b -= first[i];
-  }
+  RowJob<T> j;
+  const int b = find_job(pack, blockIdx.x, j);
   const int nbn = (j.N + TN - 1) / TN;
   const int n0 = (b % nbn) * TN, bm = b / nbn;
   int g, q0, nrows;
@@ -391,6 +412,47 @@ __global__ void __launch_bounds__(256) k_rows_gemm(const RowJob<T> one, const Ro
     j.out_exp[item[tid]] = rex[tid] + (j.Aexp ? j.Aexp[arow[tid]] : 0) + (j.gexp ? j.gexp[g] : 0);
 }
 
+// The same products for short rows (K <= 32): one thread per row and chunk of
+// 4 columns, the row in registers and scaled there.  A tile of k_rows_gemm
+// would leave most of its 32 column lanes idle below N = 32.
+template <class T, int KM>
+__device__ __forceinline__ void small_row(const RowJob<T>& j, unsigned it, unsigned nc) {
+  const int q = nc == 1 ? (int)it : (int)(it / nc), n0 = (int)(it - (unsigned)q * nc) * 4;
+  const int g = (int)((unsigned)q / (unsigned)j.rpg), ar = q - g * j.rpg;
+  const T* A = j.A + (int64_t)ar * j.K;
+  const T* B = j.B + ((int64_t)g * j.N + n0) * j.K;
+  T a[KM];
+  typename Real<T>::t m = 0;
+#pragma unroll
+  for (int k = 0; k < KM; ++k) a[k] = k < j.K ? A[k] : Sc<T>::zero();
+  int ex = n0 == 0 ? (j.Aexp ? j.Aexp[ar] : 0) + (j.gexp ? j.gexp[g] : 0) : 0;
+#pragma unroll
+  for (int k = 0; k < KM; ++k) m = mag_max(m, a[k]);
+  const int e = exponent_of(m);
+  ex += e;
+  if (e)
+#pragma unroll
+    for (int k = 0; k < KM; ++k) a[k] = scale_pow2(a[k], -e);
+  T* o = j.out + (int64_t)q * j.N + n0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (n0 + c >= j.N) break;
+    T s = Sc<T>::zero();
+#pragma unroll
+    for (int k = 0; k < KM; ++k)
+      if (k < j.K) s = Sc<T>::fma(a[k], B[c * j.K + k], s);
+    o[c] = s;
+  }
+  if (n0 == 0) j.out_exp[q] = ex;
+}
+template <class T, int KM>
+__global__ void __launch_bounds__(128) k_rows_small(const __grid_constant__ RowPack<T> pack) {
+  RowJob<T> j;
+  const int b = find_job(pack, blockIdx.x, j);
+  const unsigned nc = (j.N + 3) / 4, it = (unsigned)b * 128 + threadIdx.x;
+  if (it < (unsigned)j.rows * nc) small_row<T, KM>(j, it, nc);
+}
+
 // --------------------------------------------------- permuted tensors ----
 constexpr int MOVE_MAXD = 20;
 struct MoveJob {
@@ -402,17 +464,31 @@ struct MoveJob {
   int64_t str[MOVE_MAXD];  // strides of those axes in src
 };
 template <class T>
-__global__ void k_move(const MoveJob* __restrict__ jobs) {
-  const MoveJob& j = jobs[blockIdx.y];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < j.n; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t q = i, s = 0;
-    for (int d = j.nd - 1; d >= 0; --d) {
-      const int64_t t = q / j.dim[d];
-      s += (q - t * j.dim[d]) * j.str[d];
-      q = t;
+__device__ __forceinline__ void move_run(const MoveJob& j, int64_t i0, int64_t step) {
+  const bool small = j.n < (int64_t(1) << 31);
+  for (int64_t i = i0; i < j.n; i += step) {
+    int64_t s = 0;
+    if (small) {
+      unsigned q = (unsigned)i;
+      for (int d = j.nd - 1; d >= 0; --d) {
+        const unsigned t = q / (unsigned)j.dim[d];
+        s += (int64_t)(q - t * (unsigned)j.dim[d]) * j.str[d];
+        q = t;
+      }
+    } else {
+      int64_t q = i;
+      for (int d = j.nd - 1; d >= 0; --d) {
+        const int64_t t = q / j.dim[d];
+        s += (q - t * j.dim[d]) * j.str[d];
+        q = t;
+      }
     }
     ((T*)j.dst)[i] = ((const T*)j.src)[s];
   }
+}
+template <class T>
+__global__ void k_move(const MoveJob* __restrict__ jobs) {
+  move_run<T>(jobs[blockIdx.y], blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
 // ------------------------------------------------------------- centre ----
@@ -460,6 +536,12 @@ __device__ __forceinline__ float shfl_x(float v, int o) { return __shfl_xor_sync
 __device__ __forceinline__ double shfl_x(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ cplx shfl_x(cplx v, int o) {
   return {__shfl_xor_sync(0xffffffffu, v.re, o), __shfl_xor_sync(0xffffffffu, v.im, o)};
+}
+
+__device__ __forceinline__ float shfl_i(float v, int i) { return __shfl_sync(0xffffffffu, v, i); }
+__device__ __forceinline__ double shfl_i(double v, int i) { return __shfl_sync(0xffffffffu, v, i); }
+__device__ __forceinline__ cplx shfl_i(cplx v, int i) {
+  return {__shfl_sync(0xffffffffu, v.re, i), __shfl_sync(0xffffffffu, v.im, i)};
 }
 
 // f(p) = prod over components of sum_c A[c] B[c].  The block digitizes its
@@ -553,6 +635,389 @@ __global__ void __launch_bounds__(256) k_centre(const double* __restrict__ X, in
   }
 }
 
+__device__ __forceinline__ void copy_async16(void* d, const void* s) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(s));
+}
+__device__ __forceinline__ void copy_async4(void* d, const void* s) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(s));
+}
+
+// bytes (a multiple of 4) of global memory to shared memory, by the whole block
+__device__ __forceinline__ void copy_async_block(void* d, const void* s, int bytes) {
+  const int n16 = (((uintptr_t)s | (uintptr_t)d) & 15) == 0 ? bytes / 16 : 0;
+  for (int i = threadIdx.x; i < n16; i += blockDim.x) copy_async16((char*)d + 16 * i, (const char*)s + 16 * i);
+  for (int i = n16 * 4 + threadIdx.x; i < bytes / 4; i += blockDim.x)
+    copy_async4((char*)d + 4 * i, (const char*)s + 4 * i);
+}
+
+// The common case of k_centre -- one component, both sides tables, few digit
+// runs -- with everything but the rows in kernel parameters and registers: a
+// thread digitizes its point, then G lanes take each of the warp's points in
+// turn.  k_centre spent 350 instructions per point on job records, digit runs
+// and codes in memory.  At bond 2 the FP64 pipe (2 multiply-adds per point at
+// 2 per clock per SM) and HBM (16 bytes per point) are about even.
+constexpr int CENTRE_RUNS = 12;
+template <class T>
+struct PairParams {
+  const double* X;
+  void* out;
+  int* err;
+  int64_t P, p0;
+  const T *A, *B;
+  const int *ea, *eb;  // null: zero
+  const int *pa, *pb;  // set on the device: the side's exponents are all zero (null: not known)
+  int na, nb;          // rows
+  int ncols, Pc, nruns, chi, sa, sb, kind, scale;  // sa, sb: code slots; scale: rows of a leaf tensor
+  DigitRun runs[CENTRE_RUNS];
+};
+// SM: both tables are copied to shared memory first.  A gather of 32 different
+// rows costs a cache line per lane in L1 (32 cycles), a few bank conflicts
+// there.
+template <class T, int G, int VEC, bool SM>
+__global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ PairParams<T> W) {
+  extern __shared__ __align__(16) unsigned char pair_sh[];
+  const int lane = threadIdx.x & 31, l = lane % G;
+  const T* tabA = W.A;
+  const T* tabB = W.B;
+  if constexpr (SM) {
+    const int na = W.na * W.chi, nb = W.nb * W.chi;
+    T* sa = (T*)pair_sh;
+    T* sb = sa + (na + VEC - 1) / VEC * VEC;
+    copy_async_block(sa, W.A, na * (int)sizeof(T));
+    copy_async_block(sb, W.B, nb * (int)sizeof(T));
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    tabA = sa;
+    tabB = sb;
+  }
+  const int* xa_ = W.ea && !(W.pa && *W.pa) ? W.ea : nullptr;
+  const int* xb_ = W.eb && !(W.pb && *W.pb) ? W.eb : nullptr;
+  constexpr int PG = 32 / G;  // points per pass
+  for (int64_t base = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) - lane; base < W.Pc;
+       base += (int64_t)gridDim.x * blockDim.x) {
+    const int p = (int)min((int64_t)W.Pc - 1, base + lane);  // the padding lanes repeat the last point
+    int c[2] = {0, 0};
+    {
+      double xr = 0.0;
+      unsigned long long u = 0;
+      for (int e = 0; e < W.nruns; ++e) {
+        const DigitRun& d = W.runs[e];
+        if (d.start) {
+          xr = W.X[(int64_t)p * W.ncols + d.col];
+          const unsigned long long xb = (unsigned long long)__double_as_longlong(xr);
+          if (xb > 0x8000000000000000ull || (xb & 0x7FF0000000000000ull) == 0x7FF0000000000000ull) {
+            atomicOr(W.err, 1);
+            xr = 0.0;
+          }
+          u = unit_fraction(xr);
+        }
+        int add;
+        if (d.bits) {
+          const unsigned f = (unsigned)((u << (d.first - 1)) >> 32);
+          add = (int)(d.rev ? __brev(f) & (0xFFFFFFFFu >> (32 - d.n)) : f >> (32 - d.n)) * d.w;
+        } else {
+          int dig = 0;
+          for (int v = d.base - 1; v >= 1; --v) {
+            const double t = (double)v * d.invb;
+            if (xr >= t) {
+              dig = v;
+              xr -= t;
+              break;
+            }
+          }
+          add = dig * d.w;
+        }
+        if (d.slot == W.sa) c[0] += add;
+        else c[1] += add;
+      }
+    }
+    T v = Sc<T>::zero();
+    int ve = 0;
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const int t = i * PG + lane / G;  // the point of this pass
+      const int ra = G == 1 ? c[0] : __shfl_sync(0xffffffffu, c[0], t);
+      const int rb = G == 1 ? c[1] : __shfl_sync(0xffffffffu, c[1], t);
+      const T* A = tabA + (int64_t)ra * W.chi;
+      const T* B = tabB + (int64_t)rb * W.chi;
+      int e = (xa_ ? xa_[ra] : 0) + (xb_ ? xb_[rb] : 0), ea = 0, eb = 0;
+      if (W.scale) {
+        typename Real<T>::t ma = 0, mb = 0;
+        for (int k = l; k < W.chi; k += G) {
+          ma = mag_max(ma, A[k]);
+          mb = mag_max(mb, B[k]);
+        }
+#pragma unroll
+        for (int o = G / 2; o; o >>= 1) {
+          ma = mag_max(ma, __shfl_xor_sync(0xffffffffu, ma, o));
+          mb = mag_max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+        }
+        ea = exponent_of(ma);
+        eb = exponent_of(mb);
+        e += ea + eb;
+      }
+      T s = Sc<T>::zero();
+      for (int k = l * VEC; k < W.chi; k += G * VEC) {
+        T xa[VEC], xb[VEC];
+        if constexpr (VEC > 1) {
+          *reinterpret_cast<int4*>(xa) = *reinterpret_cast<const int4*>(A + k);
+          *reinterpret_cast<int4*>(xb) = *reinterpret_cast<const int4*>(B + k);
+        } else {
+          xa[0] = A[k];
+          xb[0] = B[k];
+        }
+#pragma unroll
+        for (int q = 0; q < VEC; ++q)
+          s = Sc<T>::fma(ea ? scale_pow2(xa[q], -ea) : xa[q], eb ? scale_pow2(xb[q], -eb) : xb[q], s);
+      }
+#pragma unroll
+      for (int o = G / 2; o; o >>= 1) s = s + shfl_x(s, o);
+      // hand the sum to the point's own lane
+      if constexpr (G == 1) {
+        v = s;
+        ve = e;
+      } else {
+        const int src = ((lane - i * PG) * G) & 31;
+        const T sv = shfl_i(s, src);
+        const int se = __shfl_sync(0xffffffffu, e, src);
+        if (lane / PG == i) {
+          v = sv;
+          ve = se;
+        }
+      }
+    }
+    if (base + lane < W.Pc) write_out<T>(W.out, W.kind, W.p0 + base + lane, W.P, v, ve);
+  }
+}
+
+// --------------------------------------------------- small-bond walk ----
+// Small bonds: a thread takes its point through every vertex that has no table
+// in one launch, and no message goes through HBM.  The two sides of the centre
+// are walked by two threads (half the chain each).  The schedule and, up to 64
+// KB, the network's tensors are copied to shared memory asynchronously while
+// the points are digitized; the tensors are read through strides, so no vertex
+// needs a copy in another axis order.  Up to bond 8 the message of a step stays
+// in registers for the next one when that reads it (a path never stores one);
+// otherwise messages are in shared memory, [slot][entry][point].  For a few
+// thousand points G lanes share a point: each makes CHI / G rows of a step and
+// the message is put together by shuffles, because one warp's FP64 multiply-add
+// takes 64 cycles of its scheduler and a chain of them on few warps leaves the
+// other schedulers idle.
+template <class T>
+struct WalkStep {
+  const T* B;       // tensor slices (vertex tensor, or one with an absorbed table)
+  const int* gexp;  // exponent of a slice, null: zero
+  const T* t1;      // first child's table, null: its message slot
+  const T* t2;      // last child's
+  const int* e1;    // the tables' exponents, null: zero
+  const int* e2;
+  int stage;        // element offset of B in the staged network tensors, -1: read in place
+  int key;          // code slot of the slice, -1: slice 0
+  int chi_a;
+  int d1, d2;       // first and last child's bonds (1 when absent)
+  int c1, c2;       // code slot (table) or message slot of the children; -1: none, -2: the previous step's registers
+  int sg, sa, s1, s2;  // strides of slice, row, first and last child in B
+  int out;          // message slot, -1: stays in registers
+};
+template <class T>
+struct WalkSide {
+  const T* tab;  // null: message slot `at`
+  const int* exps;
+  int at;        // code slot or message slot
+  int chi;       // 0: absent (a vertex centre)
+};
+template <class T>
+struct WalkParams {
+  const double* X;
+  const unsigned char* blob;  // runs, steps (side 0's, then side 1's), sides (two per component)
+  const T* tensors;
+  void* out;
+  int* err;
+  int64_t P, p0;
+  int ncols, Pc, nruns, nslots, nsteps0, nsteps, ncomp, nmsg, nstage, kind;
+};
+
+template <class T>
+__host__ __device__ inline size_t walk_blob(int nruns, int nsteps, int ncomp) {
+  return (nruns * sizeof(DigitRun) + nsteps * sizeof(WalkStep<T>) + 2 * ncomp * sizeof(WalkSide<T>) + 15) / 16 * 16;
+}
+template <class T>
+__host__ __device__ inline size_t walk_smem(int chi, int tp, int nstage, int nmsg, int nslots, int nruns, int nsteps,
+                                            int ncomp) {
+  return walk_blob<T>(nruns, nsteps, ncomp) + ((size_t)nstage * sizeof(T) + 15) / 16 * 16 +
+         (size_t)nmsg * chi * tp * sizeof(T) + (size_t)(2 + nslots) * tp * 4;
+}
+
+template <class T, int CHI, int G>
+__global__ void __launch_bounds__(256) k_walk(const __grid_constant__ WalkParams<T> W) {
+  constexpr bool REG = CHI <= 8;  // the message also in registers (unrolled rows)
+  constexpr int RL = CHI / G;     // rows per lane
+  static_assert(REG || G == 1, "lanes share a point only with the message in registers");
+  extern __shared__ __align__(16) unsigned char walk_sh[];
+  const int tl = blockDim.x >> 1, tp = tl / G;  // threads and points per side
+  const int side = threadIdx.x >= tl, t = (threadIdx.x - side * tl) / G, gl = threadIdx.x % G;
+  const DigitRun* runs = (const DigitRun*)walk_sh;
+  const WalkStep<T>* st = (const WalkStep<T>*)(runs + W.nruns);
+  const WalkSide<T>* sd = (const WalkSide<T>*)(st + W.nsteps);
+  const size_t nblob = walk_blob<T>(W.nruns, W.nsteps, W.ncomp);
+  T* ten = (T*)(walk_sh + nblob);
+  T* msg = (T*)(walk_sh + nblob + ((size_t)W.nstage * sizeof(T) + 15) / 16 * 16);
+  int* sex = (int*)(msg + (size_t)W.nmsg * CHI * tp);  // [2][tp] exponents of the sides
+  int* codes = sex + 2 * tp;                           // [nslots][tp]
+  copy_async_block(walk_sh, W.blob, (int)nblob);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  copy_async_block(ten, W.tensors, W.nstage * (int)sizeof(T));
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;" ::: "memory");
+  __syncthreads();
+  auto M = [&](int slot, int k) -> T& { return msg[((size_t)slot * CHI + k) * tp + t]; };
+  for (int base = blockIdx.x * tp; base < W.Pc; base += gridDim.x * tp) {
+    const int p = base + t;
+    if (side == 0 && gl == 0) {
+      for (int s = 0; s < W.nslots; ++s) codes[s * tp + t] = 0;
+      if (p < W.Pc) digit_codes(W.X + (int64_t)p * W.ncols, runs, W.nruns, codes + t, tp, 0, W.nslots, W.err);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    int ex_acc = 0;
+    T cur[REG ? CHI : 1];
+    const int i1 = side ? W.nsteps : W.nsteps0;
+    for (int i = side ? W.nsteps0 : 0; i < i1; ++i) {
+      const WalkStep<T>& s = st[i];
+      const int g = s.key >= 0 ? codes[s.key * tp + t] : 0;
+      const int d1 = s.d1, d2 = s.d2, chi_a = s.chi_a, sa = s.sa, s1 = s.s1, s2 = s.s2, c1 = s.c1, c2 = s.c2;
+      const T* B = (s.stage >= 0 ? ten + s.stage : s.B) + (int64_t)g * s.sg;
+      if (s.gexp) ex_acc += s.gexp[g];
+      // the last child's row in registers; a table's row is scaled here, a
+      // message was when it was made
+      T ml[CHI];
+      if (REG && c2 == -2) {
+#pragma unroll
+        for (int c = 0; c < CHI; ++c) ml[c] = cur[REG ? c : 0];
+      } else if (s.t2) {
+        const int r = codes[c2 * tp + t];
+        const T* row = s.t2 + (int64_t)r * d2;
+        typename Real<T>::t m = 0;
+#pragma unroll
+        for (int c = 0; c < CHI; ++c) {
+          ml[c] = c < d2 ? row[c] : Sc<T>::zero();
+          m = mag_max(m, ml[c]);
+        }
+        const int e = exponent_of(m);
+        ex_acc += e + (s.e2 ? s.e2[r] : 0);
+        if (e)
+#pragma unroll
+          for (int c = 0; c < CHI; ++c) ml[c] = scale_pow2(ml[c], -e);
+      } else {
+#pragma unroll
+        for (int c = 0; c < CHI; ++c) ml[c] = c < d2 ? M(c2, c) : Sc<T>::zero();
+      }
+      const T* row1 = nullptr;
+      int e1 = 0;
+      if (s.t1) {
+        const int r = codes[c1 * tp + t];
+        row1 = s.t1 + (int64_t)r * d1;
+        typename Real<T>::t m = 0;
+        for (int b = 0; b < d1; ++b) m = mag_max(m, row1[b]);
+        e1 = exponent_of(m);
+        ex_acc += e1 + (s.e1 ? s.e1[r] : 0);
+      }
+      auto row = [&](int a) {
+        const T* Ba = B + a * sa;
+        T acc = Sc<T>::zero();
+        if (c1 == -1) {
+#pragma unroll
+          for (int c = 0; c < CHI; ++c)
+            if (c < d2) acc = Sc<T>::fma(Ba[c * s2], ml[c], acc);
+        } else {
+          for (int b = 0; b < d1; ++b) {
+            T in = Sc<T>::zero();
+#pragma unroll
+            for (int c = 0; c < CHI; ++c)
+              if (c < d2) in = Sc<T>::fma(Ba[b * s1 + c * s2], ml[c], in);
+            const T x = row1 ? scale_pow2(row1[b], -e1) : M(c1, b);
+            acc = Sc<T>::fma(x, in, acc);
+          }
+        }
+        return acc;
+      };
+      typename Real<T>::t mx = 0;
+      if constexpr (REG) {
+        T mine[RL];
+#pragma unroll
+        for (int a = 0; a < RL; ++a) mine[a] = a * G + gl < chi_a ? row(a * G + gl) : Sc<T>::zero();
+#pragma unroll
+        for (int a = 0; a < CHI; ++a) {
+          cur[a] = G == 1 ? mine[a / G] : shfl_i(mine[a / G], (threadIdx.x & 31) - gl + a % G);
+          mx = mag_max(mx, cur[a]);
+        }
+        const int ex = exponent_of(mx);
+        if (ex) {
+          ex_acc += ex;
+#pragma unroll
+          for (int a = 0; a < CHI; ++a) cur[a] = scale_pow2(cur[a], -ex);
+        }
+        if (s.out >= 0) {
+          if (gl == 0)
+#pragma unroll
+            for (int a = 0; a < CHI; ++a)
+              if (a < chi_a) M(s.out, a) = cur[a];
+          if (G > 1) __syncwarp();
+        }
+      } else {
+        for (int a = 0; a < chi_a; ++a) {
+          const T x = row(a);
+          M(s.out, a) = x;
+          mx = mag_max(mx, x);
+        }
+        const int ex = exponent_of(mx);
+        ex_acc += ex;
+        if (ex)
+          for (int a = 0; a < chi_a; ++a) M(s.out, a) = scale_pow2(M(s.out, a), -ex);
+      }
+    }
+    if (gl == 0) sex[side * tp + t] = ex_acc;
+    __syncthreads();
+    if (side == 0 && gl == 0 && p < W.Pc) {
+      T v = Sc<T>::one();
+      int e = sex[t] + sex[tp + t];
+      for (int c = 0; c < W.ncomp; ++c) {
+        const WalkSide<T>&A = sd[2 * c], &B = sd[2 * c + 1];
+        const T* ra = nullptr;
+        const T* rb = nullptr;
+        if (A.tab) {
+          const int r = codes[A.at * tp + t];
+          ra = A.tab + (int64_t)r * A.chi;
+          e += A.exps ? A.exps[r] : 0;
+        }
+        if (B.tab) {
+          const int r = codes[B.at * tp + t];
+          rb = B.tab + (int64_t)r * B.chi;
+          e += B.exps ? B.exps[r] : 0;
+        }
+        T s = Sc<T>::zero();
+        if (B.chi == 0) {
+          s = ra ? ra[0] : M(A.at, 0);
+        } else {
+          typename Real<T>::t ma = 0, mb = 0;
+          if (ra)
+            for (int k = 0; k < A.chi; ++k) ma = mag_max(ma, ra[k]);
+          if (rb)
+            for (int k = 0; k < A.chi; ++k) mb = mag_max(mb, rb[k]);
+          const int ea = exponent_of(ma), eb = exponent_of(mb);
+          e += ea + eb;
+          for (int k = 0; k < A.chi; ++k) {
+            const T x = ra ? scale_pow2(ra[k], -ea) : M(A.at, k), y = rb ? scale_pow2(rb[k], -eb) : M(B.at, k);
+            s = Sc<T>::fma(x, y, s);
+          }
+        }
+        v = c == 0 ? s : v * s;
+      }
+      write_out<T>(W.out, W.kind, W.p0 + p, W.P, v, e);
+    }
+    __syncthreads();
+  }
+}
+
 // Rows of a table scaled to a largest entry in [1/2, 1), the exponents kept.
 template <class T>
 struct NormJob {
@@ -560,15 +1025,13 @@ struct NormJob {
   int* exps;
   int rows, chi;
 };
+// (8 lanes per row; per: rows in flight, r0: the caller's row of the first pass)
 template <class T>
-__global__ void k_norm_rows(const NormJob<T>* __restrict__ jobs) {
-  const NormJob<T> j = jobs[blockIdx.y];
-  // 8 lanes per row
+__device__ __forceinline__ void norm_run(const NormJob<T>& j, int r0, int per) {
   const int l = threadIdx.x & 7;
-  const int per = gridDim.x * (blockDim.x >> 3);
   const int n = (j.rows + per - 1) / per;
   for (int i = 0; i < n; ++i) {
-    const int r = i * per + (blockIdx.x * blockDim.x + threadIdx.x) / 8;
+    const int r = i * per + r0;
     const bool ok = r < j.rows;
     T* row = j.tab + (int64_t)(ok ? r : 0) * j.chi;
     typename Real<T>::t m = 0;
@@ -580,6 +1043,137 @@ __global__ void k_norm_rows(const NormJob<T>* __restrict__ jobs) {
     for (int k = l; k < j.chi; k += 8) row[k] = scale_pow2(row[k], -ex);
     if (l == 0) j.exps[r] += ex;
   }
+}
+template <class T>
+__global__ void k_norm_rows(const NormJob<T>* __restrict__ jobs) {
+  norm_run<T>(jobs[blockIdx.y], (blockIdx.x * blockDim.x + threadIdx.x) / 8, gridDim.x * (blockDim.x >> 3));
+}
+
+// The first levels of the tables, where a launch costs more than its work: one
+// block takes everything below one vertex in shared memory.  The tensors are
+// copied there in one go (read through strides, so none needs its axes
+// permuted), level follows level behind a block barrier, and only the top
+// table goes out.  Each level would be a launch otherwise, and from global
+// memory every one of them costs two or three L2 latencies (4 us, measured).
+// A side of the centre leaves with its rows scaled; if the rows' exponents lie
+// within +-range, the powers of two join the entries and *plain is set: the
+// centre then reads no exponent per point.
+struct HeadJob {
+  int A, Aexp;    // rows: element offset, exponents' offset (-1: zero)
+  int lda;        // row pitch
+  int B, gexp;    // tensor slices, their exponents' offset (-1: zero)
+  int out, oexp, ldo;
+  int K, N, rows, rpg;
+  int bg, n2, bn1, bn2, bk;  // B strides; column n = (n / n2, n % n2)
+  int level;
+};
+template <class T>
+struct HeadCopy {
+  const T* src;
+  int dst, n;
+};
+template <class T>
+struct HeadBlock {
+  T* tab;       // the top table in global memory
+  int* exps;
+  int copy0, copy1, job0, job1;
+  int top, topexp, ld, rows, chi;  // the top table in shared memory
+  int centre;   // a side of the centre: rows are scaled
+  int plain;    // index of its flag
+};
+template <class T, int KM>
+__device__ __forceinline__ void head_item(const HeadJob& j, T* sh, int* ex, int q, int n0) {
+  const int g = (int)((unsigned)q / (unsigned)j.rpg), ar = q - g * j.rpg;
+  const T* A = sh + j.A + ar * j.lda;
+  T a[KM];
+  typename Real<T>::t m = 0;
+#pragma unroll
+  for (int k = 0; k < KM; ++k) {
+    a[k] = k < j.K ? A[k] : Sc<T>::zero();
+    m = mag_max(m, a[k]);
+  }
+  const int e = exponent_of(m);
+  if (e)
+#pragma unroll
+    for (int k = 0; k < KM; ++k) a[k] = scale_pow2(a[k], -e);
+  T* o = sh + j.out + q * j.ldo + n0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int n = n0 + c;
+    if (n >= j.N) break;
+    const int n1 = j.n2 == j.N ? 0 : n / j.n2;
+    const T* B = sh + j.B + g * j.bg + n1 * j.bn1 + (n - n1 * j.n2) * j.bn2;
+    T s = Sc<T>::zero();
+#pragma unroll
+    for (int k = 0; k < KM; ++k)
+      if (k < j.K) s = Sc<T>::fma(a[k], B[k * j.bk], s);
+    o[c] = s;
+  }
+  if (n0 == 0) ex[j.oexp + q] = e + (j.Aexp >= 0 ? ex[j.Aexp + ar] : 0) + (j.gexp >= 0 ? ex[j.gexp + g] : 0);
+}
+template <class T, int KM>
+__global__ void __launch_bounds__(256) k_head(const HeadBlock<T>* __restrict__ blocks,
+                                              const HeadCopy<T>* __restrict__ copies,
+                                              const HeadJob* __restrict__ gjobs, int nelem, int nexp, int njobs,
+                                              int* __restrict__ plain, int range) {
+  extern __shared__ __align__(16) unsigned char head_sh[];
+  __shared__ int red[2];
+  T* sh = (T*)head_sh;
+  int* ex = (int*)(sh + nelem);
+  HeadJob* jobs = (HeadJob*)(ex + nexp);
+  const HeadBlock<T> h = blocks[blockIdx.x];
+  const int nj = h.job1 - h.job0;
+  const int lane = threadIdx.x & 31;
+  for (int i = h.copy0 + (threadIdx.x >> 5); i < h.copy1; i += blockDim.x >> 5) {
+    const HeadCopy<T> c = copies[i];
+    for (int k = lane; k < c.n * (int)(sizeof(T) / 4); k += 32)
+      copy_async4((int*)(sh + c.dst) + k, (const int*)c.src + k);
+  }
+  for (int i = threadIdx.x; i < nj * (int)(sizeof(HeadJob) / 4); i += blockDim.x)
+    copy_async4((int*)jobs + i, (const int*)(gjobs + h.job0) + i);
+  if (threadIdx.x == 0) red[0] = INT_MAX, red[1] = INT_MIN;
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  for (int i = 0; i < nj; ++i) {
+    const HeadJob& j = jobs[i];
+    if (i > 0 && j.level != jobs[i - 1].level) __syncthreads();
+    // rows fastest: a warp's lanes read one column of B and rows a pitch apart
+    const unsigned rows = j.rows, n = rows * ((j.N + 3) / 4);
+    for (unsigned it = threadIdx.x; it < n; it += blockDim.x) {
+      const unsigned c = it / rows;
+      head_item<T, KM>(j, sh, ex, (int)(it - c * rows), (int)c * 4);
+    }
+  }
+  __syncthreads();
+  int shift = 0;  // plain: the exponents go into the entries
+  if (h.centre) {
+    int lo = INT_MAX, hi = INT_MIN;  // of the rows that are not zero
+    for (int r = threadIdx.x; r < h.rows; r += blockDim.x) {
+      T* row = sh + h.top + r * h.ld;
+      typename Real<T>::t m = 0;
+      for (int k = 0; k < h.chi; ++k) m = mag_max(m, row[k]);
+      const int e = exponent_of(m);
+      if (e)
+        for (int k = 0; k < h.chi; ++k) row[k] = scale_pow2(row[k], -e);
+      const int t = ex[h.topexp + r] += e;
+      if (m != 0) lo = min(lo, t), hi = max(hi, t);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) {
+      atomicMin(&red[0], lo);
+      atomicMax(&red[1], hi);
+    }
+    __syncthreads();
+    shift = red[0] <= red[1] && red[1] <= range && red[0] >= -range;
+    if (threadIdx.x == 0) plain[h.plain] = shift;
+  }
+  for (int i = threadIdx.x; i < h.rows * h.chi; i += blockDim.x) {
+    const int r = i / h.chi;
+    const T v = sh[h.top + r * h.ld + (i - r * h.chi)];
+    h.tab[i] = shift ? scale_pow2(v, ex[h.topexp + r]) : v;
+  }
+  for (int r = threadIdx.x; r < h.rows; r += blockDim.x) h.exps[r] = shift ? 0 : ex[h.topexp + r];
 }
 
 }  // namespace tnfa
