@@ -51,6 +51,8 @@ struct EvalTreeOptions {
   double table_rows = 1;        // a message with at most this many combinations is a table
   double table_elems = 1e18;    // bound on the elements of one absorbed tensor
   bool absorb = true;
+  bool absorb_points = true;    // also into the tensors of vertices without a table
+  int table_kids = 1 << 30;     // a vertex with more kids has no table; with two, one is always absorbed
   bool balance = false;         // choose the centre by the costlier side, not the sum
   std::vector<char> tensor_ok;  // vertices the tensor-core kernel takes in the stored axis order
   double tensor_speed = 40.0;   // its rate over the CUDA cores' (measured: 46 for MIXED)
@@ -135,16 +137,20 @@ class EvalTreeBuilder {
     int nk = 0;
     for (int w : nb_[v]) nk += w != u;
     if (nk == 0) return 0.0;
-    const double n = below(v, u), rows = n <= o_.table_rows ? n : o_.points;
+    const bool tab = is_table(v, u);
+    const double rows = tab ? below(v, u) : o_.points;
     if (is_tensor(v, u)) return rows * W_[v] / o_.tensor_speed;
-    double best = rows * W_[v];
-    if (nk < 2 || !o_.absorb) return best;
+    const double direct = rows * W_[v];
+    double best = direct;
+    if (nk < 2 || !o_.absorb || (!tab && !o_.absorb_points)) return best;
+    if (tab && o_.table_kids < nk + 1) best = INFINITY;
     for (int w : nb_[v]) {
       if (w == u) continue;
+      if (!is_table(w, v)) continue;
       const double nw = below(w, v);
       if (nw > o_.table_rows) continue;
       const double groups = T_.site_dim[v] * nw, made = groups * W_[v];
-      if (made > o_.table_elems) continue;
+      if (made > o_.table_elems && best < INFINITY) continue;
       // a group's last tile is padded to a few rows
       const double c = made + (rows + 4.0 * groups) * W_[v] / bond(w, v);
       if (c < best) {
@@ -153,6 +159,17 @@ class EvalTreeBuilder {
       }
     }
     return best;
+  }
+  // The message v -> u has a row per digit combination (a leaf always does).
+  bool is_table(int v, int u) const {
+    int nk = 0;
+    for (int w : nb_[v]) nk += w != u;
+    if (nk == 0) return true;
+    if (below(v, u) > o_.table_rows || nk > o_.table_kids) return false;
+    if (o_.table_kids < (1 << 30))
+      for (int w : nb_[v])
+        if (w != u && !is_table(w, v)) return false;
+    return true;
   }
   bool is_tensor(int v, int u) const {
     return !o_.tensor_ok.empty() && o_.tensor_ok[v] && u == T_.parent[v];
@@ -185,7 +202,7 @@ class EvalTreeBuilder {
     e.leaf = e.kids.empty();
     e.tensor = !e.leaf && is_tensor(v, u);
     const double n = below(v, u);
-    e.tabled = e.leaf || n <= o_.table_rows;
+    e.tabled = is_table(v, u);
     e.N = e.tabled ? (int64_t)n : 0;
     auto axis = [&](int w) {  // stored axis of the bond to w
       if (w == T_.parent[v]) return 1;

@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "eval_tree.cuh"
+#include "adjoint.cuh"
 #include "evaluate.cuh"
 #include "rows.cuh"
 
@@ -544,13 +545,6 @@ static std::vector<DigitRun> make_runs(const std::vector<DigitRef>& prog, const 
   return runs;
 }
 
-// Every vertex's site value as a code of its own.
-static std::vector<DigitRun> make_site_runs(const Topo& T, const std::vector<DigitRef>& prog) {
-  std::vector<int> slot(T.V), mult(T.V, 1);
-  for (int v = 0; v < T.V; ++v) slot[v] = v;
-  return make_runs(prog, slot, mult);
-}
-
 static size_t digitize_smem(int n, int block) { return (size_t)n * block * sizeof(int); }
 
 // Codes of Pc points into C[slot][ldC].
@@ -708,9 +702,9 @@ template <class T>
 class EvalEngine {
  public:
   EvalEngine(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const std::vector<DigitRef>& prog,
-             int ncols, int64_t P, bool use_tc, bool use_oz, size_t budget)
+             int ncols, int64_t P, bool use_tc, bool use_oz, size_t budget, bool adjoint = false)
       : ctx_(ctx), net_(net), tensors_(tensors), topo_(net->topo), prog_(prog), ncols_(ncols), P_(P),
-        use_tc_(use_tc), use_oz_(use_oz) {
+        use_tc_(use_tc), use_oz_(use_oz), adjoint_(adjoint) {
     const int V = topo_.V;
     EvalTreeOptions o;
     o.points = (double)P;
@@ -735,7 +729,11 @@ class EvalEngine {
     // Tables take at most half the scratch: the row bound shrinks until they
     // fit.  Every digit code stays within 31 bits.
     double rows = std::min((double)P, 134217728.0);
-    small_ = !use_tc && !use_oz && small_bonds(topo_, sizeof(T), P);
+    if (adjoint_) {  // every product of a table is a row product (see AdjointEngine)
+      o.table_kids = 2;
+      o.absorb_points = false;
+    }
+    small_ = !adjoint_ && !use_tc && !use_oz && small_bonds(topo_, sizeof(T), P);
     if (small_) {
       // Points that a thread walks cost one launch; a level of tables costs
       // another (about 3 us).  Up to about 20 us of walking there are no tables;
@@ -770,7 +768,6 @@ class EvalEngine {
 
   int chunk() const { return Pc_; }
   void set_chunk(int pc) { Pc_ = pc; }
-  size_t per_point() const { return per_point_; }
   // Bytes of scratch for chunks of pc points.
   size_t scratch(int64_t pc) {
     Carve c;
@@ -871,7 +868,7 @@ class EvalEngine {
     centre(X, n, out, kind, Pout, pofs);
   }
 
- private:
+ protected:
   struct Level {
     std::vector<RowJob<T>> rows;
     std::vector<int> verts;  // table vertices of the multi-child kernels
@@ -931,7 +928,7 @@ class EvalEngine {
     nslots_ = n;
     // all sides are tables: the centre kernel takes the digits itself, as long
     // as its shared memory holds them
-    fused_ = fused_allowed() && npp_ == 0 && n <= 16 && prog_.size() <= 256;
+    fused_ = !adjoint_ && fused_allowed() && npp_ == 0 && n <= 16 && prog_.size() <= 256;
     runs_ = make_runs(prog_, slot_, mult_);
     walk_ = small_ && npp_ > 0 && plan_walk();
     ncodes_ = fused_ || walk_ ? 0 : n;
@@ -954,7 +951,7 @@ class EvalEngine {
       free_slots.pop_back();
       msg_chi_ = std::max(msg_chi_, e.chi);
       for (int w : e.kids)
-        if (!tree_.v[w].tabled) free_slots.push_back(msg_[w]);
+        if (!tree_.v[w].tabled && !adjoint_) free_slots.push_back(msg_[w]);
     }
     max_group_ = 1;
     for (int v = 0; v < V; ++v)
@@ -1045,7 +1042,7 @@ class EvalEngine {
       const EvalVertex& e = tree_.v[v];
       for (int w : e.kids) reader[w] = v;
       bytes[v] = topo_.size(v) * (int64_t)sizeof(T);
-      if (e.leaf || !e.tabled || !row_form(v)) continue;
+      if (adjoint_ || e.leaf || !e.tabled || !row_form(v)) continue;
       bool ok = e.kids.size() <= 2;
       for (int w : e.kids) {
         ok &= tree_.v[w].leaf || head_[w];
@@ -1139,7 +1136,7 @@ class EvalEngine {
     int nmove = 0, nnorm = 0;
     for (int v = 0; v < V; ++v) nmove += needs_move(v);
     for (const auto& cc : tree_.comps)
-      for (int v : {cc.a, cc.b}) nnorm += !walk_ && v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf && !head_[v];
+      for (int v : {cc.a, cc.b}) nnorm += !walk_ && !adjoint_ && v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf && !head_[v];
     dmoves_ = c.take<MoveJob>(nmove);
     dnorms_ = c.take<NormJob<T>>(nnorm);
     dcentre_ = c.take<CentreJob<T>>(tree_.comps.size());
@@ -1165,9 +1162,11 @@ class EvalEngine {
     tabe_.assign(V, nullptr);
     abs_.assign(V, nullptr);
     abse_.assign(V, nullptr);
+    rex_.assign(V, nullptr);
     for (int v = 0; v < V; ++v) {
       const EvalVertex& e = tree_.v[v];
       ten_[v] = needs_move(v) ? c.take<T>(topo_.size(v)) : const_cast<T*>(tensors_ + topo_.off[v]);
+      if (adjoint_ && e.tabled) rex_[v] = c.take<int>(e.N);
       if (e.leaf) {
         tab_[v] = ten_[v];
       } else if (e.tabled) {
@@ -1234,7 +1233,7 @@ class EvalEngine {
       if (c.b >= 0) j.b = side(c.b);
       cj.push_back(j);
       for (int v : {c.a, c.b})
-        if (!walk_ && v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf && !head_[v])
+        if (!walk_ && !adjoint_ && v >= 0 && tree_.v[v].tabled && !tree_.v[v].leaf && !head_[v])
           norms_.push_back({tab_[v], tabe_[v], (int)tree_.v[v].N, tree_.v[v].chi});
     }
     put(dcentre_, cj.data(), cj.size() * sizeof(CentreJob<T>));
@@ -1428,6 +1427,7 @@ class EvalEngine {
     j.B = ten_[v];
     j.out = abs_[v];
     j.out_exp = abse_[v];
+    j.rex = rex_[w];
     j.K = k.chi;
     j.N = (int)(e.W / k.chi);
     j.rpg = (int)k.N;
@@ -1447,6 +1447,7 @@ class EvalEngine {
     j.gexp = e.absorb ? abse_[v] : nullptr;
     j.out = tab_[v];
     j.out_exp = tabe_[v];
+    j.rex = rex_[w];
     j.K = k.chi;
     j.N = e.chi;
     j.rpg = (int)k.N;
@@ -1829,7 +1830,7 @@ class EvalEngine {
   const std::vector<DigitRef>& prog_;
   int ncols_;
   int64_t P_;
-  bool use_tc_, use_oz_;
+  bool use_tc_, use_oz_, adjoint_;
   EvalTree tree_;
   std::vector<int> ttile_;  // tile rows that the group table of a table vertex was made for
   std::vector<int> slot_, mult_, key_slot_, row_slot_, msg_, lvl_, lvl_m_;
@@ -1864,7 +1865,7 @@ class EvalEngine {
   MoveJob* dmoves_ = nullptr;
   NormJob<T>* dnorms_ = nullptr;
   CentreJob<T>* dcentre_ = nullptr;
-  std::vector<int*> tmeta_, tabe_, abse_;
+  std::vector<int*> tmeta_, tabe_, abse_, rex_;
   std::vector<T*> ten_, tab_, abs_;
   int *codes_ = nullptr, *perm_ = nullptr, *meta_ = nullptr, *mexp_ = nullptr;
   T* mval_ = nullptr;
@@ -2283,31 +2284,8 @@ extern "C" int tnfa_eval_plan_destroy(tnfa_eval_plan* plan) {
 }
 
 // ----------------------------------------------- vector-Jacobian product ----
-// d/dT of sum_p dout_p f(x_p).  For vertex v with outside message E_v (the
-// contraction of everything but v's subtree, as a vector over v's parent
-// bond) and inside messages m_c of its children,
-//   dT_v[s][a][c1..ck] += sum_{p: s_v(p) = s} dout_p E_v[p][a] prod_j m_cj[p][c_j].
-// Inside messages come from the forward contraction (kept for every vertex);
-// E of a child is the same contraction with that child's bond as the output
-// (the vertex tensor with the child's axis moved first, E_v as one more input);
-// the accumulation treats E_v as one more Kronecker factor and reduces over
-// the points of each digit group (split over point tiles, atomics per tile).
-#include "linalg.cuh"
-
 namespace tnfa {
 namespace {
-
-template <class T>
-__device__ inline void atomic_add_T(T* a, T v);
-template <>
-__device__ inline void atomic_add_T<double>(double* a, double v) { atomicAdd(a, v); }
-template <>
-__device__ inline void atomic_add_T<float>(float* a, float v) { atomicAdd(a, v); }
-template <>
-__device__ inline void atomic_add_T<cplx>(cplx* a, cplx v) {
-  atomicAdd(&a->re, v.re);
-  atomicAdd(&a->im, v.im);
-}
 
 // dT_v[g][k] += sum over the points p of site value g of scale_p * prod_c m_c[p][k_c]
 // (k decoded as the mixed-radix tuple of the child entries, last child
@@ -2400,88 +2378,451 @@ __global__ void __launch_bounds__(256) k_grad_acc(const VertexJob<T> j, T* __res
 }
 
 template <class T>
-__global__ void k_vjp_seed(const double* __restrict__ dout, const T* __restrict__ rootv,
-                           const int* __restrict__ roote, int nroots, int r, int Pc, T* __restrict__ E,
-                           int* __restrict__ Eexp) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < Pc; p += gridDim.x * blockDim.x) {
-    T v = Sc<T>::one();
-    if constexpr (sizeof(T) == 16)
-      v = T{dout[p], 0.0};
-    else
-      v = (T)dout[p];
-    int e = 0;
-    for (int q = 0; q < nroots; ++q) {
-      if (q == r) continue;
-      v = v * rootv[(int64_t)q * Pc + p];
-      e += roote[(int64_t)q * Pc + p];
-    }
-    E[p] = v;
-    Eexp[p] = e;
-  }
+size_t grad_acc_smem(int sumdim, int tp) {
+  return (size_t)sumdim * tp * sizeof(T) + tp * sizeof(T) + 2 * tp * sizeof(int);
 }
 
-// Group the points of a chunk by the site value of vertex v (fills the job's
-// group fields; tp = tile rows of the kernel that will consume them).
-template <class T>
-void group_by_site(tnfa_ctx* ctx, VertexJob<T>& j, const int* key, int Pc, int ng, int tp, int* meta,
-                   int* perm) {
-  j.ngroups = ng;
-  j.grp_off = meta;
-  j.grp_cnt = meta + ng;
-  j.tile_start = meta + 2 * ng;
-  j.perm = launch_group(ctx, ng > 1 ? key : nullptr, Pc, ng, tp, meta, perm);
+// dT += the job's sums (children: the outside message, then the kids).
+template <class T, int TP, int KQ>
+void launch_grad_acc(tnfa_ctx* ctx, const VertexJob<T>& j, int sumdim, int Pc, T* dT) {
+  const size_t sm = grad_acc_smem<T>(sumdim, TP);
+  auto kern = k_grad_acc<T, TP, KQ>;
+  if (sm > 48 * 1024)
+    TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  // one wave of resident CTAs, each over a run of consecutive tiles
+  int occ = 0;
+  TNFA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, sm));
+  const int ntiles = (int)((Pc + TP - 1) / TP + j.ngroups);
+  const int ky = (int)((j.K + 256 * KQ - 1) / (256 * KQ));
+  const int want = std::max(1, std::max(occ, 1) * ctx->sm_count / ky);
+  const int per = std::max(1, (ntiles + want - 1) / want);
+  dim3 grid((unsigned)((ntiles + per - 1) / per), (unsigned)ky);
+  KernelScope ks(ctx, "grad_acc", 2.0 * Pc * (double)j.K, 0.0);
+  kern<<<grid, 256, sm, ctx->stream>>>(j, dT, per);
+  TNFA_LAUNCH_CHECK();
 }
+
+// d/dT of sum_p dout_p f(x_p), on the table schedule of the evaluation.  With
+// the two rows A, B that meet at the centre for point p, the adjoint of a
+// table's row is the sum of dout_p times the other side's row over the points
+// that read it; from there the products that built the tables are run
+// backwards, once per table row instead of once per point.  A vertex without a
+// table has one adjoint row per point (E), the adjoint of its message: E of a
+// kid is the same contraction with that kid's bond as the output (the tensor
+// with the kid's axis moved first, E as one more input), and
+//   dT_v[s][a][c1..ck] += sum_{p: s_v(p) = s} E_v[p][a] prod_j m_cj[p][c_j]
+// (k_grad_acc).  All adjoints carry one common power of two per chunk, taken
+// from the largest weight, so that networks of tiny values do not lose their
+// FP32 gradients on the way.
+template <class T>
+class AdjointEngine : public EvalEngine<T> {
+  using Base = EvalEngine<T>;
+  using Base::abs_;
+  using Base::abse_;
+  using Base::codes_;
+  using Base::ctx_;
+  using Base::dcentre_;
+  using Base::druns_;
+  using Base::err_;
+  using Base::key_slot_;
+  using Base::ld_;
+  using Base::lvl_;
+  using Base::lvl_m_;
+  using Base::mexp_;
+  using Base::meta_;
+  using Base::msg_;
+  using Base::msg_chi_;
+  using Base::mval_;
+  using Base::ncodes_;
+  using Base::ncols_;
+  using Base::nmsg_;
+  using Base::Pc_;
+  using Base::perm_;
+  using Base::rex_;
+  using Base::row_slot_;
+  using Base::runs_;
+  using Base::tab_;
+  using Base::tabe_;
+  using Base::ten_;
+  using Base::topo_;
+  using Base::tree_;
+
+ public:
+  AdjointEngine(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const std::vector<DigitRef>& prog, int ncols,
+                int64_t P, size_t budget)
+      : Base(ctx, net, tensors, prog, ncols, P, false, false, budget, true) {
+    const int V = topo_.V;
+    has_e_.assign(V, 0);
+    for (int v = 0; v < V; ++v)
+      if (!tree_.v[v].tabled)
+        for (int w : tree_.v[v].kids) has_e_[w] = 1;
+    for (const EvalTree::Comp& c : tree_.comps) {
+      if (!tree_.v[c.a].tabled) has_e_[c.a] = 1;
+      if (c.b >= 0 && !tree_.v[c.b].tabled) has_e_[c.b] = 1;
+    }
+    const size_t fixed = this->scratch(0) + adjoint_scratch(0);
+    const size_t per = (this->scratch(1 << 12) + adjoint_scratch(1 << 12) - fixed) / (1 << 12) + 1;
+    const size_t left = budget > fixed ? budget - fixed : 0;
+    const int64_t pc = std::max<int64_t>(256, std::min<int64_t>((int64_t)(left / per) / 256 * 256, int64_t(1) << 30));
+    Pc_ = (int)std::min<int64_t>(P, pc);
+  }
+  size_t bytes() { return this->scratch(Pc_) + adjoint_scratch(Pc_); }
+  void bind_all(void* base, T* dT) {
+    const size_t own = (this->scratch(Pc_) + 255) / 256 * 256;
+    this->bind(base);
+    Carve c;
+    c.base = (unsigned char*)base + own;
+    lay_out_adjoint(c, Pc_);
+    fill_adjoint(dT);
+  }
+  void upload_all() {
+    this->upload();
+    h2d(ctx_, blob_, host_.data(), host_.size());
+    for (const auto& m : tmoves_) max_move_ = std::max(max_move_, m.n);
+    if (!tmoves_.empty()) {
+      k_move<T><<<dim3(grid_for(max_move_, 256, 1024), (unsigned)tmoves_.size()), 256, 0, ctx_->stream>>>(dtmoves_);
+      TNFA_LAUNCH_CHECK();
+    }
+  }
+
+  // Adds the gradient of the chunk's n points.
+  void chunk_gradient(const double* X, int n, const double* dout) {
+    cudaStream_t st = ctx_->stream;
+    if (ncodes_ > 0) launch_digitize(ctx_, X, ncols_, n, druns_, (int)runs_.size(), ncodes_, codes_, ld_, err_);
+    for (int v : tree_.order)
+      if (!tree_.v[v].tabled) this->contract_points(v, n);
+    TNFA_CUDA(cudaMemsetAsync(zero_, 0, zero_bytes_, st));
+    TNFA_CUDA(cudaMemsetAsync(S_, 0x80, sizeof(int), st));
+    const int nc = (int)tree_.comps.size();
+    const unsigned grid = grid_for(n, 256, ctx_->sm_count * 8);
+    {
+      KernelScope ks(ctx_, "adjoint", 0.0, 0.0);
+      k_adj_prep<T><<<grid, 256, 0, st>>>(dout, n, dcentre_, nc, wv_, we_, ld_, S_);
+      TNFA_LAUNCH_CHECK();
+    }
+    for (int c = 0; c < nc; ++c) {
+      const T* wv = wv_ + (int64_t)(nc + c) * ld_;
+      const int* we = we_ + (int64_t)(nc + c) * ld_;
+      const int a = tree_.comps[c].a, b = tree_.comps[c].b;
+      if (tree_.v[a].tabled || (b >= 0 && tree_.v[b].tabled)) {
+        KernelScope ks(ctx_, "adjoint", 0.0, 0.0);
+        k_adj_weight<T><<<grid, 256, 0, st>>>(wv, we, n, dcentre_, c, S_, w_);
+        TNFA_LAUNCH_CHECK();
+      }
+      for (int sd = 0; sd < (b >= 0 ? 2 : 1); ++sd) {
+        const int v = sd ? b : a, o = sd ? a : b;
+        CentreSide<T> other{};
+        if (o >= 0) other = this->side(o);
+        if (tree_.v[v].tabled) {
+          segsum(v, n, other.ptr, other.idx, w_, nullptr);
+        } else {
+          KernelScope ks(ctx_, "adjoint", 0.0, 0.0);
+          const int chi = tree_.v[v].chi;
+          k_adj_seed<T><<<grid_for((int64_t)n * chi, 256, ctx_->sm_count * 16), 256, 0, st>>>(
+              wv, we, n, other, chi, S_, ev_[v], ee_[v]);
+          TNFA_LAUNCH_CHECK();
+        }
+      }
+    }
+    for (size_t i = tree_.order.size(); i-- > 0;)
+      if (!tree_.v[tree_.order[i]].tabled) points_back(tree_.order[i], n);
+    for (size_t l = levels_.size(); l-- > 0;) {
+      const BackLevel& L = levels_[l];
+      if (L.jobs.empty()) continue;
+      KernelScope ks(ctx_, "adjoint_rows", 0.0, 0.0);
+      k_rows_back<T><<<(unsigned)L.first.back(), 256, 0, st>>>(L.djobs, L.dfirst, (int)L.jobs.size());
+      TNFA_LAUNCH_CHECK();
+    }
+    k_adj_add<T><<<dim3(grid_for(max_add_, 256, 256), (unsigned)topo_.V), 256, 0, st>>>(dadds_, S_);
+    TNFA_LAUNCH_CHECK();
+  }
+
+ private:
+  struct BackLevel {
+    std::vector<BackJob<T>> jobs;
+    std::vector<int> first;
+    BackJob<T>* djobs = nullptr;
+    int* dfirst = nullptr;
+    int njobs = 0;
+  };
+
+  size_t adjoint_scratch(int64_t pc) {
+    Carve c;
+    lay_out_adjoint(c, pc);
+    return c.used + 512;
+  }
+
+  void lay_out_adjoint(Carve& c, int64_t pc) {
+    const int V = topo_.V;
+    // job tables
+    blob_ = (unsigned char*)c.take<MoveJob>(V);
+    dadds_ = (MoveJob*)blob_;
+    int nt = 0;
+    for (int v = 0; v < V; ++v)
+      if (!tree_.v[v].tabled) nt += (int)tree_.v[v].kids.size();
+    dtmoves_ = c.take<MoveJob>(nt);
+    int top = 0;
+    for (int v = 0; v < V; ++v)
+      if (!tree_.v[v].leaf) top = std::max({top, lvl_m_[v], lvl_[v]});
+    levels_.assign(top + 1, BackLevel{});
+    for (int v : tree_.order) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.leaf || !e.tabled) continue;
+      levels_[lvl_[v]].njobs += 1;
+      if (e.absorb) levels_[lvl_m_[v]].njobs += 1;
+    }
+    for (auto& L : levels_) {
+      L.djobs = c.take<BackJob<T>>(L.njobs);
+      L.dfirst = c.take<int>(L.njobs + 1);
+    }
+    blob_bytes_ = c.used - (size_t)(blob_ - c.base);
+    // adjoints that start at zero
+    dten_.assign(V, nullptr);
+    bar_.assign(V, nullptr);
+    dabs_.assign(V, nullptr);
+    S_ = c.take<int>(1);
+    zero_ = c.take<unsigned char>(1);
+    for (int v = 0; v < V; ++v) {
+      const EvalVertex& e = tree_.v[v];
+      dten_[v] = c.take<T>(topo_.size(v));
+      if (e.leaf) bar_[v] = dten_[v];
+      else if (e.tabled) bar_[v] = c.take<T>((size_t)e.N * e.chi);
+      if (e.absorb)
+        dabs_[v] = c.take<T>((size_t)this->absorbed_rows(v) * (size_t)(e.W / tree_.v[e.kids.back()].chi));
+    }
+    zero_bytes_ = c.used - (size_t)(zero_ - c.base);
+    // tensors with a kid's axis first
+    tk_.assign(V, nullptr);
+    for (int v = 0; v < V; ++v)
+      if (!tree_.v[v].tabled)
+        for (int w : tree_.v[v].kids) tk_[w] = c.take<T>(topo_.size(v));
+    // per point
+    const size_t nc = tree_.comps.size();
+    wv_ = c.take<T>(2 * nc * pc);
+    we_ = c.take<int>(2 * nc * pc);
+    w_ = c.take<T>(pc);
+    sperm_ = c.take<int>(pc);
+    int64_t ng = 1;
+    for (int v = 0; v < V; ++v)
+      if (tree_.v[v].tabled && row_slot_[v] >= 0) ng = std::max(ng, tree_.v[v].N);
+    smeta_ = c.take<int>(group_meta_ints((int)ng));
+    ev_.assign(V, nullptr);
+    ee_.assign(V, nullptr);
+    for (int v = 0; v < V; ++v)
+      if (has_e_[v]) {
+        ev_[v] = c.take<T>((size_t)pc * tree_.v[v].chi);
+        ee_[v] = c.take<int>(pc);
+      }
+  }
+
+  BackJob<T> back_job(const RowJob<T>& f, int kid, const T* bar, T* dB) const {
+    BackJob<T> j{};
+    j.A = f.A;
+    j.rex = rex_[kid];
+    j.B = f.B;
+    j.bar = bar;
+    j.dB = dB;
+    j.dA = bar_[kid];
+    j.K = f.K;
+    j.N = f.N;
+    j.rpg = f.rpg;
+    j.ng = f.rows / f.rpg;
+    const int nk = (j.K + BACK_T - 1) / BACK_T, nn = (j.N + BACK_T - 1) / BACK_T;
+    j.sb = std::max(1, std::min(256, j.rpg / 128));
+    j.sa = (int)std::max<int64_t>(1, std::min<int64_t>(256, (int64_t)j.ng * j.N / 256));
+    j.nb = nk * nn * j.ng * j.sb;
+    return j;
+  }
+  static int64_t back_blocks(const BackJob<T>& j) {
+    return (int64_t)j.nb + (int64_t)((j.K + BACK_T - 1) / BACK_T) * ((j.rpg + BACK_T - 1) / BACK_T) * j.sa;
+  }
+
+  void fill_adjoint(T* dT) {
+    host_.assign(blob_bytes_, 0);
+    auto put = [&](const void* dev, const void* src, size_t n) {
+      if (n) std::memcpy(host_.data() + ((const unsigned char*)dev - blob_), src, n);
+    };
+    std::vector<MoveJob> adds;
+    tmoves_.clear();
+    max_add_ = max_move_ = 1;
+    for (int v = 0; v < topo_.V; ++v) {
+      MoveJob m = this->move_job(v);
+      m.src = dT + topo_.off[v];
+      m.dst = dten_[v];
+      adds.push_back(m);
+      max_add_ = std::max(max_add_, m.n);
+      const EvalVertex& e = tree_.v[v];
+      if (e.tabled) continue;
+      for (size_t i = 0; i < e.kids.size(); ++i) {  // sites, kid, up, the other kids
+        MoveJob t = this->move_job(v);
+        t.dst = tk_[e.kids[i]];
+        const int nk = (int)e.kids.size(), at = t.nd - nk + (int)i, up = t.nd - nk - 1;
+        const int dim = t.dim[at];
+        const int64_t str = t.str[at];
+        for (int d = at; d > up; --d) {
+          t.dim[d] = t.dim[d - 1];
+          t.str[d] = t.str[d - 1];
+        }
+        t.dim[up] = dim;
+        t.str[up] = str;
+        tmoves_.push_back(t);
+      }
+    }
+    put(dadds_, adds.data(), adds.size() * sizeof(MoveJob));
+    put(dtmoves_, tmoves_.data(), tmoves_.size() * sizeof(MoveJob));
+    for (int v : tree_.order) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.leaf || !e.tabled) continue;
+      levels_[lvl_[v]].jobs.push_back(
+          back_job(this->table_job(v), e.kids[0], bar_[v], e.absorb ? dabs_[v] : dten_[v]));
+      if (e.absorb) levels_[lvl_m_[v]].jobs.push_back(back_job(this->absorb_job(v), e.kids.back(), dabs_[v], dten_[v]));
+    }
+    for (auto& L : levels_) {
+      L.first.assign(1, 0);
+      int64_t b = 0;
+      for (const auto& j : L.jobs) {
+        b += back_blocks(j);
+        TNFA_CHECK(b < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "gradient block too large");
+        L.first.push_back((int)b);
+      }
+      put(L.djobs, L.jobs.data(), L.jobs.size() * sizeof(BackJob<T>));
+      put(L.dfirst, L.first.data(), L.first.size() * sizeof(int));
+    }
+  }
+
+  // bar[row] += point adjoints (weight w, or E's own exponents) of the table of v.
+  void segsum(int v, int n, const T* src, const RowIdx& sidx, const T* w, const int* we) {
+    const EvalVertex& e = tree_.v[v];
+    const int ng = (int)e.N;
+    const int* key = codes_ + (int64_t)row_slot_[v] * ld_;
+    const int* perm = launch_group(ctx_, ng > 1 ? key : nullptr, n, ng, SEG_TILE, smeta_, sperm_);
+    KernelScope ks(ctx_, "adjoint_sum", 2.0 * n * e.chi, (double)n * e.chi * sizeof(T));
+    const int64_t tiles = (n + SEG_TILE - 1) / SEG_TILE + ng;
+    k_segsum<T><<<(unsigned)((tiles + 7) / 8), 256, 0, ctx_->stream>>>(
+        src, sidx, e.chi, w, we, w ? nullptr : tabe_[v], perm, smeta_, smeta_ + ng, smeta_ + 2 * ng, ng, bar_[v]);
+    TNFA_LAUNCH_CHECK();
+  }
+
+  ChildSrc<T> kid_src(int w) const {
+    ChildSrc<T> s{};
+    s.dim = tree_.v[w].chi;
+    if (tree_.v[w].tabled) {
+      s.ptr = tab_[w];
+      s.exps = tabe_[w];
+      s.idx.codes = codes_ + (int64_t)row_slot_[w] * ld_;
+    } else {
+      s.ptr = mval_ + (int64_t)msg_[w] * ld_ * msg_chi_;
+      s.exps = mexp_ + (int64_t)msg_[w] * ld_;
+    }
+    return s;
+  }
+
+  // From E of v: E of its kids, the gradient of its tensor, and the rows of
+  // the kids' tables.
+  void points_back(int v, int n) {
+    const EvalVertex& e = tree_.v[v];
+    const int ng = topo_.site_dim[v];
+    const int* key = key_slot_[v] >= 0 ? codes_ + (int64_t)key_slot_[v] * ld_ : nullptr;
+    ChildSrc<T> E{};
+    E.ptr = ev_[v];
+    E.exps = ee_[v];
+    E.dim = e.chi;
+    bool grouped = false;
+    const int* perm = nullptr;
+    auto group = [&](VertexJob<T>& j, int tp) {
+      if (!grouped) perm = launch_group(ctx_, key, n, ng, tp, meta_, perm_);
+      else launch_retile(ctx_, key != nullptr, n, ng, tp, meta_);
+      grouped = true;
+      j.perm = perm;
+      j.ngroups = ng;
+      j.grp_off = meta_;
+      j.grp_cnt = meta_ + ng;
+      j.tile_start = meta_ + 2 * ng;
+      j.site_dim = ng;
+      j.Pc = n;
+    };
+    for (int w : e.kids) {
+      VertexJob<T> j{};
+      j.ch[j.nchild++] = E;
+      int64_t K = e.chi;
+      int sumdim = e.chi;
+      for (int o : e.kids)
+        if (o != w) {
+          TNFA_CHECK(j.nchild < EVAL_MAXC, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
+          j.ch[j.nchild++] = kid_src(o);
+          K *= tree_.v[o].chi;
+          sumdim += tree_.v[o].chi;
+        }
+      j.K = (int)K;
+      j.chi_a = tree_.v[w].chi;
+      j.B = tk_[w];
+      j.out = ev_[w];
+      j.out_exp = ee_[w];
+      group(j, contract_tile_rows(j.chi_a, sumdim, sizeof(T)));
+      launch_contract<T>(ctx_, j, n);
+    }
+    VertexJob<T> j{};
+    j.ch[j.nchild++] = E;
+    int64_t K = e.chi;
+    int sumdim = e.chi;
+    for (int w : e.kids) {
+      TNFA_CHECK(j.nchild < EVAL_MAXC, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
+      j.ch[j.nchild++] = kid_src(w);
+      K *= tree_.v[w].chi;
+      sumdim += tree_.v[w].chi;
+    }
+    j.K = (int)K;
+    j.chi_a = 1;
+    constexpr int TP = 64, KQ = 4;
+    group(j, TP);
+    launch_grad_acc<T, TP, KQ>(ctx_, j, sumdim, n, dten_[v]);
+    for (int w : e.kids)
+      if (tree_.v[w].tabled) segsum(w, n, ev_[w], RowIdx{}, nullptr, ee_[w]);
+  }
+
+  std::vector<char> has_e_;
+  std::vector<BackLevel> levels_;
+  std::vector<unsigned char> host_;
+  std::vector<MoveJob> tmoves_;
+  int64_t max_add_ = 1, max_move_ = 1;
+  size_t blob_bytes_ = 0, zero_bytes_ = 0;
+  unsigned char *blob_ = nullptr, *zero_ = nullptr;
+  MoveJob *dadds_ = nullptr, *dtmoves_ = nullptr;
+  std::vector<T*> dten_, bar_, dabs_, tk_, ev_;
+  std::vector<int*> ee_;
+  T *wv_ = nullptr, *w_ = nullptr;
+  int *we_ = nullptr, *S_ = nullptr, *sperm_ = nullptr, *smeta_ = nullptr;
+};
 
 template <class T>
 void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double* X, int64_t P,
               int ncols, const std::vector<DigitRef>& prog, int xmem, const double* dout,
               int dout_mem, T* dT) {
   const Topo& Tp = net->topo;
-  const int V = Tp.V;
-  EvalPlan plan = make_plan(Tp);
-  const int nroots = (int)plan.roots.size();
-  std::vector<int> root_index(V, -1);
-  for (int r = 0; r < nroots; ++r) root_index[plan.roots[r]] = r;
-  size_t per_point = V * 4 + 4 + (xmem == TNFA_MEM_HOST ? ncols * 8 : 0) +
-                     (dout_mem == TNFA_MEM_HOST ? 8 : 0) + nroots * (sizeof(T) + 4);
-  for (int v = 0; v < V; ++v) per_point += 2 * ((size_t)Tp.link[v] * sizeof(T) + 4);
-  int64_t Pc_max = (int64_t)(ctx->eval_budget / per_point);
-  Pc_max = std::max<int64_t>(256, std::min<int64_t>(Pc_max, int64_t(1) << 30));
-  const int Pcap = (int)std::max<int64_t>(std::min<int64_t>(P, (Pc_max / 256) * 256), 1);
-  int maxsd = 1;
-  for (int v = 0; v < V; ++v) maxsd = std::max(maxsd, Tp.site_dim[v]);
-  const std::vector<DigitRun> runs = make_site_runs(Tp, prog);
-  DBuf dprog(ctx, std::max<size_t>(runs.size(), 1) * sizeof(DigitRun));
-  h2d(ctx, dprog.p, runs.data(), runs.size() * sizeof(DigitRun));
-  DBuf dS(ctx, (size_t)V * Pcap * 4), dperm(ctx, (size_t)Pcap * 4);
-  DBuf dmeta(ctx, group_meta_ints(maxsd) * 4), derr(ctx, 4);
-  TNFA_CUDA(cudaMemsetAsync(derr.p, 0, 4, ctx->stream));
-  std::vector<DBuf> in(V), ine(V), E(V), Ee(V);
-  for (int v = 0; v < V; ++v) {
-    if (!plan.fused_leaf[v]) {
-      in[v] = DBuf(ctx, (size_t)Pcap * Tp.link[v] * sizeof(T));
-      ine[v] = DBuf(ctx, (size_t)Pcap * 4);
+  // shapes the per-point kernels take (whether or not this call runs them)
+  for (int v = 0; v < Tp.V; ++v) {
+    TNFA_CHECK(Tp.children[v].size() < (size_t)EVAL_MAXC, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
+    int64_t K = Tp.link[v], sumdim = Tp.link[v];
+    for (int c : Tp.children[v]) {
+      K *= Tp.link[c];
+      sumdim += Tp.link[c];
     }
-    E[v] = DBuf(ctx, (size_t)Pcap * Tp.link[v] * sizeof(T));
-    Ee[v] = DBuf(ctx, (size_t)Pcap * 4);
+    TNFA_CHECK(K < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "gradient block too large");
+    TNFA_CHECK(grad_acc_smem<T>((int)sumdim, 64) <= 200 * 1024, TNFA_ERR_UNSUPPORTED,
+               "bonds too large for the gradient kernel");
   }
-  DBuf droot(ctx, (size_t)nroots * Pcap * sizeof(T)), droote(ctx, (size_t)nroots * Pcap * 4);
+  const size_t staged = (xmem == TNFA_MEM_HOST ? ncols * 8 : 0) + (dout_mem == TNFA_MEM_HOST ? 8 : 0);
+  AdjointEngine<T> E(ctx, net, tensors, prog, ncols, P, ctx->eval_budget);
+  int64_t Pcap = E.chunk();
+  if (staged) Pcap = std::min(Pcap, std::max<int64_t>(256, (int64_t)(ctx->eval_budget / staged) / 256 * 256));
+  E.set_chunk((int)Pcap);
   DBuf dX(ctx, xmem == TNFA_MEM_HOST ? (size_t)Pcap * ncols * 8 : 0);
   DBuf ddout(ctx, dout_mem == TNFA_MEM_HOST ? (size_t)Pcap * 8 : 0);
-  int* meta = dmeta.as<int>();
-  auto inside_src = [&](int c) {
-    ChildSrc<T> s{};
-    s.dim = Tp.link[c];
-    if (plan.fused_leaf[c]) {
-      s.ptr = tensors + Tp.off[c];
-      s.exps = nullptr;
-      s.idx.codes = dS.as<int>() + (int64_t)c * Pcap;
-    } else {
-      s.ptr = in[c].as<T>();
-      s.exps = ine[c].as<int>();
-    }
-    return s;
-  };
+  DBuf arena(ctx, E.bytes() + 512);
+  E.bind_all(arena.p, dT);
+  E.upload_all();
+  E.clear_error();
+  E.tables();
   for (int64_t p0 = 0; p0 < P; p0 += Pcap) {
     const int Pc = (int)std::min<int64_t>(Pcap, P - p0);
     const double* Xc = X + p0 * ncols;
@@ -2494,145 +2835,9 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
       TNFA_CUDA(cudaMemcpyAsync(ddout.p, dc, (size_t)Pc * 8, cudaMemcpyHostToDevice, ctx->stream));
       dc = ddout.as<double>();
     }
-    launch_digitize(ctx, Xc, ncols, Pc, dprog.as<DigitRun>(), (int)runs.size(), V, dS.as<int>(), Pcap,
-                    derr.as<int>());
-    // forward: inside messages of every non-leaf vertex
-    for (int v : plan.order) {
-      VertexJob<T> j{};
-      j.nchild = (int)Tp.children[v].size();
-      TNFA_CHECK(j.nchild <= EVAL_MAXC, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
-      int64_t K = 1;
-      int sumdim = 0;
-      for (int i = 0; i < j.nchild; ++i) {
-        j.ch[i] = inside_src(Tp.children[v][i]);
-        K *= j.ch[i].dim;
-        sumdim += j.ch[i].dim;
-      }
-      j.K = (int)K;
-      j.chi_a = Tp.link[v];
-      j.site_dim = Tp.site_dim[v];
-      j.B = tensors + Tp.off[v];
-      j.Pc = Pc;
-      if (Tp.parent[v] < 0) {
-        j.out = (T*)droot.p + (size_t)root_index[v] * Pcap;
-        j.out_exp = droote.as<int>() + (size_t)root_index[v] * Pcap;
-      } else {
-        j.out = in[v].as<T>();
-        j.out_exp = ine[v].as<int>();
-      }
-      group_by_site(ctx, j, dS.as<int>() + (int64_t)v * Pcap, Pc, j.site_dim,
-                    contract_tile_rows(j.chi_a, sumdim, sizeof(T)), meta, dperm.as<int>());
-      launch_contract<T>(ctx, j, Pc);
-    }
-    // seeds: E of a root = dout times the other roots' values
-    for (int r = 0; r < nroots; ++r)
-      k_vjp_seed<T><<<grid_for(Pc, 256, 4096), 256, 0, ctx->stream>>>(
-          dc, (const T*)droot.p, droote.as<int>(), nroots, r, Pcap, E[plan.roots[r]].as<T>(),
-          Ee[plan.roots[r]].as<int>());
-    TNFA_LAUNCH_CHECK();
-    // top-down: outside messages of every child
-    for (int v = 0; v < V; ++v) {
-      const auto& kids = Tp.children[v];
-      std::vector<int> shp{Tp.site_dim[v], Tp.link[v]};
-      for (int c : kids) shp.push_back(Tp.link[c]);
-      for (size_t jx = 0; jx < kids.size(); ++jx) {
-        const int c = kids[jx];
-        // T_v with child c's axis moved to position 1: [s][c][parent][others]
-        DBuf perm_t(ctx, (size_t)Tp.size(v) * sizeof(T));
-        la::PermJob pj{};
-        pj.src = tensors + Tp.off[v];
-        pj.dst = perm_t.p;
-        pj.nd = (int)shp.size();
-        TNFA_CHECK(pj.nd <= la::MAXD, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
-        std::vector<int> order;
-        order.push_back(0);
-        order.push_back(2 + (int)jx);
-        for (int a = 1; a < pj.nd; ++a)
-          if (a != 2 + (int)jx) order.push_back(a);
-        pj.n = Tp.size(v);
-        for (int a = 0; a < pj.nd; ++a) {
-          pj.shape[a] = shp[a];
-          pj.perm[a] = order[a];
-        }
-        la::permute<T>(ctx, {pj});
-        VertexJob<T> j{};
-        j.nchild = 0;
-        ChildSrc<T> e{};
-        e.ptr = E[v].as<T>();
-        e.exps = Ee[v].as<int>();
-        e.dim = Tp.link[v];
-        j.ch[j.nchild++] = e;
-        int64_t K = e.dim;
-        int sumdim = e.dim;
-        for (size_t q = 0; q < kids.size(); ++q) {
-          if (q == jx) continue;
-          TNFA_CHECK(j.nchild < EVAL_MAXC, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
-          j.ch[j.nchild++] = inside_src(kids[q]);
-          K *= Tp.link[kids[q]];
-          sumdim += Tp.link[kids[q]];
-        }
-        j.K = (int)K;
-        j.chi_a = Tp.link[c];
-        j.site_dim = Tp.site_dim[v];
-        j.B = perm_t.as<T>();
-        j.Pc = Pc;
-        j.out = E[c].as<T>();
-        j.out_exp = Ee[c].as<int>();
-        group_by_site(ctx, j, dS.as<int>() + (int64_t)v * Pcap, Pc, j.site_dim,
-                      contract_tile_rows(j.chi_a, sumdim, sizeof(T)), meta, dperm.as<int>());
-        launch_contract<T>(ctx, j, Pc);
-      }
-    }
-    // accumulation: dT_v[s][(a, c...)] += sum_p E_v[p][a] prod m_c[p][c]
-    for (int v = 0; v < V; ++v) {
-      VertexJob<T> j{};
-      ChildSrc<T> e{};
-      e.ptr = E[v].as<T>();
-      e.exps = Ee[v].as<int>();
-      e.dim = Tp.link[v];
-      j.ch[j.nchild++] = e;
-      int64_t K = e.dim;
-      int sumdim = e.dim;
-      for (int c : Tp.children[v]) {
-        TNFA_CHECK(j.nchild < EVAL_MAXC, TNFA_ERR_UNSUPPORTED, "vertex degree too high");
-        j.ch[j.nchild++] = inside_src(c);
-        K *= Tp.link[c];
-        sumdim += Tp.link[c];
-      }
-      TNFA_CHECK(K < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "gradient block too large");
-      j.K = (int)K;
-      j.chi_a = 1;
-      j.site_dim = Tp.site_dim[v];
-      j.Pc = Pc;
-      constexpr int TP = 64;
-      group_by_site(ctx, j, dS.as<int>() + (int64_t)v * Pcap, Pc, j.site_dim, TP, meta,
-                    dperm.as<int>());
-      const size_t sm = (size_t)sumdim * TP * sizeof(T) + TP * sizeof(T) + 2 * TP * sizeof(int);
-      TNFA_CHECK(sm <= 200 * 1024, TNFA_ERR_UNSUPPORTED, "bonds too large for the gradient kernel");
-      constexpr int KQ = 4;
-      auto kern = k_grad_acc<T, TP, KQ>;
-      if (sm > 48 * 1024)
-        TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-      // one wave of resident CTAs, each over a run of consecutive tiles
-      int occ = 0, nsm = 0, dev = 0;
-      TNFA_CUDA(cudaGetDevice(&dev));
-      TNFA_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-      TNFA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, sm));
-      const int ntiles = (int)((Pc + TP - 1) / TP + j.ngroups);
-      const int ky = (int)((K + 256 * KQ - 1) / (256 * KQ));
-      const int want = std::max(1, std::max(occ, 1) * nsm / ky);
-      const int per = std::max(1, (ntiles + want - 1) / want);
-      dim3 grid((unsigned)((ntiles + per - 1) / per), (unsigned)ky);
-      KernelScope ks(ctx, "grad_acc", 2.0 * Pc * (double)K, 0.0);
-      kern<<<grid, 256, sm, ctx->stream>>>(j, dT + Tp.off[v], per);
-      TNFA_LAUNCH_CHECK();
-    }
+    E.chunk_gradient(Xc, Pc, dc);
   }
-  int herr = 0;
-  TNFA_CUDA(cudaMemcpyAsync(&herr, derr.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
-  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
-  TNFA_CHECK(herr == 0, TNFA_ERR_DOMAIN,
-             "a coordinate is negative or not finite (the digit map needs x >= 0)");
+  check_eval_error(ctx, E.err_flag());
 }
 
 }  // namespace

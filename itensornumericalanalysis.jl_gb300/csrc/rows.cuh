@@ -270,6 +270,7 @@ struct RowJob {
   const int* gexp;  // exponent of B[g], null: zero
   T* out;
   int* out_exp;
+  int* rex;         // receives the scaling exponent of every row of A, null: not kept
   int K, N, rows;
   int rpg;  // > 0: uniform groups, and row(q) = q % rpg
   const int* perm;  // null: identity
@@ -408,6 +409,7 @@ __global__ void __launch_bounds__(256) k_rows_gemm(const __grid_constant__ RowPa
         if (n0 + lane * CN + c < j.N) o[lane * CN + c] = acc[i][c];
     }
   }
+  if (n0 == 0 && tid < nrows && j.rex) j.rex[arow[tid]] = rex[tid];
   if (n0 == 0 && tid < nrows)
     j.out_exp[item[tid]] = rex[tid] + (j.Aexp ? j.Aexp[arow[tid]] : 0) + (j.gexp ? j.gexp[g] : 0);
 }
@@ -443,7 +445,10 @@ __device__ __forceinline__ void small_row(const RowJob<T>& j, unsigned it, unsig
       if (k < j.K) s = Sc<T>::fma(a[k], B[c * j.K + k], s);
     o[c] = s;
   }
-  if (n0 == 0) j.out_exp[q] = ex;
+  if (n0 == 0) {
+    j.out_exp[q] = ex;
+    if (j.rex) j.rex[ar] = e;
+  }
 }
 template <class T, int KM>
 __global__ void __launch_bounds__(128) k_rows_small(const __grid_constant__ RowPack<T> pack) {
