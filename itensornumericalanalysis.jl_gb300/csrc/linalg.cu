@@ -112,11 +112,16 @@ __device__ inline double shfl_xor(double v, int o) { return __shfl_xor_sync(0xff
 __device__ inline cplx shfl_xor(cplx v, int o) {
   return {__shfl_xor_sync(0xffffffffu, v.re, o), __shfl_xor_sync(0xffffffffu, v.im, o)};
 }
+__device__ inline float shfl_idx(float v, int i) { return __shfl_sync(0xffffffffu, v, i); }
+__device__ inline double shfl_idx(double v, int i) { return __shfl_sync(0xffffffffu, v, i); }
 template <class T>
 __device__ inline T warp_sum(T v) {
   for (int o = 16; o; o >>= 1) v = v + shfl_xor(v, o);
   return v;
 }
+// s + |x|^2, one multiply-add per part
+__device__ inline double add_abs2(double s, double x) { return fma(x, x, s); }
+__device__ inline double add_abs2(double s, cplx x) { return fma(x.re, x.re, fma(x.im, x.im, s)); }
 // x / |x| (1 for x = 0)
 __device__ inline double phase(double x) { return x < 0 ? -1.0 : 1.0; }
 __device__ inline cplx phase(cplx x) {
@@ -130,6 +135,9 @@ __device__ inline dfl scal(dfl x, dfl a) { return x * a; }
 template <> __host__ __device__ inline dfl from_real<dfl>(double a) { return dfl(a); }
 __device__ inline dfl absval(dfl x) { return fabs(x); }
 __device__ inline dfl phase(dfl x) { return x.hi < 0.f ? dfl(-1) : dfl(1); }
+__device__ inline dfl shfl_idx(dfl v, int i) {
+  return {__shfl_sync(0xffffffffu, v.hi, i), __shfl_sync(0xffffffffu, v.lo, i)};
+}
 __device__ inline dfl shfl_xor(dfl v, int o) {
   return {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
 }
@@ -155,12 +163,23 @@ __global__ void k_permute(const PermJob* __restrict__ jobs) {
   T* dst = (T*)jb.dst;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < jb.n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = i, si = 0;
-    for (int a = jb.nd - 1; a >= 0; --a) {
-      const int sa = jb.perm[a];
-      const int64_t x = r % jb.shape[sa];
-      r /= jb.shape[sa];
-      si += x * sstride[sa];
+    int64_t si = 0;
+    if (jb.n < (int64_t(1) << 31)) {
+      unsigned r = (unsigned)i;
+      for (int a = jb.nd - 1; a >= 0; --a) {
+        const int sa = jb.perm[a];
+        const unsigned d = (unsigned)jb.shape[sa], q = r / d;
+        si += (int64_t)(r - q * d) * sstride[sa];
+        r = q;
+      }
+    } else {
+      int64_t r = i;
+      for (int a = jb.nd - 1; a >= 0; --a) {
+        const int sa = jb.perm[a];
+        const int64_t x = r % jb.shape[sa];
+        r /= jb.shape[sa];
+        si += x * sstride[sa];
+      }
     }
     dst[i] = src[si];
   }
@@ -190,59 +209,94 @@ __device__ inline T opget(const T* X, int ld, int op, int r, int c) {
   return op == 2 ? conj(v) : v;
 }
 
-template <class T>
-__global__ void __launch_bounds__(256) k_gemm(const GemmJob* __restrict__ jobs) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  const GemmJob& jb = jobs[blockIdx.z];
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  if (m0 >= jb.m || n0 >= jb.n) return;
-  __shared__ T As[BK][BM + 1];
-  __shared__ T Bs[BK][BN + 1];
+// Tile of BT x BT outputs by 256 threads, K in chunks of 16.  An SM executes 2
+// FP64 multiply-adds a clock, so a 64 x 64 tile takes 16 us a chunk on its one
+// SM whatever part of it is real: small tiles reach more SMs and pad less, and
+// their two shared-memory words per multiply-add are far below what shared
+// memory delivers.  16 x 16 while the batch has fewer than two tiles of 32 per
+// SM (a 42 x 84 x 42 product: 48 -> 5 us), else 32 x 32.
+template <class T, int BT>
+__global__ void __launch_bounds__(256) k_gemm(const GemmJob* __restrict__ jobs, const int* __restrict__ first,
+                                              int njobs) {
+  constexpr int BK = 16, RT = BT / 16;
+  int lo = 0, hi = njobs;  // first[lo] <= blockIdx.x < first[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (first[mid] <= (int)blockIdx.x) lo = mid;
+    else hi = mid;
+  }
+  const GemmJob jb = jobs[lo];
+  const int t = blockIdx.x - first[lo], nt = (jb.n + BT - 1) / BT;
+  const int m0 = t / nt * BT, n0 = t % nt * BT;
+  __shared__ T As[BK][BT + 1];
+  __shared__ T Bs[BK][BT + 1];
   const T* A = (const T*)jb.A;
   const T* B = (const T*)jb.B;
   T* C = (T*)jb.C;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  T acc[4][4];
+  T acc[RT][RT], pa[RT], pb[RT];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = from_real<T>(0.0);
-  for (int k0 = 0; k0 < jb.k; k0 += BK) {
-    for (int idx = threadIdx.x; idx < BM * BK; idx += 256) {
-      int r, kk;
-      if (jb.opA == 0) { r = idx / BK; kk = idx % BK; }   // contiguous along k
-      else { kk = idx / BM; r = idx % BM; }              // contiguous along m
-      const int gr = m0 + r, gk = k0 + kk;
-      As[kk][r] = (gr < jb.m && gk < jb.k) ? opget(A, jb.lda, jb.opA, gr, gk) : from_real<T>(0.0);
+    for (int j = 0; j < RT; ++j) acc[i][j] = from_real<T>(0.0);
+  // element i of a thread's share of a chunk, contiguous along the operand's rows
+  auto at_a = [&](int i, int& r, int& kk) {
+    const int x = threadIdx.x + 256 * i;
+    if (jb.opA == 0) r = x / BK, kk = x % BK;
+    else kk = x / BT, r = x % BT;
+  };
+  auto at_b = [&](int i, int& c, int& kk) {
+    const int x = threadIdx.x + 256 * i;
+    if (jb.opB == 0) kk = x / BT, c = x % BT;
+    else c = x / BK, kk = x % BK;
+  };
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+      int r, c, kk;
+      at_a(i, r, kk);
+      pa[i] = m0 + r < jb.m && k0 + kk < jb.k ? opget(A, jb.lda, jb.opA, m0 + r, k0 + kk) : from_real<T>(0.0);
+      at_b(i, c, kk);
+      pb[i] = n0 + c < jb.n && k0 + kk < jb.k ? opget(B, jb.ldb, jb.opB, k0 + kk, n0 + c) : from_real<T>(0.0);
     }
-    for (int idx = threadIdx.x; idx < BN * BK; idx += 256) {
-      int c, kk;
-      if (jb.opB == 0) { kk = idx / BN; c = idx % BN; }   // contiguous along n
-      else { c = idx / BK; kk = idx % BK; }              // contiguous along k
-      const int gc = n0 + c, gk = k0 + kk;
-      Bs[kk][c] = (gc < jb.n && gk < jb.k) ? opget(B, jb.ldb, jb.opB, gk, gc) : from_real<T>(0.0);
+  };
+  load(0);
+  // (a warp whose rows all lie outside only helps with the loads)
+  const bool mine = m0 + (ty & ~1) < jb.m;
+  for (int k0 = 0; k0 < jb.k; k0 += BK) {
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+      int r, c, kk;
+      at_a(i, r, kk);
+      As[kk][r] = pa[i];
+      at_b(i, c, kk);
+      Bs[kk][c] = pb[i];
     }
     __syncthreads();
+    if (k0 + BK < jb.k) load(k0 + BK);  // in flight behind the products
+    if (mine) {
+      const int kn = min(BK, jb.k - k0);
+#pragma unroll 4
+      for (int kk = 0; kk < kn; ++kk) {
+        T a[RT], b[RT];
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      T a[4], b[4];
+        for (int i = 0; i < RT; ++i) a[i] = As[kk][ty + 16 * i];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
+        for (int j = 0; j < RT; ++j) b[j] = Bs[kk][tx + 16 * j];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
+        for (int i = 0; i < RT; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = Sc<T>::fma(a[i], b[j], acc[i][j]);
+          for (int j = 0; j < RT; ++j) acc[i][j] = Sc<T>::fma(a[i], b[j], acc[i][j]);
+      }
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < RT; ++i) {
     const int r = m0 + ty + 16 * i;
     if (r >= jb.m) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < RT; ++j) {
       const int c = n0 + tx + 16 * j;
       if (c >= jb.n) continue;
       T v = scal(acc[i][j], jb.alpha);
@@ -254,19 +308,38 @@ __global__ void __launch_bounds__(256) k_gemm(const GemmJob* __restrict__ jobs) 
 
 template <class T>
 void gemm(tnfa_ctx* ctx, const std::vector<GemmJob>& jobs) {
-  if (jobs.empty()) return;
-  int mt = 1, nt = 1;
   double fl = 0;
+  std::vector<GemmJob> js;
   for (const auto& j : jobs) {
-    mt = std::max(mt, (j.m + 63) / 64);
-    nt = std::max(nt, (j.n + 63) / 64);
+    if (j.m <= 0 || j.n <= 0) continue;
+    js.push_back(j);
     fl += 2.0 * j.m * j.n * j.k;
   }
-  TNFA_CHECK(jobs.size() <= 65535 && mt <= 65535, TNFA_ERR_UNSUPPORTED, "gemm batch too large");
-  DBuf d = upload(ctx, jobs);
-  dim3 grid(nt, mt, (unsigned)jobs.size());
+  if (js.empty()) return;
+  auto tiles = [&](int bt) {
+    std::vector<int> f(1, 0);
+    int64_t n = 0;
+    for (const auto& j : js) {
+      n += (int64_t)((j.m + bt - 1) / bt) * ((j.n + bt - 1) / bt);
+      TNFA_CHECK(n < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "gemm batch too large");
+      f.push_back((int)n);
+    }
+    return f;
+  };
+  std::vector<int> first = tiles(32);
+  const bool fine = first.back() < 2 * ctx->sm_count;
+  if (fine) first = tiles(16);
+  // the jobs and their first tiles in one upload
+  const size_t nb = js.size() * sizeof(GemmJob);
+  std::vector<unsigned char> blob(nb + first.size() * sizeof(int));
+  std::memcpy(blob.data(), js.data(), nb);
+  std::memcpy(blob.data() + nb, first.data(), first.size() * sizeof(int));
+  DBuf d(ctx, blob.size());
+  h2d(ctx, d.p, blob.data(), blob.size());
+  const int* df = (const int*)(d.as<unsigned char>() + nb);
   KernelScope ks(ctx, sizeof(T) == 8 ? "gemm_f64" : "gemm_c128", fl, 0.0);
-  k_gemm<T><<<grid, 256, 0, ctx->stream>>>(d.as<GemmJob>());
+  if (fine) k_gemm<T, 16><<<(unsigned)first.back(), 256, 0, ctx->stream>>>(d.as<GemmJob>(), df, (int)js.size());
+  else k_gemm<T, 32><<<(unsigned)first.back(), 256, 0, ctx->stream>>>(d.as<GemmJob>(), df, (int)js.size());
   TNFA_LAUNCH_CHECK();
 }
 
@@ -722,24 +795,312 @@ __global__ void __launch_bounds__(512) k_qrcp(const QrJob* __restrict__ jobs, T*
   if (crank == 0 && threadIdx.x == 0) ranks[ji] = r_keep;
 }
 
+
+// --- the same factorisation with the columns in shared memory ---------------
+// k_qrcp keeps its columns in global memory: a step waits for two cluster
+// barriers and several L2 round trips, about 13 us for 0.3-3 us of FP64 work.
+// Here every CTA of the cluster holds its columns (and its columns of Q) in
+// shared memory.  A step has one cluster barrier: the CTAs post their best
+// column to each other's slots, then each copies the winner from its owner's
+// shared memory and builds the reflector itself (the winning column is never
+// written again).  The weight that decides the stop is summed in FP32, scaled
+// by the matrix norm: it is only compared with tol^2, and an FP64 addition
+// costs a warp 64 cycles.
+struct QrSlot {
+  double best;
+  int idx;
+  float sum;
+};
+constexpr int QRS_MAXM = 512;  // rows: one element of a column per thread
+
+struct QrSmem {
+  int pitch, nc, qc;
+  size_t q, x, nrm, v0, beta, bytes;
+};
+__host__ __device__ inline QrSmem qr_smem(int m, int n, int C, size_t ts) {
+  QrSmem L;
+  const int k = m < n ? m : n;
+  L.pitch = m | 1;
+  L.nc = (n + C - 1) / C;
+  L.qc = (k + C - 1) / C;
+  L.q = (size_t)L.nc * L.pitch * ts;
+  L.x = L.q + (size_t)L.qc * L.pitch * ts;
+  L.nrm = (L.x + 2 * (size_t)m * ts + 15) / 16 * 16;
+  L.v0 = (L.nrm + (size_t)L.nc * 8 + 15) / 16 * 16;
+  L.beta = L.v0 + (size_t)k * ts;
+  L.bytes = L.beta + (size_t)k * 8 + (size_t)k * 4;  // beta, then the pivots
+  return L;
+}
+
+// sqrt(x), and 1 / (sqrt(x) (sqrt(x) + |y|)), for a normal x > 0: FP32 starts
+// on the mantissas, third-order Newton for the root, two Newton steps for the
+// reciprocal (an FP64 division or root is some 20 operations on the slow pipe).
+__device__ __forceinline__ void root_and_beta(double x, double y, double& nrm, double& beta) {
+  const int e = (((int)(__double2hiint(x) >> 20) - 1023) & ~1);  // even: x = X 2^e, X in [1, 4)
+  const double X = x * __hiloint2double((1023 - e) << 20, 0);
+  double r = (double)rsqrtf((float)X);
+  const double f = fma(-X * r, r, 1.0);
+  r = fma(r * f, fma(f, 0.375, 0.5), r);
+  double s = X * r;
+  s = fma(0.5 * r, fma(-s, s, X), s);  // one correction of the root itself
+  const double half = __hiloint2double((1023 + e / 2) << 20, 0), inv = __hiloint2double((1023 - e / 2) << 20, 0);
+  nrm = s * half;
+  const double d = s + fabs(y) * inv;  // in [1, 4): |y| <= sqrt(x)
+  double q = (double)(1.0f / (float)d);
+  q = fma(q, fma(-d, q, 1.0), q);
+  q = fma(q, fma(-d, q, 1.0), q);
+  beta = r * q * inv * inv;
+}
+
+template <class T>
+__global__ void __launch_bounds__(512) k_qrcp_sm(const QrJob* __restrict__ jobs, double tol2, int* __restrict__ ranks) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), crank = (int)cl.block_rank();
+  const int ji = blockIdx.x / C;
+  const QrJob jb = jobs[ji];
+  const int m = jb.m, n = jb.n, kq = min(m, n);
+  extern __shared__ __align__(16) unsigned char qr_sh[];
+  __shared__ QrSlot slot[2][QR_CLUSTER];
+  __shared__ double tot[QR_CLUSTER];
+  __shared__ T red[32];
+  __shared__ int piv_now;
+  __shared__ double beta_now;
+  __shared__ T v0_now, alpha_now;
+  const QrSmem L = qr_smem(m, n, C, sizeof(T));
+  T* W = (T*)qr_sh;
+  T* Qc = (T*)(qr_sh + L.q);
+  T* xs = (T*)(qr_sh + L.x);
+  double* nrm = (double*)(qr_sh + L.nrm);
+  T* v0s = (T*)(qr_sh + L.v0);
+  double* betas = (double*)(qr_sh + L.beta);
+  int* piv = (int*)(betas + kq);
+  const T* A = (const T*)jb.A;
+  T* R = (T*)jb.R;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int nc = crank < n ? (n - crank + C - 1) / C : 0;  // own columns: crank + C k
+  for (int i = tid; i < m * nc; i += blockDim.x) {
+    const int r = i / nc, k = i - r * nc;
+    W[k * L.pitch + r] = A[(int64_t)r * n + crank + C * k];
+  }
+  for (int i = tid; i < kq * nc; i += blockDim.x) {
+    const int r = i / nc, k = i - r * nc;
+    R[(int64_t)r * n + crank + C * k] = from_real<T>(0.0);
+  }
+  __syncthreads();
+  for (int k = warp; k < nc; k += nw) {
+    double s = 0.0;
+    for (int r = lane; r < m; r += 32) s += abs2(W[k * L.pitch + r]);
+    s = warp_sum(s);
+    if (lane == 0) nrm[k] = s;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    double s = 0.0;
+    for (int k = lane; k < nc; k += 32) s += nrm[k];
+    s = warp_sum(s);
+    if (lane < C) *cl.map_shared_rank(&tot[crank], lane) = s;
+  }
+  cl.sync();
+  double total = 0.0;
+  for (int i = 0; i < C; ++i) total += tot[i];
+  // 2^-E total is in [1, 2) (left alone when zero or not finite)
+  const int te = (int)(__double2hiint(total) >> 20) & 0x7FF;
+  const double sc = te > 0 && te < 2046 ? __hiloint2double((2046 - te) << 20, 0) : 1.0;
+  const float thr = (float)(tol2 * (total * sc));
+  int r_keep = kq;
+  for (int j = 0; j < kq; ++j) {
+    if (warp == 0) {
+      long long best = -1;  // norms are >= 0: their bits order like the values
+      int bi = INT_MAX;
+      float sum = 0.f;
+      for (int k = lane; k < nc; k += 32) {
+        const double v = nrm[k];
+        const long long b = __double_as_longlong(v);
+        if (b < 0 || b > 0x7FF0000000000000ll) continue;  // pivoted (-1), NaN
+        sum += (float)(v * sc);
+        if (b > best) best = b, bi = crank + C * k;
+      }
+      for (int o = 16; o; o >>= 1) {
+        const long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (ob > best || (ob == best && oi < bi)) best = ob, bi = oi;
+      }
+      if (lane < C) *cl.map_shared_rank(&slot[j & 1][crank], lane) = QrSlot{__longlong_as_double(best), bi, sum};
+    }
+    cl.sync();
+    long long gbest = -1;
+    int p = INT_MAX;
+    float gsum = 0.f;
+    for (int i = 0; i < C; ++i) {
+      const QrSlot& o = slot[j & 1][i];
+      const long long ob = __double_as_longlong(o.best);
+      gsum += o.sum;
+      if (o.idx < n && (ob > gbest || (ob == gbest && o.idx < p))) gbest = ob, p = o.idx;
+    }
+    if (p >= n || (j > 0 && (gsum <= thr || gbest <= 0))) {
+      r_keep = j;  // 0 only when no column has a finite norm
+      break;
+    }
+    const T* rem = cl.map_shared_rank(W, p % C) + (p / C) * L.pitch;
+    for (int r = j + tid; r < m; r += blockDim.x) xs[r] = rem[r];
+    if (tid == 0) {
+      const T x0 = rem[j];
+      const double nrm2 = __longlong_as_double(gbest);
+      T v0 = x0, alpha = x0;
+      double beta = 0.0;
+      // (an almost eliminated column is not reflected: 2 / |v|^2 would overflow)
+      if (nrm2 > 1e-300) {
+        if constexpr (sizeof(T) == 8) {
+          double nv;
+          root_and_beta(nrm2, x0, nv, beta);
+          alpha = x0 < 0 ? nv : -nv;
+          v0 = x0 - alpha;
+        } else {
+          const double nv = sqrt(nrm2);
+          alpha = scal(phase(x0), -nv);
+          v0 = x0 - alpha;
+          const double vn2 = nrm2 - abs2(x0) + abs2(v0);
+          beta = vn2 > 0.0 ? 2.0 / vn2 : 0.0;
+        }
+      }
+      piv[j] = p;
+      betas[j] = beta;
+      v0s[j] = v0;
+      beta_now = beta;
+      v0_now = v0;
+      if (p % C == crank) {
+        R[(int64_t)j * n + p] = alpha;
+        nrm[p / C] = -1.0;
+      }
+    }
+    __syncthreads();
+    const double beta = beta_now;
+    const T v0 = v0_now;
+    for (int k = warp; k < nc; k += nw) {
+      if (__double_as_longlong(nrm[k]) < 0) continue;
+      T* y = W + k * L.pitch;
+      const T yj = y[j];
+      T bw = from_real<T>(0.0);
+      if (beta != 0.0) {
+        T w = lane == 0 ? Sc<T>::fma(conj(v0), yj, from_real<T>(0.0)) : from_real<T>(0.0);
+        for (int r = j + 1 + lane; r < m; r += 32) w = Sc<T>::fma(conj(xs[r]), y[r], w);
+        w = warp_sum(w);
+        bw = scal(w, beta);
+      }
+      double s = 0.0;
+      for (int r = j + 1 + lane; r < m; r += 32) {
+        const T v = Sc<T>::fma(scal(xs[r], -1.0), bw, y[r]);
+        y[r] = v;
+        s = add_abs2(s, v);
+      }
+      s = warp_sum(s);
+      if (lane == 0) {
+        nrm[k] = s;
+        R[(int64_t)j * n + crank + C * k] = yj - v0 * bw;
+      }
+    }
+    __syncthreads();
+  }
+  // Q = H_0 ... H_{r-1} [I; 0] (m x r): reflector after reflector, the next one
+  // on its way from its owner while this one is applied
+  const int nq = crank < r_keep ? (r_keep - crank + C - 1) / C : 0;
+  for (int i = tid; i < m * nq; i += blockDim.x) {
+    const int k = i / m, r = i - k * m;
+    Qc[k * L.pitch + r] = from_real<T>(r == crank + C * k ? 1.0 : 0.0);
+  }
+  __syncthreads();
+  auto reflector = [&](int j) {  // this thread's element
+    if (tid <= j || tid >= m) return from_real<T>(0.0);
+    const int p = piv[j];
+    return (cl.map_shared_rank(W, p % C) + (p / C) * L.pitch)[tid];
+  };
+  T nx = r_keep > 0 ? reflector(r_keep - 1) : from_real<T>(0.0);
+  for (int j = r_keep - 1; j >= 0; --j) {
+    T* x = xs + (j & 1) * m;
+    if (tid < m) x[tid] = tid == j ? v0s[j] : nx;
+    __syncthreads();
+    if (j > 0) nx = reflector(j - 1);
+    const double beta = betas[j];
+    if (beta == 0.0) continue;
+    for (int k = warp; k < nq; k += nw) {
+      if (crank + C * k < j) continue;
+      T* y = Qc + k * L.pitch;
+      T w = from_real<T>(0.0);
+      for (int r = j + lane; r < m; r += 32) w = Sc<T>::fma(conj(x[r]), y[r], w);
+      w = warp_sum(w);
+      const T bw = scal(w, -beta);
+      for (int r = j + lane; r < m; r += 32) y[r] = Sc<T>::fma(x[r], bw, y[r]);
+    }
+  }
+  __syncthreads();
+  T* Q = (T*)jb.Q;
+  for (int i = tid; i < m * nq; i += blockDim.x) {
+    const int r = i / nq, k = i - r * nq;
+    Q[(int64_t)r * r_keep + crank + C * k] = Qc[k * L.pitch + r];
+  }
+  if (crank == 0 && tid == 0) ranks[ji] = r_keep;
+  cl.sync();  // no CTA leaves while another reads its columns
+}
+
+template <class T>
+void launch_qrcp_sm(tnfa_ctx* ctx, const std::vector<QrJob>& js, int C, double tol, int* ranks) {
+  size_t sm = 0;
+  for (const auto& j : js) sm = std::max(sm, qr_smem(j.m, j.n, C, sizeof(T)).bytes);
+  DBuf d = upload(ctx, js);
+  TNFA_CUDA(cudaFuncSetAttribute(k_qrcp_sm<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(js.size() * C));
+  cfg.blockDim = dim3(512);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  TNFA_CUDA(cudaLaunchKernelEx(&cfg, k_qrcp_sm<T>, (const QrJob*)d.as<QrJob>(), tol * tol, ranks));
+  TNFA_LAUNCH_CHECK();
+}
+constexpr size_t QRS_SMEM = 200 * 1024;
+
 template <class T>
 void qr_rank(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, std::vector<int>& ranks) {
   ranks.assign(jobs.size(), 0);
   if (jobs.empty()) return;
-  std::vector<size_t> big, small;
+  std::vector<size_t> big, small, sm1, sm8;
   const bool few = jobs.size() * 8 <= (size_t)ctx->sm_count;
   for (size_t i = 0; i < jobs.size(); ++i) {
     const QrJob& j = jobs[i];
     TNFA_CHECK(std::min(j.m, j.n) <= QRCP_MAXK, TNFA_ERR_UNSUPPORTED,
                "rank-revealing QR handles at most 1024 reflectors");
-    (((double)j.m * j.n * std::min(j.m, j.n) >= 4.0e6 && std::min(j.m, j.n) >= 64) ||
-             (few && std::min(j.m, j.n) >= 32)
-         ? big
-         : small)
-        .push_back(i);
+    const bool spread = ((double)j.m * j.n * std::min(j.m, j.n) >= 4.0e6 && std::min(j.m, j.n) >= 64) ||
+                        (few && std::min(j.m, j.n) >= 32);
+    auto fits = [&](int C) { return j.m <= QRS_MAXM && qr_smem(j.m, j.n, C, sizeof(T)).bytes <= QRS_SMEM; };
+    // columns in shared memory: of one SM, or of a cluster's
+    if (!spread && fits(1)) sm1.push_back(i);
+    else if (fits(QR_CLUSTER)) sm8.push_back(i);
+    else (spread ? big : small).push_back(i);
   }
   // ranks of the cluster launch first, then of the single-CTA launch
   DBuf rk(ctx, jobs.size() * sizeof(int));
+  std::vector<size_t> order(big);
+  order.insert(order.end(), small.begin(), small.end());
+  for (const std::vector<size_t>* idx : {&sm8, &sm1}) {
+    if (idx->empty()) continue;
+    std::vector<QrJob> js;
+    double fl = 0;
+    for (size_t i : *idx) {
+      js.push_back(jobs[i]);
+      fl += 4.0 * jobs[i].m * jobs[i].n * std::min(jobs[i].m, jobs[i].n);
+    }
+    KernelScope ks(ctx, sizeof(T) == 8 ? "qr_rank_f64" : "qr_rank_c128", fl, 0.0);
+    if (trace_on()) ks.note = "shared " + size_note(js);
+    launch_qrcp_sm<T>(ctx, js, idx == &sm8 ? QR_CLUSTER : 1, tol, rk.as<int>() + order.size());
+    order.insert(order.end(), idx->begin(), idx->end());
+  }
   for (int pass = 0; pass < 2; ++pass) {
     const std::vector<size_t>& idx = pass == 0 ? big : small;
     if (idx.empty()) continue;
@@ -787,8 +1148,7 @@ void qr_rank(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, std::vec
   std::vector<int> h(jobs.size());
   TNFA_CUDA(cudaMemcpyAsync(h.data(), rk.p, jobs.size() * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
-  for (size_t i = 0; i < big.size(); ++i) ranks[big[i]] = h[i];
-  for (size_t i = 0; i < small.size(); ++i) ranks[small[i]] = h[big.size() + i];
+  for (size_t i = 0; i < order.size(); ++i) ranks[order[i]] = h[i];
   for (int r : ranks)
     TNFA_CHECK(r >= 1, TNFA_ERR_DOMAIN, "rank-revealing QR: no column with a finite norm (NaN or Inf input)");
   if (trace_on()) {
@@ -1065,6 +1425,316 @@ __global__ void __launch_bounds__(512) k_jacobi(const SvdJob* __restrict__ jobs,
   if (crank == 0 && threadIdx.x == 0 && jb.sweeps) *jb.sweeps = converged ? sweep : -1;
 }
 
+
+// --- one-sided Jacobi with the columns in shared memory ---------------------
+// The same iteration for a matrix (and V) that fits one SM's shared memory: a
+// round is then bound by its arithmetic and one block barrier, not by two L2
+// round trips (k_jacobi: about 8 us a round at 42 columns).  G lanes share a
+// column pair.  On the FP64 pipe (a warp instruction takes 64 cycles of its
+// scheduler) few lanes per pair waste the fewest instructions, the three dot
+// products are reduced together (each halving step hands half of the partial
+// sums to the partner: 6 additions instead of 15 for 32 lanes), and the angle
+// comes from FP32: only c^2 + s^2 = 1 has to hold to FP64, an angle off by
+// 1e-7 leaves 1e-7 of the off-diagonal for the next sweep.
+
+// 1 / sqrt(x) to FP64 for x in [1, 2]: FP32 root, one third-order Newton step
+// (y e (1/2 + 3/8 e), e = 1 - x y^2: the error term is e^3).
+__device__ __forceinline__ double rsqrt_1_2(double x) {
+  const double y = (double)rsqrtf((float)x);
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// Sums over G lanes of a, b and the parts of g.
+template <int G, class R>
+__device__ __forceinline__ void group_sum4(R& a, R& b, R& g, R& h, bool four) {
+  if constexpr (G < 4) {
+#pragma unroll
+    for (int o = G / 2; o; o >>= 1) {
+      a = a + shfl_xor(a, o);
+      b = b + shfl_xor(b, o);
+      g = g + shfl_xor(g, o);
+      h = h + shfl_xor(h, o);
+    }
+  } else {
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & (G / 2), bit = lane & (G / 4);
+    R x0 = hi ? g : a, x1 = hi ? h : b;
+    const R y0 = hi ? a : g, y1 = hi ? b : h;
+    x0 = x0 + shfl_xor(y0, G / 2);
+    x1 = x1 + shfl_xor(y1, G / 2);
+    R z = bit ? x1 : x0;
+    const R w = bit ? x0 : x1;
+    z = z + shfl_xor(w, G / 4);
+#pragma unroll
+    for (int o = G / 8; o; o >>= 1) z = z + shfl_xor(z, o);
+    const int base = lane & ~(G - 1);
+    a = shfl_idx(z, base);
+    b = shfl_idx(z, base + G / 4);
+    g = shfl_idx(z, base + G / 2);
+    if (four) h = shfl_idx(z, base + G / 2 + G / 4);
+  }
+}
+
+template <class T> struct Parts {  // real types
+  __device__ static T re(T x) { return x; }
+  __device__ static T im(T) { return T(0); }
+  __device__ static T make(T r, T) { return r; }
+};
+template <> struct Parts<cplx> {
+  __device__ static double re(cplx x) { return x.re; }
+  __device__ static double im(cplx x) { return x.im; }
+  __device__ static cplx make(double r, double i) { return {r, i}; }
+};
+
+struct JacobiSmem {
+  size_t u, v, sig, rank, bytes;  // byte offsets of a job's parts
+  int pu, pv;                     // column pitches
+};
+__host__ __device__ inline JacobiSmem jacobi_smem(int m, int n, bool v, size_t ts) {
+  JacobiSmem L;
+  L.pu = m | 1;
+  L.pv = n | 1;
+  L.u = 0;
+  L.v = (size_t)n * L.pu * ts;
+  L.sig = (L.v + (v ? (size_t)n * L.pv * ts : 0) + 15) / 16 * 16;
+  L.rank = L.sig + (size_t)n * 8;
+  L.bytes = L.rank + (size_t)n * 4;
+  return L;
+}
+
+template <class T, int G, int NE>
+__global__ void __launch_bounds__(sizeof(T) == 16 ? 512 : 1024) k_jacobi_sm(const SvdJob* __restrict__ jobs, int max_sweeps, JacobiOpts opt) {
+  using R = typename RealOf<T>::type;
+  extern __shared__ __align__(16) unsigned char jac_sh[];
+  __shared__ double red[32];
+  __shared__ int busy_sh[3];
+  const SvdJob jb = jobs[blockIdx.x];
+  const int m = jb.m, n = jb.n;
+  const bool want_v = jb.V != nullptr;
+  const JacobiSmem L = jacobi_smem(m, n, want_v, sizeof(T));
+  T* U = (T*)(jac_sh + L.u);
+  T* V = (T*)(jac_sh + L.v);
+  double* sig = (double*)(jac_sh + L.sig);
+  int* rank = (int*)(jac_sh + L.rank);
+  const T* A = (const T*)jb.A;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  double part = 0.0;
+  for (int i = tid; i < m * n; i += blockDim.x) {
+    const int r = i / n, c = i - r * n;
+    const T x = A[i];
+    U[c * L.pu + r] = x;
+    part += (double)abs2(x);
+  }
+  if (want_v)
+    for (int i = tid; i < n * n; i += blockDim.x) {
+      const int c = i / n, r = i - c * n;
+      V[c * L.pv + r] = from_real<T>(r == c ? 1.0 : 0.0);
+    }
+  if (tid < 3) busy_sh[tid] = 0;
+  const double fro2 = block_sum<double>(part, red);
+  const double negl = JacobiTraits<R>::negl * fro2;
+  const R tol = (R)(8.0 * sqrt((double)m) * JacobiTraits<R>::eps);
+  const R stop = (R)fmax((double)tol, opt.stop_rel);
+  const float tolf = (float)(double)tol, stopf = (float)(double)stop;
+  const double small = opt.small_rel * fro2 / n;
+  const int n2 = (n + 1) & ~1;
+  constexpr int PG = 32 / G;
+  const int gl = lane & (G - 1), sub = lane / G;
+  int sweep = 0;
+  bool converged = n < 2;
+  while (!converged && sweep < max_sweeps) {
+    if (tid == 0) busy_sh[(sweep + 1) % 3] = 0;
+    bool busy = false;
+    for (int r = 0; r < n2 - 1; ++r) {
+      for (int base = warp * PG; base < n2 / 2; base += nw * PG) {
+        const int slot = base + sub;
+        int p = r + slot, q = r - slot;
+        if (p >= n2 - 1) p -= n2 - 1;
+        if (q < 0) q += n2 - 1;
+        if (slot == 0) p = n2 - 1, q = r;
+        if (p > q) {
+          const int t = p;
+          p = q;
+          q = t;
+        }
+        const bool act = slot < n2 / 2 && q < n;
+        T* up = U + (act ? p : 0) * L.pu;
+        T* uq = U + (act ? q : 0) * L.pu;
+        R a = R(0), b = R(0);
+        T g = from_real<T>(0.0);
+        T xp[NE], xq[NE];
+#pragma unroll
+        for (int k = 0; k < NE; ++k) {
+          const int i = gl + G * k;
+          const bool in = act && i < m;
+          xp[k] = in ? up[i] : from_real<T>(0.0);
+          xq[k] = in ? uq[i] : from_real<T>(0.0);
+          if (G * k < m) {  // (uniform: a chunk beyond the columns costs nothing)
+            a += abs2(xp[k]);
+            b += abs2(xq[k]);
+            g = fmaT(conj(xp[k]), xq[k], g);
+          }
+        }
+        R gr = Parts<T>::re(g), gi = Parts<T>::im(g);
+        group_sum4<G, R>(a, b, gr, gi, sizeof(T) == 16);
+        if (!act) continue;
+        if ((double)a < negl || (double)b < negl) continue;
+        if ((double)a < small && (double)b < small) continue;
+        T se, sec;
+        R c;
+        if constexpr (std::is_same<T, double>::value) {
+          // FP32 on numbers scaled so that the larger column is about 1
+          const int e = max((int)((unsigned)__double2hiint(a) >> 20), (int)((unsigned)__double2hiint(b) >> 20)) - 1023;
+          const double sc = __hiloint2double((1023 - e) << 20, 0);
+          const float af = (float)(a * sc), bf = (float)(b * sc), gf = (float)(gr * sc);
+          const float agf = fabsf(gf), nab = sqrtf(af) * sqrtf(bf);
+          if (agf > stopf * nab) busy = true;
+          if (!(agf > tolf * nab)) continue;
+          const float zeta = (float)((b - a) * sc) / (2.f * agf);
+          const float az = fabsf(zeta);
+          float t = az > 1e18f ? 0.5f / az : 1.f / (az + sqrtf(1.f + zeta * zeta));
+          if (t == 0.f) continue;
+          if (zeta < 0.f) t = -t;
+          const double td = (double)t;
+          c = rsqrt_1_2(fma(td, td, 1.0));
+          const double sn = c * td;
+          se = sec = gf < 0.f ? -sn : sn;
+        } else if constexpr (std::is_same<T, float>::value) {
+          // squares instead of roots, and the hardware's reciprocal root: an
+          // FP32 pass hands its V on to be made orthonormal in FP64
+          const float ag = fabsf(gr), g2 = gr * gr, ab = a * b;
+          if (g2 > stopf * stopf * ab) busy = true;
+          if (!(g2 > tolf * tolf * ab)) continue;
+          const float zeta = __fdividef(b - a, 2.f * ag), az = fabsf(zeta), x = fmaf(zeta, zeta, 1.f);
+          float t = az > 1e9f ? __fdividef(0.5f, az) : __fdividef(1.f, az + x * rsqrtf(x));
+          if (!(t > 0.f)) continue;
+          if (zeta < 0.f) t = -t;
+          c = rsqrtf(fmaf(t, t, 1.f));
+          const float sn = c * t;
+          se = sec = gr < 0.f ? -sn : sn;
+        } else {
+          const T gg = Parts<T>::make(gr, gi);
+          const R ag = absval(gg);
+          const R nab = sqrt(a) * sqrt(b);
+          if (ag > stop * nab) busy = true;
+          if (ag <= tol * nab || ag == R(0)) continue;
+          const R zeta = (b - a) / (R(2) * ag);
+          const R big = (R)JacobiTraits<R>::big;
+          const R t = fabs(zeta) > big
+                          ? (R)0.5 / zeta
+                          : (zeta >= R(0) ? R(1) : R(-1)) / (fabs(zeta) + sqrt(R(1) + zeta * zeta));
+          if (t == R(0)) continue;
+          c = R(1) / sqrt(R(1) + t * t);
+          const R sn = c * t;
+          const T e = phase(gg);
+          se = scal(e, sn);
+          sec = scal(conj(e), sn);
+        }
+#pragma unroll
+        for (int k = 0; k < NE; ++k) {
+          const int i = gl + G * k;
+          if (i < m) {
+            up[i] = scal(xp[k], c) - sec * xq[k];
+            uq[i] = se * xp[k] + scal(xq[k], c);
+          }
+        }
+        if (want_v) {
+          T* vp = V + p * L.pv;
+          T* vq = V + q * L.pv;
+          for (int i = gl; i < n; i += G) {
+            const T x = vp[i], y = vq[i];
+            vp[i] = scal(x, c) - sec * y;
+            vq[i] = se * x + scal(y, c);
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (busy) busy_sh[sweep % 3] = 1;
+    __syncthreads();
+    converged = busy_sh[sweep % 3] == 0;
+    ++sweep;
+  }
+  // singular values, ranks (descending, stable), normalised outputs
+  for (int c = warp; c < n; c += nw) {
+    double s2 = 0.0;
+    for (int i = lane; i < m; i += 32) s2 += (double)abs2(U[c * L.pu + i]);
+    s2 = warp_sum(s2);
+    if (lane == 0) sig[c] = sqrt(s2);
+  }
+  __syncthreads();
+  for (int c = tid; c < n; c += blockDim.x) {
+    const double sc = sig[c];
+    int rk = 0;
+    for (int d = 0; d < n; ++d) rk += (sig[d] > sc) || (sig[d] == sc && d < c);
+    rank[c] = rk;
+    jb.S[rk] = sc;
+  }
+  __syncthreads();
+  T* Uo = (T*)jb.U;
+  for (int i = tid; i < m * n; i += blockDim.x) {
+    const int c = i / m, r = i - c * m;
+    const double sc = sig[c];
+    // a negligible column was never orthogonalised: it leaves U as zeros
+    Uo[(int64_t)r * n + rank[c]] =
+        sc * sc > negl && sc > 0 ? scal(U[c * L.pu + r], (R)(1.0 / sc)) : from_real<T>(0.0);
+  }
+  if (want_v) {
+    T* Vo = (T*)jb.V;
+    for (int i = tid; i < n * n; i += blockDim.x) {
+      const int c = i / n, r = i - c * n;
+      Vo[(int64_t)r * n + rank[c]] = V[c * L.pv + r];
+    }
+  }
+  if (tid == 0 && jb.sweeps) *jb.sweeps = converged ? sweep : -1;
+}
+
+constexpr size_t JACOBI_SMEM_MAX = 220 * 1024;
+constexpr int JACOBI_SMEM_M = 256;  // column elements that the lanes hold
+
+// One block per matrix in shared memory, if it fits -- unless it is a large
+// FP64 matrix in a batch that leaves most SMs idle: a round of more than about
+// 12000 FP64 cycles is shorter on the 8 SMs of a cluster, barrier included.
+template <class T>
+bool jacobi_fits(const SvdJob& j, size_t njobs, int sms) {
+  if (j.m > JACOBI_SMEM_M || jacobi_smem(j.m, j.n, j.V != nullptr, sizeof(T)).bytes > JACOBI_SMEM_MAX) return false;
+  const bool fp64 = std::is_same<T, double>::value || std::is_same<T, cplx>::value;
+  return !(fp64 && njobs * 8 <= (size_t)sms && 1.75 * j.n * j.m * (sizeof(T) / 8) * (sizeof(T) / 8) > 12000.0);
+}
+
+template <class T>
+void launch_jacobi_sm(tnfa_ctx* ctx, const std::vector<SvdJob>& js, int max_sweeps, JacobiOpts opt) {
+  size_t sm = 0;
+  int maxm = 1, pairs = 1;
+  for (const auto& j : js) {
+    sm = std::max(sm, jacobi_smem(j.m, j.n, j.V != nullptr, sizeof(T)).bytes);
+    maxm = std::max(maxm, j.m);
+    pairs = std::max(pairs, (j.n + 1) / 2);
+  }
+  DBuf d = upload(ctx, js);
+  auto go = [&](auto kern, int G) {
+    // as many warps as the pairs of a round fill evenly
+    constexpr int top = sizeof(T) == 16 ? 16 : 32;
+    const int need = (pairs * G + 31) / 32, passes = (need + top - 1) / top;
+    const int warps = std::max(4, std::min(top, (need + passes - 1) / passes));
+    TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)JACOBI_SMEM_MAX));
+    kern<<<(unsigned)js.size(), 32 * warps, sm, ctx->stream>>>(d.as<SvdJob>(), max_sweeps, opt);
+  };
+  if constexpr (std::is_same<T, double>::value) {
+    if (maxm <= 64) go(k_jacobi_sm<T, 8, 8>, 8);
+    else if (maxm <= 128) go(k_jacobi_sm<T, 16, 8>, 16);
+    else go(k_jacobi_sm<T, 32, 8>, 32);
+  } else if constexpr (std::is_same<T, cplx>::value) {
+    if (maxm <= 64) go(k_jacobi_sm<T, 16, 4>, 16);
+    else go(k_jacobi_sm<T, 32, 8>, 32);
+  } else {
+    if (maxm <= 64) go(k_jacobi_sm<T, 16, 4>, 16);
+    else go(k_jacobi_sm<T, 32, 8>, 32);
+  }
+  TNFA_LAUNCH_CHECK();
+}
+
 constexpr int SVD_CLUSTER = 8;  // CTAs (SMs) per large matrix
 
 // A job goes to the cluster kernel when its Jacobi work is large enough to
@@ -1106,8 +1776,20 @@ template <class T>
 void jacobi(tnfa_ctx* ctx, const std::vector<SvdJob>& jobs, int max_sweeps, JacobiOpts stop_rel,
             const char* family) {
   if (ctx->jacobi_sweep_cap > 0) max_sweeps = std::min(max_sweeps, ctx->jacobi_sweep_cap);
-  std::vector<SvdJob> big, small;
-  for (const auto& j : jobs) (svd_big(j, jobs.size(), ctx->sm_count) ? big : small).push_back(j);
+  std::vector<SvdJob> big, small, sm;
+  for (const auto& j : jobs)
+    (jacobi_fits<T>(j, jobs.size(), ctx->sm_count) ? sm : svd_big(j, jobs.size(), ctx->sm_count) ? big : small)
+        .push_back(j);
+  if (!sm.empty()) {
+    double fl = 0;
+    for (const auto& j : sm) {
+      TNFA_CHECK(j.m >= j.n, TNFA_ERR_INVALID_ARGUMENT, "svd needs m >= n");
+      fl += 5.0 * j.m * j.n * j.n * 8;
+    }
+    KernelScope ks(ctx, family, fl, 0.0);
+    if (trace_on()) ks.note = "shared " + size_note(sm);
+    launch_jacobi_sm<T>(ctx, sm, max_sweeps, stop_rel);
+  }
   for (int pass = 0; pass < 2; ++pass) {
     const std::vector<SvdJob>& js = pass == 0 ? big : small;
     if (js.empty()) continue;
@@ -1811,7 +2493,15 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
   std::vector<double> extra(nj, 0.0);
   std::vector<double> polish_scale;  // mixed: sum of squares of each polish input
   std::vector<SvdJob> sj;
-  if (!mixed) {
+  // FP64 with FP32 in front: the same two FP32 passes find V, nothing is
+  // dropped, and FP64 Jacobi on C V -- whose columns are orthogonal to FP32
+  // accuracy -- takes two or three sweeps instead of eight or nine, to the same
+  // stop.  From 32 columns on (42: 1.0 -> 0.5 ms a matrix); below, the extra
+  // launches cost more than the sweeps.
+  int maxn = 0;
+  for (size_t q = 0; q < nj; ++q) maxn = std::max(maxn, n[q]);
+  const bool front = real64 && !mixed && maxn >= 32;
+  if (!mixed && !front) {
     for (size_t q = 0; q < nj; ++q) {
       ku[q] = n[q];
       U[q] = DBuf(ctx, (size_t)cm[q] * n[q] * sizeof(T));
@@ -1862,7 +2552,9 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
       // pass 1 only has to split kept from dropped directions and hand pass 2
       // a nearly diagonal start: stop at 1e-4; pass 2 runs to FP32 accuracy
       jacobi<float>(ctx, s32, 60, JacobiOpts{pass == 0 ? 1e-4 : 0.0, opts.small_rel}, "svd_f32");
-      if (pass == 0) {
+      if (pass == 0 && front) {
+        for (size_t q = 0; q < nj; ++q) ku[q] = n[q];
+      } else if (pass == 0) {
         // keep the FP32 directions that a 10^6 times smaller cutoff would
         // keep (all of them without a cutoff).  What pass 1 drops cannot be
         // recovered: a kept direction s_k tilts by ~eps32 s_max / s_k into
@@ -1929,6 +2621,13 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
       }
       if (pass == 1) ss_keep = std::move(ss);
     }
+    if (front) {
+      for (size_t q = 0; q < nj; ++q) {
+        U[q] = DBuf(ctx, (size_t)cm[q] * n[q] * sizeof(T));
+        sj.push_back({X[q].p, U[q].p, S_of(q), nullptr, cm[q], n[q], sw_of(q)});
+      }
+      jacobi<T>(ctx, sj, 60, opts, "svd_f64");
+    } else {
     TNFA_CUDA(cudaMemcpyAsync(ss_kept.data(), ss_keep.p, nj * sizeof(double), cudaMemcpyDeviceToHost,
                               ctx->stream));
     TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1987,6 +2686,7 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
           fclose(fp);
         }
       }
+    }
     }
   }
   // (3) ranks on the host (one read-back of every job's values and sweeps)

@@ -900,8 +900,13 @@ void absorb_batched(std::vector<Work<T>>& W, const std::vector<BSlot>& sl, const
 // directions (a few hundred times the FP64 rounding of a QR step).
 constexpr double kRevealTol = 1e-13;
 
+// A single call keeps directions down to 1e-14, where the truncation rule
+// stops keeping them too (s^2 <= 1e-28 of the weight).
+constexpr double kRevealTolOne = 1e-14;
+
 template <class T>
-void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& prm) {
+void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& prm,
+                            double reveal_tol = kRevealTol) {
   if (W.empty()) return;
   tnfa_ctx* ctx = W[0].ctx;
   int maxV = 0;
@@ -919,7 +924,7 @@ void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& pr
     }
     std::vector<DBuf> Rs;
     std::vector<int> ks;
-    qr_parent_axis_batched(W, sl, Rs, ks, kRevealTol);
+    qr_parent_axis_batched(W, sl, Rs, ks, reveal_tol);
     std::vector<BSlot> ps;
     std::vector<int> ax;
     std::vector<const void*> Ms;
@@ -956,7 +961,7 @@ void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& pr
     }
     move_axes<T>(ctx, mv);
     std::vector<la::FactorResult> res;
-    la::trunc_factor<T>(ctx, fj, prm.cutoff, prm.maxdim, prm.mindim, prm.precision, res, kRevealTol);
+    la::trunc_factor<T>(ctx, fj, prm.cutoff, prm.maxdim, prm.mindim, prm.precision, res, reveal_tol);
     mv.clear();
     for (size_t q = 0; q < n; ++q) {
       TNFA_CHECK(res[q].sweeps >= 0, TNFA_ERR_NOT_CONVERGED, "Jacobi SVD hit its sweep cap");
@@ -996,7 +1001,8 @@ void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& pr
 
 template <class T>
 void batch_apply_truncate(tnfa_ctx* ctx, int n, const tnfa_net* const* ops, const tnfa_net* const* fs,
-                          const tnfa_trunc_params& prm, int dtype, tnfa_net** outs) {
+                          const tnfa_trunc_params& prm, int dtype, tnfa_net** outs,
+                          double reveal_tol = kRevealTol) {
   std::vector<Work<T>> W;
   if (ops) {
     apply_exact_many<T>(ctx, n, ops, fs, W);
@@ -1004,7 +1010,7 @@ void batch_apply_truncate(tnfa_ctx* ctx, int n, const tnfa_net* const* ops, cons
     W.reserve(n);
     for (int i = 0; i < n; ++i) W.push_back(load_work<T>(ctx, fs[i]));
   }
-  truncate_paths_batched(W, prm);
+  truncate_paths_batched(W, prm, reveal_tol);
   store_works(W, dtype, outs);
 }
 
@@ -2276,6 +2282,25 @@ using namespace tnfa;
 
 extern "C" {
 
+// One path through the batched sweeps: their rank-revealing QR cuts the bonds
+// of an exact product (D chi) to its rank before anything is factorised at
+// full width.  Null when the sweeps do not take it (another tree, a matrix of
+// more than 1024 columns, NaN or Inf entries): the general form then does.
+static tnfa_net* one_path(tnfa_ctx* ctx, const tnfa_net* op, const tnfa_net* f, const tnfa_trunc_params& prm) {
+  if (!is_rooted_path(f->topo) || (op && op->dtype != f->dtype)) return nullptr;
+  tnfa_net* out = nullptr;
+  try {
+    if (f->dtype == TNFA_F64)
+      batch_apply_truncate<double>(ctx, 1, op ? &op : nullptr, &f, prm, TNFA_F64, &out, kRevealTolOne);
+    else if (f->dtype == TNFA_C128)
+      batch_apply_truncate<cplx>(ctx, 1, op ? &op : nullptr, &f, prm, TNFA_C128, &out, kRevealTolOne);
+  } catch (const Error& e) {
+    if (e.status != TNFA_ERR_DOMAIN && e.status != TNFA_ERR_UNSUPPORTED) throw;
+    return nullptr;
+  }
+  return out;
+}
+
 int tnfa_apply(tnfa_ctx* ctx, const tnfa_net* op, const tnfa_net* f,
                const tnfa_trunc_params* params, tnfa_net** out) {
   TNFA_API_BEGIN(ctx);
@@ -2284,7 +2309,8 @@ int tnfa_apply(tnfa_ctx* ctx, const tnfa_net* op, const tnfa_net* f,
   require_net(f, "apply function");
   check_params(params);
   TNFA_CHECK(out, TNFA_ERR_INVALID_ARGUMENT, "null out");
-  *out = apply_truncate(ctx, op, f, *params);
+  *out = one_path(ctx, op, f, *params);
+  if (!*out) *out = apply_truncate(ctx, op, f, *params);
   TNFA_API_END
 }
 
@@ -2367,7 +2393,8 @@ int tnfa_truncate(tnfa_ctx* ctx, const tnfa_net* f, const tnfa_trunc_params* par
   require_net(f, "truncate");
   check_params(params);
   TNFA_CHECK(out, TNFA_ERR_INVALID_ARGUMENT, "null out");
-  *out = truncate_net(ctx, f, *params);
+  *out = one_path(ctx, nullptr, f, *params);
+  if (!*out) *out = truncate_net(ctx, f, *params);
   TNFA_API_END
 }
 
