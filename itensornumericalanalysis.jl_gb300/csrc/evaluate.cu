@@ -845,7 +845,18 @@ class EvalEngine {
         if (tuned) tune(ctx_, key, RowTiles<T>::n, fl, go);
         else go(0);
       }
-      for (int v : L.verts) contract_table(v);
+      if constexpr (std::is_same<T, double>::value) {
+        // the sliced tensor-core tables of a level in one launch
+        std::vector<std::pair<int, VertexJob<double>>> oz;
+        for (int v : L.verts) {
+          if (!tree_.v[v].tensor) continue;
+          oz.push_back({v, vertex_job(v)});
+          bind_groups(oz.back().second, tmeta_[v]);
+        }
+        if (!oz.empty()) oz_contract(ctx_, net_, oz, err_);
+      }
+      for (int v : L.verts)
+        if (!std::is_same<T, double>::value || !tree_.v[v].tensor) contract_table(v);
     }
     if (!norms_.empty()) {
       int n = 1;
@@ -1644,18 +1655,21 @@ class EvalEngine {
   }
 
   // Runs a multi-child job whose groups are in meta with tile rows tp.
+  static void bind_groups(VertexJob<T>& j, int* meta) {
+    j.grp_off = meta;
+    j.grp_cnt = meta + j.ngroups;
+    j.tile_start = meta + 2 * j.ngroups;
+  }
   void contract_vertex(int v, VertexJob<T>& j, int* meta, bool keyed, int tp) {
     const int ng = j.ngroups;
-    j.grp_off = meta;
-    j.grp_cnt = meta + ng;
-    j.tile_start = meta + 2 * ng;
+    bind_groups(j, meta);
     if (tree_.v[v].tensor) {
       if constexpr (std::is_same<T, float>::value) {
         tc_contract_vertex(ctx_, net_, v, j, tp, err_);
         return;
       }
       if constexpr (std::is_same<T, double>::value) {
-        oz_contract_vertex(ctx_, net_, v, j, tp, err_);
+        oz_contract(ctx_, net_, {{v, j}}, err_);
         return;
       }
     }

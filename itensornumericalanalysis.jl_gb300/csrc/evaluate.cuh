@@ -73,8 +73,9 @@ CUtensorMap tc_make_map3(const void* base, int x_dim, int y_dim, int64_t z_dim, 
 // children evaluated from FP64 messages to FP64 messages on tcgen05.
 bool oz_vertex_eligible(int nchild, const int* child_dims, int chi_a);
 void oz_prepare_net(tnfa_ctx* ctx, const tnfa_net* net);  // digit planes of the tensors
-void oz_contract_vertex(tnfa_ctx* ctx, const tnfa_net* net, int v, const VertexJob<double>& job,
-                        int tile_rows, int* err);
+// independent vertices together
+void oz_contract(tnfa_ctx* ctx, const tnfa_net* net, const std::vector<std::pair<int, VertexJob<double>>>& jobs,
+                 int* err);
 int oz_tile_rows();
 
 }  // namespace tnfa

@@ -189,9 +189,19 @@ __device__ __forceinline__ void dd_add(float& ah, float& al, float bh, float bl)
   al = __fsub_rn(e, __fsub_rn(ah, s2));
 }
 
+// Vertices of one launch.  A tile is `split` CTAs, each with its part of the
+// blocks of 32 parent values.
+constexpr int OZ_BATCH = 8;
+struct OzBatch {
+  CUtensorMap map[OZ_BATCH];
+  OzParams job[OZ_BATCH];
+  int blk0[OZ_BATCH + 1];  // first CTA of each
+  int split[OZ_BATCH];
+  int n;
+};
+
 template <int KCH>
-__global__ void __launch_bounds__(OZ_THREADS, 1)
-    k_contract_oz(const __grid_constant__ CUtensorMap mapB, const OzParams P) {
+__global__ void __launch_bounds__(OZ_THREADS, 1) k_contract_oz(const __grid_constant__ OzBatch batch) {
   constexpr int PP = OZ_DIG / KCH;  // digit planes resident per phase
   constexpr int NPH = KCH;          // phases over the digit planes of A
   constexpr int CHI2 = KCH * OZ_KC;
@@ -205,7 +215,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   unsigned char* Asm = smem;
   unsigned char* Bsm = smem + OZ_SLOTS * OZ_SLOT_BYTES;
 
-  const int blk = blockIdx.x;
+  int bj = 0;
+  while (bj + 1 < batch.n && batch.blk0[bj + 1] <= (int)blockIdx.x) ++bj;
+  const OzParams& P = batch.job[bj];
+  const CUtensorMap& mapB = batch.map[bj];
+  const int split = batch.split[bj];
+  const int blk = ((int)blockIdx.x - batch.blk0[bj]) / split;
+  const int part = ((int)blockIdx.x - batch.blk0[bj]) % split;
   const int ng = P.ngroups;
   if (blk >= P.tile_start[ng]) return;
   int g = 0;
@@ -213,7 +229,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   const int row0 = P.grp_off[g] + (blk - P.tile_start[g]) * OZ_M;
   const int nrows = min(OZ_M, P.grp_off[g] + P.grp_cnt[g] - row0);
   if (nrows <= 0) return;
-  const int nab = P.chi_a / OZ_NA, nbb = P.chi1 / OZ_NB;
+  const int nbb = P.chi1 / OZ_NB;
+  const int ab0 = P.chi_a / OZ_NA * part / split, ab1 = P.chi_a / OZ_NA * (part + 1) / split;
   const uint32_t lim = P.wait_limit;
 
   if (tid == 0) {
@@ -301,7 +318,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       fence_proxy_async();
       if (!(P.drop_arrive && ph == 0)) mbar_arrive(&a_ready);
 
-      for (int ab = 0; ab < nab && ok; ++ab) {
+      for (int ab = ab0; ab < ab1 && ok; ++ab) {
         float ah[16], al[16];  // the a-block's sums (double-float)
         float sh[16], sl[16];  // the current four N-tiles' sums
 #pragma unroll
@@ -414,14 +431,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       }
     }
     if (!ok) atomicOr(P.err, ERR_TIMEOUT);
-    if (ok && valid && h == 0) P.out_exp[p] = e_in + E1 + E2;
+    if (ok && valid && h == 0 && part == 0) P.out_exp[p] = e_in + E1 + E2;
   } else if (warp == 8) {
     // ------------------------------------------------------------ TMA ----
     if (lane == 0) {
       bool ok = true;
       uint32_t si = 0;
       for (int ph = 0; ph < NPH && ok; ++ph)
-        for (int ab = 0; ab < nab && ok; ++ab)
+        for (int ab = ab0; ab < ab1 && ok; ++ab)
           for (int bb = 0; bb < nbb && ok; ++bb)
             for (int gi = 0; gi < oz_ngroups(ph, PP) && ok; ++gi) {
               const int k = oz_group(ph, gi, PP);
@@ -458,7 +475,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           break;
         }
         tc_fence_after();
-        for (int ab = 0; ab < nab && ok; ++ab)
+        for (int ab = ab0; ab < ab1 && ok; ++ab)
           for (int bb = 0; bb < nbb && ok; ++bb)
             for (int gi = 0; gi < oz_ngroups(ph, PP) && ok; ++gi) {
               const int k = oz_group(ph, gi, PP);
@@ -579,11 +596,40 @@ OzLayout oz_layout(const Topo& T) {
 }
 
 template <int KCH>
-void launch_oz(tnfa_ctx* ctx, const CUtensorMap& map, const OzParams& p, unsigned grid) {
+void launch_oz(tnfa_ctx* ctx, const OzBatch& b) {
   TNFA_CUDA(cudaFuncSetAttribute(k_contract_oz<KCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  OZ_SMEM));
-  k_contract_oz<KCH><<<grid, OZ_THREADS, OZ_SMEM, ctx->stream>>>(map, p);
+  k_contract_oz<KCH><<<(unsigned)b.blk0[b.n], OZ_THREADS, OZ_SMEM, ctx->stream>>>(b);
   TNFA_LAUNCH_CHECK();
+}
+
+// Parts per tile: a CTA alone on its SM takes the same time whether its tile
+// holds 128 rows or 8, so a launch of fewer tiles than SMs (the tables), or
+// with a nearly empty last wave, is cut finer along the parent's values.  Of
+// the cuts 1, 2, 4, ... the one with the least (waves x CTA time), a CTA's
+// time being its blocks of 32 parent values plus about a tenth of one for
+// building its digit planes.
+int oz_split(int sms, const std::vector<std::pair<int64_t, int>>& tiles_nab) {
+  int best = 1, most = 1;
+  for (const auto& t : tiles_nab) most = std::max(most, t.second);
+  double cost = 0;
+  for (int s = 1;; s *= 2) {
+    const int cut = std::min(s, most);
+    int64_t n = 0;
+    int longest = 0;
+    for (const auto& t : tiles_nab) {
+      const int c = std::min(cut, t.second);
+      n += t.first * c;
+      longest = std::max(longest, (t.second + c - 1) / c);
+    }
+    const double x = (double)((n + sms - 1) / sms) * (longest + 0.1);
+    if (s == 1 || x < cost) {
+      cost = x;
+      best = cut;
+    }
+    if (s >= most) break;
+  }
+  return best;
 }
 
 }  // namespace
@@ -629,46 +675,66 @@ void oz_prepare_net(tnfa_ctx* ctx, const tnfa_net* net) {
   TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 
-void oz_contract_vertex(tnfa_ctx* ctx, const tnfa_net* net, int v, const VertexJob<double>& j,
-                        int tile_rows, int* err) {
-  TNFA_CHECK(tile_rows == OZ_M, TNFA_ERR_INVALID_ARGUMENT, "tile rows mismatch");
+void oz_contract(tnfa_ctx* ctx, const tnfa_net* net, const std::vector<std::pair<int, VertexJob<double>>>& jobs,
+                 int* err) {
   TNFA_CHECK(net->d_oz != nullptr, TNFA_ERR_INVALID_ARGUMENT, "digit planes not prepared");
   const Topo& T = net->topo;
   const OzLayout L = oz_layout(T);
-  TNFA_CHECK(L.doff[v] >= 0 && j.nchild == 2, TNFA_ERR_UNSUPPORTED,
-             "vertex shape outside the sliced tensor-core kernel");
-  const int chi1 = j.ch[0].dim, chi2 = j.ch[1].dim;
-  const __nv_bfloat16* planes = (const __nv_bfloat16*)net->d_oz + L.doff[v];
-  const CUtensorMap map =
-      tc_make_map3(planes, chi2, chi1, (int64_t)OZ_DIG * j.site_dim * j.chi_a, OZ_NB, OZ_NA);
-  OzParams p{};
-  p.m1_ptr = j.ch[0].ptr;
-  p.m1_exp = j.ch[0].exps;
-  p.m1_idx = j.ch[0].idx;
-  p.m2_ptr = j.ch[1].ptr;
-  p.m2_exp = j.ch[1].exps;
-  p.m2_idx = j.ch[1].idx;
-  p.chi_a = j.chi_a;
-  p.chi1 = chi1;
-  p.site_dim = j.site_dim;
-  p.bexp = net->d_ozexp + L.eoff[v];
-  p.out = j.out;
-  p.out_exp = j.out_exp;
-  p.perm = j.perm;
-  p.grp_off = j.grp_off;
-  p.grp_cnt = j.grp_cnt;
-  p.tile_start = j.tile_start;
-  p.ngroups = j.ngroups;
-  p.err = err;
-  p.wait_limit = ctx->tc_wait_limit;
-  p.drop_arrive = ctx->tc_drop_arrive;
-  const unsigned grid = (unsigned)((j.Pc + OZ_M - 1) / OZ_M + j.ngroups);
-  // 26 digit-pair passes per product (the algorithmic count is one)
-  KernelScope ks(ctx, "contract_oz", 2.0 * j.Pc * (double)j.K * j.chi_a,
-                 8.0 * ((double)j.Pc * (chi1 + chi2 + j.chi_a)) +
-                     2.0 * OZ_DIG * j.site_dim * (double)j.chi_a * j.K);
-  if (chi2 == 128) launch_oz<2>(ctx, map, p, grid);
-  else launch_oz<1>(ctx, map, p, grid);
+  for (const int chi2 : {64, 128}) {
+    size_t at = 0;
+    while (at < jobs.size()) {
+      OzBatch b{};
+      std::vector<std::pair<int64_t, int>> tiles_nab;
+      double flops = 0, bytes = 0;
+      for (; at < jobs.size() && b.n < OZ_BATCH; ++at) {
+        const int v = jobs[at].first;
+        const VertexJob<double>& j = jobs[at].second;
+        TNFA_CHECK(L.doff[v] >= 0 && j.nchild == 2, TNFA_ERR_UNSUPPORTED,
+                   "vertex shape outside the sliced tensor-core kernel");
+        if (j.ch[1].dim != chi2 || j.Pc == 0) continue;
+        const int chi1 = j.ch[0].dim;
+        b.map[b.n] = tc_make_map3((const __nv_bfloat16*)net->d_oz + L.doff[v], chi2, chi1,
+                                  (int64_t)OZ_DIG * j.site_dim * j.chi_a, OZ_NB, OZ_NA);
+        OzParams& p = b.job[b.n];
+        p.m1_ptr = j.ch[0].ptr;
+        p.m1_exp = j.ch[0].exps;
+        p.m1_idx = j.ch[0].idx;
+        p.m2_ptr = j.ch[1].ptr;
+        p.m2_exp = j.ch[1].exps;
+        p.m2_idx = j.ch[1].idx;
+        p.chi_a = j.chi_a;
+        p.chi1 = chi1;
+        p.site_dim = j.site_dim;
+        p.bexp = net->d_ozexp + L.eoff[v];
+        p.out = j.out;
+        p.out_exp = j.out_exp;
+        p.perm = j.perm;
+        p.grp_off = j.grp_off;
+        p.grp_cnt = j.grp_cnt;
+        p.tile_start = j.tile_start;
+        p.ngroups = j.ngroups;
+        p.err = err;
+        p.wait_limit = ctx->tc_wait_limit;
+        p.drop_arrive = ctx->tc_drop_arrive;
+        tiles_nab.push_back({(j.Pc + OZ_M - 1) / OZ_M + j.ngroups, j.chi_a / OZ_NA});
+        flops += 2.0 * j.Pc * (double)j.K * j.chi_a;
+        bytes += 8.0 * ((double)j.Pc * (chi1 + chi2 + j.chi_a)) + 2.0 * OZ_DIG * j.site_dim * (double)j.chi_a * j.K;
+        ++b.n;
+      }
+      if (b.n == 0) break;
+      const int s = oz_split(ctx->sm_count, tiles_nab);
+      for (int i = 0; i < b.n; ++i) {
+        b.split[i] = std::min(s, tiles_nab[i].second);
+        const int64_t next = b.blk0[i] + tiles_nab[i].first * b.split[i];
+        TNFA_CHECK(next < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
+        b.blk0[i + 1] = (int)next;
+      }
+      // 26 digit-pair passes per product (the algorithmic count is one)
+      KernelScope ks(ctx, "contract_oz", flops, bytes);
+      if (chi2 == 128) launch_oz<2>(ctx, b);
+      else launch_oz<1>(ctx, b);
+    }
+  }
 }
 
 }  // namespace tnfa
