@@ -149,10 +149,32 @@ static DBuf upload(tnfa_ctx* ctx, const std::vector<Job>& jobs) {
   return d;
 }
 
+// A launch's jobs: in its parameters when there are few, else uploaded.  A
+// single network's sweep is thousands of launches of one job each, and the
+// upload is a copy on the stream between two kernels (about 3 us of the 6 us
+// that a small permutation or product took).
+constexpr int ARG_JOBS = 4;
+template <class Job>
+struct JobArgs {
+  Job few[ARG_JOBS];
+  const Job* many;
+  __device__ const Job& operator[](int i) const { return many ? many[i] : few[i]; }
+};
+template <class Job>
+static JobArgs<Job> pass(tnfa_ctx* ctx, const std::vector<Job>& jobs, DBuf& keep) {
+  JobArgs<Job> a{};
+  if (jobs.size() <= (size_t)ARG_JOBS) {
+    std::copy(jobs.begin(), jobs.end(), a.few);
+  } else {
+    keep = upload(ctx, jobs);
+    a.many = keep.as<Job>();
+  }
+  return a;
+}
+
 // ------------------------------------------------------------- permute --
 template <class T>
-__global__ void k_permute(const PermJob* __restrict__ jobs) {
-  const PermJob& jb = jobs[blockIdx.y];
+__device__ inline void permute_job(const PermJob& jb) {
   int64_t sstride[MAXD];
   int64_t st = 1;
   for (int a = jb.nd - 1; a >= 0; --a) {
@@ -184,6 +206,14 @@ __global__ void k_permute(const PermJob* __restrict__ jobs) {
     dst[i] = src[si];
   }
 }
+template <class T>
+__global__ void k_permute(const PermJob* __restrict__ jobs) {
+  permute_job<T>(jobs[blockIdx.y]);
+}
+template <class T>
+__global__ void k_permute_few(const __grid_constant__ JobArgs<PermJob> jobs) {
+  permute_job<T>(jobs.few[blockIdx.y]);
+}
 
 template <class T>
 void permute(tnfa_ctx* ctx, const std::vector<PermJob>& jobs) {
@@ -193,10 +223,12 @@ void permute(tnfa_ctx* ctx, const std::vector<PermJob>& jobs) {
   TNFA_CHECK(jobs.size() <= 65535, TNFA_ERR_UNSUPPORTED, "permute batch too large");
   for (const auto& j : jobs)
     TNFA_CHECK(j.nd >= 1 && j.nd <= MAXD, TNFA_ERR_UNSUPPORTED, "permute: tensor order above 16");
-  DBuf d = upload(ctx, jobs);
+  DBuf d;
+  const auto args = pass(ctx, jobs, d);
   dim3 grid(grid_for(nmax, 256, 2048), (unsigned)jobs.size());
   KernelScope ks(ctx, "permute", 0.0, 2.0 * sizeof(T) * nmax * jobs.size());
-  k_permute<T><<<grid, 256, 0, ctx->stream>>>(d.as<PermJob>());
+  if (args.many) k_permute<T><<<grid, 256, 0, ctx->stream>>>(args.many);
+  else k_permute_few<T><<<grid, 256, 0, ctx->stream>>>(args);
   TNFA_LAUNCH_CHECK();
 }
 
@@ -215,10 +247,19 @@ __device__ inline T opget(const T* X, int ld, int op, int r, int c) {
 // their two shared-memory words per multiply-add are far below what shared
 // memory delivers.  16 x 16 while the batch has fewer than two tiles of 32 per
 // SM (a 42 x 84 x 42 product: 48 -> 5 us), else 32 x 32.
+struct GemmArgs {
+  GemmJob jobs[ARG_JOBS];
+  int first[ARG_JOBS + 1];  // first tile of each job, and their number
+  int n;
+  const GemmJob* more;
+  const int* more_first;
+};
 template <class T, int BT>
-__global__ void __launch_bounds__(256) k_gemm(const GemmJob* __restrict__ jobs, const int* __restrict__ first,
-                                              int njobs) {
+__global__ void __launch_bounds__(256) k_gemm(const __grid_constant__ GemmArgs args) {
   constexpr int BK = 16, RT = BT / 16;
+  const GemmJob* jobs = args.more ? args.more : args.jobs;
+  const int* first = args.more ? args.more_first : args.first;
+  const int njobs = args.n;
   int lo = 0, hi = njobs;  // first[lo] <= blockIdx.x < first[hi]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -329,17 +370,25 @@ void gemm(tnfa_ctx* ctx, const std::vector<GemmJob>& jobs) {
   std::vector<int> first = tiles(32);
   const bool fine = first.back() < 2 * ctx->sm_count;
   if (fine) first = tiles(16);
-  // the jobs and their first tiles in one upload
-  const size_t nb = js.size() * sizeof(GemmJob);
-  std::vector<unsigned char> blob(nb + first.size() * sizeof(int));
-  std::memcpy(blob.data(), js.data(), nb);
-  std::memcpy(blob.data() + nb, first.data(), first.size() * sizeof(int));
-  DBuf d(ctx, blob.size());
-  h2d(ctx, d.p, blob.data(), blob.size());
-  const int* df = (const int*)(d.as<unsigned char>() + nb);
+  GemmArgs args{};
+  args.n = (int)js.size();
+  DBuf d;
+  if (js.size() <= (size_t)ARG_JOBS) {
+    std::copy(js.begin(), js.end(), args.jobs);
+    std::copy(first.begin(), first.end(), args.first);
+  } else {  // the jobs and their first tiles in one upload
+    const size_t nb = js.size() * sizeof(GemmJob);
+    std::vector<unsigned char> blob(nb + first.size() * sizeof(int));
+    std::memcpy(blob.data(), js.data(), nb);
+    std::memcpy(blob.data() + nb, first.data(), first.size() * sizeof(int));
+    d = DBuf(ctx, blob.size());
+    h2d(ctx, d.p, blob.data(), blob.size());
+    args.more = d.as<GemmJob>();
+    args.more_first = (const int*)(d.as<unsigned char>() + nb);
+  }
   KernelScope ks(ctx, sizeof(T) == 8 ? "gemm_f64" : "gemm_c128", fl, 0.0);
-  if (fine) k_gemm<T, 16><<<(unsigned)first.back(), 256, 0, ctx->stream>>>(d.as<GemmJob>(), df, (int)js.size());
-  else k_gemm<T, 32><<<(unsigned)first.back(), 256, 0, ctx->stream>>>(d.as<GemmJob>(), df, (int)js.size());
+  if (fine) k_gemm<T, 16><<<(unsigned)first.back(), 256, 0, ctx->stream>>>(args);
+  else k_gemm<T, 32><<<(unsigned)first.back(), 256, 0, ctx->stream>>>(args);
   TNFA_LAUNCH_CHECK();
 }
 
@@ -398,7 +447,10 @@ __device__ inline T block_sum(T v, T* red) {
 }
 
 // Workspace per job: A copied column-major into W (m*n), Q column-major
-// into Qw (m*kq); reflector j is stored in W column j rows j..m-1.
+// into Qw (m*kq); reflector j is stored in W column j rows j..m-1.  One CTA
+// whose workspace fits shared memory keeps it there (SM): a column step's
+// loads then take tens of cycles where they were L2 round trips (the QRs of
+// a linsolve sweep with bonds up to 16: 47 -> 37 us on average).
 //
 // Columns are dealt round-robin to the CTAs of a cluster (CL; one CTA
 // otherwise): the owner of column j builds reflector j in place, a barrier
@@ -412,21 +464,33 @@ __device__ inline void qsync() {
     __syncthreads();
 }
 
-template <class T, bool CL>
-__global__ void __launch_bounds__(512) k_qr(const QrJob* __restrict__ jobs, T* __restrict__ work,
-                                            const int64_t* __restrict__ woff) {
+struct QrTask {
+  QrJob job;
+  int64_t woff;
+};
+template <class T, bool CL, bool SM>
+__global__ void __launch_bounds__(512) k_qr(const __grid_constant__ JobArgs<QrTask> tasks, T* __restrict__ work) {
+  extern __shared__ __align__(16) unsigned char qr_work[];
   int C = 1, crank = 0;
   if constexpr (CL) {
     C = (int)cg::this_cluster().num_blocks();
     crank = (int)cg::this_cluster().block_rank();
   }
   const int ji = blockIdx.x / C;
-  const QrJob jb = jobs[ji];
+  const QrJob jb = tasks[ji].job;
   const int m = jb.m, n = jb.n, kq = min(m, n);
-  T* W = work + woff[ji];
+  T* W = SM ? (T*)qr_work : work + tasks[ji].woff;
   T* Qw = W + (int64_t)m * n;
   T* alpha_g = Qw + (int64_t)m * kq;  // kq diagonal entries of R
-  T* tau = (T*)jb.tau;
+  T* tau = SM ? alpha_g + kq : (T*)jb.tau;
+  auto ld = [](const T* p) {
+    if constexpr (SM) return *p;
+    else return ldcg(p);
+  };
+  auto st = [](T* p, T v) {
+    if constexpr (SM) *p = v;
+    else stcg(p, v);
+  };
   const T* A = (const T*)jb.A;
   __shared__ T red[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -448,36 +512,36 @@ __global__ void __launch_bounds__(512) k_qr(const QrJob* __restrict__ jobs, T* _
         if (!(nrm > 1e-150)) {
           // an (almost) eliminated column: no reflection.  A residue this
           // small (rounding left by earlier steps) would make 2 / |v|^2 overflow.
-          stcg(tau + j, from_real<T>(0.0));
-          stcg(alpha_g + j, x0);
+          st(tau + j, from_real<T>(0.0));
+          st(alpha_g + j, x0);
         } else {
           const T alpha = scal(phase(x0), -nrm);
           const T v0 = x0 - alpha;
           const double vn2 = nrm2 - abs2(x0) + abs2(v0);
-          stcg(tau + j, from_real<T>(vn2 > 0.0 ? 2.0 / vn2 : 0.0));
-          stcg(x + j, v0);
-          stcg(alpha_g + j, alpha);
+          st(tau + j, from_real<T>(vn2 > 0.0 ? 2.0 / vn2 : 0.0));
+          st(x + j, v0);
+          st(alpha_g + j, alpha);
         }
       }
     }
     qsync<CL>();
-    const double beta = re(ldcg(tau + j));
+    const double beta = re(ld(tau + j));
     if (beta != 0.0) {
       // this CTA's columns c > j: c = crank + C * k
       const int c0 = j + 1 + ((crank - (j + 1)) % C + C) % C;
       for (int c = c0 + C * warp; c < n; c += C * nw) {
         T* y = W + (int64_t)c * m;
         T w = from_real<T>(0.0);
-        for (int r = j + lane; r < m; r += 32) w = Sc<T>::fma(conj(ldcg(x + r)), y[r], w);
+        for (int r = j + lane; r < m; r += 32) w = Sc<T>::fma(conj(ld(x + r)), y[r], w);
         w = warp_sum(w);
         const T bw = scal(w, beta);
-        for (int r = j + lane; r < m; r += 32) y[r] = y[r] - ldcg(x + r) * bw;
+        for (int r = j + lane; r < m; r += 32) y[r] = y[r] - ld(x + r) * bw;
       }
     }
     __syncthreads();
     // R row j: diagonal alpha, then the updated row j of this CTA's columns
     for (int c = crank + C * threadIdx.x; c < n; c += C * blockDim.x)
-      R[(int64_t)j * n + c] = c < j ? from_real<T>(0.0) : (c == j ? ldcg(alpha_g + j) : W[(int64_t)c * m + j]);
+      R[(int64_t)j * n + c] = c < j ? from_real<T>(0.0) : (c == j ? ld(alpha_g + j) : W[(int64_t)c * m + j]);
   }
   // Q = H_0 ... H_{kq-1} [I; 0], columns owned as above
   for (int c = crank + C * warp; c < kq; c += C * nw) {
@@ -486,7 +550,7 @@ __global__ void __launch_bounds__(512) k_qr(const QrJob* __restrict__ jobs, T* _
   }
   __syncthreads();
   for (int j = kq - 1; j >= 0; --j) {
-    const double beta = re(ldcg(tau + j));
+    const double beta = re(ld(tau + j));
     if (beta == 0.0) continue;
     const T* x = W + (int64_t)j * m;
     // a column stays with one warp for all j (no barrier between the j)
@@ -494,10 +558,10 @@ __global__ void __launch_bounds__(512) k_qr(const QrJob* __restrict__ jobs, T* _
       if (c < j) continue;
       T* y = Qw + (int64_t)c * m;
       T w = from_real<T>(0.0);
-      for (int r = j + lane; r < m; r += 32) w = Sc<T>::fma(conj(ldcg(x + r)), y[r], w);
+      for (int r = j + lane; r < m; r += 32) w = Sc<T>::fma(conj(ld(x + r)), y[r], w);
       w = warp_sum(w);
       const T bw = scal(w, beta);
-      for (int r = j + lane; r < m; r += 32) y[r] = y[r] - ldcg(x + r) * bw;
+      for (int r = j + lane; r < m; r += 32) y[r] = y[r] - ld(x + r) * bw;
     }
   }
   __syncthreads();
@@ -509,6 +573,7 @@ __global__ void __launch_bounds__(512) k_qr(const QrJob* __restrict__ jobs, T* _
 }
 
 constexpr int QR_CLUSTER = 8;
+constexpr size_t QR_SMEM = 200 * 1024;
 
 template <class T>
 void qr(tnfa_ctx* ctx, const std::vector<QrJob>& jobs) {
@@ -523,8 +588,8 @@ void qr(tnfa_ctx* ctx, const std::vector<QrJob>& jobs) {
          ? big
          : small)
         .push_back(j);
-  for (int pass = 0; pass < 2; ++pass) {
-    const std::vector<QrJob>& js = pass == 0 ? big : small;
+  for (int pass_ = 0; pass_ < 2; ++pass_) {
+    const std::vector<QrJob>& js = pass_ == 0 ? big : small;
     if (js.empty()) continue;
     std::vector<int64_t> woff(js.size() + 1, 0);
     double fl = 0;
@@ -534,12 +599,24 @@ void qr(tnfa_ctx* ctx, const std::vector<QrJob>& jobs) {
       woff[i + 1] = woff[i] + m * n + m * k + k;
       fl += 4.0 * m * n * k;
     }
-    DBuf work(ctx, (size_t)woff.back() * sizeof(T));
-    DBuf dw = upload(ctx, woff);
-    DBuf d = upload(ctx, js);
+    // in shared memory where the largest job's workspace (and its kq taus) fits
+    size_t sm = 0;
+    int maxm = 1, maxn = 1;
+    for (const auto& j : js) {
+      const size_t k = std::min(j.m, j.n);
+      sm = std::max(sm, ((size_t)j.m * j.n + j.m * k + 2 * k) * sizeof(T));
+      maxm = std::max(maxm, j.m);
+      maxn = std::max(maxn, j.n);
+    }
+    const bool shared = pass_ == 1 && sm <= QR_SMEM;
+    DBuf work(ctx, shared ? 0 : (size_t)woff.back() * sizeof(T));
+    std::vector<QrTask> tasks;
+    for (size_t i = 0; i < js.size(); ++i) tasks.push_back({js[i], woff[i]});
+    DBuf d;
+    const auto args = pass(ctx, tasks, d);
     KernelScope ks(ctx, sizeof(T) == 8 ? "qr_f64" : "qr_c128", fl, 0.0);
-    if (trace_on()) ks.note = (pass == 0 ? "cluster " : "single ") + size_note(js);
-    if (pass == 0) {
+    if (trace_on()) ks.note = (pass_ == 0 ? "cluster " : "single ") + size_note(js);
+    if (pass_ == 0) {
       cudaLaunchConfig_t cfg{};
       cfg.gridDim = dim3((unsigned)(js.size() * QR_CLUSTER));
       cfg.blockDim = dim3(512);
@@ -551,11 +628,14 @@ void qr(tnfa_ctx* ctx, const std::vector<QrJob>& jobs) {
       at[0].val.clusterDim.z = 1;
       cfg.attrs = at;
       cfg.numAttrs = 1;
-      TNFA_CUDA(cudaLaunchKernelEx(&cfg, k_qr<T, true>, (const QrJob*)d.as<QrJob>(), work.as<T>(),
-                                   (const int64_t*)dw.as<int64_t>()));
+      TNFA_CUDA(cudaLaunchKernelEx(&cfg, k_qr<T, true, false>, args, work.as<T>()));
+    } else if (shared) {
+      // a warp per column or 32 rows, whichever are more
+      const int warps = std::min(16, std::max({4, (maxm + 31) / 32, maxn}));
+      TNFA_CUDA(cudaFuncSetAttribute(k_qr<T, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QR_SMEM));
+      k_qr<T, false, true><<<(unsigned)js.size(), 32 * warps, sm, ctx->stream>>>(args, nullptr);
     } else {
-      k_qr<T, false><<<(unsigned)js.size(), 512, 0, ctx->stream>>>(d.as<QrJob>(), work.as<T>(),
-                                                                  dw.as<int64_t>());
+      k_qr<T, false, false><<<(unsigned)js.size(), 512, 0, ctx->stream>>>(args, work.as<T>());
     }
     TNFA_LAUNCH_CHECK();
   }
@@ -2197,23 +2277,22 @@ __global__ void __launch_bounds__(128) k_lu_trsm_reg(double* A, int n, int k, in
 // of 32 rows: the block's right-hand side first takes the product with the
 // solved part (all warps, one row each), then one warp solves the 32 x 32
 // triangle with shuffles.
-__global__ void __launch_bounds__(512) k_lu_subst(const double* A, int n, const int* piv, double* b) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (threadIdx.x == 0)
-    for (int j = 0; j < n; ++j) {
-      const int p = piv[j];
-      if (p != j) {
-        const double t = b[j];
-        b[j] = b[p];
-        b[p] = t;
-      }
+__device__ inline void lu_swaps(const int* piv, double* b, int n) {
+  for (int j = 0; j < n; ++j) {
+    const int p = piv[j];
+    if (p != j) {
+      const double t = b[j];
+      b[j] = b[p];
+      b[p] = t;
     }
-  __syncthreads();
+  }
+}
+__device__ inline void lu_triangles(const double* A, int ld, int n, double* b, int lane, int warp, int nw) {
   // forward: rows r0..r0+31 after rows < r0 are final
   for (int r0 = 0; r0 < n; r0 += 32) {
     const int rb = min(32, n - r0);
     for (int i = warp; i < rb; i += nw) {
-      const double* Ar = A + (int64_t)(r0 + i) * n;
+      const double* Ar = A + (int64_t)(r0 + i) * ld;
       double part = 0.0;
       for (int t = lane; t < r0; t += 32) part += Ar[t] * b[t];
       for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -2224,7 +2303,7 @@ __global__ void __launch_bounds__(512) k_lu_subst(const double* A, int n, const 
       double y = lane < rb ? b[r0 + lane] : 0.0;
       for (int i = 0; i < rb; ++i) {
         const double yi = __shfl_sync(0xffffffffu, y, i);
-        if (lane > i && lane < rb) y -= A[(int64_t)(r0 + lane) * n + r0 + i] * yi;
+        if (lane > i && lane < rb) y -= A[(int64_t)(r0 + lane) * ld + r0 + i] * yi;
       }
       if (lane < rb) b[r0 + lane] = y;
     }
@@ -2234,7 +2313,7 @@ __global__ void __launch_bounds__(512) k_lu_subst(const double* A, int n, const 
   for (int r1 = n; r1 > 0; r1 -= 32) {
     const int r0 = max(0, r1 - 32), rb = r1 - r0;
     for (int i = warp; i < rb; i += nw) {
-      const double* Ar = A + (int64_t)(r0 + i) * n;
+      const double* Ar = A + (int64_t)(r0 + i) * ld;
       double part = 0.0;
       for (int t = r1 + lane; t < n; t += 32) part += Ar[t] * b[t];
       for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -2244,15 +2323,114 @@ __global__ void __launch_bounds__(512) k_lu_subst(const double* A, int n, const 
     if (warp == 0) {
       double y = lane < rb ? b[r0 + lane] : 0.0;
       for (int i = rb - 1; i >= 0; --i) {
-        const double di = A[(int64_t)(r0 + i) * n + r0 + i];
+        const double di = A[(int64_t)(r0 + i) * ld + r0 + i];
         if (lane == i) y /= di;
         const double yi = __shfl_sync(0xffffffffu, y, i);
-        if (lane < i) y -= A[(int64_t)(r0 + lane) * n + r0 + i] * yi;
+        if (lane < i) y -= A[(int64_t)(r0 + lane) * ld + r0 + i] * yi;
       }
       if (lane < rb) b[r0 + lane] = y;
     }
     __syncthreads();
   }
+}
+__global__ void __launch_bounds__(512) k_lu_subst(const double* A, int n, const int* piv, double* b) {
+  if (threadIdx.x == 0) lu_swaps(piv, b, n);
+  __syncthreads();
+  lu_triangles(A, n, n, b, threadIdx.x & 31, threadIdx.x >> 5, blockDim.x >> 5);
+}
+
+// The whole solve of a small system on one SM, matrix and right-hand side in
+// shared memory (row stride odd): the panels, row swaps, triangular solves and
+// trailing updates of the launches below with the same arithmetic, without
+// four launches a panel.  Every warp searches the pivot column itself, so a
+// column step has three barriers.  The 92 two-site systems of a linsolve sweep
+// (24 bits, bonds up to 16): 292 -> 107 us each on average.
+constexpr int LU_SMALL = 165;  // (n | 1) n doubles in 220 KB
+__global__ void __launch_bounds__(512) k_lu_small(const double* __restrict__ Ag, double* __restrict__ bg, int n,
+                                                  int* singular) {
+  extern __shared__ __align__(16) double P[];
+  __shared__ double b[LU_SMALL];
+  __shared__ int piv[LU_SMALL];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, ld = n | 1;
+  for (int i = threadIdx.x; i < n * n; i += blockDim.x) P[i / n * ld + i % n] = Ag[i];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) b[i] = bg[i];
+  bool sing = false;
+  __syncthreads();
+  for (int k = 0; k < n; k += LU_RB) {
+    const int kb = min(LU_RB, n - k);
+    for (int j = k; j < k + kb; ++j) {
+      // the largest |entry| on or below the diagonal, the first of equals
+      // (ordered as integers; a NaN is never larger)
+      long long best = -1;
+      int p = j;
+      for (int r = j + lane; r < n; r += 32) {
+        const double x = fabs(P[r * ld + j]);
+        const long long key = x == x ? __double_as_longlong(x) : -1;
+        if (key > best) best = key, p = r;
+      }
+      for (int o = 16; o; o >>= 1) {
+        const long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int op = __shfl_xor_sync(0xffffffffu, p, o);
+        if (ob > best || (ob == best && op < p)) best = ob, p = op;
+      }
+      if (best < 0) p = j;
+      if (!(best > 0)) sing = true;
+      __syncthreads();
+      if (threadIdx.x == 0) piv[j] = p;
+      if (p != j)
+        for (int c = threadIdx.x; c < n; c += blockDim.x) {
+          const double t = P[j * ld + c];
+          P[j * ld + c] = P[p * ld + c];
+          P[p * ld + c] = t;
+        }
+      __syncthreads();
+      const double d = P[j * ld + j];
+      if (d != 0.0)
+        for (int r = j + 1 + threadIdx.x; r < n; r += blockDim.x) {
+          double* row = P + r * ld;
+          const double l = row[j] / d;
+          row[j] = l;
+          for (int c = j + 1; c < k + kb; ++c) row[c] -= l * P[j * ld + c];
+        }
+      __syncthreads();
+    }
+    const int n2 = n - k - kb;
+    if (n2 <= 0) break;
+    for (int c = k + kb + threadIdx.x; c < n; c += blockDim.x) {
+      double v[LU_RB];
+#pragma unroll
+      for (int r = 0; r < LU_RB; ++r) v[r] = P[(k + r) * ld + c];
+#pragma unroll
+      for (int r = 1; r < LU_RB; ++r)
+#pragma unroll
+        for (int t = 0; t < r; ++t) v[r] -= P[(k + r) * ld + k + t] * v[t];
+#pragma unroll
+      for (int r = 0; r < LU_RB; ++r) P[(k + r) * ld + c] = v[r];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n2 * n2; i += blockDim.x) {
+      const int r = k + kb + i / n2, c = k + kb + i % n2;
+      double acc = 0.0;
+#pragma unroll
+      for (int t = 0; t < LU_RB; ++t) acc = fma(P[r * ld + k + t], P[(k + t) * ld + c], acc);
+      P[r * ld + c] -= acc;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    if (sing) *singular = 1;
+    lu_swaps(piv, b, n);
+  }
+  __syncthreads();
+  lu_triangles(P, ld, n, b, lane, warp, nw);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) bg[i] = b[i];
+}
+
+static bool lu_regular(tnfa_ctx* ctx, const int* singular) {
+  int hs = 0;
+  TNFA_CUDA(cudaMemcpyAsync(&hs, singular, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
+  return hs == 0;
 }
 
 bool lu_solve(tnfa_ctx* ctx, double* A, double* b, int n) {
@@ -2260,6 +2438,13 @@ bool lu_solve(tnfa_ctx* ctx, double* A, double* b, int n) {
   DBuf piv(ctx, (size_t)n * sizeof(int)), sing(ctx, sizeof(int));
   TNFA_CUDA(cudaMemsetAsync(sing.p, 0, sizeof(int), ctx->stream));
   KernelScope ks(ctx, "lu_f64", 2.0 / 3.0 * (double)n * n * n, 0.0);
+  if (n <= LU_SMALL) {
+    const size_t sm = (size_t)n * (n | 1) * 8;
+    TNFA_CUDA(cudaFuncSetAttribute(k_lu_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    k_lu_small<<<1, n <= 64 ? 256 : 512, sm, ctx->stream>>>(A, b, n, sing.as<int>());
+    TNFA_LAUNCH_CHECK();
+    return lu_regular(ctx, sing.as<int>());
+  }
   TNFA_CUDA(cudaFuncSetAttribute(k_lu_panel_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)LU_SMEM_PANEL));
   for (int k = 0; k < n;) {
@@ -2296,10 +2481,7 @@ bool lu_solve(tnfa_ctx* ctx, double* A, double* b, int n) {
   }
   k_lu_subst<<<1, 512, 0, ctx->stream>>>(A, n, piv.as<int>(), b);
   TNFA_LAUNCH_CHECK();
-  int hs = 0;
-  TNFA_CUDA(cudaMemcpyAsync(&hs, sing.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
-  return hs == 0;
+  return lu_regular(ctx, sing.as<int>());
 }
 
 // --------------------------------------------------------- factorise --
@@ -2346,7 +2528,7 @@ __device__ inline dfl cvt(double x, dfl*) { return dfl(x); }
 __device__ inline double cvt(dfl x, double*) { return (double)x; }
 
 template <class S, class D>
-__global__ void k_copy_block(const CopyJob* __restrict__ jobs) {
+__global__ void k_copy_block(const __grid_constant__ JobArgs<CopyJob> jobs) {
   const CopyJob jb = jobs[blockIdx.y];
   const S* src = (const S*)jb.src;
   D* dst = (D*)jb.dst;
@@ -2368,9 +2550,9 @@ void copy_blocks(tnfa_ctx* ctx, const std::vector<CopyJob>& jobs) {
   int64_t nmax = 1;
   for (const auto& j : jobs) nmax = std::max<int64_t>(nmax, (int64_t)j.rows * j.cols);
   TNFA_CHECK(jobs.size() <= 65535, TNFA_ERR_UNSUPPORTED, "more than 65535 copies in one batch");
-  DBuf d = upload(ctx, jobs);
-  k_copy_block<S, D><<<dim3(grid_for(nmax, 256, 1024), (unsigned)jobs.size()), 256, 0, ctx->stream>>>(
-      d.as<CopyJob>());
+  DBuf d;
+  const auto args = pass(ctx, jobs, d);
+  k_copy_block<S, D><<<dim3(grid_for(nmax, 256, 1024), (unsigned)jobs.size()), 256, 0, ctx->stream>>>(args);
   TNFA_LAUNCH_CHECK();
 }
 
