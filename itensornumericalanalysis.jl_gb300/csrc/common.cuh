@@ -181,6 +181,10 @@ struct tnfa_ctx {
   };
   std::vector<PinnedBlock> pinned;
   size_t pinned_bytes = 0;
+  // Error words that kernels of synchronous calls set in host memory, one per
+  // call in turn (tnfa::error_word)
+  int* err_words = nullptr;
+  unsigned err_next = 0;
 };
 
 struct tnfa_net {
@@ -208,6 +212,12 @@ void dfree(tnfa_ctx* ctx, void* p);
 // context's stream that returns without waiting for the stream: the source
 // may be reused as soon as the call returns.
 void h2d(tnfa_ctx* ctx, void* dst, const void* src, size_t bytes);
+// A zeroed word of page-locked host memory that kernels write (only when
+// something is wrong) and the host reads after the stream has drained: no
+// clearing and no copy on the stream.  The context's words are used in turn,
+// so kernels left behind by a call that failed meet a later call's word only
+// 1024 calls on.
+int* error_word(tnfa_ctx* ctx);
 
 // RAII scratch buffer.
 struct DBuf {

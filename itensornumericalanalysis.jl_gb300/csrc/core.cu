@@ -129,6 +129,18 @@ void dfree(tnfa_ctx* ctx, void* p) {
 constexpr size_t kPageableAsyncMax = size_t(64) << 10;
 constexpr size_t kPinnedMaxBytes = size_t(256) << 20;
 
+int* error_word(tnfa_ctx* ctx) {
+  constexpr unsigned n = 1024;
+  if (!ctx->err_words) {
+    void* p = nullptr;
+    TNFA_CUDA(cudaHostAlloc(&p, n * sizeof(int), cudaHostAllocMapped));
+    ctx->err_words = (int*)p;
+  }
+  int* w = ctx->err_words + ctx->err_next++ % n;
+  *(volatile int*)w = 0;
+  return w;
+}
+
 void h2d(tnfa_ctx* ctx, void* dst, const void* src, size_t bytes) {
   if (bytes == 0) return;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -212,6 +224,7 @@ static void ctx_free(tnfa_ctx* ctx) {
       cudaEventDestroy(ev.second);
     }
   for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
+  if (ctx->err_words) cudaFreeHost(ctx->err_words);
   for (auto& b : ctx->pinned) {
     cudaEventDestroy(b.ev);
     cudaFreeHost(b.p);

@@ -789,6 +789,7 @@ class EvalEngine {
     h2d(ctx_, blob_, host_.data(), host_.size());
   }
   void clear_error() { TNFA_CUDA(cudaMemsetAsync(err_, 0, 4, ctx_->stream)); }
+  void use_error(int* word) { err_ = word; }  // after bind: a synchronous call's own word
 
   // Tables: permuted tensors, then every level.
   void tables() {
@@ -1889,14 +1890,17 @@ static size_t out_elem_size(int out_kind) {
   return out_kind == TNFA_OUT_F64 ? 8 : out_kind == TNFA_OUT_F32 ? 4 : out_kind == TNFA_OUT_F32_SCALED ? 8 : 16;
 }
 
-static void check_eval_error(tnfa_ctx* ctx, const int* derr) {
-  int herr = 0;
-  TNFA_CUDA(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, ctx->stream));
-  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
+static void check_error_word(int herr) {
   TNFA_CHECK((herr & 2) == 0, TNFA_ERR_TIMEOUT,
              "a tensor-core pipeline wait ran out of its iteration budget");
   TNFA_CHECK(herr == 0, TNFA_ERR_DOMAIN,
              "a coordinate is negative or not finite (the digit map needs x >= 0)");
+}
+static void check_eval_error(tnfa_ctx* ctx, const int* derr) {
+  int herr = 0;
+  TNFA_CUDA(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
+  check_error_word(herr);
 }
 
 template <class T>
@@ -1916,7 +1920,8 @@ static void evaluate_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, 
   DBuf arena(ctx, E.scratch(Pcap));
   E.bind(arena.p);
   E.upload();
-  E.clear_error();
+  int* const err = error_word(ctx);
+  E.use_error(err);
   E.tables();
   for (int64_t p0 = 0; p0 < P; p0 += Pcap) {
     const int Pc = (int)std::min<int64_t>(Pcap, P - p0);
@@ -1940,7 +1945,8 @@ static void evaluate_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, 
       }
     }
   }
-  check_eval_error(ctx, E.err_flag());
+  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
+  check_error_word(*(volatile int*)err);
 }
 
 }  // namespace tnfa
@@ -2835,7 +2841,8 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
   DBuf arena(ctx, E.bytes() + 512);
   E.bind_all(arena.p, dT);
   E.upload_all();
-  E.clear_error();
+  int* const err = error_word(ctx);
+  E.use_error(err);
   E.tables();
   for (int64_t p0 = 0; p0 < P; p0 += Pcap) {
     const int Pc = (int)std::min<int64_t>(Pcap, P - p0);
@@ -2851,7 +2858,8 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
     }
     E.chunk_gradient(Xc, Pc, dc);
   }
-  check_eval_error(ctx, E.err_flag());
+  TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
+  check_error_word(*(volatile int*)err);
 }
 
 }  // namespace

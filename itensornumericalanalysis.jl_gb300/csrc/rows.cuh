@@ -40,6 +40,12 @@ __device__ __forceinline__ unsigned long long unit_fraction(double x) {
   return sh > -53 ? m >> -sh : 0ull;
 }
 
+// Sets the error word (which may lie in host memory: one lane asks for the
+// warp, and writes only until the word is seen set).
+__device__ __noinline__ void raise_domain(int* err) {
+  if ((int)(threadIdx.x & 31) == __ffs(__activemask()) - 1 && !(*(volatile int*)err & 1)) atomicOr(err, 1);
+}
+
 // Adds every run to codes[slot * ld] for the slots [s0, s1).
 __device__ __forceinline__ void digit_codes(const double* __restrict__ Xp, const DigitRun* runs, int nruns,
                                             int* codes, int ld, int s0, int s1, int* err) {
@@ -52,7 +58,7 @@ __device__ __forceinline__ void digit_codes(const double* __restrict__ Xp, const
       const unsigned long long xb = (unsigned long long)__double_as_longlong(xr);
       // negative (not -0), infinite or NaN
       if (xb > 0x8000000000000000ull || (xb & 0x7FF0000000000000ull) == 0x7FF0000000000000ull) {
-        atomicOr(err, 1);
+        raise_domain(err);
         xr = 0.0;
       }
       u = unit_fraction(xr);
@@ -711,7 +717,7 @@ __global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ Pai
           xr = W.X[(int64_t)p * W.ncols + d.col];
           const unsigned long long xb = (unsigned long long)__double_as_longlong(xr);
           if (xb > 0x8000000000000000ull || (xb & 0x7FF0000000000000ull) == 0x7FF0000000000000ull) {
-            atomicOr(W.err, 1);
+            raise_domain(W.err);
             xr = 0.0;
           }
           u = unit_fraction(xr);
