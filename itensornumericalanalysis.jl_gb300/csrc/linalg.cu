@@ -254,7 +254,11 @@ struct GemmArgs {
   const GemmJob* more;
   const int* more_first;
 };
-template <class T, int BT>
+__device__ inline int64_t view_row(const MatView& v, int r) { return (int64_t)(r / v.r1) * v.R1 + (int64_t)(r % v.r1) * v.R0; }
+__device__ inline int64_t view_col(const MatView& v, int c) { return (int64_t)(c / v.c1) * v.C1 + (int64_t)(c % v.c1) * v.C0; }
+
+// (VIEW: some operand of the launch is viewed)
+template <class T, int BT, bool VIEW>
 __global__ void __launch_bounds__(256) k_gemm(const __grid_constant__ GemmArgs args) {
   constexpr int BK = 16, RT = BT / 16;
   const GemmJob* jobs = args.more ? args.more : args.jobs;
@@ -296,9 +300,14 @@ __global__ void __launch_bounds__(256) k_gemm(const __grid_constant__ GemmArgs a
     for (int i = 0; i < RT; ++i) {
       int r, c, kk;
       at_a(i, r, kk);
-      pa[i] = m0 + r < jb.m && k0 + kk < jb.k ? opget(A, jb.lda, jb.opA, m0 + r, k0 + kk) : from_real<T>(0.0);
+      auto get = [&](const T* X, const MatView& v, int ld, int op, int row, int col) -> T {
+        if constexpr (VIEW)
+          if (v.r1) return X[view_row(v, row) + view_col(v, col)];
+        return opget(X, ld, op, row, col);
+      };
+      pa[i] = m0 + r < jb.m && k0 + kk < jb.k ? get(A, jb.va, jb.lda, jb.opA, m0 + r, k0 + kk) : from_real<T>(0.0);
       at_b(i, c, kk);
-      pb[i] = n0 + c < jb.n && k0 + kk < jb.k ? opget(B, jb.ldb, jb.opB, k0 + kk, n0 + c) : from_real<T>(0.0);
+      pb[i] = n0 + c < jb.n && k0 + kk < jb.k ? get(B, jb.vb, jb.ldb, jb.opB, k0 + kk, n0 + c) : from_real<T>(0.0);
     }
   };
   load(0);
@@ -387,8 +396,11 @@ void gemm(tnfa_ctx* ctx, const std::vector<GemmJob>& jobs) {
     args.more_first = (const int*)(d.as<unsigned char>() + nb);
   }
   KernelScope ks(ctx, sizeof(T) == 8 ? "gemm_f64" : "gemm_c128", fl, 0.0);
-  if (fine) k_gemm<T, 16><<<(unsigned)first.back(), 256, 0, ctx->stream>>>(args);
-  else k_gemm<T, 32><<<(unsigned)first.back(), 256, 0, ctx->stream>>>(args);
+  bool view = false;
+  for (const auto& j : js) view |= j.va.r1 > 0 || j.vb.r1 > 0;
+  auto go = [&](auto kern) { kern<<<(unsigned)first.back(), 256, 0, ctx->stream>>>(args); };
+  if (view) fine ? go(k_gemm<T, 16, true>) : go(k_gemm<T, 32, true>);
+  else fine ? go(k_gemm<T, 16, false>) : go(k_gemm<T, 32, false>);
   TNFA_LAUNCH_CHECK();
 }
 
@@ -495,7 +507,13 @@ __global__ void __launch_bounds__(512) k_qr(const __grid_constant__ JobArgs<QrTa
   __shared__ T red[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int64_t i = threadIdx.x; i < (int64_t)m * n; i += blockDim.x) {
-    const int r = (int)(i / n), c = (int)(i % n);
+    int r, c;
+    if (jb.inner) {
+      const int64_t rc = i / jb.inner;
+      r = (int)(rc / n) * jb.inner + (int)(i % jb.inner), c = (int)(rc % n);
+    } else {
+      r = (int)(i / n), c = (int)(i % n);
+    }
     if (c % C == crank) W[(int64_t)c * m + r] = A[i];
   }
   __syncthreads();
@@ -543,6 +561,7 @@ __global__ void __launch_bounds__(512) k_qr(const __grid_constant__ JobArgs<QrTa
     for (int c = crank + C * threadIdx.x; c < n; c += C * blockDim.x)
       R[(int64_t)j * n + c] = c < j ? from_real<T>(0.0) : (c == j ? ld(alpha_g + j) : W[(int64_t)c * m + j]);
   }
+  if (!jb.Q) return;
   // Q = H_0 ... H_{kq-1} [I; 0], columns owned as above
   for (int c = crank + C * warp; c < kq; c += C * nw) {
     T* y = Qw + (int64_t)c * m;
@@ -567,7 +586,13 @@ __global__ void __launch_bounds__(512) k_qr(const __grid_constant__ JobArgs<QrTa
   __syncthreads();
   T* Q = (T*)jb.Q;
   for (int64_t i = threadIdx.x; i < (int64_t)m * kq; i += blockDim.x) {
-    const int r = (int)(i / kq), c = (int)(i % kq);
+    int r, c;
+    if (jb.inner) {
+      const int64_t rc = i / jb.inner;
+      r = (int)(rc / kq) * jb.inner + (int)(i % jb.inner), c = (int)(rc % kq);
+    } else {
+      r = (int)(i / kq), c = (int)(i % kq);
+    }
     if (c % C == crank) Q[i] = Qw[(int64_t)c * m + r];
   }
 }

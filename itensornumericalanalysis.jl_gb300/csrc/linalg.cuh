@@ -21,7 +21,15 @@ struct PermJob {
 template <class T>
 void permute(tnfa_ctx* ctx, const std::vector<PermJob>& jobs);
 
-// C = alpha * op(A) * op(B) + beta * C; op(X) = X, X^T or X^H (conj).
+// An operand read where it lies in a tensor whose axes are in another order:
+// element (r, c) at (r / r1) R1 + (r % r1) R0 + (c / c1) C1 + (c % c1) C0.
+struct MatView {
+  int r1 = 0, c1 = 0;  // r1 = 0: no view
+  int64_t R1 = 0, R0 = 0, C1 = 0, C0 = 0;
+};
+
+// C = alpha * op(A) * op(B) + beta * C; op(X) = X, X^T or X^H (conj).  A viewed
+// operand has op N and no leading dimension.
 struct GemmJob {
   const void* A;
   const void* B;
@@ -30,18 +38,22 @@ struct GemmJob {
   int lda, ldb, ldc;
   int opA, opB;  // 0: N, 1: T, 2: C (conjugate transpose)
   double alpha, beta;
+  MatView va{}, vb{};
 };
 template <class T>
 void gemm(tnfa_ctx* ctx, const std::vector<GemmJob>& jobs);
 
 // Householder QR of A (m x n, lda = n, destroyed): Q (m x kq, kq = min(m, n))
-// and R (kq x n) written to separate buffers.
+// and R (kq x n) written to separate buffers; without a Q buffer R alone is
+// formed.  inner > 0 (qr only): A's columns are the middle axis of a tensor
+// [m / inner][n][inner], and Q's of [m / inner][kq][inner].
 struct QrJob {
   void* A;
   void* Q;
   void* R;
   void* tau;  // kq scalars of workspace
   int m, n;
+  int inner = 0;
 };
 template <class T>
 void qr(tnfa_ctx* ctx, const std::vector<QrJob>& jobs);

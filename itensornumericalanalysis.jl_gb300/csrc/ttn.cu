@@ -139,67 +139,80 @@ void move_axis(tnfa_ctx* ctx, const void* src, void* dst, const std::vector<int>
 }
 
 // T_v <- M x_ax T_v : contract axis `ax` of v's tensor with the columns of M
-// (newdim x shape[ax]).
+// (newdim x shape[ax]).  One product per value of the axes before ax, or T M^T
+// where it is the last one: nothing is permuted.
 template <class T>
 void absorb(Work<T>& w, int v, int ax, const void* M, int newdim) {
   tnfa_ctx* ctx = w.ctx;
-  std::vector<int> shp = w.shape(v);
+  const std::vector<int> shp = w.shape(v);
   const int old = shp[ax];
-  const int64_t rest = w.size(v) / old;
-  DBuf a(ctx, (size_t)w.size(v) * sizeof(T));
-  move_axis<T>(ctx, w.t[v].p, a.p, shp, ax, 0);  // [old][rest]
-  DBuf b(ctx, (size_t)newdim * rest * sizeof(T));
-  la::GemmJob g{M, a.p, b.p, newdim, (int)rest, old, old, (int)rest, (int)rest, 0, 0, 1.0, 0.0};
-  la::gemm<T>(ctx, {g});
-  std::vector<int> nshp = shp;
-  nshp.erase(nshp.begin() + ax);
-  nshp.insert(nshp.begin(), newdim);  // current layout [newdim][rest...]
-  nan_check<T>(ctx, a.p, w.size(v), "absorb/permute-in", v);
+  int64_t lead = 1, tail = 1;
+  for (int a = 0; a < ax; ++a) lead *= shp[a];
+  for (size_t a = ax + 1; a < shp.size(); ++a) tail *= shp[a];
+  DBuf c(ctx, (size_t)lead * newdim * tail * sizeof(T));
+  nan_check<T>(ctx, w.t[v].p, w.size(v), "absorb/tensor", v);
   nan_check<T>(ctx, M, (int64_t)newdim * old, "absorb/matrix", v);
-  nan_check<T>(ctx, b.p, newdim * rest, "absorb/gemm", v);
-  DBuf c(ctx, (size_t)newdim * rest * sizeof(T));
-  move_axis<T>(ctx, b.p, c.p, nshp, 0, ax);
-  nan_check<T>(ctx, c.p, newdim * rest, "absorb/permute-out", v);
+  constexpr int64_t kLead = 64;  // products of a launch
+  if (tail == 1) {
+    TNFA_CHECK(lead < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "matrix too large");
+    la::gemm<T>(ctx, {la::GemmJob{w.t[v].p, M, c.p, (int)lead, newdim, old, old, old, newdim, 0, 1, 1.0, 0.0}});
+  } else if (lead <= kLead) {
+    TNFA_CHECK(tail < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "matrix too large");
+    std::vector<la::GemmJob> js;
+    for (int64_t i = 0; i < lead; ++i)
+      js.push_back({M, w.t[v].template as<T>() + i * old * tail, c.as<T>() + i * newdim * tail, newdim, (int)tail, old, old,
+                    (int)tail, (int)tail, 0, 0, 1.0, 0.0});
+    la::gemm<T>(ctx, js);
+  } else {
+    const int64_t rest = w.size(v) / old;
+    DBuf a(ctx, (size_t)w.size(v) * sizeof(T));
+    move_axis<T>(ctx, w.t[v].p, a.p, shp, ax, 0);  // [old][rest]
+    DBuf b(ctx, (size_t)newdim * rest * sizeof(T));
+    la::gemm<T>(ctx, {la::GemmJob{M, a.p, b.p, newdim, (int)rest, old, old, (int)rest, (int)rest, 0, 0, 1.0, 0.0}});
+    std::vector<int> nshp = shp;
+    nshp.erase(nshp.begin() + ax);
+    nshp.insert(nshp.begin(), newdim);  // current layout [newdim][rest...]
+    move_axis<T>(ctx, b.p, c.p, nshp, 0, ax);
+  }
+  nan_check<T>(ctx, c.p, lead * newdim * tail, "absorb/product", v);
   w.t[v] = std::move(c);
 }
 
 // Thin QR of v's tensor with axis `ax` as the columns: T = Q R.  v keeps Q
-// (axis ax now of dim k = min(rows, cols)); R (k x cols) is returned.
+// (axis ax now of dim k = min(rows, cols)), or its old tensor when only R is
+// wanted; R (k x cols) is returned.
 template <class T>
-int qr_axis(Work<T>& w, int v, int ax, DBuf& R) {
+int qr_axis(Work<T>& w, int v, int ax, DBuf& R, bool want_q = true) {
   tnfa_ctx* ctx = w.ctx;
-  std::vector<int> shp = w.shape(v);
+  const std::vector<int> shp = w.shape(v);
   const int cols = shp[ax];
   const int64_t rows = w.size(v) / cols;
   TNFA_CHECK(rows < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "matrix too large");
   const int k = (int)std::min<int64_t>(rows, cols);
-  DBuf M(ctx, (size_t)w.size(v) * sizeof(T));
-  move_axis<T>(ctx, w.t[v].p, M.p, shp, ax, (int)shp.size() - 1);  // [rest][cols]
-  DBuf Q(ctx, (size_t)rows * k * sizeof(T));
+  int64_t inner = 1;
+  for (size_t a = ax + 1; a < shp.size(); ++a) inner *= shp[a];
+  DBuf Q(ctx, want_q ? (size_t)rows * k * sizeof(T) : 0);
   R = DBuf(ctx, (size_t)k * cols * sizeof(T));
   DBuf tau(ctx, (size_t)k * sizeof(T));
-  nan_check<T>(ctx, M.p, w.size(v), "qr_axis/permute-in", v);
-  la::qr<T>(ctx, {la::QrJob{M.p, Q.p, R.p, tau.p, (int)rows, cols}});
-  nan_check<T>(ctx, Q.p, rows * k, "qr_axis/Q", v);
+  nan_check<T>(ctx, w.t[v].p, w.size(v), "qr_axis/tensor", v);
+  la::qr<T>(ctx, {la::QrJob{w.t[v].p, Q.p, R.p, tau.p, (int)rows, cols, inner > 1 ? (int)inner : 0}});
+  if (want_q) nan_check<T>(ctx, Q.p, rows * k, "qr_axis/Q", v);
   nan_check<T>(ctx, R.p, (int64_t)k * cols, "qr_axis/R", v);
-  std::vector<int> qshp = shp;
-  qshp.erase(qshp.begin() + ax);
-  qshp.push_back(k);
-  DBuf back(ctx, (size_t)rows * k * sizeof(T));
-  move_axis<T>(ctx, Q.p, back.p, qshp, (int)qshp.size() - 1, ax);
-  w.t[v] = std::move(back);
+  if (want_q) w.t[v] = std::move(Q);
   return k;
 }
 
+// (r_only: the roots' tensors alone are wanted)
 template <class T>
-void orthogonalize_to_roots(Work<T>& w) {
+void orthogonalize_to_roots(Work<T>& w, bool r_only = false) {
   for (int v = w.topo.V - 1; v >= 0; --v) {
     const int p = w.topo.parent[v];
     if (p < 0) continue;
     DBuf R;
     const int ax_p = w.child_axis(p, v);
-    const int k = qr_axis(w, v, 1, R);
+    const int k = qr_axis(w, v, 1, R, !r_only);
     absorb(w, p, ax_p, R.p, k);
+    if (r_only) w.t[v].reset();
     w.topo.link[v] = k;
   }
 }
@@ -209,6 +222,17 @@ struct TruncStats {
   int max_sweeps = 0;
   bool nonconv = false;
 };
+
+// Truncated factorisation of one bond matrix (overwritten).
+template <class T>
+la::FactorResult factor_bond(tnfa_ctx* ctx, void* M, int rows, int cols, const tnfa_trunc_params& prm, TruncStats& st) {
+  std::vector<la::FactorResult> res;
+  la::trunc_factor<T>(ctx, {la::FactorJob{M, rows, cols}}, prm.cutoff, prm.maxdim, prm.mindim, prm.precision, res);
+  if (res[0].sweeps < 0) st.nonconv = true;
+  st.max_sweeps = std::max(st.max_sweeps, res[0].sweeps);
+  st.max_discarded = std::max(st.max_discarded, res[0].discarded);
+  return std::move(res[0]);
+}
 
 // SVD of v's tensor across the bond to child c, truncated; the centre moves
 // into c.
@@ -223,13 +247,7 @@ void split_bond(Work<T>& w, int v, int c, const tnfa_trunc_params& prm, TruncSta
   const int rows = (int)rows64;
   DBuf M(ctx, (size_t)w.size(v) * sizeof(T));
   move_axis<T>(ctx, w.t[v].p, M.p, shp, ax, (int)shp.size() - 1);  // [rows][cols]
-  std::vector<la::FactorResult> res;
-  la::trunc_factor<T>(ctx, {la::FactorJob{M.p, rows, cols}}, prm.cutoff, prm.maxdim, prm.mindim,
-                      prm.precision, res);
-  la::FactorResult& o = res[0];
-  if (o.sweeps < 0) st.nonconv = true;
-  st.max_sweeps = std::max(st.max_sweeps, o.sweeps);
-  st.max_discarded = std::max(st.max_discarded, o.discarded);
+  const la::FactorResult o = factor_bond<T>(ctx, M.p, rows, cols, prm, st);
   const int r = o.r;
   std::vector<int> nshp = shp;
   nshp.erase(nshp.begin() + ax);
@@ -1177,6 +1195,57 @@ Dense mm(tnfa_ctx* ctx, const double* A, const double* B, int m, int n, int k, i
   return d;
 }
 
+// A tensor with its axes in another order, read in place.
+struct Axes {
+  const double* p;
+  std::vector<int> shp;
+  std::vector<int64_t> str;
+};
+Axes axes(const double* p, const std::vector<int>& shp, const std::vector<int>& order) {
+  Axes x{p, {}, {}};
+  std::vector<int64_t> st(shp.size(), 1);
+  for (int a = (int)shp.size() - 2; a >= 0; --a) st[a] = st[a + 1] * shp[a + 1];
+  for (int a : order) {
+    x.shp.push_back(shp[a]);
+    x.str.push_back(st[a]);
+  }
+  return x;
+}
+Axes axes(const Dense& d, const std::vector<int>& order) { return axes(d.p(), d.shp, order); }
+
+// The matrix of the first nr axes by the others; false: more than two strides
+// on a side.
+bool matrix_view(const Axes& x, int nr, la::MatView& v) {
+  auto side = [&](int a0, int a1, int& n1, int64_t& s1, int64_t& s0) {
+    std::vector<std::pair<int, int64_t>> g;  // (dim, stride), merged
+    for (int a = a0; a < a1; ++a) {
+      if (x.shp[a] == 1) continue;
+      if (!g.empty() && g.back().second == x.str[a] * x.shp[a]) g.back() = {g.back().first * x.shp[a], x.str[a]};
+      else g.push_back({x.shp[a], x.str[a]});
+    }
+    if (g.size() > 2) return false;
+    n1 = g.empty() ? 1 : g.back().first;
+    s0 = g.empty() ? 0 : g.back().second;
+    s1 = g.size() == 2 ? g[0].second : 0;
+    return true;
+  };
+  return side(0, nr, v.r1, v.R1, v.R0) && side(nr, (int)x.shp.size(), v.c1, v.C1, v.C0);
+}
+
+// C = A B, A's first ra axes by B's axes from kb on, the axes between summed.
+Dense mm(tnfa_ctx* ctx, const Axes& A, int ra, const Axes& B, int kb, std::vector<int> shp) {
+  Dense d;
+  d.shp = std::move(shp);
+  int m = 1, n = 1, k = 1;
+  for (size_t a = 0; a < A.shp.size(); ++a) ((int)a < ra ? m : k) *= A.shp[a];
+  for (size_t a = kb; a < B.shp.size(); ++a) n *= B.shp[a];
+  d.b = DBuf(ctx, (size_t)m * n * 8);
+  la::GemmJob j{A.p, B.p, d.b.p, m, n, k, k, n, n, 0, 0, 1.0, 0.0};
+  TNFA_CHECK(matrix_view(A, ra, j.va) && matrix_view(B, kb, j.vb), TNFA_ERR_UNSUPPORTED, "product: axes too scattered");
+  la::gemm<double>(ctx, {j});
+  return d;
+}
+
 Dense ones(tnfa_ctx* ctx, std::vector<int> shp) {
   Dense d;
   d.shp = std::move(shp);
@@ -1209,19 +1278,19 @@ void left_env(LinsolveState& S, int i) {
   const int l = S.bond(S.x, i), r = S.bond(S.x, i + 1);
   const int wl = S.bond(S.A, i), wr = S.bond(S.A, i + 1);
   const double* xi = S.x.t[i].as<double>();
-  Dense xp = permuted(ctx, xi, {d, l, r}, {1, 0, 2});                     // [l][s][r]
-  Dense t1 = mm(ctx, S.LA[i].p(), xp.p(), l * wl, d * r, l, 0, 0, {l, wl, d, r});  // [l'][wl][s][r]
-  Dense t1p = permuted(ctx, t1.p(), t1.shp, {0, 3, 1, 2});                // [l'][r][wl][s]
-  Dense Ap = permuted(ctx, S.A.t[i].as<double>(), {d, d, wl, wr}, {2, 1, 0, 3});  // [wl][s][o][wr]
-  Dense t2 = mm(ctx, t1p.p(), Ap.p(), l * r, d * wr, wl * d, 0, 0, {l, r, d, wr});  // [l'][r][o][wr]
-  Dense t2p = permuted(ctx, t2.p(), t2.shp, {2, 0, 3, 1});                // [o][l'][wr][r]
-  S.LA[i + 1] = mm(ctx, xi, t2p.p(), r, wr * r, d * l, 1, 0, {r, wr, r});
+  const Axes x3 = axes(xi, {d, l, r}, {0, 1, 2});  // [s][l][r]
+  Dense t1 = mm(ctx, axes(S.LA[i], {0, 1, 2}), 2, axes(xi, {d, l, r}, {1, 0, 2}), 1, {l, wl, d, r});  // [l'][wl][s][r]
+  Dense t2 = mm(ctx, axes(t1, {0, 3, 1, 2}), 2,                                     // [l'][r][wl][s]
+                axes(S.A.t[i].as<double>(), {d, d, wl, wr}, {2, 1, 0, 3}), 2, {l, r, d, wr});  // [wl][s][o][wr]
+  Axes xt = x3;  // [r'][o l']
+  std::rotate(xt.shp.begin(), xt.shp.begin() + 2, xt.shp.end());
+  std::rotate(xt.str.begin(), xt.str.begin() + 2, xt.str.end());
+  S.LA[i + 1] = mm(ctx, xt, 1, axes(t2, {2, 0, 3, 1}), 2, {r, wr, r});              // [o][l'][wr][r]
   if (!S.has_b) return;
   const int bl = S.bond(S.b, i), br = S.bond(S.b, i + 1);
-  Dense bp = permuted(ctx, S.b.t[i].as<double>(), {d, bl, br}, {1, 0, 2});  // [bl][s][br]
-  Dense u1 = mm(ctx, S.Lb[i].p(), bp.p(), l, d * br, bl, 0, 0, {l, d, br});   // [l'][s][br]
-  Dense u1p = permuted(ctx, u1.p(), u1.shp, {1, 0, 2});                   // [s][l'][br]
-  S.Lb[i + 1] = mm(ctx, xi, u1p.p(), r, br, d * l, 1, 0, {r, br});
+  Dense u1 = mm(ctx, axes(S.Lb[i], {0, 1}), 1, axes(S.b.t[i].as<double>(), {d, bl, br}, {1, 0, 2}), 1,
+                {l, d, br});                                                        // [l'][s][br]
+  S.Lb[i + 1] = mm(ctx, xt, 1, axes(u1, {1, 0, 2}), 2, {r, br});                    // [s][l'][br]
 }
 
 // RA_i and Rb_i from RA_{i+1}, Rb_{i+1} and the right-orthonormal x_i.
@@ -1231,19 +1300,15 @@ void right_env(LinsolveState& S, int i) {
   const int l = S.bond(S.x, i), r = S.bond(S.x, i + 1);
   const int wl = S.bond(S.A, i), wr = S.bond(S.A, i + 1);
   const double* xi = S.x.t[i].as<double>();
-  Dense Rp = permuted(ctx, S.RA[i + 1].p(), S.RA[i + 1].shp, {2, 0, 1});  // [r][r'][wr]
-  Dense t1 = mm(ctx, xi, Rp.p(), d * l, r * wr, r, 0, 0, {d, l, r, wr});  // [s][l][r'][wr]
-  Dense t1p = permuted(ctx, t1.p(), t1.shp, {0, 3, 1, 2});                // [s][wr][l][r']
-  Dense Ap = permuted(ctx, S.A.t[i].as<double>(), {d, d, wl, wr}, {0, 2, 1, 3});  // [o][wl][s][wr]
-  Dense t2 = mm(ctx, Ap.p(), t1p.p(), d * wl, l * r, d * wr, 0, 0, {d, wl, l, r});  // [o][wl][l][r']
-  Dense t2p = permuted(ctx, t2.p(), t2.shp, {0, 3, 1, 2});                // [o][r'][wl][l]
-  Dense xp = permuted(ctx, xi, {d, l, r}, {1, 0, 2});                     // [l'][o][r']
-  S.RA[i] = mm(ctx, xp.p(), t2p.p(), l, wl * l, d * r, 0, 0, {l, wl, l});
+  Dense t1 = mm(ctx, axes(xi, {d, l, r}, {0, 1, 2}), 2, axes(S.RA[i + 1], {2, 0, 1}), 1, {d, l, r, wr});  // [s][l][r'][wr]
+  Dense t2 = mm(ctx, axes(S.A.t[i].as<double>(), {d, d, wl, wr}, {0, 2, 1, 3}), 2,  // [o][wl][s][wr]
+                axes(t1, {0, 3, 1, 2}), 2, {d, wl, l, r});                          // [s][wr][l][r']
+  const Axes xp = axes(xi, {d, l, r}, {1, 0, 2});                                   // [l'][o][r']
+  S.RA[i] = mm(ctx, xp, 1, axes(t2, {0, 3, 1, 2}), 2, {l, wl, l});                  // [o][r'][wl][l]
   if (!S.has_b) return;
   const int bl = S.bond(S.b, i), br = S.bond(S.b, i + 1);
   Dense v1 = mm(ctx, S.b.t[i].as<double>(), S.Rb[i + 1].p(), d * bl, r, br, 0, 1, {d, bl, r});
-  Dense v1p = permuted(ctx, v1.p(), v1.shp, {0, 2, 1});                   // [s][r'][bl]
-  S.Rb[i] = mm(ctx, xp.p(), v1p.p(), l, bl, d * r, 0, 0, {l, bl});
+  S.Rb[i] = mm(ctx, xp, 1, axes(v1, {0, 2, 1}), 2, {l, bl});                        // [s][r'][bl]
 }
 
 // y += a x
@@ -1282,12 +1347,10 @@ Dense local_H(LinsolveState& S, int i, double a0, double a1, const char* what) {
                  " above the dense limit " + std::to_string(kLocalDenseMax) + " (lower maxdim)");
   const int n = (int)n64;
   // H[l' s1' s2' r'][l s1 s2 r] = LA_i A_i A_{i+1} RA_{i+2}
-  Dense Lp = permuted(ctx, S.LA[i].p(), S.LA[i].shp, {0, 2, 1});                       // [l'][l][wl]
-  Dense A1 = permuted(ctx, S.A.t[i].as<double>(), {d, d, wl, wm}, {2, 0, 1, 3});      // [wl][o][in][wm]
-  Dense P1 = mm(ctx, Lp.p(), A1.p(), l * l, d * d * wm, wl, 0, 0, {l, l, d, d, wm});
-  Dense A2 = permuted(ctx, S.A.t[i + 1].as<double>(), {d, d, wm, wr}, {2, 0, 1, 3});  // [wm][o][in][wr]
-  Dense Rp = permuted(ctx, S.RA[i + 2].p(), S.RA[i + 2].shp, {1, 0, 2});              // [wr][r'][r]
-  Dense P2 = mm(ctx, A2.p(), Rp.p(), wm * d * d, r * r, wr, 0, 0, {wm, d, d, r, r});
+  Dense P1 = mm(ctx, axes(S.LA[i], {0, 2, 1}), 2,                                    // [l'][l][wl]
+                axes(S.A.t[i].as<double>(), {d, d, wl, wm}, {2, 0, 1, 3}), 1, {l, l, d, d, wm});  // [wl][o][in][wm]
+  Dense P2 = mm(ctx, axes(S.A.t[i + 1].as<double>(), {d, d, wm, wr}, {2, 0, 1, 3}), 3,  // [wm][o][in][wr]
+                axes(S.RA[i + 2], {1, 0, 2}), 1, {wm, d, d, r, r});                     // [wr][r'][r]
   Dense Hr = mm(ctx, P1.p(), P2.p(), l * l * d * d, d * d * r * r, wm, 0, 0,
                 {l, l, d, d, d, d, r, r});  // [l'][l][s1'][s1][s2'][s2][r'][r]
   Dense H = permuted(ctx, Hr.p(), Hr.shp, {0, 2, 4, 6, 1, 3, 5, 7});
@@ -1304,31 +1367,13 @@ void store_two_site(LinsolveState& S, int i, const Dense& v, const tnfa_trunc_pa
   tnfa_ctx* ctx = S.ctx;
   const int d = S.d;
   const int l = S.bond(S.x, i), r = S.bond(S.x, i + 2);
-  // a two-vertex work: vertex 0 = v as [(l s1)][1][(s2 r)], vertex 1 = the
-  // identity on (s2 r); split_bond leaves U in vertex 0 and S V^T in vertex 1
-  Work<double> two{ctx, Topo{}, {}};
-  two.topo.V = 2;
-  two.topo.parent = {-1, 0};
-  two.topo.link = {1, d * r};
-  two.topo.nlegs = {0, 0};
-  two.topo.finalize();
-  two.topo.site_dim = {l * d, d * r};
-  const int64_t nv = (int64_t)l * d * d * r;
-  two.t.emplace_back(ctx, (size_t)nv * 8);
-  TNFA_CUDA(cudaMemcpyAsync(two.t[0].p, v.p(), (size_t)nv * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-  {
-    const int q = d * r;
-    std::vector<double> eye((size_t)q * q, 0.0);
-    for (int k = 0; k < q; ++k) eye[(size_t)k * q + k] = 1.0;
-    two.t.emplace_back(ctx, eye.size() * 8);
-    TNFA_CUDA(cudaMemcpyAsync(two.t[1].p, eye.data(), eye.size() * 8, cudaMemcpyHostToDevice,
-                              ctx->stream));
-    TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
-  }
-  split_bond(two, 0, 1, tp, st);
-  const int k = two.topo.link[1];
-  Dense x0 = permuted(ctx, two.t[0].as<double>(), {l, d, k}, {1, 0, 2});  // [s1][l][k]
-  Dense x1 = permuted(ctx, two.t[1].as<double>(), {d, r, k}, {0, 2, 1});  // [s2][k][r]
+  // L [l][s1][k] and X [k][s2][r]; v stays the caller's
+  DBuf M(ctx, (size_t)l * d * d * r * 8);
+  TNFA_CUDA(cudaMemcpyAsync(M.p, v.p(), (size_t)l * d * d * r * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+  const la::FactorResult f = factor_bond<double>(ctx, M.p, l * d, d * r, tp, st);
+  const int k = f.r;
+  Dense x0 = permuted(ctx, f.L.as<double>(), {l, d, k}, {1, 0, 2});  // [s1][l][k]
+  Dense x1 = permuted(ctx, f.X.as<double>(), {k, d, r}, {1, 0, 2});  // [s2][k][r]
   S.x.t[i] = std::move(x0.b);
   S.x.t[i + 1] = std::move(x1.b);
   S.x.topo.link[i + 1] = k;
@@ -1581,9 +1626,8 @@ Dense two_site(LinsolveState& S, int i) {
   tnfa_ctx* ctx = S.ctx;
   const int d = S.d;
   const int l = S.bond(S.x, i), k = S.bond(S.x, i + 1), r = S.bond(S.x, i + 2);
-  Dense a = permuted(ctx, S.x.t[i].as<double>(), {d, l, k}, {1, 0, 2});      // [l][s1][k]
-  Dense b = permuted(ctx, S.x.t[i + 1].as<double>(), {d, k, r}, {1, 0, 2});  // [k][s2][r]
-  return mm(ctx, a.p(), b.p(), l * d, d * r, k, 0, 0, {l, d, d, r});
+  return mm(ctx, axes(S.x.t[i].as<double>(), {d, l, k}, {1, 0, 2}), 2,         // [l][s1][k]
+            axes(S.x.t[i + 1].as<double>(), {d, k, r}, {1, 0, 2}), 1, {l, d, d, r});  // [k][s2][r]
 }
 
 // Solve the projected system at bond (i, i+1); returns v [l][s1][s2][r].
@@ -1596,10 +1640,10 @@ Dense local_solve(LinsolveState& S, int i, double a0, double a1) {
   const int n = (int)n64;
   // g[l][s1][s2][r] = Lb_i b_i b_{i+1} Rb_{i+2}
   const int bl = S.bond(S.b, i), bm = S.bond(S.b, i + 1), br = S.bond(S.b, i + 2);
-  Dense b1 = permuted(ctx, S.b.t[i].as<double>(), {d, bl, bm}, {1, 0, 2});      // [bl][s][bm]
-  Dense G1 = mm(ctx, S.Lb[i].p(), b1.p(), l, d * bm, bl, 0, 0, {l, d, bm});
-  Dense b2 = permuted(ctx, S.b.t[i + 1].as<double>(), {d, bm, br}, {1, 0, 2});  // [bm][s][br]
-  Dense G2 = mm(ctx, G1.p(), b2.p(), l * d, d * br, bm, 0, 0, {l, d, d, br});
+  Dense G1 = mm(ctx, axes(S.Lb[i], {0, 1}), 1, axes(S.b.t[i].as<double>(), {d, bl, bm}, {1, 0, 2}), 1,
+                {l, d, bm});                                                              // [bl][s][bm]
+  Dense G2 = mm(ctx, axes(G1, {0, 1, 2}), 2, axes(S.b.t[i + 1].as<double>(), {d, bm, br}, {1, 0, 2}), 1,
+                {l, d, d, br});                                                           // [bm][s][br]
   Dense g = mm(ctx, G2.p(), S.Rb[i + 2].p(), l * d * d, r, br, 0, 1, {l, d, d, r});
   if (n64 <= kLocalDenseMax && !force_matrix_free()) {
     Dense H = local_H(S, i, a0, a1, "linsolve");
@@ -1617,7 +1661,7 @@ Dense local_solve(LinsolveState& S, int i, double a0, double a1) {
 // ||net|| through a QR sweep toward the root (backward stable).
 double qr_norm(tnfa_ctx* ctx, const tnfa_net* net) {
   Work<double> w = load_work<double>(ctx, net);
-  orthogonalize_to_roots(w);
+  orthogonalize_to_roots(w, true);
   double s2 = 0;
   for (int r : w.topo.roots()) {
     const double x = host_norm<double>(ctx, w.t[r], w.size(r));
