@@ -2385,21 +2385,19 @@ __global__ void __launch_bounds__(512) k_lu_small(const double* __restrict__ Ag,
     const int kb = min(LU_RB, n - k);
     for (int j = k; j < k + kb; ++j) {
       // the largest |entry| on or below the diagonal, the first of equals
-      // (ordered as integers; a NaN is never larger)
-      long long best = -1;
+      // (ordered as integers, high and low word; a NaN is never larger)
+      unsigned bh = 0, bl = 0;
       int p = j;
       for (int r = j + lane; r < n; r += 32) {
         const double x = fabs(P[r * ld + j]);
-        const long long key = x == x ? __double_as_longlong(x) : -1;
-        if (key > best) best = key, p = r;
+        if (!(x == x)) continue;
+        const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+        if (h > bh || (h == bh && l > bl)) bh = h, bl = l, p = r;
       }
-      for (int o = 16; o; o >>= 1) {
-        const long long ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int op = __shfl_xor_sync(0xffffffffu, p, o);
-        if (ob > best || (ob == best && op < p)) best = ob, p = op;
-      }
-      if (best < 0) p = j;
-      if (!(best > 0)) sing = true;
+      const unsigned mh = __reduce_max_sync(0xffffffffu, bh);
+      const unsigned ml = __reduce_max_sync(0xffffffffu, bh == mh ? bl : 0u);
+      p = (int)__reduce_min_sync(0xffffffffu, bh == mh && bl == ml ? (unsigned)p : 0xffffffffu);
+      if (mh == 0 && ml == 0) p = j, sing = true;
       __syncthreads();
       if (threadIdx.x == 0) piv[j] = p;
       if (p != j)
