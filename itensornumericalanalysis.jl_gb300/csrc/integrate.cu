@@ -74,12 +74,12 @@ __global__ void k_site_reduce<cplx>(const cplx* __restrict__ src, cplx* __restri
 // 32 * NCH * VE entries and 8 / NCH loads are in flight per lane.
 //
 // Bound by HBM at large bonds in FP32 and by the FP64 pipe in FP64 (one FMA per
-// entry, 203 us of the 306 below: there the rows are summed with their weights
+// entry, 203 us of the 295 below: there the rows are summed with their weights
 // before the last child's message comes in, once per task).  A call on
 // the 60-vertex binary tree, against one persistent launch fed by bulk copies
 // whose consumers waited for their children's flags task by task: bond 128
-// (117 M entries) FP32 133 us (194), FP64 306 us (350); bond 48 FP32 106 us (129);
-// path of 60 vertices, bond 256, FP64 393 us (1312), bond 6 235 us (425).
+// (117 M entries) FP32 121 us (194), FP64 295 us (350); bond 48 FP32 50 us (129);
+// path of 60 vertices, bond 256, FP64 389 us (1312), bond 6 236 us (425).
 template <class T> struct IntAcc { using type = double; };
 template <> struct IntAcc<cplx> { using type = cplx; };
 __device__ inline void atomicAddAcc(double* a, double v) { atomicAdd(a, v); }
@@ -476,7 +476,7 @@ void integrate_levels(tnfa_ctx* ctx, const tnfa_net* net, int take_sum, double* 
   // are not 16-byte aligned, take the generic path)
   int nch = 1;
   while (nch < 8 && 32 * VE * nch < maxlast) nch *= 2;
-  const int64_t warps = (int64_t)ctx->sm_count * 32;
+  const int64_t slots = (int64_t)ctx->sm_count * INT_WARPS * (sizeof(T) == 16 ? 2 : 3);
   {
     KernelScope ks(ctx, "integrate", 2.0 * (double)Tp.n_elem, (double)dtype_size(net->dtype) * Tp.n_elem);
     bool first = true;
@@ -491,8 +491,23 @@ void integrate_levels(tnfa_ctx* ctx, const tnfa_net* net, int take_sum, double* 
         for (size_t c = 0; c + 1 < Tp.children[v].size(); ++c) r *= Tp.link[Tp.children[v][c]];
         if (!Tp.children[v].empty()) rows += r * Tp.site_dim[v] * Tp.link[v];
       }
-      int kb = 1;
-      while (kb < 32 && kb * 2 <= rows / (2 * warps)) kb *= 2;
+      // Rows per task: the level in w full waves of the warps the GPU holds, w
+      // the one with the least w (rows + about three loads of rows, a block's
+      // start).  Powers of two left a second wave of a few blocks at the narrow
+      // levels (60-vertex binary tree, bond 128, FP32: @KB@).
+      const int start = 3 * (nch >= 8 ? 1 : 8 / nch) * std::max(1, 32 * VE / std::max(1, maxlast));
+      int kb = 32;
+      int64_t least = -1;
+      for (int w = 1; w <= 8; ++w) {
+        const int64_t k = std::max<int64_t>(1, (rows + slots * w - 1) / (slots * w));
+        if (k > 32) continue;
+        const int64_t cost = w * (k + start);
+        if (least < 0 || cost < least) {
+          least = cost;
+          kb = (int)k;
+        }
+        if (k == 1) break;
+      }
       int nc = 0;
       int64_t blocks = 0;
       size_t smem = 0;
@@ -538,8 +553,11 @@ void integrate_levels(tnfa_ctx* ctx, const tnfa_net* net, int take_sum, double* 
         iv.last = cs.empty() ? 1 : Tp.link[cs.back()];
         iv.kb = iv.nkb = 1;
         if (!cs.empty()) {
-          iv.kb = (int)std::min<int64_t>(kb, kouter);
-          const int64_t nkb = (kouter + iv.kb - 1) / iv.kb;
+          // the tasks of an (s, a) of even length, as many as stay within the wave
+          int64_t nkb = std::max<int64_t>(1, kouter / kb);
+          if ((kouter + nkb - 1) / nkb > 32) nkb = (kouter + 31) / 32;
+          iv.kb = (int)((kouter + nkb - 1) / nkb);
+          nkb = (kouter + iv.kb - 1) / iv.kb;
           ntask = (int64_t)iv.sd * iv.chi_a * nkb;
           TNFA_CHECK(ntask < (int64_t(1) << 31) - 64, TNFA_ERR_UNSUPPORTED, "integrate: vertex too large");
           iv.nkb = (int)nkb;
