@@ -1787,23 +1787,33 @@ class EvalEngine {
     const bool shared = W.chi * sizeof(T) <= 64 && sm <= 48 * 1024 &&
                         (double)n >= 8.0 * (W.na + W.nb) * ctx_->sm_count;
     const unsigned grid = grid_for(n, 256, ctx_->sm_count * (shared ? 4 : 8));
-    auto go = [&](auto kern, auto kern_sm) {
-      if (shared) kern_sm<<<grid, 256, sm, ctx_->stream>>>(W);
-      else kern<<<grid, 256, 0, ctx_->stream>>>(W);
+    bool few = W.nruns >= 1 && W.nruns <= 2;
+    for (int i = 0; i < std::min(W.nruns, 2); ++i) few &= W.runs[i].bits != 0;
+    auto run = [&](auto kern, size_t bytes) { kern<<<grid, 256, bytes, ctx_->stream>>>(W); };
+    auto go = [&](auto g, auto v, auto may_share) {
+      constexpr int GG = decltype(g)::value, VV = decltype(v)::value;
+      if constexpr (decltype(may_share)::value) {
+        if (shared) {
+          few ? run(k_centre_pair<T, GG, VV, true, true>, sm) : run(k_centre_pair<T, GG, VV, true, false>, sm);
+          return;
+        }
+      }
+      few ? run(k_centre_pair<T, GG, VV, false, true>, 0) : run(k_centre_pair<T, GG, VV, false, false>, 0);
     };
+    using std::integral_constant;
     if constexpr (vec > 1) {
       if (centre_vec_) {
         const int lanes = (W.chi + vec - 1) / vec;
-        if (lanes <= 2) go(k_centre_pair<T, 1, vec, false>, k_centre_pair<T, 1, vec, true>);
-        else if (lanes <= 4) go(k_centre_pair<T, 4, vec, false>, k_centre_pair<T, 4, vec, true>);
-        else go(k_centre_pair<T, 8, vec, false>, k_centre_pair<T, 8, vec, false>);
+        if (lanes <= 2) go(integral_constant<int, 1>{}, integral_constant<int, vec>{}, std::true_type{});
+        else if (lanes <= 4) go(integral_constant<int, 4>{}, integral_constant<int, vec>{}, std::true_type{});
+        else go(integral_constant<int, 8>{}, integral_constant<int, vec>{}, std::false_type{});
         TNFA_LAUNCH_CHECK();
         return;
       }
     }
-    if (W.chi <= 4) go(k_centre_pair<T, 1, 1, false>, k_centre_pair<T, 1, 1, true>);
-    else if (W.chi <= 8) go(k_centre_pair<T, 4, 1, false>, k_centre_pair<T, 4, 1, true>);
-    else go(k_centre_pair<T, 8, 1, false>, k_centre_pair<T, 8, 1, true>);
+    if (W.chi <= 4) go(integral_constant<int, 1>{}, integral_constant<int, 1>{}, std::true_type{});
+    else if (W.chi <= 8) go(integral_constant<int, 4>{}, integral_constant<int, 1>{}, std::true_type{});
+    else go(integral_constant<int, 8>{}, integral_constant<int, 1>{}, std::true_type{});
     TNFA_LAUNCH_CHECK();
   }
 

@@ -56,8 +56,7 @@ __global__ void k_site_reduce<cplx>(const cplx* __restrict__ src, cplx* __restri
 // reads it than a launch does, so it has no height of its own.
 //
 // A block belongs to one vertex and its 8 warps take a task each: up to kb <= 32
-// consecutive rows (s, a, k) with the same (s, a), kb chosen so that the level
-// has about two tasks per warp the GPU holds.  A warp issues the loads of its
+// consecutive rows (s, a, k) with the same (s, a).  A warp issues the loads of its
 // first rows, and only then the block waits for the launch before it
 // (programmatic dependent launch: the next level's blocks start, and their
 // tensors stream in, while this level's last tasks run).  The block brings the
@@ -494,7 +493,8 @@ void integrate_levels(tnfa_ctx* ctx, const tnfa_net* net, int take_sum, double* 
       // Rows per task: the level in w full waves of the warps the GPU holds, w
       // the one with the least w (rows + about three loads of rows, a block's
       // start).  Powers of two left a second wave of a few blocks at the narrow
-      // levels (60-vertex binary tree, bond 128, FP32: @KB@).
+      // levels and tasks of 4 rows at the middle ones (60-vertex binary tree,
+      // FP32: bond 128 133 -> 121 us, bond 48 106 -> 50 us).
       const int start = 3 * (nch >= 8 ? 1 : 8 / nch) * std::max(1, 32 * VE / std::max(1, maxlast));
       int kb = 32;
       int64_t least = -1;

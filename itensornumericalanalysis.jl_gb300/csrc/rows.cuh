@@ -524,7 +524,7 @@ __device__ inline void write_out(void* out, int kind, int64_t p, int64_t P, T v,
 template <>
 __device__ inline void write_out<double>(void* out, int kind, int64_t p, int64_t P, double v, int e) {
   if (kind == TNFA_OUT_F64) {
-    ((double*)out)[p] = scale_pow2(v, e);
+    ((double*)out)[p] = e ? scale_pow2(v, e) : v;
   } else if (kind == TNFA_OUT_F32) {
     ((float*)out)[p] = (float)scale_pow2(v, e);
   } else {  // scaled f32
@@ -684,7 +684,13 @@ struct PairParams {
 // SM: both tables are copied to shared memory first.  A gather of 32 different
 // rows costs a cache line per lane in L1 (32 cycles), a few bank conflicts
 // there.
-template <class T, int G, int VEC, bool SM>
+// FEW: at most two runs, both bit fields (a side's digits are one block of a
+// variable's): their fields stay in registers and the next point's coordinates
+// are on their way while this one's rows are summed.  With the loop over run
+// records, and each thread waiting for its coordinate, 10^7 points at bond 2
+// took 104 us of k_centre_pair (256 instructions a point), now 63 (180), of
+// which the two multiply-adds a point are 34.
+template <class T, int G, int VEC, bool SM, bool FEW>
 __global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ PairParams<T> W) {
   extern __shared__ __align__(16) unsigned char pair_sh[];
   const int lane = threadIdx.x & 31, l = lane % G;
@@ -704,11 +710,47 @@ __global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ Pai
   const int* xa_ = W.ea && !(W.pa && *W.pa) ? W.ea : nullptr;
   const int* xb_ = W.eb && !(W.pb && *W.pb) ? W.eb : nullptr;
   constexpr int PG = 32 / G;  // points per pass
-  for (int64_t base = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) - lane; base < W.Pc;
-       base += (int64_t)gridDim.x * blockDim.x) {
-    const int p = (int)min((int64_t)W.Pc - 1, base + lane);  // the padding lanes repeat the last point
+  // (unsigned: below 2^31 points, and a grid's step more stays below 2^32)
+  const unsigned Pc = (unsigned)W.Pc, step = gridDim.x * blockDim.x;
+  const unsigned base0 = blockIdx.x * blockDim.x + threadIdx.x - lane;
+  const bool two = W.nruns > 1, own = two && W.runs[1].start;  // the second run's column is its own
+  const int f0 = W.runs[0].first - 1, n0 = 32 - W.runs[0].n, w0 = W.runs[0].w, r0 = W.runs[0].rev;
+  const int f1 = two ? W.runs[1].first - 1 : 0, n1 = two ? 32 - W.runs[1].n : 0, w1 = two ? W.runs[1].w : 0;
+  const int r1 = two ? W.runs[1].rev : 0;
+  const bool a0 = W.runs[0].slot == W.sa, a1 = two && W.runs[1].slot == W.sa;
+  double x0 = 0.0, x1 = 0.0;
+  auto fetch = [&](unsigned b) {
+    const double* Xp = W.X + (int64_t)min(Pc - 1, b + lane) * W.ncols;  // the padding lanes repeat the last point
+    x0 = Xp[W.runs[0].col];
+    if (own) x1 = Xp[W.runs[1].col];
+  };
+  auto in_domain = [&](double& x) {
+    const unsigned long long xb = (unsigned long long)__double_as_longlong(x);
+    if (xb > 0x8000000000000000ull || (xb & 0x7FF0000000000000ull) == 0x7FF0000000000000ull) {
+      raise_domain(W.err);
+      x = 0.0;
+    }
+  };
+  if (FEW && base0 < Pc) fetch(base0);
+  for (unsigned base = base0; base < Pc; base += step) {
+    const int p = (int)min(Pc - 1, base + lane);
     int c[2] = {0, 0};
-    {
+    if constexpr (FEW) {
+      double xa = x0, xb = x1;
+      if (base + step < Pc) fetch(base + step);
+      in_domain(xa);
+      const unsigned long long u = unit_fraction(xa);
+      unsigned long long v = u;
+      if (own) {
+        in_domain(xb);
+        v = unit_fraction(xb);
+      }
+      const unsigned g0 = (unsigned)((u << f0) >> 32), g1 = (unsigned)((v << f1) >> 32);
+      const int c0 = (int)(r0 ? __brev(g0) & (0xFFFFFFFFu >> n0) : g0 >> n0) * w0;
+      const int c1 = (int)(r1 ? __brev(g1) & (0xFFFFFFFFu >> n1) : g1 >> n1) * w1;
+      c[0] = (a0 ? c0 : 0) + (a1 ? c1 : 0);
+      c[1] = (a0 ? 0 : c0) + (a1 ? 0 : c1);
+    } else {
       double xr = 0.0;
       unsigned long long u = 0;
       for (int e = 0; e < W.nruns; ++e) {
@@ -749,8 +791,8 @@ __global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ Pai
       const int t = i * PG + lane / G;  // the point of this pass
       const int ra = G == 1 ? c[0] : __shfl_sync(0xffffffffu, c[0], t);
       const int rb = G == 1 ? c[1] : __shfl_sync(0xffffffffu, c[1], t);
-      const T* A = tabA + (int64_t)ra * W.chi;
-      const T* B = tabB + (int64_t)rb * W.chi;
+      const T* A = SM ? tabA + ra * W.chi : tabA + (int64_t)ra * W.chi;
+      const T* B = SM ? tabB + rb * W.chi : tabB + (int64_t)rb * W.chi;
       int e = (xa_ ? xa_[ra] : 0) + (xb_ ? xb_[rb] : 0), ea = 0, eb = 0;
       if (W.scale) {
         typename Real<T>::t ma = 0, mb = 0;
@@ -768,19 +810,27 @@ __global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ Pai
         e += ea + eb;
       }
       T s = Sc<T>::zero();
-      for (int k = l * VEC; k < W.chi; k += G * VEC) {
-        T xa[VEC], xb[VEC];
-        if constexpr (VEC > 1) {
-          *reinterpret_cast<int4*>(xa) = *reinterpret_cast<const int4*>(A + k);
-          *reinterpret_cast<int4*>(xb) = *reinterpret_cast<const int4*>(B + k);
-        } else {
-          xa[0] = A[k];
-          xb[0] = B[k];
-        }
+      auto dot = [&](auto scaled) {
+        for (int k = l * VEC; k < W.chi; k += G * VEC) {
+          T xa[VEC], xb[VEC];
+          if constexpr (VEC > 1) {
+            *reinterpret_cast<int4*>(xa) = *reinterpret_cast<const int4*>(A + k);
+            *reinterpret_cast<int4*>(xb) = *reinterpret_cast<const int4*>(B + k);
+          } else {
+            xa[0] = A[k];
+            xb[0] = B[k];
+          }
 #pragma unroll
-        for (int q = 0; q < VEC; ++q)
-          s = Sc<T>::fma(ea ? scale_pow2(xa[q], -ea) : xa[q], eb ? scale_pow2(xb[q], -eb) : xb[q], s);
-      }
+          for (int q = 0; q < VEC; ++q) {
+            if constexpr (decltype(scaled)::value)
+              s = Sc<T>::fma(ea ? scale_pow2(xa[q], -ea) : xa[q], eb ? scale_pow2(xb[q], -eb) : xb[q], s);
+            else
+              s = Sc<T>::fma(xa[q], xb[q], s);
+          }
+        }
+      };
+      if (W.scale) dot(std::true_type{});
+      else dot(std::false_type{});
 #pragma unroll
       for (int o = G / 2; o; o >>= 1) s = s + shfl_x(s, o);
       // hand the sum to the point's own lane
@@ -797,7 +847,7 @@ __global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ Pai
         }
       }
     }
-    if (base + lane < W.Pc) write_out<T>(W.out, W.kind, W.p0 + base + lane, W.P, v, ve);
+    if (base + lane < Pc) write_out<T>(W.out, W.kind, W.p0 + base + lane, W.P, v, ve);
   }
 }
 
