@@ -277,10 +277,10 @@ def _timed(fn, reps=1):
 
 def integrate_rates(f32net, f64net, peaks) -> dict:
     """integrate() over [0,1)^3 of the benchmark network: the HBM-bound member
-    of the path (one persistent k_integrate launch reads every tensor byte
+    of the path (the k_integrate_level launches read every tensor byte
     once), FP32 and FP64 copies.  Per call: CUDA events on the current stream
     around 5 calls (host set-up and the read-back included); per kernel: the
-    library's own CUDA events around each k_integrate launch (on its
+    library's own CUDA events around a call's k_integrate_level launches (on its
     stream)."""
     import torch
 

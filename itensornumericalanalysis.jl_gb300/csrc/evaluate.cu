@@ -6,18 +6,22 @@
 // (one-hot slice of every site leg, :84-94) -> scalar(tn; alg="bp") (exact on
 // a tree).  It handles one point per call.
 //
-// Here all points of a chunk go through the tree vertex by vertex (children
-// before parents):
-//   1. k_digitize: coordinates -> site value s_v(p) of every vertex (u8).
-//   2. per vertex: group the points by s_v (count / scan / scatter), so that a
-//      tile of points shares one slice T_v[s].
-//   3. per vertex: out[p, a] = sum_k A[p, k] T_v[s][a][k] with A the row-wise
-//      Kronecker product of the children's messages.  Leaves are never
-//      materialised: a parent reads the leaf slice T_leaf[s_leaf(p)] directly.
-//      Each message row is rescaled by a power of two when it is read (exact)
-//      and the exponent is carried per point, so deep trees neither underflow
-//      nor overflow.
-//   4. k_combine: product over the roots of the forest, times 2^exponent.
+// Here a message is formed once for every combination of the digits below its
+// edge where there are fewer combinations than points, and once per point
+// elsewhere (the schedule: eval_tree.cuh; EvalEngine lays it out and runs it):
+//   1. tables, level by level: row r of a vertex is its message for digit
+//      combination r; the products of a level are one launch.
+//   2. k_digitize: coordinates -> the codes (table rows, site values) that the
+//      points read (in the kernels of 4 where those do it themselves).
+//   3. vertices without a table, per chunk of points: group the points by site
+//      value (count / scan / scatter), so that a tile of points shares one slice
+//      T_v[s]; out[p, a] = sum_k A[p, k] T_v[s][a][k] with A the row-wise
+//      Kronecker product of the children's messages, read from their tables by
+//      code.  At small bonds one launch walks a point through all of them.
+//   4. the centre, any one edge: f(p) = sum_c A[p, c] B[p, c] over the two
+//      messages that meet there, times the other components' values.
+// Each row is rescaled by a power of two when it is made or read (exact) and the
+// exponent is carried per row, so deep trees neither underflow nor overflow.
 #include <algorithm>
 #include <memory>
 #include <type_traits>
