@@ -70,15 +70,16 @@ __global__ void k_site_reduce<cplx>(const cplx* __restrict__ src, cplx* __restri
 // Row loads are 16-byte vectors (4 FP32, 2 FP64 or 1 complex value per lane)
 // when the vertex's rows allow it; G = 2^lg lanes share a row (rows of few
 // vectors leave no lane idle), NCH vectors a lane cover a row of up to
-// 32 * NCH * VE entries and 8 / NCH loads are in flight per lane.
+// 32 * NCH * VE entries and max(NCH, 4) loads are in flight per lane (twice as
+// many and 24 instead of 32 warps per SM took 121 us where this takes 115).
 //
 // Bound by HBM at large bonds in FP32 and by the FP64 pipe in FP64 (one FMA per
-// entry, 203 us of the 295 below: there the rows are summed with their weights
+// entry, 203 us of the 284 below: there the rows are summed with their weights
 // before the last child's message comes in, once per task).  A call on
 // the 60-vertex binary tree, against one persistent launch fed by bulk copies
 // whose consumers waited for their children's flags task by task: bond 128
-// (117 M entries) FP32 121 us (194), FP64 295 us (350); bond 48 FP32 50 us (129);
-// path of 60 vertices, bond 256, FP64 389 us (1312), bond 6 236 us (425).
+// (117 M entries) FP32 117 us (194), FP64 284 us (350); bond 48 FP32 50 us (129);
+// path of 60 vertices, bond 256, FP64 284 us (1312), bond 6 208 us (425).
 template <class T> struct IntAcc { using type = double; };
 template <> struct IntAcc<cplx> { using type = cplx; };
 __device__ inline void atomicAddAcc(double* a, double v) { atomicAdd(a, v); }
@@ -131,6 +132,8 @@ template <> struct Vec<cplx> {
 constexpr int INT_MAXV = 24, INT_MAXCH = 56;  // of a launch: its parameters stay below 4 KB
 constexpr int INT_WARPS = 8;
 constexpr int kFoldSites = 8;
+// blocks per SM: 64 registers a thread, 128 where a row's vectors need them
+constexpr int int_blocks(size_t size, int nch) { return size == 16 || nch >= 8 ? 2 : 4; }
 constexpr int INT_SMEM = 48 * 1024;  // messages of a vertex's children kept on chip
 
 struct IntChild {
@@ -183,9 +186,9 @@ __device__ inline int msg_exponent(unsigned hw) {
 }
 
 template <class T, int NCH>
-__global__ void __launch_bounds__(32 * INT_WARPS, sizeof(T) == 16 ? 2 : 3) k_integrate_level(const __grid_constant__ IntLevel<T> L) {
+__global__ void __launch_bounds__(32 * INT_WARPS, int_blocks(sizeof(T), NCH)) k_integrate_level(const __grid_constant__ IntLevel<T> L) {
   using A = typename IntAcc<T>::type;
-  constexpr int VE = Vec<T>::VE, U = NCH >= 8 ? 1 : 8 / NCH;
+  constexpr int VE = Vec<T>::VE, U = NCH >= 4 ? 1 : 4 / NCH;
   extern __shared__ __align__(16) unsigned char int_smem[];
   __shared__ unsigned red[EVAL_MAXC][INT_WARPS];
   asm volatile("griddepcontrol.launch_dependents;");
@@ -475,7 +478,7 @@ void integrate_levels(tnfa_ctx* ctx, const tnfa_net* net, int take_sum, double* 
   // are not 16-byte aligned, take the generic path)
   int nch = 1;
   while (nch < 8 && 32 * VE * nch < maxlast) nch *= 2;
-  const int64_t slots = (int64_t)ctx->sm_count * INT_WARPS * (sizeof(T) == 16 ? 2 : 3);
+  const int64_t slots = (int64_t)ctx->sm_count * INT_WARPS * int_blocks(sizeof(T), nch);
   {
     KernelScope ks(ctx, "integrate", 2.0 * (double)Tp.n_elem, (double)dtype_size(net->dtype) * Tp.n_elem);
     bool first = true;
@@ -495,7 +498,7 @@ void integrate_levels(tnfa_ctx* ctx, const tnfa_net* net, int take_sum, double* 
       // start).  Powers of two left a second wave of a few blocks at the narrow
       // levels and tasks of 4 rows at the middle ones (60-vertex binary tree,
       // FP32: bond 128 133 -> 121 us, bond 48 106 -> 50 us).
-      const int start = 3 * (nch >= 8 ? 1 : 8 / nch) * std::max(1, 32 * VE / std::max(1, maxlast));
+      const int start = 3 * (nch >= 4 ? 1 : 4 / nch) * std::max(1, 32 * VE / std::max(1, maxlast));
       int kb = 32;
       int64_t least = -1;
       for (int w = 1; w <= 8; ++w) {
