@@ -743,13 +743,25 @@ class EvalEngine {
       // another (about 3 us).  Up to about 20 us of walking there are no tables;
       // beyond, a table of half as many rows as points or less pays.
       double w = 0;
+      bool path = true;
+      int top = 1;
       for (int v = 0; v < V; ++v) {
         double x = topo_.link[v];
         for (int c : topo_.children[v]) x *= topo_.link[c];
         w += x;
+        path &= topo_.children[v].size() <= (topo_.parent[v] < 0 ? 2u : 1u);
+        top = std::max(top, topo_.link[v]);
       }
+      bool walk = w * P <= 20e-6 * WalkRate<T>::v;
+      // FP64 paths of bond 5 to 8: their tables are too large for k_head and
+      // take a launch of 10 us for every two vertices beyond about ten, 6 V -
+      // 39 us in all; the walk takes 1.4 us a vertex and 64 multiply-adds per
+      // vertex and point at 5.1e11 a second.  17 vertices, bond 7: 12662
+      // points 51 us walked, 63 from tables; 20000 points 67 and 62.
+      if (std::is_same<T, double>::value && path && top > 4 && top <= 8)
+        walk |= 64.0 * V * P <= (4.6e-6 * V - 39e-6) * 5.1e11;
       o.balance = true;
-      rows = w * P <= 20e-6 * WalkRate<T>::v ? 0 : std::floor(rows / 2);
+      rows = walk ? 0 : std::floor(rows / 2);
     }
     for (;;) {
       o.table_rows = rows;

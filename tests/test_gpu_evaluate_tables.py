@@ -44,3 +44,18 @@ def test_tables_match_oracle(ina, monkeypatch, gname, chi, base, nd, dtype):
         got = f.evaluate_batch(X[:n], dims, precision="f32" if dtype == "f32" else "f64")
         assert np.max(np.abs(got - ref[:n])) <= tol * scale, n
     assert rel_err(got, ref) < tol
+
+
+@pytest.mark.parametrize("V,chi", [(9, 8), (12, 5), (17, 7), (24, 8)])
+def test_walk_or_tables(ina, V, chi):
+    """FP64 paths of bond 5 to 8 on both sides of the point count where tables
+    take over from the walk, against the oracle."""
+    rng = np.random.default_rng(3000 + V)
+    net = O.random_net(O.siteinds(O.path_graph(V)), chi, rng, normalize=True)
+    f, _ = upload_oracle(ina, O.path_graph(V), net)
+    limit = int((4.6e-6 * V - 39e-6) * 5.1e11 / (64 * V))
+    X = rng.random((limit + 40, 1))
+    ref = O.evaluate_batch(net, X, [1])
+    scale = np.max(np.abs(ref))
+    for n in (limit - 33, limit, limit + 1, limit + 40):
+        assert np.max(np.abs(f.evaluate_batch(X[:n]) - ref[:n])) <= 1e-12 * scale, n
