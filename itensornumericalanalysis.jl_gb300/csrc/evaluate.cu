@@ -755,11 +755,11 @@ class EvalEngine {
       bool walk = w * P <= 20e-6 * WalkRate<T>::v;
       // FP64 paths of bond 5 to 8: their tables are too large for k_head and
       // take a launch of 10 us for every two vertices beyond about ten, 6 V -
-      // 39 us in all; the walk takes 1.4 us a vertex and 64 multiply-adds per
-      // vertex and point at 5.1e11 a second.  17 vertices, bond 7: 12662
-      // points 51 us walked, 63 from tables; 20000 points 67 and 62.
+      // 39 us in all; the walk takes 1.4 us a vertex and up to 64 multiply-adds
+      // per vertex and point at 5.4e11 a second.  Calls on 17 vertices, bond 7:
+      // 15000 points 85 us walked, 94 from tables; 22000 points 114 and 94.
       if (std::is_same<T, double>::value && path && top > 4 && top <= 8)
-        walk |= 64.0 * V * P <= (4.6e-6 * V - 39e-6) * 5.1e11;
+        walk |= 64.0 * V * P <= (4.6e-6 * V - 39e-6) * 5.4e11;
       o.balance = true;
       rows = walk ? 0 : std::floor(rows / 2);
     }
@@ -1034,13 +1034,15 @@ class EvalEngine {
     nstage_ = (size_t)topo_.n_elem * sizeof(T) <= 64 * 1024 ? (int)topo_.n_elem : 0;
     // points per block: spread over the SMs first, then as many as the shared
     // memory allows two blocks per SM with
-    wtp_ = P_ <= 32 * 2 * ctx_->sm_count ? 32 : P_ <= 64 * 4 * ctx_->sm_count ? 64 : 128;
+    wtp_ = P_ <= 64 * 4 * ctx_->sm_count ? 32 : 128;
     while (wtp_ > 32 && walk_bytes() > 100 * 1024) wtp_ /= 2;
     // lanes per point: up to four while the points alone do not give every
-    // scheduler (four per SM) a warp
+    // second scheduler (four per SM) a warp.  Twice as many lanes cost more in
+    // shuffles than their warps hide: 26 vertices, bond 6, FP64, 8000 points 104
+    // us a call against 91, 19078 points 124 against 108
     wlanes_ = 1;
     if (wchi_ <= 8)
-      while (wlanes_ < std::min(4, wchi_) && 2 * P_ * wlanes_ < 128 * 2 * (int64_t)ctx_->sm_count) wlanes_ *= 2;
+      while (wlanes_ < std::min(4, wchi_) && 2 * P_ * wlanes_ < 64 * 2 * (int64_t)ctx_->sm_count) wlanes_ *= 2;
     if (wlanes_ > 1) wtp_ = 32 / wlanes_ * (wlanes_ == 4 ? 2 : 1);
     return walk_bytes() <= 200 * 1024;
   }

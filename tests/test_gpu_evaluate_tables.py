@@ -53,7 +53,7 @@ def test_walk_or_tables(ina, V, chi):
     rng = np.random.default_rng(3000 + V)
     net = O.random_net(O.siteinds(O.path_graph(V)), chi, rng, normalize=True)
     f, _ = upload_oracle(ina, O.path_graph(V), net)
-    limit = int((4.6e-6 * V - 39e-6) * 5.1e11 / (64 * V))
+    limit = int((4.6e-6 * V - 39e-6) * 5.4e11 / (64 * V))
     X = rng.random((limit + 40, 1))
     ref = O.evaluate_batch(net, X, [1])
     scale = np.max(np.abs(ref))
