@@ -998,7 +998,7 @@ __global__ void __launch_bounds__(512) k_qrcp_sm(const QrJob* __restrict__ jobs,
     s = warp_sum(s);
     if (lane == 0) nrm[k] = s;
   }
-  __syncthreads();
+  cl.sync();  // every CTA of the cluster runs: their shared memory may be written
   if (warp == 0) {
     double s = 0.0;
     for (int k = lane; k < nc; k += 32) s += nrm[k];
