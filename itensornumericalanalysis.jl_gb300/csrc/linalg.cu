@@ -2607,25 +2607,34 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
   DBuf swall(ctx, nj * sizeof(int));
   auto S_of = [&](size_t q) { return Sall.as<double>() + soff[q]; };
   auto sw_of = [&](size_t q) { return swall.as<int>() + q; };
-  // Rank-revealing front end (reveal_tol > 0, tall jobs): M = Q1 R1 by
-  // pivoted QR with R1 (r x cols), r the numerical rank; when r < cols the
-  // square core is R2^H from R1^H = Q2 R2, else R1 itself.  The left vectors
-  // of M are Q1 times those of the core, so L = Q1 U_r and X = U_r^H R1, as
-  // for the plain tall case with (Q, R) = (Q1, R1).
+  // Rank-revealing front end (reveal_tol > 0): M = Q1 R1 by pivoted QR with
+  // R1 (r x cols), r the numerical rank; when r < cols the square core is R2^H
+  // from R1^H = Q2 R2, else R1 itself.  The left vectors of M are Q1 times
+  // those of the core, so L = Q1 U_r and X = U_r^H R1, as for the plain tall
+  // case with (Q, R) = (Q1, R1).  A wide M: M^H = Q1 R1, and the core R1^H
+  // (rows x r) has M's own left vectors.
   std::vector<char> rev(nj, 0);
   if (reveal_tol > 0.0) {
     std::vector<QrJob> pj;
     std::vector<size_t> pidx;
     for (size_t q = 0; q < nj; ++q) {
       const FactorJob& f = jobs[q];
-      if (f.rows < f.cols) continue;
+      const bool wide = f.rows < f.cols;
+      if (wide && f.rows > QRCP_MAXK) continue;
       rev[q] = 1;
-      Q[q] = DBuf(ctx, (size_t)f.rows * f.cols * sizeof(T));
-      R[q] = DBuf(ctx, (size_t)f.cols * f.cols * sizeof(T));
-      tau[q] = DBuf(ctx, (size_t)f.cols * sizeof(T));
-      pj.push_back({f.M, Q[q].p, R[q].p, tau[q].p, f.rows, f.cols});
+      const int m = std::max(f.rows, f.cols), k = std::min(f.rows, f.cols);
+      if (wide) {
+        Mt[q] = DBuf(ctx, (size_t)m * k * sizeof(T));
+        adj.push_back({f.M, Mt[q].p, f.rows, f.cols, f.cols, f.rows, 1, 1});
+      }
+      Q[q] = DBuf(ctx, (size_t)m * k * sizeof(T));
+      R[q] = DBuf(ctx, (size_t)k * k * sizeof(T));
+      tau[q] = DBuf(ctx, (size_t)k * sizeof(T));
+      pj.push_back({wide ? Mt[q].p : f.M, Q[q].p, R[q].p, tau[q].p, m, k});
       pidx.push_back(q);
     }
+    copy_blocks<T, T>(ctx, adj);
+    adj.clear();
     std::vector<int> rk;
     qr_rank<T>(ctx, pj, reveal_tol, rk);
     // R1^H = Q2 R2 for the jobs with r < cols; the core is R2^H
@@ -2636,6 +2645,13 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
       const size_t q = pidx[i];
       const int r = rk[i], cols = jobs[q].cols;
       n[q] = cm[q] = r;
+      if (jobs[q].rows < cols) {
+        const int rows = cm[q] = jobs[q].rows;
+        J[q] = DBuf(ctx, (size_t)rows * r * sizeof(T));
+        back.push_back({R[q].p, J[q].p, r, rows, rows, r, 1, 1});
+        core[q] = J[q].p;
+        continue;
+      }
       tall[q] = useq[q] = 1;
       if (r == cols) {
         core[q] = R[q].p;
@@ -2687,7 +2703,7 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
   qr<T>(ctx, qj);
   adj.clear();
   for (size_t q = 0; q < nj; ++q)
-    if (!tall[q]) adj.push_back({R[q].p, J[q].p, n[q], n[q], n[q], n[q], 1, 1});
+    if (!tall[q] && !rev[q]) adj.push_back({R[q].p, J[q].p, n[q], n[q], n[q], n[q], 1, 1});
   copy_blocks<T, T>(ctx, adj);
   const JacobiOpts opts{1e-10, cutoff > 0 ? cutoff * 1e-2 : 0.0};
   // the polish starts from FP32-converged columns (offsets ~1e-7), already in

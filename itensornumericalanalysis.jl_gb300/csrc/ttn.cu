@@ -918,22 +918,29 @@ void absorb_batched(std::vector<Work<T>>& W, const std::vector<BSlot>& sl, const
 // directions (a few hundred times the FP64 rounding of a QR step).
 constexpr double kRevealTol = 1e-13;
 
-// A single call keeps directions down to 1e-14, where the truncation rule
-// stops keeping them too (s^2 <= 1e-28 of the weight).
-constexpr double kRevealTolOne = 1e-14;
+// Where a sweep may cut a matrix to its numerical rank before factorising it
+// (0: nowhere).  first: the orthogonalising sweep, where the rest of the
+// network is not orthonormal and a direction's size in the matrix is not its
+// weight in the function.  centre: the SVD sweep, whose matrix is the function.
+struct Reveal {
+  double first = 0.0, centre = 0.0;
+};
+
+// A single call cuts at the centre alone, where the truncation rule stops
+// keeping directions too (s^2 <= 1e-28 of the weight).
+constexpr Reveal kRevealMany{kRevealTol, kRevealTol}, kRevealOne{0.0, 1e-14};
 
 template <class T>
-void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& prm,
-                            double reveal_tol = kRevealTol) {
+void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& prm, Reveal reveal) {
   if (W.empty()) return;
   tnfa_ctx* ctx = W[0].ctx;
   int maxV = 0;
   for (auto& w : W) maxV = std::max(maxV, w.topo.V);
-  // (1) orthogonalise toward vertex 0, from the far end of every path.  The
-  // QR is rank revealing: an operator's exact product carries bonds of D chi
-  // whose numerical rank is often far lower (a shift adds one direction per
-  // bond), and dropping the directions at the FP64 rounding floor here
-  // shrinks every later factorisation.
+  // (1) orthogonalise toward vertex 0, from the far end of every path.  For a
+  // batch the QR is rank revealing: an operator's exact product carries bonds
+  // of D chi whose numerical rank is often far lower (a shift adds one
+  // direction per bond), and dropping the directions at the FP64 rounding
+  // floor here shrinks every later factorisation.
   for (int t = 0; t + 1 < maxV; ++t) {
     std::vector<BSlot> sl;
     for (int i = 0; i < (int)W.size(); ++i) {
@@ -942,7 +949,7 @@ void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& pr
     }
     std::vector<DBuf> Rs;
     std::vector<int> ks;
-    qr_parent_axis_batched(W, sl, Rs, ks, reveal_tol);
+    qr_parent_axis_batched(W, sl, Rs, ks, reveal.first);
     std::vector<BSlot> ps;
     std::vector<int> ax;
     std::vector<const void*> Ms;
@@ -979,7 +986,7 @@ void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& pr
     }
     move_axes<T>(ctx, mv);
     std::vector<la::FactorResult> res;
-    la::trunc_factor<T>(ctx, fj, prm.cutoff, prm.maxdim, prm.mindim, prm.precision, res, reveal_tol);
+    la::trunc_factor<T>(ctx, fj, prm.cutoff, prm.maxdim, prm.mindim, prm.precision, res, reveal.centre);
     mv.clear();
     for (size_t q = 0; q < n; ++q) {
       TNFA_CHECK(res[q].sweeps >= 0, TNFA_ERR_NOT_CONVERGED, "Jacobi SVD hit its sweep cap");
@@ -1020,7 +1027,7 @@ void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& pr
 template <class T>
 void batch_apply_truncate(tnfa_ctx* ctx, int n, const tnfa_net* const* ops, const tnfa_net* const* fs,
                           const tnfa_trunc_params& prm, int dtype, tnfa_net** outs,
-                          double reveal_tol = kRevealTol) {
+                          Reveal reveal = kRevealMany) {
   std::vector<Work<T>> W;
   if (ops) {
     apply_exact_many<T>(ctx, n, ops, fs, W);
@@ -1028,7 +1035,7 @@ void batch_apply_truncate(tnfa_ctx* ctx, int n, const tnfa_net* const* ops, cons
     W.reserve(n);
     for (int i = 0; i < n; ++i) W.push_back(load_work<T>(ctx, fs[i]));
   }
-  truncate_paths_batched(W, prm, reveal_tol);
+  truncate_paths_batched(W, prm, reveal);
   store_works(W, dtype, outs);
 }
 
@@ -2326,18 +2333,21 @@ using namespace tnfa;
 
 extern "C" {
 
-// One path through the batched sweeps: their rank-revealing QR cuts the bonds
-// of an exact product (D chi) to its rank before anything is factorised at
-// full width.  Null when the sweeps do not take it (another tree, a matrix of
-// more than 1024 columns, NaN or Inf entries): the general form then does.
+// One path through the batched sweeps: a plain QR sweep, then at the centre the
+// rank-revealing QR cuts the matrix of an exact product (D chi) to its rank
+// before the Jacobi iteration (24 vertices, bond 40, first derivative: 44.5 ms,
+// the tree sweep 141; cutting in the first sweep already took 27 and lost every
+// part of a function whose tensors there are small).  Null when the sweeps do
+// not take it (another tree, a matrix of more than 1024 columns, NaN or Inf
+// entries): the general form then does.
 static tnfa_net* one_path(tnfa_ctx* ctx, const tnfa_net* op, const tnfa_net* f, const tnfa_trunc_params& prm) {
   if (!is_rooted_path(f->topo) || (op && op->dtype != f->dtype)) return nullptr;
   tnfa_net* out = nullptr;
   try {
     if (f->dtype == TNFA_F64)
-      batch_apply_truncate<double>(ctx, 1, op ? &op : nullptr, &f, prm, TNFA_F64, &out, kRevealTolOne);
+      batch_apply_truncate<double>(ctx, 1, op ? &op : nullptr, &f, prm, TNFA_F64, &out, kRevealOne);
     else if (f->dtype == TNFA_C128)
-      batch_apply_truncate<cplx>(ctx, 1, op ? &op : nullptr, &f, prm, TNFA_C128, &out, kRevealTolOne);
+      batch_apply_truncate<cplx>(ctx, 1, op ? &op : nullptr, &f, prm, TNFA_C128, &out, kRevealOne);
   } catch (const Error& e) {
     if (e.status != TNFA_ERR_DOMAIN && e.status != TNFA_ERR_UNSUPPORTED) throw;
     return nullptr;

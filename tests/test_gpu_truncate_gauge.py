@@ -1,0 +1,71 @@
+"""Truncation where the tensors behind a bond say nothing about the weight in
+the function: sums whose blocks differ by many orders of magnitude at a vertex
+(an exponential's amplitude is spread over all vertices), and a summand whose
+scale sits on one vertex.
+
+Unless the cutoff is larger, 1e-24 leaves sqrt(20 bonds x 1e-24) < 5e-12 of the
+norm and the factorisations a few n eps per bond, below 1e-11: 1e-10.  A first
+difference loses 2 |f| / |f(x + d) - f(x - d)| < 2^20 / 10 of that rounding:
+20 bonds x 10 eps x 1e5 = 2e-9, 1e-8."""
+import numpy as np
+import pytest
+
+import oracle as O
+from _helpers import upload_oracle
+
+pytestmark = pytest.mark.gpu
+
+L = 20
+X = np.linspace(0.0, 1.0, 4001, endpoint=False)
+
+
+def _cosh(ina, k):
+    s = ina.continuous_siteinds(ina.named_path_graph(L))
+    f = ina.cosh_itensornetwork(s, k=float(k), a=-k / 2)
+    return s, f, np.cosh(k * np.floor(X * 2**L) / 2**L - k / 2)
+
+
+def _l2(got, ref):
+    return np.linalg.norm(got - ref) / np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("k", [10, 44, 60, 100])
+@pytest.mark.parametrize("cutoff", [0.0, 1e-24])
+def test_truncate_cosh(ina, k, cutoff):
+    _, f, ref = _cosh(ina, k)
+    assert _l2(f.evaluate_batch(X), ref) < 1e-12
+    assert _l2(ina.truncate(f, cutoff=cutoff).evaluate_batch(X), ref) < 1e-10
+
+
+@pytest.mark.parametrize("k", [10, 44, 100])
+@pytest.mark.parametrize("op", ["shift", "derivative"])
+def test_operate_cosh(ina, k, op):
+    s, f, _ = _cosh(ina, k)
+    o = ina.forward_shift_op(s) if op == "shift" else ina.first_derivative_operator(s)
+    ref = ina.operate_exact(o, f).evaluate_batch(X)
+    got = ina.operate(o, f, cutoff=1e-24).evaluate_batch(X)
+    assert _l2(got, ref) < (1e-10 if op == "shift" else 1e-8)
+
+
+def _lopsided(ina, seed, dtype):
+    """f + g with f's scale 1e-20 at the last vertex and 1e20 at the root; the values of f + g."""
+    graph, rng = O.path_graph(12), np.random.default_rng(seed)
+    fs, vals = [], 0
+    for i in range(2):
+        f, s = upload_oracle(ina, graph, O.random_net(O.siteinds(graph), 3, rng, normalize=True))
+        if dtype == "c128":
+            f = f.astype(ina._lib.C128)
+            f.scale_vertex(s.layout.order[0], 0.6 - 0.8j)
+        vals = vals + f.evaluate_batch(X)
+        fs.append((f, s))
+    f, s = fs[0]
+    f.scale_vertex(s.layout.order[-1], 1e-20)
+    f.scale_vertex(s.layout.order[0], 1e20)
+    return f + fs[1][0], vals
+
+
+@pytest.mark.parametrize("dtype", ["f64", "c128"])
+@pytest.mark.parametrize("cutoff,tol", [(0.0, 1e-10), (1e-24, 1e-10), (1e-12, 1e-5)])
+def test_truncate_lopsided(ina, dtype, cutoff, tol):
+    h, ref = _lopsided(ina, 5, dtype)
+    assert _l2(ina.truncate(h, cutoff=cutoff).evaluate_batch(X), ref) < tol
