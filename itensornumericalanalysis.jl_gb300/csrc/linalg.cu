@@ -1272,6 +1272,75 @@ void qr_rank(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, std::vec
   }
 }
 
+// Columns brought to a norm in [1, 2) by a power of two (exact), its exponent
+// kept per column; columns without a normal squared norm stay as they are.
+struct ColScaleJob {
+  void* A;
+  int* exps;
+  int m, n;
+};
+template <class T>
+__global__ void __launch_bounds__(256) k_scale_cols(const ColScaleJob* __restrict__ jobs) {
+  __shared__ double part[8][32];
+  const ColScaleJob jb = jobs[blockIdx.y];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
+  if (blockIdx.x * 32 >= jb.n) return;
+  T* A = (T*)jb.A;
+  double s = 0.0;
+  if (c < jb.n)
+    for (int r = ty; r < jb.m; r += 8) s += abs2(A[(int64_t)r * jb.n + c]);
+  part[ty][tx] = s;
+  __syncthreads();
+  s = 0.0;
+  for (int i = 0; i < 8; ++i) s += part[i][tx];
+  if (c >= jb.n) return;
+  const int e = s >= 2.2250738585072014e-308 && s <= 1.7976931348623157e308 ? ilogb(sqrt(s)) : 0;
+  if (ty == 0) jb.exps[c] = e;
+  if (e == 0) return;
+  const double f = scalbn(1.0, -e);
+  for (int r = ty; r < jb.m; r += 8) A[(int64_t)r * jb.n + c] = scal(A[(int64_t)r * jb.n + c], f);
+}
+// Back to the columns' own sizes in R (A: R, m: its rows).
+template <class T>
+__global__ void __launch_bounds__(256) k_unscale_cols(const ColScaleJob* __restrict__ jobs) {
+  const ColScaleJob jb = jobs[blockIdx.y];
+  T* A = (T*)jb.A;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)jb.m * jb.n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int e = jb.exps[i % jb.n];
+    if (e) A[i] = scal(A[i], scalbn(1.0, e));
+  }
+}
+
+template <class T>
+void qr_rank_columns(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, std::vector<int>& ranks) {
+  TNFA_CHECK(jobs.size() <= 65535, TNFA_ERR_UNSUPPORTED, "QR batch too large");
+  if (jobs.empty()) return qr_rank<T>(ctx, jobs, tol, ranks);
+  std::vector<size_t> at(1, 0);
+  int maxn = 1;
+  for (const auto& j : jobs) {
+    at.push_back(at.back() + j.n);
+    maxn = std::max(maxn, j.n);
+  }
+  DBuf exps(ctx, at.back() * sizeof(int));
+  auto launch = [&](auto kern, bool back) {
+    std::vector<ColScaleJob> cj;
+    int64_t most = 1;
+    for (size_t i = 0; i < jobs.size(); ++i) {
+      const int m = back ? ranks[i] : jobs[i].m;
+      cj.push_back({back ? jobs[i].R : jobs[i].A, exps.as<int>() + at[i], m, jobs[i].n});
+      most = std::max(most, (int64_t)m * jobs[i].n);
+    }
+    DBuf d = upload(ctx, cj);
+    const unsigned gx = back ? grid_for(most, 256, 256) : (unsigned)((maxn + 31) / 32);
+    kern<<<dim3(gx, (unsigned)jobs.size()), 256, 0, ctx->stream>>>(d.as<ColScaleJob>());
+    TNFA_LAUNCH_CHECK();
+  };
+  launch(k_scale_cols<T>, false);
+  qr_rank<T>(ctx, jobs, tol, ranks);
+  launch(k_unscale_cols<T>, true);
+}
+
 // ----------------------------------------------------------------- svd --
 void trace_sweeps(tnfa_ctx* ctx, const std::vector<SvdJob>& jobs) {
   int mx = 0, capped = 0, cnt = 0;
@@ -2998,6 +3067,8 @@ template void qr<double>(tnfa_ctx*, const std::vector<QrJob>&);
 template void qr<cplx>(tnfa_ctx*, const std::vector<QrJob>&);
 template void qr_rank<double>(tnfa_ctx*, const std::vector<QrJob>&, double, std::vector<int>&);
 template void qr_rank<cplx>(tnfa_ctx*, const std::vector<QrJob>&, double, std::vector<int>&);
+template void qr_rank_columns<double>(tnfa_ctx*, const std::vector<QrJob>&, double, std::vector<int>&);
+template void qr_rank_columns<cplx>(tnfa_ctx*, const std::vector<QrJob>&, double, std::vector<int>&);
 template void trunc_factor<double>(tnfa_ctx*, const std::vector<FactorJob>&, double, int, int, int,
                                    std::vector<FactorResult>&, double);
 template void trunc_factor<cplx>(tnfa_ctx*, const std::vector<FactorJob>&, double, int, int, int,

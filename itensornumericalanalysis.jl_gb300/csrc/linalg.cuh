@@ -65,6 +65,11 @@ void qr(tnfa_ctx* ctx, const std::vector<QrJob>& jobs);
 // at most tol^2 of |A|_F^2 (r = min(m, n) if none).  ranks[i] = r of job i.
 template <class T>
 void qr_rank(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, std::vector<int>& ranks);
+// The same on columns of about unit norm (A is rescaled in place, R comes out
+// in A's own sizes): what is left of each column is at most tol sqrt(n) of that
+// column, however the columns differ in size.
+template <class T>
+void qr_rank_columns(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, std::vector<int>& ranks);
 
 // One job of the one-sided Jacobi SVD used by trunc_factor: A (m x n, m >=
 // n, lda = n, read only) = U diag(S) V^H with U (m x n, orthonormal columns

@@ -827,8 +827,10 @@ struct BSlot {
 // QR of the listed vertices with their parent axis (1) as columns; each keeps
 // Q and returns R (k x old) in Rs[i]; ks[i] = k.  With reveal_tol > 0 the
 // factorisation is rank revealing (column pivoting): k is the numerical rank,
-// the directions left out holding at most reveal_tol of the matrix's
-// Frobenius norm.
+// the directions left out holding at most about reveal_tol of every column.
+// (Not of the whole matrix: the rest of the network, by which the columns are
+// multiplied, is not orthonormal, and a sum's summands are columns of any
+// size.)
 template <class T>
 void qr_parent_axis_batched(std::vector<Work<T>>& W, const std::vector<BSlot>& sl,
                             std::vector<DBuf>& Rs, std::vector<int>& ks, double reveal_tol = 0.0) {
@@ -859,7 +861,7 @@ void qr_parent_axis_batched(std::vector<Work<T>>& W, const std::vector<BSlot>& s
   }
   move_axes<T>(ctx, mv);
   if (reveal_tol > 0.0)
-    la::qr_rank<T>(ctx, qj, reveal_tol, ks);
+    la::qr_rank_columns<T>(ctx, qj, reveal_tol, ks);
   else
     la::qr<T>(ctx, qj);
   mv.clear();
@@ -914,7 +916,7 @@ void absorb_batched(std::vector<Work<T>>& W, const std::vector<BSlot>& sl, const
   for (size_t i = 0; i < n; ++i) W[sl[i].net].t[sl[i].v] = std::move(c[i]);
 }
 
-// Relative Frobenius weight below which the batched orthogonalisation drops
+// Part of every column below which the batched orthogonalisation drops
 // directions (a few hundred times the FP64 rounding of a QR step).
 constexpr double kRevealTol = 1e-13;
 

@@ -69,3 +69,28 @@ def _lopsided(ina, seed, dtype):
 def test_truncate_lopsided(ina, dtype, cutoff, tol):
     h, ref = _lopsided(ina, 5, dtype)
     assert _l2(ina.truncate(h, cutoff=cutoff).evaluate_batch(X), ref) < tol
+
+
+# the batched sweep may leave 1e-13 sqrt(40 columns) of every column per bond: 20 bonds, 2e-11
+@pytest.mark.parametrize("precision", ["f64", "mixed"])
+@pytest.mark.parametrize("cutoff", [0.0, 1e-24])
+def test_truncate_batched_cosh(ina, precision, cutoff):
+    nets = [_cosh(ina, k)[1:] for k in (10, 44, 60, 100)]
+    gs = ina.truncate_batched([f for f, _ in nets], cutoff=cutoff, precision=precision)
+    for g, (_, ref) in zip(gs, nets):
+        assert _l2(g.evaluate_batch(X), ref) < 1e-10
+
+
+def test_operate_batched_cosh(ina):
+    nets = [_cosh(ina, k) for k in (10, 44, 100)]
+    ops = [ina.forward_shift_op(s) for s, _, _ in nets]
+    for (_, f, _), o, g in zip(nets, ops, ina.operate_batched(ops, [f for _, f, _ in nets], cutoff=1e-24)):
+        assert _l2(g.evaluate_batch(X), ina.operate_exact(o, f).evaluate_batch(X)) < 1e-10
+
+
+@pytest.mark.parametrize("dtype", ["f64", "c128"])
+@pytest.mark.parametrize("cutoff,tol", [(0.0, 1e-10), (1e-12, 1e-5)])
+def test_truncate_batched_lopsided(ina, dtype, cutoff, tol):
+    nets = [_lopsided(ina, 5 + i, dtype) for i in range(3)]
+    for g, (_, ref) in zip(ina.truncate_batched([h for h, _ in nets], cutoff=cutoff), nets):
+        assert _l2(g.evaluate_batch(X), ref) < tol
