@@ -3024,15 +3024,22 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
     r = std::max(r, std::min(std::max(mindim, 1), c));
     drop = extra[q];
     for (int i = r; i < c; ++i) drop += o.s[i] * o.s[i];
-    o.r = r;
+    // mindim counts the matrix's own directions: what the rank-revealing QR cut
+    // (nothing above the rounding floor) comes back as zeros
+    const int rp = std::max(r, std::min(std::max(mindim, 1), std::min(f.rows, f.cols)));
+    o.r = rp;
     o.discarded = tot > 0 ? drop / tot : 0.0;
-    o.L = DBuf(ctx, (size_t)f.rows * r * sizeof(T));
-    o.X = DBuf(ctx, (size_t)r * f.cols * sizeof(T));
+    o.L = DBuf(ctx, (size_t)f.rows * rp * sizeof(T));
+    o.X = DBuf(ctx, (size_t)rp * f.cols * sizeof(T));
+    if (rp > r) {
+      TNFA_CUDA(cudaMemsetAsync(o.L.p, 0, (size_t)f.rows * rp * sizeof(T), ctx->stream));
+      TNFA_CUDA(cudaMemsetAsync(o.X.p, 0, (size_t)rp * f.cols * sizeof(T), ctx->stream));
+    }
     if (useq[q]) {
-      gl.push_back({Q[q].p, U[q].p, o.L.p, f.rows, r, k, k, c, r, 0, 0, 1.0, 0.0});
+      gl.push_back({Q[q].p, U[q].p, o.L.p, f.rows, r, k, k, c, rp, 0, 0, 1.0, 0.0});
       gx.push_back({U[q].p, R[q].p, o.X.p, r, f.cols, k, c, f.cols, f.cols, 2, 0, 1.0, 0.0});
     } else {
-      cl.push_back({U[q].p, o.L.p, m, r, c, r, 0, 0});
+      cl.push_back({U[q].p, o.L.p, m, r, c, rp, 0, 0});
       gx.push_back({U[q].p, f.M, o.X.p, r, f.cols, m, c, f.cols, f.cols, 2, 0, 1.0, 0.0});
     }
   }

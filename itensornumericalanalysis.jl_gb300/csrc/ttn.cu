@@ -830,10 +830,12 @@ struct BSlot {
 // the directions left out holding at most about reveal_tol of every column.
 // (Not of the whole matrix: the rest of the network, by which the columns are
 // multiplied, is not orthonormal, and a sum's summands are columns of any
-// size.)
+// size.)  A rank below mindim is filled up to it, as far as the matrix goes,
+// with zero columns of Q and zero rows of R.
 template <class T>
 void qr_parent_axis_batched(std::vector<Work<T>>& W, const std::vector<BSlot>& sl,
-                            std::vector<DBuf>& Rs, std::vector<int>& ks, double reveal_tol = 0.0) {
+                            std::vector<DBuf>& Rs, std::vector<int>& ks, double reveal_tol = 0.0,
+                            int mindim = 1) {
   if (sl.empty()) return;
   tnfa_ctx* ctx = W[sl[0].net].ctx;
   const size_t n = sl.size();
@@ -866,10 +868,21 @@ void qr_parent_axis_batched(std::vector<Work<T>>& W, const std::vector<BSlot>& s
     la::qr<T>(ctx, qj);
   mv.clear();
   for (size_t i = 0; i < n; ++i) {
+    const int64_t rows = W[sl[i].net].size(sl[i].v) / shp[i][1];
+    const int cols = shp[i][1], k = ks[i], least = (int)std::min<int64_t>(mindim, std::min<int64_t>(rows, cols));
+    if (k < least) {
+      DBuf wide(ctx, (size_t)rows * least * sizeof(T));
+      TNFA_CUDA(cudaMemsetAsync(wide.p, 0, (size_t)rows * least * sizeof(T), ctx->stream));
+      TNFA_CUDA(cudaMemcpy2DAsync(wide.p, least * sizeof(T), Q[i].p, k * sizeof(T), k * sizeof(T), rows,
+                                  cudaMemcpyDeviceToDevice, ctx->stream));
+      TNFA_CUDA(cudaMemsetAsync(Rs[i].template as<T>() + (size_t)k * cols, 0, (size_t)(least - k) * cols * sizeof(T),
+                                ctx->stream));
+      Q[i] = std::move(wide);
+      ks[i] = least;
+    }
     std::vector<int> qshp = shp[i];
     qshp.erase(qshp.begin() + 1);
     qshp.push_back(ks[i]);
-    const int64_t rows = W[sl[i].net].size(sl[i].v) / shp[i][1];
     back[i] = DBuf(ctx, (size_t)rows * ks[i] * sizeof(T));
     mv.push_back({Q[i].p, back[i].p, qshp, (int)qshp.size() - 1, 1});
   }
@@ -951,7 +964,7 @@ void truncate_paths_batched(std::vector<Work<T>>& W, const tnfa_trunc_params& pr
     }
     std::vector<DBuf> Rs;
     std::vector<int> ks;
-    qr_parent_axis_batched(W, sl, Rs, ks, reveal.first);
+    qr_parent_axis_batched(W, sl, Rs, ks, reveal.first, prm.mindim);
     std::vector<BSlot> ps;
     std::vector<int> ax;
     std::vector<const void*> Ms;

@@ -94,3 +94,19 @@ def test_truncate_batched_lopsided(ina, dtype, cutoff, tol):
     nets = [_lopsided(ina, 5 + i, dtype) for i in range(3)]
     for g, (_, ref) in zip(ina.truncate_batched([h for h, _ in nets], cutoff=cutoff), nets):
         assert _l2(g.evaluate_batch(X), ref) < tol
+
+
+@pytest.mark.parametrize("mindim", [3, 5, 8, 20])
+@pytest.mark.parametrize("precision,dtype", [("f64", "f64"), ("f64", "c128"), ("mixed", "f64")])
+@pytest.mark.parametrize("batched", [False, True])
+def test_mindim_of_a_low_rank(ina, mindim, precision, dtype, batched):
+    graph = O.path_graph(8)
+    f, _ = upload_oracle(ina, graph, O.random_net(O.siteinds(graph), 2, np.random.default_rng(7), normalize=True))
+    if dtype == "c128":
+        f = f.astype(ina._lib.C128)
+    g = f + f
+    h = g + g  # rank 2, stored with bonds of 8
+    kw = dict(cutoff=1e-20, mindim=mindim, precision=precision)
+    for t in ina.truncate_batched([h, h], **kw) if batched else [ina.truncate(h, **kw)]:
+        assert [t.linkdims()[e] for e in h.linkdims()] == [min(mindim, 8, 2**i, 2 ** (8 - i)) for i in range(1, 8)]
+        assert _l2(t.evaluate_batch(X), 4 * f.evaluate_batch(X)) < 1e-9
