@@ -782,8 +782,9 @@ __global__ void __launch_bounds__(512) k_qrcp(const QrJob* __restrict__ jobs, T*
   }
   const double thr = tol2 * total;
   T* R = (T*)jb.R;
-  int r_keep = kq;
-  for (int j = 0; j < kq; ++j) {
+  // (an Inf or NaN entry, or one whose square overflows, leaves no rank)
+  int r_keep = total <= 1.7976931348623157e308 ? kq : 0;
+  for (int j = 0; j < r_keep; ++j) {
     double best = -1.0, sum = 0.0;
     int bi = INT_MAX;
     for (int c = crank + C * threadIdx.x; c < n; c += C * blockDim.x) {
@@ -817,7 +818,7 @@ __global__ void __launch_bounds__(512) k_qrcp(const QrJob* __restrict__ jobs, T*
       }
     }
     if (p >= n || (j > 0 && (gsum <= thr || !(gbest > 0.0)))) {
-      r_keep = j;  // 0 only when no column has a finite norm
+      r_keep = j;
       break;
     }
     if (threadIdx.x == 0) piv[j] = p;
@@ -1012,8 +1013,9 @@ __global__ void __launch_bounds__(512) k_qrcp_sm(const QrJob* __restrict__ jobs,
   const int te = (int)(__double2hiint(total) >> 20) & 0x7FF;
   const double sc = te > 0 && te < 2046 ? __hiloint2double((2046 - te) << 20, 0) : 1.0;
   const float thr = (float)(tol2 * (total * sc));
-  int r_keep = kq;
-  for (int j = 0; j < kq; ++j) {
+  // (an Inf or NaN entry, or one whose square overflows, leaves no rank)
+  int r_keep = total <= 1.7976931348623157e308 ? kq : 0;
+  for (int j = 0; j < r_keep; ++j) {
     if (warp == 0) {
       long long best = -1;  // norms are >= 0: their bits order like the values
       int bi = INT_MAX;
@@ -1044,7 +1046,7 @@ __global__ void __launch_bounds__(512) k_qrcp_sm(const QrJob* __restrict__ jobs,
       if (o.idx < n && (ob > gbest || (ob == gbest && o.idx < p))) gbest = ob, p = o.idx;
     }
     if (p >= n || (j > 0 && (gsum <= thr || gbest <= 0))) {
-      r_keep = j;  // 0 only when no column has a finite norm
+      r_keep = j;
       break;
     }
     const T* rem = cl.map_shared_rank(W, p % C) + (p / C) * L.pitch;
@@ -1255,7 +1257,7 @@ void qr_rank(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, std::vec
   TNFA_CUDA(cudaStreamSynchronize(ctx->stream));
   for (size_t i = 0; i < order.size(); ++i) ranks[order[i]] = h[i];
   for (int r : ranks)
-    TNFA_CHECK(r >= 1, TNFA_ERR_DOMAIN, "rank-revealing QR: no column with a finite norm (NaN or Inf input)");
+    TNFA_CHECK(r >= 1, TNFA_ERR_DOMAIN, "rank-revealing QR: a column without a finite norm (NaN or Inf input)");
   if (trace_on()) {
     long sr = 0, sk = 0, mx_m = 0, mx_n = 0, mx_r = 0;
     for (size_t i = 0; i < jobs.size(); ++i) {

@@ -110,3 +110,18 @@ def test_mindim_of_a_low_rank(ina, mindim, precision, dtype, batched):
     for t in ina.truncate_batched([h, h], **kw) if batched else [ina.truncate(h, **kw)]:
         assert [t.linkdims()[e] for e in h.linkdims()] == [min(mindim, 8, 2**i, 2 ** (8 - i)) for i in range(1, 8)]
         assert _l2(t.evaluate_batch(X), 4 * f.evaluate_batch(X)) < 1e-9
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("at", [0, 3, 7])
+@pytest.mark.parametrize("chi", [4, 40])
+def test_not_finite(ina, value, at, chi):
+    """A batch refuses entries that are not finite; a single call answers with them."""
+    graph = O.path_graph(8)
+    f, s = upload_oracle(ina, graph, O.random_net(O.siteinds(graph, base=3), chi, np.random.default_rng(0)))
+    ts = {v: t.copy() for v, t in f.tensors().items()}
+    ts[s.layout.order[at]].flat[1] = value
+    f = ina.ITensorNetworkFunction.from_tensors(s, ts)
+    with pytest.raises(ina.TnfaError, match="TNFA_ERR_DOMAIN"):
+        ina.truncate_batched([f, f], cutoff=1e-20)
+    assert not np.any(np.isfinite(ina.truncate(f, cutoff=1e-20).evaluate_batch(X[::100])))
