@@ -134,7 +134,9 @@ constexpr int INT_WARPS = 8;
 constexpr int kFoldSites = 8;
 // blocks per SM: 64 registers a thread, 128 where a row's vectors need them
 constexpr int int_blocks(size_t size, int nch) { return size == 16 || nch >= 8 ? 2 : 4; }
-constexpr int INT_SMEM = 48 * 1024;  // messages of a vertex's children kept on chip
+// messages of a vertex's children kept on chip: with the block's static
+// reductions (4 bytes a child and warp) within the 48 KB of a plain launch
+constexpr int INT_SMEM = 48 * 1024 - EVAL_MAXC * INT_WARPS * 4;
 
 struct IntChild {
   int64_t src;  // offset of its message, or of its tensor (sd > 0)
