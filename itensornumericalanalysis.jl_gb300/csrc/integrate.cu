@@ -137,6 +137,7 @@ constexpr int int_blocks(size_t size, int nch) { return size == 16 || nch >= 8 ?
 // messages of a vertex's children kept on chip: with the block's static
 // reductions (4 bytes a child and warp) within the 48 KB of a plain launch
 constexpr int INT_SMEM = 48 * 1024 - EVAL_MAXC * INT_WARPS * 4;
+constexpr int INT_SMEM_LONG = 200 * 1024;  // where rows are long
 
 struct IntChild {
   int64_t src;  // offset of its message, or of its tensor (sd > 0)
@@ -152,7 +153,9 @@ struct IntVertex {
   int nkb, kb;     // tasks per (s, a); rows per task
   int sd, chi_a, last;    // last: entries of the last child
   int nchild, ch0;        // its children in the launch's list
-  short lg, vec, staged;  // vec: rows are read as 16-byte vectors
+  short lg, vec;   // vec: rows are read as 16-byte vectors, 2: rows longer than the lanes hold
+  short staged;    // the messages are in shared memory (2: without an unscaled copy)
+  short tpw;       // tasks per warp
 };
 
 template <class T>
@@ -185,6 +188,88 @@ __device__ inline unsigned hi_abs(cplx z) { return max(hi_abs(z.re), hi_abs(z.im
 __device__ inline int msg_exponent(unsigned hw) {
   const int e = (int)(hw >> 20);
   return e == 0x7ff ? 0 : min(e - 1022, 1022);  // none where an entry is not finite
+}
+
+template <class T>
+__device__ inline T warp_total(T v) {
+  for (int o = 16; o; o >>= 1) {
+    if constexpr (sizeof(T) == 16) {
+      cplx z = *(cplx*)&v;
+      z.re += __shfl_xor_sync(0xffffffffu, z.re, o);
+      z.im += __shfl_xor_sync(0xffffffffu, z.im, o);
+      v = *(T*)&z;
+    } else {
+      v = v + __shfl_xor_sync(0xffffffffu, v, o);
+    }
+  }
+  return v;
+}
+
+// Rows longer than the lanes of the main path hold (over 1024 FP32, 512 FP64
+// or 256 complex entries): a warp walks its row with 8 vectors per lane in
+// flight, each summed on its own, and takes several tasks, because a message of
+// that length costs its block about as long to stage as eight rows to read.  A
+// path of 4 vertices, against the scalar loop of the unaligned rows and against
+// one persistent launch: bond 4096 FP32 158 us (741, 480), bond 6000 FP64 356
+// us (1233, 982).
+template <class T, class Unscale, class Entry>
+__device__ inline void long_rows(const IntLevel<T>& L, const IntVertex& iv, const IntChild* ch, const T* cm,
+                                 const Unscale& unscale, const Entry& entry) {
+  using A = typename IntAcc<T>::type;
+  constexpr int VE = Vec<T>::VE, LU = 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nchild = iv.nchild, last = iv.last;
+  const IntChild& cl = ch[nchild - 1];
+  const double ul = unscale(nchild - 1);
+  int olast = 0;
+  for (int c = 0; c + 1 < nchild; ++c) olast += ch[c].dim;
+  for (int i = 0; i < iv.tpw; ++i) {
+    const int64_t t64 = ((int64_t)((int)blockIdx.x - iv.b0) * iv.tpw + i) * INT_WARPS + warp;
+    if (t64 >= iv.ntask) return;
+    const int t = (int)t64, sa = t / iv.nkb, a = sa % iv.chi_a;
+    const int64_t k0 = (int64_t)(t - sa * iv.nkb) * iv.kb;
+    const int nr = (int)min((int64_t)iv.kb, iv.kouter - k0);
+    T w = Sc<T>::one();  // lane r: the weight of row r
+    if (nchild > 1 && lane < nr) {
+      int64_t kk = k0 + lane;
+      int o = olast;
+      for (int c = nchild - 2; c >= 0; --c) {
+        const int d = ch[c].dim, j = c ? (int)(kk % d) : (int)kk;
+        o -= d;
+        w = w * (iv.staged ? cm[o + j] : to_dot(mulw(entry(ch[c], j), unscale(c)), T{}));
+        if (c) kk /= d;
+      }
+    }
+    T partial = Sc<T>::zero();
+    for (int r = 0; r < nr; ++r) {
+      const T* row = L.tensors + iv.off + ((int64_t)sa * iv.kouter + k0 + r) * last;
+      T acc[LU];
+#pragma unroll
+      for (int u = 0; u < LU; ++u) acc[u] = Sc<T>::zero();
+      for (int j0 = lane * VE; j0 < last; j0 += 32 * VE * LU) {
+        T x[LU][VE];
+#pragma unroll
+        for (int u = 0; u < LU; ++u) {
+          const int j = j0 + 32 * VE * u;
+          if (j < last) Vec<T>::load(row + j, x[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < LU; ++u) {
+          const int j = j0 + 32 * VE * u;
+          if (j >= last) break;
+#pragma unroll
+          for (int e = 0; e < VE; ++e) {
+            const T m = iv.staged ? cm[olast + j + e] : to_dot(mulw(entry(cl, j + e), ul), T{});
+            acc[u] = Sc<T>::fma(x[u][e], m, acc[u]);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 1; u < LU; ++u) acc[0] = acc[0] + acc[u];
+      partial = Sc<T>::fma(shfl_t(w, r), acc[0], partial);
+    }
+    partial = warp_total(partial);
+    if (lane == 0) atomicAddAcc(L.msgs + iv.out + a, mulw(to_acc(partial, A{}), iv.w));
+  }
 }
 
 template <class T, int NCH>
@@ -238,7 +323,7 @@ __global__ void __launch_bounds__(32 * INT_WARPS, int_blocks(sizeof(T), NCH)) k_
         }
       }
   };
-  if (iv.vec) load(0);
+  if (iv.vec == 1) load(0);
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // the children's messages
@@ -255,7 +340,7 @@ __global__ void __launch_bounds__(32 * INT_WARPS, int_blocks(sizeof(T), NCH)) k_
     if (iv.staged) {
       int sum = 0;
       for (int c = 0; c < nchild; ++c) sum += ch[c].dim;
-      cm = (T*)(raw + sum);
+      if (iv.staged == 1) cm = (T*)(raw + sum);
     }
   }
   int at = 0;
@@ -263,7 +348,7 @@ __global__ void __launch_bounds__(32 * INT_WARPS, int_blocks(sizeof(T), NCH)) k_
     unsigned hw = 0;
     for (int j = threadIdx.x; j < ch[c].dim; j += 32 * INT_WARPS) {
       const A e = entry(ch[c], j);
-      if (iv.staged) raw[at + j] = e;
+      if (iv.staged == 1) raw[at + j] = e;
       hw = max(hw, hi_abs(e));
     }
     hw = __reduce_max_sync(0xffffffffu, hw);
@@ -283,10 +368,17 @@ __global__ void __launch_bounds__(32 * INT_WARPS, int_blocks(sizeof(T), NCH)) k_
     at = 0;
     for (int c = 0; c < nchild; ++c) {
       const double f = unscale(c);
-      for (int j = threadIdx.x; j < ch[c].dim; j += 32 * INT_WARPS) cm[at + j] = to_dot(mulw(raw[at + j], f), T{});
+      for (int j = threadIdx.x; j < ch[c].dim; j += 32 * INT_WARPS) 
+        cm[at + j] = to_dot(mulw(iv.staged == 1 ? raw[at + j] : entry(ch[c], j), f), T{});
       at += ch[c].dim;
     }
     __syncthreads();
+  }
+  if constexpr (NCH == 8) {  // (the other forms are launched where every row fits)
+    if (iv.vec == 2) {
+      long_rows<T>(L, iv, ch, cm, unscale, entry);
+      return;
+    }
   }
   if (nr <= 0) return;
   // entry j of child c's scaled message (o: where its entries start)
@@ -308,7 +400,7 @@ __global__ void __launch_bounds__(32 * INT_WARPS, int_blocks(sizeof(T), NCH)) k_
     }
   }
   T partial = Sc<T>::zero();
-  if (iv.vec) {
+  if (iv.vec == 1) {
     auto lastval = [&](int c, int e) -> T {
       const int j = (jl + (c << lg)) * VE + e;
       return j < last ? cm[olast + j] : Sc<T>::zero();
@@ -370,7 +462,7 @@ __global__ void __launch_bounds__(32 * INT_WARPS, int_blocks(sizeof(T), NCH)) k_
           if ((jl + (c << lg)) * VE + e < last) partial = Sc<T>::fma(acc[c][e], lastval(c, e), partial);
     }
   } else {
-    // rows that are not 16-byte aligned or longer than the lanes hold
+    // rows that are not 16-byte aligned
     for (int r = 0; r < nr; ++r) {
       const T* row = rows + (int64_t)r * last;
       T dot = Sc<T>::zero();
@@ -378,16 +470,7 @@ __global__ void __launch_bounds__(32 * INT_WARPS, int_blocks(sizeof(T), NCH)) k_
       partial = Sc<T>::fma(shfl_t(w32, r), dot, partial);
     }
   }
-  for (int o = 16; o; o >>= 1) {
-    if constexpr (sizeof(T) == 16) {
-      cplx z = *(cplx*)&partial;
-      z.re += __shfl_xor_sync(0xffffffffu, z.re, o);
-      z.im += __shfl_xor_sync(0xffffffffu, z.im, o);
-      partial = *(T*)&z;
-    } else {
-      partial = partial + __shfl_xor_sync(0xffffffffu, partial, o);
-    }
-  }
+  partial = warp_total(partial);
   if (lane == 0) atomicAddAcc(L.msgs + iv.out + a, mulw(to_acc(partial, A{}), iv.w));
 }
 
@@ -530,6 +613,8 @@ void integrate_levels(tnfa_ctx* ctx, const tnfa_net* net, int take_sum, double* 
         cfg.attrs = pdl;
         cfg.numAttrs = first ? 0 : 1;  // the first launch follows the clearing
         first = false;
+        if (smem > INT_SMEM)
+          TNFA_CUDA(cudaFuncSetAttribute(k_integrate_level<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, INT_SMEM_LONG));
         switch (nch) {
           case 1: TNFA_CUDA(cudaLaunchKernelEx(&cfg, k_integrate_level<T, 1>, L)); break;
           case 2: TNFA_CUDA(cudaLaunchKernelEx(&cfg, k_integrate_level<T, 2>, L)); break;
@@ -568,14 +653,25 @@ void integrate_levels(tnfa_ctx* ctx, const tnfa_net* net, int take_sum, double* 
           iv.nkb = (int)nkb;
         }
         iv.ntask = (int)ntask;
-        const size_t need = (size_t)sum * (sizeof(A) + (sizeof(A) != sizeof(T) ? sizeof(T) : 0));
+        size_t need = (size_t)sum * (sizeof(A) + (sizeof(A) != sizeof(T) ? sizeof(T) : 0));
         iv.staged = need <= INT_SMEM;
-        iv.vec = !cs.empty() && iv.staged && iv.off % VE == 0 && iv.last % VE == 0 &&
-                 iv.last <= 32 * VE * nch && ((uintptr_t)net->d & 15) == 0;
+        iv.vec = !cs.empty() && iv.off % VE == 0 && iv.last % VE == 0 && ((uintptr_t)net->d & 15) == 0;
+        iv.tpw = 1;
+        if (iv.vec && iv.last > 32 * VE * nch) {
+          iv.vec = 2;
+          if (!iv.staged && (size_t)sum * sizeof(T) <= INT_SMEM_LONG) {
+            iv.staged = sizeof(A) == sizeof(T) ? 1 : 2;
+            need = (size_t)sum * sizeof(T);
+          }
+          const int64_t wave = (int64_t)ctx->sm_count * int_blocks(sizeof(T), nch) * INT_WARPS;
+          iv.tpw = (short)std::min<int64_t>(32, (ntask + wave - 1) / wave);
+        } else if (!iv.staged) {
+          iv.vec = 0;
+        }
         iv.lg = 5;
-        if (iv.vec)
+        if (iv.vec == 1)
           while (iv.lg > 0 && (1 << (iv.lg - 1)) * VE >= iv.last) --iv.lg;
-        const int64_t nb = (ntask + INT_WARPS - 1) / INT_WARPS;
+        const int64_t nb = (ntask + INT_WARPS * iv.tpw - 1) / (INT_WARPS * iv.tpw);
         if (L.nv == INT_MAXV || nc + iv.nchild > INT_MAXCH || blocks + nb > 0x7fffffff) launch();
         iv.b0 = (int)blocks;
         iv.ch0 = nc;
