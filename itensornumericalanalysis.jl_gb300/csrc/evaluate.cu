@@ -706,7 +706,8 @@ template <class T>
 class EvalEngine {
  public:
   EvalEngine(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const std::vector<DigitRef>& prog,
-             int ncols, int64_t P, bool use_tc, bool use_oz, size_t budget, bool adjoint = false)
+             int ncols, int64_t P, bool use_tc, bool use_oz, size_t budget, bool adjoint = false,
+             double max_rows = 134217728.0)
       : ctx_(ctx), net_(net), tensors_(tensors), topo_(net->topo), prog_(prog), ncols_(ncols), P_(P),
         use_tc_(use_tc), use_oz_(use_oz), adjoint_(adjoint) {
     const int V = topo_.V;
@@ -730,9 +731,11 @@ class EvalEngine {
                                 : oz_vertex_eligible((int)kids.size(), cd, topo_.link[v]);
       }
     }
-    // Tables take at most half the scratch: the row bound shrinks until they
-    // fit.  Every digit code stays within 31 bits.
-    double rows = std::min((double)P, 134217728.0);
+    // Tables (and their adjoints, of the same size) take at most half the
+    // scratch: the row bound shrinks until they fit.  Every digit code stays
+    // within 31 bits.
+    const double copies = adjoint_ ? 2.0 : 1.0;
+    double rows = std::min((double)P, max_rows);
     if (adjoint_) {  // every product of a table is a row product (see AdjointEngine)
       o.table_kids = 2;
       o.absorb_points = false;
@@ -767,7 +770,7 @@ class EvalEngine {
       o.table_rows = rows;
       o.table_elems = std::min(1073741824.0, (double)(budget / 2) / sizeof(T));
       tree_ = EvalTreeBuilder(topo_, o).build();
-      if (table_bytes() <= budget / 2 || rows < 1) break;
+      if (copies * table_bytes() <= budget / 2 || rows < 1) break;
       rows = std::floor(rows / 4);
       if (rows < 1 && !small_) {  // the stored order, nothing but points
         o.rule = CentreRule::ROOT;
@@ -783,6 +786,12 @@ class EvalEngine {
   }
 
   int chunk() const { return Pc_; }
+  int64_t table_rows() const {  // of the longest table
+    int64_t n = 0;
+    for (const EvalVertex& e : tree_.v)
+      if (e.tabled && !e.leaf) n = std::max(n, e.N);
+    return n;
+  }
   void set_chunk(int pc) { Pc_ = pc; }
   // Bytes of scratch for chunks of pc points.
   size_t scratch(int64_t pc) {
@@ -2497,8 +2506,8 @@ class AdjointEngine : public EvalEngine<T> {
 
  public:
   AdjointEngine(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const std::vector<DigitRef>& prog, int ncols,
-                int64_t P, size_t budget)
-      : Base(ctx, net, tensors, prog, ncols, P, false, false, budget, true) {
+                int64_t P, size_t budget, double max_rows)
+      : Base(ctx, net, tensors, prog, ncols, P, false, false, budget, true, max_rows) {
     const int V = topo_.V;
     has_e_.assign(V, 0);
     for (int v = 0; v < V; ++v)
@@ -2860,7 +2869,17 @@ void vjp_impl(tnfa_ctx* ctx, const tnfa_net* net, const T* tensors, const double
                "bonds too large for the gradient kernel");
   }
   const size_t staged = (xmem == TNFA_MEM_HOST ? ncols * 8 : 0) + (dout_mem == TNFA_MEM_HOST ? 8 : 0);
-  AdjointEngine<T> E(ctx, net, tensors, prog, ncols, P, ctx->eval_budget);
+  // The tables run backwards once per chunk: no table may be longer than one.
+  // (A path of 48 vertices, bond 46, FP64, 4 x 10^6 points: 120 chunks behind
+  // tables of 2 x 10^6 rows took 13.4 s, the points alone 6.0.)
+  double rows = 134217728.0;
+  std::unique_ptr<AdjointEngine<T>> engine;
+  for (;;) {
+    engine.reset(new AdjointEngine<T>(ctx, net, tensors, prog, ncols, P, ctx->eval_budget, rows));
+    if (engine->chunk() >= P || engine->table_rows() <= engine->chunk()) break;
+    rows = engine->chunk();
+  }
+  AdjointEngine<T>& E = *engine;
   int64_t Pcap = E.chunk();
   if (staged) Pcap = std::min(Pcap, std::max<int64_t>(256, (int64_t)(ctx->eval_budget / staged) / 256 * 256));
   E.set_chunk((int)Pcap);
