@@ -160,7 +160,16 @@ __global__ void __launch_bounds__(256) k_segsum(const T* __restrict__ src, const
 //   dA[r][k]    += 2^-rex sum_(g, n) bar[(g, r)][n] B[g][n][k]
 // One launch takes every product of a level; a block makes one 32 x 32 tile of
 // either sum over a slice of its terms and adds it atomically, so that a sum
-// over thousands of rows into a small tensor still fills the SMs.
+// over thousands of rows into a small tensor still fills the SMs.  A table also
+// has the rows that no point reads, whose adjoint is zero: where they (or the
+// tensor's slices behind them) are not finite the zeros are left out.
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7F800000u) == 0x7F800000u; }
+__device__ __forceinline__ bool not_finite(double x) { return ((unsigned)__double2hiint(x) & 0x7FF00000u) == 0x7FF00000u; }
+__device__ __forceinline__ bool not_finite(cplx z) { return not_finite(z.re) || not_finite(z.im); }
+__device__ __forceinline__ bool is_zero(float x) { return x == 0.f; }
+__device__ __forceinline__ bool is_zero(double x) { return x == 0.0; }
+__device__ __forceinline__ bool is_zero(cplx z) { return z.re == 0.0 && z.im == 0.0; }
+
 template <class T>
 struct BackJob {
   const T* A;
@@ -184,7 +193,18 @@ __global__ void __launch_bounds__(256) k_rows_back(const BackJob<T>* __restrict_
   const int nk = (j.K + BACK_T - 1) / BACK_T;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   T acc[2][2] = {{Sc<T>::zero(), Sc<T>::zero()}, {Sc<T>::zero(), Sc<T>::zero()}};
-  auto multiply = [&]() {
+  auto multiply = [&](bool guard) {  // guard: some y is not finite
+    if (guard) {
+      for (int z = 0; z < BACK_C; ++z)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const T x = xs[z][ty + 16 * i];
+            if (!is_zero(x)) acc[i][q] = Sc<T>::fma(x, ys[z][tx + 16 * q], acc[i][q]);
+          }
+      return;
+    }
 #pragma unroll
     for (int z = 0; z < BACK_C; ++z) {
       const T x0 = xs[z][ty], x1 = xs[z][ty + 16], y0 = ys[z][tx], y1 = ys[z][tx + 16];
@@ -203,6 +223,7 @@ __global__ void __launch_bounds__(256) k_rows_back(const BackJob<T>* __restrict_
     const int g = b % j.ng, sl = b / j.ng;
     const int per = (j.rpg + j.sb - 1) / j.sb, r0 = sl * per, r1 = min(j.rpg, r0 + per);
     for (int r = r0; r < r1; r += BACK_C) {
+      bool bad = false;
       __syncthreads();
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -216,9 +237,9 @@ __global__ void __launch_bounds__(256) k_rows_back(const BackJob<T>* __restrict_
           if (e) y = scale_pow2(y, -e);
         }
         ys[z][c] = y;
+        bad |= not_finite(y);
       }
-      __syncthreads();
-      multiply();
+      multiply(__syncthreads_or(bad));
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -237,6 +258,7 @@ __global__ void __launch_bounds__(256) k_rows_back(const BackJob<T>* __restrict_
   const int64_t tot = (int64_t)j.ng * j.N;
   const int64_t per = (tot + j.sa - 1) / j.sa, z0 = sl * per, z1 = min(tot, z0 + per);
   for (int64_t zz = z0; zz < z1; zz += BACK_C) {
+    bool bad = false;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -252,10 +274,11 @@ __global__ void __launch_bounds__(256) k_rows_back(const BackJob<T>* __restrict_
         xs[z][c] = x;
       }
       const int z = t >> 5, c = t & 31;
-      ys[z][c] = zz + z < z1 && k0 + c < j.K ? j.B[(zz + z) * j.K + k0 + c] : Sc<T>::zero();
+      const T y = zz + z < z1 && k0 + c < j.K ? j.B[(zz + z) * j.K + k0 + c] : Sc<T>::zero();
+      ys[z][c] = y;
+      bad |= not_finite(y);
     }
-    __syncthreads();
-    multiply();
+    multiply(__syncthreads_or(bad));
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
