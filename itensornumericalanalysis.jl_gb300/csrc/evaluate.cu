@@ -829,7 +829,7 @@ class EvalEngine {
       KernelScope ks(ctx_, FamilyName<T>::v, 0.0, 0.0);
       const size_t sm = head_elems_ * sizeof(T) + head_exps_ * 4 + head_jobs_ * sizeof(HeadJob);
       auto go = [&](auto kern) {
-        if (sm > 48 * 1024)
+        if (sm > 47 * 1024)  // (48 KB with the kernel's static words)
           TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         // exponents of a side within +-range: its entries stay far from the type's limits
         kern<<<(unsigned)hgroups_.size(), 256, sm, ctx_->stream>>>(dhblocks_, dhcopies_, dhjobs_, head_elems_,
