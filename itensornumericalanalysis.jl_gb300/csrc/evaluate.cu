@@ -831,7 +831,7 @@ class EvalEngine {
       auto go = [&](auto kern) {
         if (sm > 47 * 1024)  // (48 KB with the kernel's static words)
           TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        // exponents of a side within +-range: its entries stay far from the type's limits
+        // range of a side's exponents: products of two sides stay far below the type's limit
         kern<<<(unsigned)hgroups_.size(), 256, sm, ctx_->stream>>>(dhblocks_, dhcopies_, dhjobs_, head_elems_,
                                                                     head_exps_, head_jobs_, plain_,
                                                                     sizeof(T) == 4 ? 40 : 400);
@@ -1902,7 +1902,7 @@ class EvalEngine {
   std::vector<int> plain_of_;  // head block of its top vertex
   std::vector<std::vector<int>> hgroups_;
   int nhead_jobs_ = 0, nhead_copies_ = 0, head_k_ = 1, head_elems_ = 0, head_exps_ = 0, head_jobs_ = 0;
-  int* plain_ = nullptr;  // per head block: its rows carry no exponents
+  int* plain_ = nullptr;  // per head block: the exponent that all its rows carry, or INT_MIN
   HeadBlock<T>* dhblocks_ = nullptr;
   HeadCopy<T>* dhcopies_ = nullptr;
   HeadJob* dhjobs_ = nullptr;

@@ -676,7 +676,7 @@ struct PairParams {
   int64_t P, p0;
   const T *A, *B;
   const int *ea, *eb;  // null: zero
-  const int *pa, *pb;  // set on the device: the side's exponents are all zero (null: not known)
+  const int *pa, *pb;  // set on the device: the exponent of all rows of the side, INT_MIN if they differ (null: not known)
   int na, nb;          // rows
   int ncols, Pc, nruns, chi, sa, sb, kind, scale;  // sa, sb: code slots; scale: rows of a leaf tensor
   DigitRun runs[CENTRE_RUNS];
@@ -707,8 +707,10 @@ __global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ Pai
     tabA = sa;
     tabB = sb;
   }
-  const int* xa_ = W.ea && !(W.pa && *W.pa) ? W.ea : nullptr;
-  const int* xb_ = W.eb && !(W.pb && *W.pb) ? W.eb : nullptr;
+  const int ca = W.ea && W.pa ? *W.pa : INT_MIN, cb = W.eb && W.pb ? *W.pb : INT_MIN;
+  const int* xa_ = ca == INT_MIN ? W.ea : nullptr;
+  const int* xb_ = cb == INT_MIN ? W.eb : nullptr;
+  const int e0 = (ca == INT_MIN ? 0 : ca) + (cb == INT_MIN ? 0 : cb);
   constexpr int PG = 32 / G;  // points per pass
   // (unsigned: below 2^31 points, and a grid's step more stays below 2^32)
   const unsigned Pc = (unsigned)W.Pc, step = gridDim.x * blockDim.x;
@@ -793,7 +795,7 @@ __global__ void __launch_bounds__(256) k_centre_pair(const __grid_constant__ Pai
       const int rb = G == 1 ? c[1] : __shfl_sync(0xffffffffu, c[1], t);
       const T* A = SM ? tabA + ra * W.chi : tabA + (int64_t)ra * W.chi;
       const T* B = SM ? tabB + rb * W.chi : tabB + (int64_t)rb * W.chi;
-      int e = (xa_ ? xa_[ra] : 0) + (xb_ ? xb_[rb] : 0), ea = 0, eb = 0;
+      int e = e0 + (xa_ ? xa_[ra] : 0) + (xb_ ? xb_[rb] : 0), ea = 0, eb = 0;
       if (W.scale) {
         typename Real<T>::t ma = 0, mb = 0;
         for (int k = l; k < W.chi; k += G) {
@@ -1117,8 +1119,10 @@ __global__ void k_norm_rows(const NormJob<T>* __restrict__ jobs) {
 // table goes out.  Each level would be a launch otherwise, and from global
 // memory every one of them costs two or three L2 latencies (4 us, measured).
 // A side of the centre leaves with its rows scaled; if the rows' exponents lie
-// within +-range, the powers of two join the entries and *plain is set: the
-// centre then reads no exponent per point.
+// within range of their least, the powers of two above that one join the
+// entries and *plain receives it (else INT_MIN): the centre then reads no
+// exponent per point.  Entries only grow by it, so none becomes subnormal that
+// was not, and their products stay below the type's limit.
 struct HeadJob {
   int A, Aexp;    // rows: element offset, exponents' offset (-1: zero)
   int lda;        // row pitch
@@ -1140,7 +1144,7 @@ struct HeadBlock {
   int copy0, copy1, job0, job1;
   int top, topexp, ld, rows, chi;  // the top table in shared memory
   int centre;   // a side of the centre: rows are scaled
-  int plain;    // index of its flag
+  int plain;    // index of its word
 };
 template <class T, int KM>
 __device__ __forceinline__ void head_item(const HeadJob& j, T* sh, int* ex, int q, int n0) {
@@ -1206,7 +1210,7 @@ __global__ void __launch_bounds__(256) k_head(const HeadBlock<T>* __restrict__ b
     }
   }
   __syncthreads();
-  int shift = 0;  // plain: the exponents go into the entries
+  int shift = 0, least = 0;  // plain: the exponents above the least go into the entries
   if (h.centre) {
     int lo = INT_MAX, hi = INT_MIN;  // of the rows that are not zero
     for (int r = threadIdx.x; r < h.rows; r += blockDim.x) {
@@ -1226,15 +1230,16 @@ __global__ void __launch_bounds__(256) k_head(const HeadBlock<T>* __restrict__ b
       atomicMax(&red[1], hi);
     }
     __syncthreads();
-    shift = red[0] <= red[1] && red[1] <= range && red[0] >= -range;
-    if (threadIdx.x == 0) plain[h.plain] = shift;
+    least = red[0];
+    shift = least <= red[1] && red[1] - least <= range;
+    if (threadIdx.x == 0) plain[h.plain] = shift ? least : INT_MIN;
   }
   for (int i = threadIdx.x; i < h.rows * h.chi; i += blockDim.x) {
     const int r = i / h.chi;
     const T v = sh[h.top + r * h.ld + (i - r * h.chi)];
-    h.tab[i] = shift ? scale_pow2(v, ex[h.topexp + r]) : v;
+    h.tab[i] = shift ? scale_pow2(v, ex[h.topexp + r] - least) : v;
   }
-  for (int r = threadIdx.x; r < h.rows; r += blockDim.x) h.exps[r] = shift ? 0 : ex[h.topexp + r];
+  for (int r = threadIdx.x; r < h.rows; r += blockDim.x) h.exps[r] = shift ? least : ex[h.topexp + r];
 }
 
 }  // namespace tnfa

@@ -26,3 +26,39 @@ def test_shared_memory_of_a_plain_launch(ina):
         t = ts[v] if i + 1 < V else ts[v][..., None]
         row = np.einsum("pa,pab->pb", row, t[digits[:, i]])
     assert np.max(np.abs(got[some] / row[:, 0] - 1)) < 3e-5
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32", "c128"])
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_entries_far_apart(ina, dtype, sign):
+    """Two terms whose sizes differ by 2^96 (FP32) or 2^704 at the centre; the last
+    digit leaves the smaller one alone.  The terms of either side of the centre
+    carry 2^39 or 2^399, in turn.  16 vertices x 2 roundings and the centre's: 40 eps."""
+    V, f32 = 16, dtype == "f32"
+    step, side, eps = (2.0**-12, 2.0**39, 2.0**-24) if f32 else (2.0**-88, 2.0**399, 2.0**-53)
+    s = ina.continuous_siteinds(ina.named_path_graph(V))
+    ts, small = {}, []
+    for i, v in enumerate(s.layout.order):
+        # FP32 values, so that both networks hold the same ones
+        x = np.float32([1.7, 1.3]) * np.float32(1 + 0.01 * i)
+        big, low = np.ones(2), x * (step if i < V // 2 else 1.0)
+        if i == V - 1:
+            big = np.array([1.0, 0.0])
+        scale = side**sign if i == 0 else side**-sign if i == V - 1 else 1.0
+        small.append(np.float64(x))
+        if i == 0:
+            ts[v] = np.stack([big, low], -1)[:, None, :] * scale
+        elif i < V - 1:
+            ts[v] = np.stack([np.diag([big[d], low[d]]) for d in range(2)])
+        else:
+            ts[v] = np.stack([big, low], -1) * scale
+    f = ina.ITensorNetworkFunction.from_tensors(s, ts, dtype=ina._lib.F32 if f32 else ina._lib.F64)
+    if dtype == "c128":
+        f = f.astype(ina._lib.C128)
+    n = 1 << 21
+    cells = np.random.default_rng(0).integers(0, 2 ** (V - 1), n) * 2 + 1
+    got = f.evaluate_batch((cells / 2.0**V)[:, None], precision="f32" if f32 else "f64")
+    ref = np.ones(n)
+    for i in range(V):
+        ref *= small[i][(cells >> (V - 1 - i)) & 1]
+    assert np.max(np.abs(got / (ref * step ** (V // 2)) - 1)) < 40 * eps
