@@ -395,6 +395,8 @@ template <> struct FamilyName<double> { static constexpr const char* v = "contra
 template <> struct FamilyName<float> { static constexpr const char* v = "contract_f32"; };
 template <> struct FamilyName<cplx> { static constexpr const char* v = "contract_c128"; };
 
+constexpr size_t CONTRACT_SMEM = 200 * 1024;
+
 template <class T>
 static void launch_contract(tnfa_ctx* ctx, const VertexJob<T>& j, int Pc,
                             const GemmTile* tile = nullptr) {
@@ -406,7 +408,7 @@ static void launch_contract(tnfa_ctx* ctx, const VertexJob<T>& j, int Pc,
   if (j.chi_a <= 16) {
     constexpr int TP = 8;
     size_t sm = (size_t)sumdim * TP * sizeof(T) + 2 * TP * sizeof(int);
-    TNFA_CHECK(sm <= 200 * 1024, TNFA_ERR_UNSUPPORTED, "children bonds too large for evaluation");
+    TNFA_CHECK(sm <= CONTRACT_SMEM, TNFA_ERR_UNSUPPORTED, "children bonds too large for evaluation");
     if (sm > 48 * 1024)
       for (auto kern : {k_contract_narrow<T, 1>, k_contract_narrow<T, 4>, k_contract_narrow<T, 16>})
         TNFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -419,7 +421,7 @@ static void launch_contract(tnfa_ctx* ctx, const VertexJob<T>& j, int Pc,
     const GemmTile t = tile ? *tile : gemm_tile(j.chi_a, sumdim, sizeof(T));
     const size_t sm = (size_t)sumdim * sizeof(T) * t.tp + (size_t)16 * (t.tp + t.ta) * sizeof(T) +
                       2 * t.tp * sizeof(int);
-    TNFA_CHECK(sm <= 200 * 1024, TNFA_ERR_UNSUPPORTED, "children bonds too large for evaluation");
+    TNFA_CHECK(sm <= CONTRACT_SMEM, TNFA_ERR_UNSUPPORTED, "children bonds too large for evaluation");
     dim3 grid((unsigned)((Pc + t.tp - 1) / t.tp + j.ngroups), (unsigned)((j.chi_a + t.ta - 1) / t.ta));
     auto go = [&](auto kern) {
       if (sm > 48 * 1024)
@@ -431,6 +433,13 @@ static void launch_contract(tnfa_ctx* ctx, const VertexJob<T>& j, int Pc,
     else t.tp == 32 ? go(k_contract_gemm<T, 32, 128>) : go(k_contract_gemm<T, 8, 128>);
   }
   TNFA_LAUNCH_CHECK();
+}
+
+// Shared memory of launch_contract for one vertex.
+static size_t contract_smem(int chi_a, int64_t sumdim, size_t tsize) {
+  if (chi_a <= 16) return sumdim * 8 * tsize + 2 * 8 * sizeof(int);
+  const GemmTile t = gemm_tile(chi_a, (int)sumdim, tsize);
+  return sumdim * tsize * t.tp + (size_t)16 * (t.tp + t.ta) * tsize + 2 * t.tp * sizeof(int);
 }
 
 static int contract_tile_rows(int chi_a, int sumdim, size_t tsize) {
@@ -731,6 +740,7 @@ class EvalEngine {
                                 : oz_vertex_eligible((int)kids.size(), cd, topo_.link[v]);
       }
     }
+    check_shapes(o.tensor_ok);
     // Tables (and their adjoints, of the same size) take at most half the
     // scratch: the row bound shrinks until they fit.  Every digit code stays
     // within 31 bits.
@@ -770,6 +780,11 @@ class EvalEngine {
       o.table_rows = rows;
       o.table_elems = std::min(1073741824.0, (double)(budget / 2) / sizeof(T));
       tree_ = EvalTreeBuilder(topo_, o).build();
+      if (!jobs_fit()) {  // the stored order does (check_shapes)
+        o.rule = CentreRule::ROOT;
+        o.absorb = false;
+        tree_ = EvalTreeBuilder(topo_, o).build();
+      }
       if (copies * table_bytes() <= budget / 2 || rows < 1) break;
       rows = std::floor(rows / 4);
       if (rows < 1 && !small_) {  // the stored order, nothing but points
@@ -918,6 +933,37 @@ class EvalEngine {
     std::vector<int> first[3];
     int* dfirst[3] = {nullptr, nullptr, nullptr};
   };
+
+  // The networks that evaluation takes, whatever the schedule: those whose
+  // contraction in the stored order the per-point kernels take.
+  void check_shapes(const std::vector<char>& tensor_ok) const {
+    for (int v = 0; v < topo_.V; ++v) {
+      const auto& kids = topo_.children[v];
+      if (topo_.parent[v] >= 0 && kids.empty()) continue;
+      TNFA_CHECK(kids.size() <= (size_t)EVAL_MAXC, TNFA_ERR_UNSUPPORTED,
+                 "vertex degree above " + std::to_string(EVAL_MAXC) + " children");
+      int64_t K = 1, sum = 0;
+      for (int c : kids) {
+        K = std::min(K * topo_.link[c], int64_t(1) << 31);
+        sum += topo_.link[c];
+      }
+      TNFA_CHECK(K < (int64_t(1) << 31), TNFA_ERR_UNSUPPORTED, "contraction too large");
+      TNFA_CHECK((!tensor_ok.empty() && tensor_ok[v]) || contract_smem(topo_.link[v], sum, sizeof(T)) <= CONTRACT_SMEM,
+                 TNFA_ERR_UNSUPPORTED, "children bonds too large for evaluation");
+    }
+  }
+  // (in another orientation a vertex may have to take its parent's bond in)
+  bool jobs_fit() const {
+    for (int v = 0; v < topo_.V; ++v) {
+      const EvalVertex& e = tree_.v[v];
+      if (e.leaf || e.tensor || row_form(v)) continue;
+      int64_t K = 1;
+      for (size_t i = 0; i + (e.absorb ? 1 : 0) < e.kids.size(); ++i)
+        K = std::min(K * tree_.v[e.kids[i]].chi, int64_t(1) << 31);
+      if (K >= (int64_t(1) << 31) || contract_smem(e.chi, job_sumdim(v), sizeof(T)) > CONTRACT_SMEM) return false;
+    }
+    return true;
+  }
 
   size_t table_bytes() const {
     double b = 0;
