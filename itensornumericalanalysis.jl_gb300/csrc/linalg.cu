@@ -1284,9 +1284,9 @@ struct ColScaleJob {
 template <class T>
 __global__ void __launch_bounds__(256) k_scale_cols(const ColScaleJob* __restrict__ jobs) {
   __shared__ double part[8][32];
-  const ColScaleJob jb = jobs[blockIdx.y];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
-  if (blockIdx.x * 32 >= jb.n) return;
+  const ColScaleJob jb = jobs[blockIdx.x];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.y * 32 + tx;
+  if (blockIdx.y * 32 >= jb.n) return;
   T* A = (T*)jb.A;
   double s = 0.0;
   if (c < jb.n)
@@ -1305,10 +1305,10 @@ __global__ void __launch_bounds__(256) k_scale_cols(const ColScaleJob* __restric
 // Back to the columns' own sizes in R (A: R, m: its rows).
 template <class T>
 __global__ void __launch_bounds__(256) k_unscale_cols(const ColScaleJob* __restrict__ jobs) {
-  const ColScaleJob jb = jobs[blockIdx.y];
+  const ColScaleJob jb = jobs[blockIdx.x];
   T* A = (T*)jb.A;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)jb.m * jb.n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)jb.m * jb.n;
+       i += (int64_t)gridDim.y * blockDim.x) {
     const int e = jb.exps[i % jb.n];
     if (e) A[i] = scal(A[i], scalbn(1.0, e));
   }
@@ -1316,7 +1316,6 @@ __global__ void __launch_bounds__(256) k_unscale_cols(const ColScaleJob* __restr
 
 template <class T>
 void qr_rank_columns(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, std::vector<int>& ranks) {
-  TNFA_CHECK(jobs.size() <= 65535, TNFA_ERR_UNSUPPORTED, "QR batch too large");
   if (jobs.empty()) return qr_rank<T>(ctx, jobs, tol, ranks);
   std::vector<size_t> at(1, 0);
   int maxn = 1;
@@ -1334,8 +1333,8 @@ void qr_rank_columns(tnfa_ctx* ctx, const std::vector<QrJob>& jobs, double tol, 
       most = std::max(most, (int64_t)m * jobs[i].n);
     }
     DBuf d = upload(ctx, cj);
-    const unsigned gx = back ? grid_for(most, 256, 256) : (unsigned)((maxn + 31) / 32);
-    kern<<<dim3(gx, (unsigned)jobs.size()), 256, 0, ctx->stream>>>(d.as<ColScaleJob>());
+    const unsigned gy = back ? grid_for(most, 256, 256) : (unsigned)((maxn + 31) / 32);
+    kern<<<dim3((unsigned)jobs.size(), gy), 256, 0, ctx->stream>>>(d.as<ColScaleJob>());
     TNFA_LAUNCH_CHECK();
   };
   launch(k_scale_cols<T>, false);
