@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 
 #include "linalg.cuh"
+#include "roots.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -938,26 +939,6 @@ __host__ __device__ inline QrSmem qr_smem(int m, int n, int C, size_t ts) {
   return L;
 }
 
-// sqrt(x), and 1 / (sqrt(x) (sqrt(x) + |y|)), for a normal x > 0: FP32 starts
-// on the mantissas, third-order Newton for the root, two Newton steps for the
-// reciprocal (an FP64 division or root is some 20 operations on the slow pipe).
-__device__ __forceinline__ void root_and_beta(double x, double y, double& nrm, double& beta) {
-  const int e = (((int)(__double2hiint(x) >> 20) - 1023) & ~1);  // even: x = X 2^e, X in [1, 4)
-  const double X = x * __hiloint2double((1023 - e) << 20, 0);
-  double r = (double)rsqrtf((float)X);
-  const double f = fma(-X * r, r, 1.0);
-  r = fma(r * f, fma(f, 0.375, 0.5), r);
-  double s = X * r;
-  s = fma(0.5 * r, fma(-s, s, X), s);  // one correction of the root itself
-  const double half = __hiloint2double((1023 + e / 2) << 20, 0), inv = __hiloint2double((1023 - e / 2) << 20, 0);
-  nrm = s * half;
-  const double d = s + fabs(y) * inv;  // in [1, 4): |y| <= sqrt(x)
-  double q = (double)(1.0f / (float)d);
-  q = fma(q, fma(-d, q, 1.0), q);
-  q = fma(q, fma(-d, q, 1.0), q);
-  beta = r * q * inv * inv;
-}
-
 template <class T>
 __global__ void __launch_bounds__(512) k_qrcp_sm(const QrJob* __restrict__ jobs, double tol2, int* __restrict__ ranks) {
   cg::cluster_group cl = cg::this_cluster();
@@ -1611,14 +1592,6 @@ __global__ void __launch_bounds__(512) k_jacobi(const SvdJob* __restrict__ jobs,
 // sums to the partner: 6 additions instead of 15 for 32 lanes), and the angle
 // comes from FP32: only c^2 + s^2 = 1 has to hold to FP64, an angle off by
 // 1e-7 leaves 1e-7 of the off-diagonal for the next sweep.
-
-// 1 / sqrt(x) to FP64 for x in [1, 2]: FP32 root, one third-order Newton step
-// (y e (1/2 + 3/8 e), e = 1 - x y^2: the error term is e^3).
-__device__ __forceinline__ double rsqrt_1_2(double x) {
-  const double y = (double)rsqrtf((float)x);
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
 
 // Sums over G lanes of a, b and the parts of g.
 template <int G, class R>
