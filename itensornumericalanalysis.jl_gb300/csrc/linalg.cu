@@ -910,13 +910,10 @@ __global__ void __launch_bounds__(512) k_qrcp(const QrJob* __restrict__ jobs, T*
 // shared memory.  A step has one cluster barrier: the CTAs post their best
 // column to each other's slots, then each copies the winner from its owner's
 // shared memory and builds the reflector itself (the winning column is never
-// written again).  The weight that decides the stop is summed in FP32, scaled
-// by the matrix norm: it is only compared with tol^2, and an FP64 addition
-// costs a warp 64 cycles.
+// written again).
 struct QrSlot {
-  double best;
+  double best, sum;
   int idx;
-  float sum;
 };
 constexpr int QRS_MAXM = 512;  // rows: one element of a column per thread
 
@@ -990,22 +987,19 @@ __global__ void __launch_bounds__(512) k_qrcp_sm(const QrJob* __restrict__ jobs,
   cl.sync();
   double total = 0.0;
   for (int i = 0; i < C; ++i) total += tot[i];
-  // 2^-E total is in [1, 2) (left alone when zero or not finite)
-  const int te = (int)(__double2hiint(total) >> 20) & 0x7FF;
-  const double sc = te > 0 && te < 2046 ? __hiloint2double((2046 - te) << 20, 0) : 1.0;
-  const float thr = (float)(tol2 * (total * sc));
+  const double thr = tol2 * total;
   // (an Inf or NaN entry, or one whose square overflows, leaves no rank)
   int r_keep = total <= 1.7976931348623157e308 ? kq : 0;
   for (int j = 0; j < r_keep; ++j) {
     if (warp == 0) {
       long long best = -1;  // norms are >= 0: their bits order like the values
       int bi = INT_MAX;
-      float sum = 0.f;
+      double sum = 0.0;
       for (int k = lane; k < nc; k += 32) {
         const double v = nrm[k];
         const long long b = __double_as_longlong(v);
         if (b < 0 || b > 0x7FF0000000000000ll) continue;  // pivoted (-1), NaN
-        sum += (float)(v * sc);
+        sum += v;
         if (b > best) best = b, bi = crank + C * k;
       }
       for (int o = 16; o; o >>= 1) {
@@ -1014,12 +1008,12 @@ __global__ void __launch_bounds__(512) k_qrcp_sm(const QrJob* __restrict__ jobs,
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (ob > best || (ob == best && oi < bi)) best = ob, bi = oi;
       }
-      if (lane < C) *cl.map_shared_rank(&slot[j & 1][crank], lane) = QrSlot{__longlong_as_double(best), bi, sum};
+      if (lane < C) *cl.map_shared_rank(&slot[j & 1][crank], lane) = QrSlot{__longlong_as_double(best), sum, bi};
     }
     cl.sync();
     long long gbest = -1;
     int p = INT_MAX;
-    float gsum = 0.f;
+    double gsum = 0.0;
     for (int i = 0; i < C; ++i) {
       const QrSlot& o = slot[j & 1][i];
       const long long ob = __double_as_longlong(o.best);
