@@ -2657,7 +2657,7 @@ void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cuto
     for (size_t q = 0; q < nj; ++q) {
       const FactorJob& f = jobs[q];
       const bool wide = f.rows < f.cols;
-      if (wide && f.rows > QRCP_MAXK) continue;
+      if (std::min(f.rows, f.cols) > QRCP_MAXK) continue;
       rev[q] = 1;
       const int m = std::max(f.rows, f.cols), k = std::min(f.rows, f.cols);
       if (wide) {

@@ -111,9 +111,10 @@ struct FactorResult {
   int sweeps = 0;          // FP64 Jacobi sweeps; -1: the sweep cap was hit
   std::vector<double> s;   // singular values, descending
 };
-// reveal_tol > 0: jobs first go through the rank-revealing QR (qr_rank with
-// that tolerance; wide ones on the adjoint) and the core has as many columns
-// as the numerical rank r, so the SVD runs on r rather than min(rows, cols).
+// reveal_tol > 0: jobs of up to 1024 reflectors first go through the
+// rank-revealing QR (qr_rank with that tolerance; wide ones on the adjoint) and
+// the core has as many columns as the numerical rank r, so the SVD runs on r
+// rather than min(rows, cols).
 template <class T>
 void trunc_factor(tnfa_ctx* ctx, const std::vector<FactorJob>& jobs, double cutoff, int maxdim,
                   int mindim, int precision, std::vector<FactorResult>& out, double reveal_tol = 0.0);

@@ -2353,8 +2353,7 @@ extern "C" {
 // before the Jacobi iteration (24 vertices, bond 40, first derivative: 44.5 ms,
 // the tree sweep 141; cutting in the first sweep already took 27 and lost every
 // part of a function whose tensors there are small).  Null when the sweeps do
-// not take it (another tree, a matrix of more than 1024 columns, NaN or Inf
-// entries): the general form then does.
+// not take it (another tree, NaN or Inf entries): the general form then does.
 static tnfa_net* one_path(tnfa_ctx* ctx, const tnfa_net* op, const tnfa_net* f, const tnfa_trunc_params& prm) {
   if (!is_rooted_path(f->topo) || (op && op->dtype != f->dtype)) return nullptr;
   tnfa_net* out = nullptr;
