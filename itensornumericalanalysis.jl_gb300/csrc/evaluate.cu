@@ -309,57 +309,6 @@ static bool small_bonds(const Topo& T, size_t tsize, int64_t npoints) {
 }
 
 // -------------------------------------------------------------- driver ----
-struct EvalPlan {
-  std::vector<int> order;        // vertices computed, children before parents
-  std::vector<char> fused_leaf;  // non-root leaf read directly by its parent
-  std::vector<int> slot;         // message slot of a computed non-root vertex
-  int nslots = 0;
-  std::vector<int> roots;
-  int chimax = 1;
-};
-
-// A vertex's output slot is taken while its children still hold theirs, so
-// that it never shares memory with the messages it reads: the contraction
-// kernels write their output as they go (tiles split over columns, the
-// sliced kernel's two phases) and the autotuner runs one contraction several
-// times over the same inputs.
-static EvalPlan make_plan(const Topo& T) {
-  EvalPlan P;
-  P.fused_leaf.assign(T.V, 0);
-  P.slot.assign(T.V, -1);
-  P.roots = T.roots();
-  for (int v = 0; v < T.V; ++v)
-    if (T.parent[v] >= 0 && T.children[v].empty()) P.fused_leaf[v] = 1;
-  // Post-order DFS per root keeps the number of live messages near the depth.
-  for (int r : P.roots) {
-    std::vector<std::pair<int, int>> st{{r, 0}};
-    while (!st.empty()) {
-      auto& [v, i] = st.back();
-      if (i < (int)T.children[v].size()) {
-        int c = T.children[v][i++];
-        st.push_back({c, 0});
-      } else {
-        if (!P.fused_leaf[v]) P.order.push_back(v);
-        st.pop_back();
-      }
-    }
-  }
-  std::vector<int> free_slots;
-  int n = 0;
-  for (int v : P.order) {
-    if (T.parent[v] >= 0) {
-      if (free_slots.empty()) free_slots.push_back(n++);
-      P.slot[v] = free_slots.back();
-      free_slots.pop_back();
-      P.chimax = std::max(P.chimax, T.link[v]);
-    }
-    for (int c : T.children[v])
-      if (!P.fused_leaf[c]) free_slots.push_back(P.slot[c]);
-  }
-  P.nslots = n;
-  return P;
-}
-
 // Tile of k_contract_gemm for a parent bond chi_a > 16 and children rows of
 // sumdim entries: TP x TA with TA the smallest of 32 / 64 / 128 covering
 // chi_a, and TP = 4096 / TA (a 4 x 4 micro-tile per thread) while the
@@ -780,7 +729,9 @@ class EvalEngine {
       o.table_rows = rows;
       o.table_elems = std::min(1073741824.0, (double)(budget / 2) / sizeof(T));
       tree_ = EvalTreeBuilder(topo_, o).build();
-      if (!jobs_fit()) {  // the stored order does (check_shapes)
+      // The stored order fits (check_shapes).  (Never a gradient's case, whose
+      // two-kid tables need absorption: its narrower bonds fit in any order.)
+      if (!jobs_fit()) {
         o.rule = CentreRule::ROOT;
         o.absorb = false;
         tree_ = EvalTreeBuilder(topo_, o).build();
@@ -2132,17 +2083,35 @@ unsigned char* noalloc_base(int device) {
   return addr[device];
 }
 
-// Scratch bytes by which a request is accepted: digit program, fused schedule,
-// digits, permutation, group tables, error flag, message slots of every point
-// and root values, in 256-byte pieces.  The calls that fit are part of the
-// interface; the schedule itself works in chunks that fit (FixedRun).
+// Scratch bytes by which a request is accepted: a limit of the interface, not
+// what a call uses (it works in chunks that fit, FixedRun).  Requests are taken
+// up to the point count whose digits, permutation, group tables, root values
+// and messages, one row per point for every message alive at once in a
+// depth-first contraction, fit the array.
 template <class T>
 size_t noalloc_bytes(const tnfa_net* net, int64_t P, size_t prog_entries) {
   const Topo& Tp = net->topo;
-  const EvalPlan plan = make_plan(Tp);
-  const size_t nroots = plan.roots.size();
-  int maxsd = 1;
+  int maxsd = 1, chimax = 1;
   for (int v = 0; v < Tp.V; ++v) maxsd = std::max(maxsd, Tp.site_dim[v]);
+  // messages alive at once below and at every vertex (a leaf's is read in place)
+  std::vector<int> alive(Tp.V, 0);
+  size_t nroots = 0;
+  int nslots = 0;
+  for (int v = Tp.V - 1; v >= 0; --v) {  // children before parents
+    const bool root = Tp.parent[v] < 0;
+    nroots += root;
+    int held = 0;
+    for (int c : Tp.children[v]) {
+      alive[v] = std::max(alive[v], held + alive[c]);
+      held += !Tp.children[c].empty();
+    }
+    if (root) {
+      nslots = std::max(nslots, alive[v]);
+    } else if (!Tp.children[v].empty()) {
+      alive[v] = std::max(alive[v], held + 1);
+      chimax = std::max(chimax, Tp.link[v]);
+    }
+  }
   std::array<size_t, 10> sizes{prog_entries * 32, 0, 0, 0, 0, 4, 0, 0, 0, 0};
   if (small_bonds(Tp, sizeof(T), P)) {
     sizes[1] = (size_t)Tp.V * 36;
@@ -2150,8 +2119,8 @@ size_t noalloc_bytes(const tnfa_net* net, int64_t P, size_t prog_entries) {
     sizes[2] = (size_t)Tp.V * P;
     sizes[3] = (size_t)P * 4;
     sizes[4] = group_meta_ints(maxsd) * 4;
-    sizes[6] = (size_t)plan.nslots * P * plan.chimax * sizeof(T);
-    sizes[7] = (size_t)plan.nslots * P * sizeof(int);
+    sizes[6] = (size_t)nslots * P * chimax * sizeof(T);
+    sizes[7] = (size_t)nslots * P * sizeof(int);
     sizes[8] = nroots * P * sizeof(T);
     sizes[9] = nroots * P * sizeof(int);
   }
