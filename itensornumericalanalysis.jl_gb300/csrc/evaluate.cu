@@ -638,11 +638,36 @@ static void launch_small_rows(tnfa_ctx* ctx, int64_t blocks, int kmax, const Row
   TNFA_LAUNCH_CHECK();
 }
 
-// Multiply-adds per second of the walk, for choosing between it and tables.
+// Multiply-adds per second by which the walk of a call is counted against the
+// 20 us up to which no tables are laid out at all.  Its latency is in them: the
+// rate of many points alone is higher (SmallCosts::point_madd).
 template <class T> struct WalkRate;
 template <> struct WalkRate<float> { static constexpr double v = 4e12; };
 template <> struct WalkRate<double> { static constexpr double v = 3e11; };
 template <> struct WalkRate<cplx> { static constexpr double v = 8e10; };
+
+// Microseconds of a call beyond what every call costs, where the walk and tables
+// are close: fitted to 1485 calls (paths, combs and binary trees of 12 to 30
+// vertices, bonds 2 to 8, 500 to 128000 points), each by the walk and from
+// tables; 8 % rms off in FP32 and FP64, 13 % in complex.  The walk: a vertex
+// and a multiply-add of one point's chain, and of all points (work counted with
+// bonds padded to 2, 4 or 8).  Tables: a level's launch, a table with launches
+// of its own (two kids, neither absorbed), the permuted tensors, the head and
+// one of its vertices, a multiply-add of the tables beyond it, the centre.
+struct SmallCosts {
+  double vertex, madd, point_vertex, point_madd;
+  double level, table, move, head, head_vertex, table_madd, centre;
+};
+template <class T> struct SmallCost;
+template <> struct SmallCost<double> {
+  static constexpr SmallCosts v{0.98, 0.0085, 4.9e-6, 2.1e-6, 7.2, 10, 12, 14, 0.83, 7.0e-6, 31e-6};
+};
+template <> struct SmallCost<float> {
+  static constexpr SmallCosts v{0.81, 0.0031, 3.6e-6, 0.33e-6, 5.9, 11, 12, 8.8, 1.0, 6.0e-6, 10e-6};
+};
+template <> struct SmallCost<cplx> {
+  static constexpr SmallCosts v{1.0, 0.027, 23e-6, 4.7e-6, 10, 9.5, 14, 23, 0.35, 18e-6, 58e-6};
+};
 
 // ------------------------------------------------------------- engine ----
 // Scratch handed out in 256-byte pieces from one block (or counted, base null).
@@ -744,6 +769,24 @@ class EvalEngine {
       }
     }
     plan();
+    if (small_ && rows > 0) {
+      // Where the walk by itself is cheaper than these tables by more than the
+      // second schedule (about 10 us) and the costs' error, it is taken after all.
+      // Trees have many levels of small tables: 30-vertex binary tree, bond 2,
+      // complex, 16000 points 184 us from tables, 92 so; bond 4, FP64, 8000 points
+      // 161 and 94.  The same with bond 8, FP64: 113 from tables, 220 walked.
+      const double error = sizeof(T) == 16 ? 1.2 : 1.1;
+      if (error * walk_cost(true) + 12.0 <= table_cost()) {
+        EvalTree kept = std::move(tree_);
+        o.table_rows = 0;
+        tree_ = EvalTreeBuilder(topo_, o).build();
+        plan();
+        if (!walk_) {  // (not in this order's shared memory)
+          tree_ = std::move(kept);
+          plan();
+        }
+      }
+    }
     per_point_ = (size_t)nmsg_ * (msg_chi_ * sizeof(T) + sizeof(int)) + (size_t)ncodes_ * 4 + (npp_ ? 4 : 0);
     const size_t tab = scratch(0);
     const size_t left = budget > tab ? budget - tab : 0;
@@ -914,6 +957,47 @@ class EvalEngine {
       if (K >= (int64_t(1) << 31) || contract_smem(e.chi, job_sumdim(v), sizeof(T)) > CONTRACT_SMEM) return false;
     }
     return true;
+  }
+
+  // Microseconds of walking all vertices, or those without a table (SmallCosts).
+  double walk_cost(bool all) const {
+    constexpr SmallCosts c = SmallCost<T>::v;
+    double n = 0, w = 0;
+    int top = 1;
+    for (int v = 0; v < topo_.V; ++v) {
+      top = std::max(top, topo_.link[v]);
+      if (!all && tree_.v[v].tabled) continue;
+      n += 1;
+      w += tree_.v[v].W;
+    }
+    w *= (top <= 2 ? 2.0 : top <= 4 ? 4.0 : top <= 8 ? 8.0 : top) / top;
+    return n * c.vertex + w * c.madd + P_ * (n * c.point_vertex + w * c.point_madd);
+  }
+  // Microseconds of the schedule as planned: its tables and its points.
+  double table_cost() const {
+    constexpr SmallCosts c = SmallCost<T>::v;
+    double t = 0, n = 0;
+    bool moves = false;
+    for (const Level& L : levels_) {
+      if (L.njobs > 0 || !L.verts.empty()) t += c.level;
+      t += c.table * L.verts.size();
+    }
+    for (int v = 0; v < topo_.V; ++v) {
+      const EvalVertex& e = tree_.v[v];
+      moves |= needs_move(v);
+      if (e.leaf) continue;
+      if (!e.tabled) {
+        n += 1;
+      } else if (head_[v]) {
+        t += c.head_vertex;
+      } else {
+        const double k = e.absorb ? e.W / tree_.v[e.kids.back()].chi : e.W;
+        t += c.table_madd * (e.N * k + (e.absorb ? absorbed_rows(v) * e.W : 0.0));
+      }
+    }
+    if (moves) t += c.move;
+    if (!hgroups_.empty()) t += c.head;
+    return t + (n > 0 ? walk_cost(false) : P_ * c.centre);
   }
 
   size_t table_bytes() const {
