@@ -71,14 +71,14 @@ __global__ void k_site_reduce<cplx>(const cplx* __restrict__ src, cplx* __restri
 // when the vertex's rows allow it; G = 2^lg lanes share a row (rows of few
 // vectors leave no lane idle), NCH vectors a lane cover a row of up to
 // 32 * NCH * VE entries and max(NCH, 4) loads are in flight per lane (twice as
-// many and 24 instead of 32 warps per SM took 121 us where this takes 115).
+// many and 24 instead of 32 warps per SM took 2-5 us longer a call).
 //
 // Bound by HBM at large bonds in FP32 and by the FP64 pipe in FP64 (one FMA per
 // entry, 203 us of the 284 below: there the rows are summed with their weights
 // before the last child's message comes in, once per task).  A call on
 // the 60-vertex binary tree, against one persistent launch fed by bulk copies
 // whose consumers waited for their children's flags task by task: bond 128
-// (117 M entries) FP32 117 us (194), FP64 284 us (350); bond 48 FP32 50 us (129);
+// (117 M entries) FP32 120 us (194), FP64 284 us (350); bond 48 FP32 50 us (129);
 // path of 60 vertices, bond 256, FP64 284 us (1312), bond 6 208 us (425).
 template <class T> struct IntAcc { using type = double; };
 template <> struct IntAcc<cplx> { using type = cplx; };
@@ -133,6 +133,7 @@ constexpr int INT_MAXV = 24, INT_MAXCH = 56;  // of a launch: its parameters sta
 constexpr int INT_WARPS = 8;
 constexpr int kFoldSites = 8;
 // blocks per SM: 64 registers a thread, 128 where a row's vectors need them
+// (FP32 rows of 257 to 512 entries, NCH = 4, spill 24 bytes a thread at 64)
 constexpr int int_blocks(size_t size, int nch) { return size == 16 || nch >= 8 ? 2 : 4; }
 // messages of a vertex's children kept on chip: with the block's static
 // reductions (4 bytes a child and warp) within the 48 KB of a plain launch
